@@ -496,6 +496,24 @@ def test_device_topk_order(midi):
         assert am2[r] == order[0]
 
 
+@pytest.mark.parametrize("vocab,run,k", [(5003, 5003, 40), (5003, 2500, 64), (5003, 511, 40), (5003, 3, 1), (50, 1, 40), (9000, 600, 64)])
+def test_device_topk_of_equal_logits(vocab, run, k):
+    """Blocks of `run` equal rows of the output matrix: more equal logits at the k-th place than the kernel keeps candidates for
+    (512), just fewer, rows shorter than its 1024 threads. Order by index among equals."""
+    cfg = dict(synthetic.preset("mini"), vocab_size=vocab)
+    w = synthetic.perturbed_weights(cfg, 5)
+    w["wte.weight"] = np.ascontiguousarray(w["wte.weight"][np.arange(vocab) // run * run])
+    g = pg.Gpt2Model(cfg, w)
+    cache = g.new_kv_cache(max_batch=2)
+    _, am = g.prefill_batch([synthetic.uniform_prompt(600 + i, 9, vocab) for i in range(2)], cache)
+    logits, am2, tv, ti = g.forward_one_batch(am, cache, want_logits=True, top_k=k)
+    for r in range(2):
+        order = sorted(range(vocab), key=lambda i: (-float(logits[r, i]), i))[:k]
+        assert list(ti[r]) == order
+        assert np.array_equal(tv[r], logits[r, order])
+        assert am2[r] == order[0]
+
+
 @pytest.mark.parametrize("kw", [dict(temperature=0.8, top_k=40), dict(temperature=0.9, top_p=0.95),
                                 dict(temperature=0.0, repeat_penalty=1.4), dict(temperature=0.0)])
 def test_generate_with_config_matches_oracle_loop(midi, oracle, kw):
