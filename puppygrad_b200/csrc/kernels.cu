@@ -679,65 +679,6 @@ __global__ void gather_rows_kernel(const float* src, const int* rows, float* dst
   for (int i = threadIdx.x; i < c; i += blockDim.x) dst[(size_t)r * c + i] = s[i];
 }
 
-// ------------------------------------------------------------------ FP32 GEMM (prefill parity path)
-// 128x128x8 tiles, 256 threads, 8x8 outputs per thread.
-constexpr int GB = 128, GK = 8;
-__global__ void __launch_bounds__(256) gemm_f32_kernel(LinearArgs a, int epi) {
-  __shared__ __align__(16) float As[GK][GB + 4];
-  __shared__ __align__(16) float Ws[GK][GB + 4];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * GB, n0 = blockIdx.x * GB;
-  const int lr = tid >> 1, lk = (tid & 1) * 4;  // loader: row within tile, k offset
-  const int ty = tid >> 4, tx = tid & 15;
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-
-  const bool arow_ok = (m0 + lr) < a.m, wrow_ok = (n0 + lr) < a.n;
-  const float* ap = a.x + (size_t)(m0 + lr) * a.k + lk;
-  const float* wp = a.w + (size_t)(n0 + lr) * a.k + lk;
-  for (int k0 = 0; k0 < a.k; k0 += GK) {
-    float4 av = make_float4(0, 0, 0, 0), wv = make_float4(0, 0, 0, 0);
-    if (k0 + lk < a.k) {  // k is a multiple of 4
-      if (arow_ok) av = *reinterpret_cast<const float4*>(ap + k0);
-      if (wrow_ok) wv = *reinterpret_cast<const float4*>(wp + k0);
-    }
-    As[lk + 0][lr] = av.x; As[lk + 1][lr] = av.y; As[lk + 2][lr] = av.z; As[lk + 3][lr] = av.w;
-    Ws[lk + 0][lr] = wv.x; Ws[lk + 1][lr] = wv.y; Ws[lk + 2][lr] = wv.z; Ws[lk + 3][lr] = wv.w;
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < GK; ++kk) {
-      float4 a0 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      float4 a1 = *reinterpret_cast<const float4*>(&As[kk][64 + ty * 4]);
-      float4 b0 = *reinterpret_cast<const float4*>(&Ws[kk][tx * 4]);
-      float4 b1 = *reinterpret_cast<const float4*>(&Ws[kk][64 + tx * 4]);
-      float af[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      float bf[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(af[i], bf[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-    if (m >= a.m) continue;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-      if (n >= a.n) continue;
-      float v = a.bias ? a.bias[n] + acc[i][j] : acc[i][j];
-      if (epi == EPI_GELU) v = gelu_ref(v);
-      if (epi == EPI_RESID) v = a.resid[(size_t)m * a.n + n] + v;
-      a.out[(size_t)m * a.n + n] = v;
-    }
-  }
-}
-
 // ------------------------------------------------------------------ paged KV helpers
 __device__ __forceinline__ size_t kv_row_offset(const KvLayout& kv, int page, int which, int head, int off) {
   // [page][2][head][page_tokens][head_dim]
@@ -1545,13 +1486,13 @@ cudaError_t launch_layernorm_rows_split(const float* x, const float* g, const fl
   return launch(layernorm_rows_split_kernel, dim3(rows), dim3(128), 0, s, pdl, x, g, b, eps, hi, lo, rows, c);
 }
 
-cudaError_t launch_gemm_f32(const LinearArgs& a, int epilogue, cudaStream_t s) {
-  if (a.k % 4 != 0) {
-    size_t total = (size_t)a.m * a.n;
-    return launch(linear_generic_kernel, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, s, false, a, epilogue);
-  }
-  dim3 grid((a.n + GB - 1) / GB, (a.m + GB - 1) / GB);
-  return launch(gemm_f32_kernel, grid, dim3(256), 0, s, false, a, epilogue);
+// The decode kernels stream the weights once per 8 rows. GPT-2 small's products on them and on the tiles: 9 rows
+// 14.3 / 10.3 / 18.5 and 14.4 / 11.5 / 18.4 us, 16 rows 15.8 / 11.3 / 21.3 and 14.4 / 11.7 / 18.4 us, 64 rows 42 / 28 / 65 and
+// 18.5 / 12.3 / 24.4 us (n 2304, k 768 / n 768, k 768 / n 768, k 3072); a whole prefill of 11 rows 917 and 990 us. The tiles win
+// earlier where the weights are many: lm_head of 12 rows 150 and 82 us.
+cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s) {
+  if (a.m <= 8 || a.k % 4 != 0 || (a.m <= 12 && a.n <= 16384)) return launch_linear_decode(a, epilogue, pdl, s, nullptr);
+  return launch_gemm_f32_tiles(a, epilogue, s);
 }
 
 cudaError_t launch_transpose(const float* src, float* dst, int in_f, int out_f, cudaStream_t s) {

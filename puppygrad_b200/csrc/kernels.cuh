@@ -41,8 +41,11 @@ cudaError_t launch_embed(const float* wte, const float* wpe, const int* ids, con
 // out = LayerNorm(x) row-wise; lo (optional; needs c % 4 == 0 and c <= 4096) = out - hi(out), the TF32 lo part of the result
 cudaError_t launch_layernorm_rows(const float* x, const float* g, const float* b, float eps, float* out,
                                   int rows, int c, bool pdl, cudaStream_t s, float* lo = nullptr);
-// General FP32 GEMM out[m,n] = x[m,k] . w[n,k]^T (+bias)(+GELU | +resid), CUDA-core FMA.
-cudaError_t launch_gemm_f32(const LinearArgs& a, int epilogue, cudaStream_t s);
+// General FP32 GEMM out[m,n] = x[m,k] . w[n,k]^T (+bias)(+GELU | +resid), CUDA-core FMA (gemm_f32.cu); k % 4 == 0.
+cudaError_t launch_gemm_f32_tiles(const LinearArgs& a, int epilogue, cudaStream_t s);
+cudaError_t init_gemm_f32_attributes();
+// The faster of the two FP32 products for any number of rows (no LayerNorm prologue, no arg-max partials).
+cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s);
 // dst[o, i] = src[i, o]
 cudaError_t launch_transpose(const float* src, float* dst, int in_f, int out_f, cudaStream_t s);
 

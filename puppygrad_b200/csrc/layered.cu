@@ -780,7 +780,7 @@ cudaError_t product(const LayeredModel* m, const Matrix& w, const void* x, float
   a.w = static_cast<const float*>(w.w); a.x = static_cast<const float*>(x); a.out = out ? out : static_cast<float*>(out_h);
   a.m = rows; a.n = n_out; a.k = w.kp;
   if (ldo != n_out) return cudaErrorInvalidValue;  // the FP32 products store packed rows
-  cudaError_t e = rows <= 16 ? launch_linear_decode(a, EPI_NONE, false, s, nullptr) : launch_gemm_f32(a, EPI_NONE, s);
+  cudaError_t e = launch_linear_rows(a, EPI_NONE, false, s);
   if (e == cudaSuccess && act) e = launch_activation(a.out, ldo, a.out, ldo, rows, n_out, *act, false, s);
   return e;
 }

@@ -129,6 +129,7 @@ int ensure_device(int device) {
                                     std::to_string(prop.major) + "." + std::to_string(prop.minor) +
                                     "; this library is built for sm_100a only");
     PG_CUDA_TRY(init_kernel_attributes());
+    PG_CUDA_TRY(init_gemm_f32_attributes());
     PG_CUDA_TRY(init_tc_kernel_attributes());
     PG_CUDA_TRY(init_attn_tc_attributes());
     g_device_inited[device] = true;
@@ -779,8 +780,8 @@ static cudaError_t enqueue_decode_step(pg_cache* c, int batch, int splits, cudaS
       if (e2 != cudaSuccess) return e2;
       a.x = c->norm;
     }
-    if (batch > 64 && k % 4 == 0) return launch_gemm_f32(a, epi, s);
-    return launch_linear_decode(a, epi, pdl, s, nullptr);
+    if (a.ln_g) return launch_linear_decode(a, epi, pdl, s, nullptr);
+    return launch_linear_rows(a, epi, pdl, s);
   };
   for (int l = 0; l < m->layers_n(); ++l) {
     const LayerWeights& w = m->layers[l];
@@ -917,7 +918,6 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
     LinearArgs a{};
     a.w = w; a.bias = bias; a.x = x; a.out = out; a.resid = resid; a.eps = eps;
     a.m = rows; a.n = n_out; a.k = k;
-    if (rows <= 16 && k % 4 == 0) return launch_linear_decode(a, epi, false, s, nullptr);
     if (x3_rows && w_lo && x_lo) {
       // FP32-grade product on the tensor cores: x.w + x.w_lo + x_lo.w as three TF32 MMAs per k step
       TcGemmArgs t{};
@@ -933,7 +933,7 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
       t.m = rows; t.n = n_out; t.k = k; t.epilogue = epi;
       return launch_tc_gemm_tf32(t, s);
     }
-    return launch_gemm_f32(a, epi, s);
+    return launch_linear_rows(a, epi, false, s);
   };
   static const bool no_tc_attn = getenv("PG_NO_TC_ATTN") != nullptr;
   for (int l = 0; l < m->layers_n(); ++l) {
@@ -1199,8 +1199,7 @@ static int do_prefill(const pg_model* m, pg_cache* c, const int32_t* ids, const 
   PG_CUDA_TRY(launch_layernorm_rows(c->x, m->lnf_g, m->lnf_b, m->cfg.layer_norm_epsilon, c->norm, batch, m->c(), false, s));
   LinearArgs a{};
   a.w = m->head_w; a.x = c->norm; a.out = c->logits; a.m = batch; a.n = m->v(); a.k = m->c();
-  if (batch > 64 && a.k % 4 == 0) PG_CUDA_TRY(launch_gemm_f32(a, EPI_NONE, s));
-  else PG_CUDA_TRY(launch_linear_decode(a, EPI_NONE, false, s, nullptr));
+  PG_CUDA_TRY(launch_linear_rows(a, EPI_NONE, false, s));
   PG_CUDA_TRY(launch_argmax_rows(c->logits, batch, m->v(), c->d_argmax, s));
   // device-side sequence state: pos = lens, next id = argmax
   PG_CUDA_TRY(cudaMemcpyAsync(c->d_pos, lens, batch * sizeof(int), cudaMemcpyHostToDevice, s));
@@ -1374,8 +1373,7 @@ static int do_forward(const pg_model* m, const int32_t* ids, int t, float* logit
   PG_CUDA_TRY(launch_layernorm_rows(hidden, m->lnf_g, m->lnf_b, m->cfg.layer_norm_epsilon, ws.norm, (int)out_rows, (int)C, false, s));
   LinearArgs a{};
   a.w = m->head_w; a.x = ws.norm; a.out = ws.logits; a.m = (int)out_rows; a.n = (int)V; a.k = (int)C;
-  if (out_rows > 16 && C % 4 == 0) PG_CUDA_TRY(launch_gemm_f32(a, EPI_NONE, s));
-  else PG_CUDA_TRY(launch_linear_decode(a, EPI_NONE, false, s, nullptr));
+  PG_CUDA_TRY(launch_linear_rows(a, EPI_NONE, false, s));
   PG_CUDA_TRY(cudaMemcpyAsync(logits_out, ws.logits, out_rows * V * sizeof(float), cudaMemcpyDeviceToHost, s));
   PG_CUDA_TRY(cudaStreamSynchronize(s));  // also keeps `hm` alive long enough
   return PG_OK;

@@ -71,8 +71,7 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
       LinearArgs a{};
       a.w = dw.as<float>(); a.bias = db.as<float>(); a.x = dx.as<float>(); a.out = dout.as<float>();
       a.resid = dr.as<float>(); a.m = m; a.n = n; a.k = k;
-      if (m <= 64 || k % 4 != 0) return launch_linear_decode(a, epilogue, false, st, nullptr);
-      return launch_gemm_f32(a, epilogue, st);
+      return launch_linear_rows(a, epilogue, false, st);
     }
     TcGemmArgs a{};
     a.w = dw.as<float>(); a.bias = db.as<float>(); a.resid = dr.as<float>(); a.out = dout.as<float>();

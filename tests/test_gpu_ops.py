@@ -34,6 +34,21 @@ def test_linear_fp32_matches_oracle(oracle, m, n, k, epilogue):
     np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
 
 
+# Tiles of 32 and 64 rows by 64 columns, k in blocks of 32 shared out over up to 8 CTAs: edges of all of these, a last share
+# without any block (k 1600: 50 blocks in shares of 7), k that ends inside a block.
+@pytest.mark.parametrize("m,n,k", [(9, 1, 4), (31, 63, 36), (32, 64, 64), (33, 65, 516), (128, 130, 1600), (129, 64, 512),
+                                   (65, 777, 100), (200, 2304, 768)])
+@pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
+def test_linear_fp32_tiles_match_oracle(oracle, m, n, k, epilogue):
+    rng = np.random.default_rng(m * 31 + n * 7 + k + 3)
+    x = rng.standard_normal((m, k), dtype=np.float32)
+    w = rng.standard_normal((n, k), dtype=np.float32) * np.float32(0.05)
+    b = rng.standard_normal(n, dtype=np.float32)
+    r = rng.standard_normal((m, n), dtype=np.float32)
+    got, _ = ops.linear(x, w, b, r if epilogue == "resid" else None, epilogue, "fp32")
+    np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
+
+
 @pytest.mark.parametrize("m,n,k", [(9, 4800, 1600), (16, 1600, 1600), (64, 6400, 1600), (33, 1600, 6400),
                                    (64, 50257, 1024), (40, 1000, 256)])
 @pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
