@@ -18,6 +18,7 @@
 //               without bank conflicts).
 // Every mbarrier wait is bounded; on expiry the error word is raised and all roles fall through.
 #include "kernels.cuh"
+#include "pair.cuh"
 #include "tc_common.cuh"
 
 namespace pg {
@@ -670,8 +671,7 @@ __global__ void __launch_bounds__(X3_THREADS, 1)
       tc_fence_after();
       const float inv = 1.0f / l;
       const int c0 = hf * 32;
-      float* orow = a.out + (size_t)(r0 + qpos) * c + h * AT_D + c0;
-      float* lrow = a.out_lo ? a.out_lo + (size_t)(r0 + qpos) * c + h * AT_D + c0 : nullptr;
+      const size_t at = (size_t)(r0 + qpos) * c + h * AT_D + c0;
       float v[32], v2[32];
       tmem_ld32(tmem_base + X3_O_COL + lane_addr + (uint32_t)c0, v);
       tmem_ld32(tmem_base + X3_OS_COL + lane_addr + (uint32_t)c0, v2);
@@ -680,10 +680,8 @@ __global__ void __launch_bounds__(X3_THREADS, 1)
         for (int j = 0; j < 32; j += 4) {
           const float y0 = (v[j] + v2[j]) * inv, y1 = (v[j + 1] + v2[j + 1]) * inv, y2 = (v[j + 2] + v2[j + 2]) * inv,
                       y3 = (v[j + 3] + v2[j + 3]) * inv;
-          *reinterpret_cast<float4*>(orow + j) = make_float4(y0, y1, y2, y3);
-          if (lrow)
-            *reinterpret_cast<float4*>(lrow + j) =
-                make_float4(y0 - tf32_hi(y0), y1 - tf32_hi(y1), y2 - tf32_hi(y2), y3 - tf32_hi(y3));
+          if (a.pair.hi) store_pair4(a.pair.hi + at + j, a.pair.lo + at + j, make_float4(y0, y1, y2, y3), a.pair.scale);
+          else *reinterpret_cast<float4*>(a.out + at + j) = make_float4(y0, y1, y2, y3);
         }
       }
     }
@@ -714,7 +712,7 @@ cudaError_t launch_prefill_attention_tc(const PrefillAttnArgs& a, int rows, int*
   return cudaGetLastError();
 }
 
-// FP32-grade variant; a.out_lo (optional) receives out - hi(out)
+// FP32-grade variant; a.pair (optional) receives the result as FP16 pairs
 cudaError_t launch_prefill_attention_x3(const PrefillAttnArgs& a, int rows, int* error_flag, cudaStream_t s) {
   if (!prefill_attention_tc_supported(a)) return cudaErrorInvalidValue;
   const int c = a.n_head * 64;

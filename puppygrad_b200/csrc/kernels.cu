@@ -13,6 +13,7 @@
 
 #include "common.h"
 #include "kernels.cuh"
+#include "pair.cuh"
 
 namespace pg {
 namespace {
@@ -39,7 +40,6 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
   return acc;
 }
 
-__device__ __forceinline__ float tf32_trunc(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFFE000u); }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
@@ -534,11 +534,10 @@ __global__ void layernorm_rows_kernel(const float* x, const float* __restrict__ 
 }
 
 // One 128-thread CTA per row, 128-bit loads, row kept in registers between the passes (c % 4 == 0, c <= 4096):
-// the row is read from memory once. `lo` (optional) receives y - hi(y), hi = the upper 19 bits a TF32 tensor
-// core reads, for the FP32-grade GEMM that consumes the row.
+// the row is read from memory once. With `pair` the result goes out as FP16 pairs for the product that reads the row.
 __global__ void __launch_bounds__(128) layernorm_rows_vec_kernel(const float* x, const float* __restrict__ g,
                                                                  const float* __restrict__ b, float eps, float* out,
-                                                                 float* lo, int rows, int c) {
+                                                                 PairOut pair, int rows, int c) {
   __shared__ float red[4];
   pdl_launch();
   pdl_wait();
@@ -574,7 +573,6 @@ __global__ void __launch_bounds__(128) layernorm_rows_vec_kernel(const float* x,
   const float4* g4 = reinterpret_cast<const float4*>(g);
   const float4* b4 = reinterpret_cast<const float4*>(b);
   float4* o4 = reinterpret_cast<float4*>(out + (size_t)r * c);
-  float4* lo4 = lo ? reinterpret_cast<float4*>(lo + (size_t)r * c) : nullptr;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int idx = tid + i * 128;
@@ -582,8 +580,9 @@ __global__ void __launch_bounds__(128) layernorm_rows_vec_kernel(const float* x,
       const float4 gg = g4[idx], bb = b4[idx];
       const float4 y = make_float4((v[i].x - mean) * inv_std * gg.x + bb.x, (v[i].y - mean) * inv_std * gg.y + bb.y,
                                    (v[i].z - mean) * inv_std * gg.z + bb.z, (v[i].w - mean) * inv_std * gg.w + bb.w);
-      o4[idx] = y;
-      if (lo4) lo4[idx] = make_float4(y.x - tf32_trunc(y.x), y.y - tf32_trunc(y.y), y.z - tf32_trunc(y.z), y.w - tf32_trunc(y.w));
+      const size_t at = (size_t)r * c + 4 * idx;
+      if (pair.hi) store_pair4(pair.hi + at, pair.lo + at, y, pair.scale);
+      else o4[idx] = y;
     }
   }
 }
@@ -1078,14 +1077,14 @@ __global__ void __launch_bounds__(128) prefill_attention_kernel(PrefillAttnArgs 
       float y[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) y[e] = o[i][e] * inv;
-      *reinterpret_cast<float4*>(orow + tx * 4) = make_float4(y[0], y[1], y[2], y[3]);
-      *reinterpret_cast<float4*>(orow + 32 + tx * 4) = make_float4(y[4], y[5], y[6], y[7]);
-      if (a.out_lo) {
-        float* lrow = a.out_lo + (size_t)(r0 + qpos) * c + h * D;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) y[e] -= tf32_trunc(y[e]);
-        *reinterpret_cast<float4*>(lrow + tx * 4) = make_float4(y[0], y[1], y[2], y[3]);
-        *reinterpret_cast<float4*>(lrow + 32 + tx * 4) = make_float4(y[4], y[5], y[6], y[7]);
+      const float4 ya = make_float4(y[0], y[1], y[2], y[3]), yb = make_float4(y[4], y[5], y[6], y[7]);
+      if (a.pair.hi) {
+        const size_t at = (size_t)(r0 + qpos) * c + h * D + tx * 4;
+        store_pair4(a.pair.hi + at, a.pair.lo + at, ya, a.pair.scale);
+        store_pair4(a.pair.hi + at + 32, a.pair.lo + at + 32, yb, a.pair.scale);
+      } else {
+        *reinterpret_cast<float4*>(orow + tx * 4) = ya;
+        *reinterpret_cast<float4*>(orow + 32 + tx * 4) = yb;
       }
     }
   }
@@ -1468,10 +1467,10 @@ cudaError_t launch_embed(const float* wte, const float* wpe, const int* ids, con
 }
 
 cudaError_t launch_layernorm_rows(const float* x, const float* g, const float* b, float eps, float* out, int rows,
-                                  int c, bool pdl, cudaStream_t s, float* lo) {
+                                  int c, bool pdl, cudaStream_t s, const PairOut& pair) {
   if (c % 4 == 0 && c <= 4096)
-    return launch(layernorm_rows_vec_kernel, dim3(rows), dim3(128), 0, s, pdl, x, g, b, eps, out, lo, rows, c);
-  if (lo) return cudaErrorInvalidValue;
+    return launch(layernorm_rows_vec_kernel, dim3(rows), dim3(128), 0, s, pdl, x, g, b, eps, out, pair, rows, c);
+  if (pair.hi) return cudaErrorInvalidValue;
   return launch(layernorm_rows_kernel, dim3((rows + 3) / 4), dim3(128), 0, s, pdl, x, g, b, eps, out, rows, c);
 }
 

@@ -38,9 +38,15 @@ int linear_decode_grid(int n, int num_sms);
 // out[r, :] = wte[ids[r]] + wpe[pos[r]]
 cudaError_t launch_embed(const float* wte, const float* wpe, const int* ids, const int* pos, float* out,
                          int rows, int c, bool pdl, cudaStream_t s);
-// out = LayerNorm(x) row-wise; lo (optional; needs c % 4 == 0 and c <= 4096) = out - hi(out), the TF32 lo part of the result
+// A matrix as pairs of FP16 numbers of v * scale (gemm_pair.cu): what the producers of its inputs write instead of FP32.
+struct PairOut {
+  uint16_t* hi = nullptr;
+  uint16_t* lo = nullptr;
+  float scale = 1.f;
+};
+// out = LayerNorm(x) row-wise; with `pair` (needs c % 4 == 0 and c <= 4096) the result goes there instead
 cudaError_t launch_layernorm_rows(const float* x, const float* g, const float* b, float eps, float* out,
-                                  int rows, int c, bool pdl, cudaStream_t s, float* lo = nullptr);
+                                  int rows, int c, bool pdl, cudaStream_t s, const PairOut& pair = {});
 // General FP32 GEMM out[m,n] = x[m,k] . w[n,k]^T (+bias)(+GELU | +resid), CUDA-core FMA (gemm_f32.cu); k % 4 == 0.
 cudaError_t launch_gemm_f32_tiles(const LinearArgs& a, int epilogue, cudaStream_t s);
 cudaError_t init_gemm_f32_attributes();
@@ -67,7 +73,7 @@ cudaError_t launch_decode_attention(const DecodeAttnArgs& a, bool pdl, cudaStrea
 struct PrefillAttnArgs {
   const float* qkv;      // [rows, 3c], sequences concatenated
   float* out;            // [rows, c]
-  float* out_lo;         // optional (head_dim 64, FP32 kernel): out - hi(out), the lo part the FP32-grade GEMM after it reads
+  PairOut pair;          // optional (head_dim 64; not the single TF32 pass): receives the result instead of out
   const int* seq_start;  // [batch + 1] row offsets
   int n_head, head_dim, batch, max_len;
 };
@@ -117,12 +123,11 @@ struct TcGemmArgs {
   const float* x;     // [m, k] activations (x3: the hi part)
   const float* x_lo;  // [m, k] lo part (x3 only)
   const float* w;     // [n, k] row-major; for the x3 kernel the tiled copy made by launch_tile_weights
-  const float* w_lo;  // [n, k] row-major lo parts of w (launch_tc_gemm_tf32x3_rows only)
   const float* bias;  // [n] or nullptr
   const float* resid; // [m, n], EPI_RESID
   float* out;         // [m, n] (may be nullptr in x3 when only the split outputs are wanted)
   float* out_hi;      // x3: optional TF32 hi/lo pair of the result, [m, n] each
-  float* out_lo;      // launch_tc_gemm_tf32x3_rows: optional, out - hi(out) (out_hi unused there)
+  float* out_lo;
   int* error_flag;    // set non-zero if a bounded wait inside the kernel expired
   unsigned long long* trace;  // optional tuning aid (x3 kernel): 16 words per CTA, phase timestamps and cycle counts
   int m, n, k, epilogue;
@@ -135,9 +140,28 @@ size_t tc_tiled_weight_floats(int n, int k);
 cudaError_t launch_tile_weights(const float* src, float* dst, int n, int k, cudaStream_t s);
 // single TF32 pass, any m (prefill)
 cudaError_t launch_tc_gemm_tf32(const TcGemmArgs& a, cudaStream_t s);
-// three TF32 passes (FP32-grade), any m (prefill): x_lo and w_lo hold v - hi(v) of x and w (launch_tf32_lo)
-cudaError_t launch_tc_gemm_tf32x3_rows(const TcGemmArgs& a, cudaStream_t s);
-cudaError_t launch_tf32_lo(const float* x, float* lo, size_t n, cudaStream_t s);
+
+// FP32-grade product of FP16 pairs, any m (prefill; gemm_pair.cu): out[m, n] = x[m, k] . w[n, k]^T (+bias)(+GELU | +resid).
+struct PairGemmArgs {
+  const uint16_t *x_hi, *x_lo;  // [m, k]
+  const uint16_t *w_hi, *w_lo;  // [n, k]; w_lo nullptr: all zero (BF16 weights)
+  float inv_x, inv_w;           // reciprocals of the two scales
+  const float* bias;            // [n] or nullptr
+  const float* resid;           // [m, n], EPI_RESID (may alias out)
+  float* out;                   // [m, n], or nullptr when the result goes out as pairs:
+  uint16_t *out_hi, *out_lo;    // [m, n], n even, no residual
+  float out_scale;
+  int* error_flag;
+  int m, n, k, epilogue;
+};
+bool pair_gemm_supported(int k);
+cudaError_t launch_tc_gemm_pair(const PairGemmArgs& a, cudaStream_t s);
+cudaError_t init_pair_gemm_attributes();
+// Scale for values that stay below `bound`; pairs of n values (n % 4 == 0; lo nullptr: only hi parts); {largest |w|, largest norm of a row from
+// `norm_from` on} as bit patterns into out[2], which starts at zero.
+float pair_scale(float bound);
+cudaError_t launch_make_pairs(const float* x, uint16_t* hi, uint16_t* lo, size_t n, float scale, cudaStream_t s);
+cudaError_t launch_matrix_bounds(const float* w, int rows, int cols, int norm_from, unsigned* out, cudaStream_t s);
 // three TF32 passes (FP32-grade), m <= 64 (decode)
 int tc_gemm_x3_splits(int n, int k, int num_sms);
 cudaError_t launch_tc_gemm_x3(const TcGemmArgs& a, int splits, bool pdl, cudaStream_t s);

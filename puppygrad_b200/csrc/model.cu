@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -27,7 +28,7 @@ pg_model::~pg_model() {
     cudaSetDevice(device);
     cudaFree(arena);
     if (tiled_arena) cudaFree(tiled_arena);
-    if (lo_arena) cudaFree(lo_arena);
+    if (pair_arena) cudaFree(pair_arena);
     if (packed_arena) cudaFree(packed_arena);
     if (scale_arena) cudaFree(scale_arena);
     if (head_deq) cudaFree(head_deq);
@@ -93,7 +94,7 @@ pg_cache::~pg_cache() {
   for (void* p : {(void*)kv_pool, (void*)d_ids, (void*)d_pos, (void*)d_argmax, (void*)d_token_log,
                   (void*)x, (void*)norm, (void*)qkv, (void*)attn, (void*)hbuf, (void*)logits, (void*)part_val,
                   (void*)part_idx, (void*)attn_part, (void*)attn_counters, (void*)topk_vals, (void*)topk_idx,
-                  (void*)px, (void*)pnorm, (void*)pqkv, (void*)pattn, (void*)ph, (void*)plo, (void*)prow, (void*)norm_lo,
+                  (void*)px, (void*)pnorm, (void*)pqkv, (void*)pattn, (void*)ph, (void*)prow, (void*)norm_lo,
                   (void*)attn_lo, (void*)h_lo, (void*)d_error, (void*)d_stream_ll, (void*)d_stream_epoch,
                   (void*)chain_partials, (void*)d_chain_barrier, (void*)d_chain_trace, (void*)d_chain_best})
     if (p) cudaFree(p);
@@ -131,6 +132,7 @@ int ensure_device(int device) {
     PG_CUDA_TRY(init_kernel_attributes());
     PG_CUDA_TRY(init_gemm_f32_attributes());
     PG_CUDA_TRY(init_tc_kernel_attributes());
+    PG_CUDA_TRY(init_pair_gemm_attributes());
     PG_CUDA_TRY(init_attn_tc_attributes());
     g_device_inited[device] = true;
   }
@@ -138,6 +140,73 @@ int ensure_device(int device) {
 }
 
 static size_t align_up(size_t n, size_t a) { return (n + a - 1) / a * a; }
+
+// FP16 pairs of the dense matrices, and the scales of their inputs: what the values of each can reach at most, from the
+// weights alone. `tensors`: the host tensors of the model.
+static int make_pair_weights(pg_model* m, const float* const* tensors) {
+  const size_t C = m->c(), F = m->f(), L = m->layers.size();
+  if (!pair_gemm_supported((int)C) || !pair_gemm_supported((int)F)) return PG_OK;
+  const bool exact = m->backend.math_mode == PG_MATH_BF16;  // BF16 values fit the hi part
+  const size_t per_layer = 4 * C * C + 2 * C * F;
+  PG_CUDA_TRY(cudaMalloc(&m->pair_arena, per_layer * L * (exact ? 1 : 2) * sizeof(uint16_t)));
+  unsigned* d_bounds = nullptr;
+  PG_CUDA_TRY(cudaMalloc(&d_bounds, L * 8 * sizeof(unsigned)));
+  std::vector<float> bounds(L * 8);
+  int rc = [&]() -> int {
+    PG_CUDA_TRY(cudaMemsetAsync(d_bounds, 0, L * 8 * sizeof(unsigned), 0));
+    for (size_t l = 0; l < L; ++l) {
+      const LayerWeights& w = m->layers[l];
+      unsigned* b = d_bounds + 8 * l;
+      PG_CUDA_TRY(launch_matrix_bounds(w.w_qkv, (int)(3 * C), (int)C, (int)(2 * C), b, 0));  // norms of the value rows
+      PG_CUDA_TRY(launch_matrix_bounds(w.w_proj, (int)C, (int)C, 0, b + 2, 0));
+      PG_CUDA_TRY(launch_matrix_bounds(w.w_fc, (int)F, (int)C, 0, b + 4, 0));
+      PG_CUDA_TRY(launch_matrix_bounds(w.w_proj2, (int)C, (int)F, 0, b + 6, 0));
+    }
+    PG_CUDA_TRY(cudaMemcpy(bounds.data(), d_bounds, L * 8 * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    return PG_OK;
+  }();
+  cudaFree(d_bounds);
+  if (rc != PG_OK) return rc;
+  uint16_t* at = m->pair_arena;
+  auto pairs = [&](const float* w, size_t n, float top, PairWeights* out) -> int {
+    out->scale = pair_scale(top);
+    uint16_t *hi = at, *lo = at + n;
+    if (exact) lo = nullptr;
+    PG_CUDA_TRY(launch_make_pairs(w, hi, lo, n, out->scale, 0));
+    out->hi = hi;
+    out->lo = lo;
+    at += exact ? n : 2 * n;
+    return PG_OK;
+  };
+  auto largest = [](const float* v, size_t n) {
+    float top = 0.f;
+    for (size_t i = 0; i < n; ++i) top = std::max(top, std::fabs(v[i]));
+    return top;
+  };
+  auto norm = [](const float* v, size_t n) {
+    double sq = 0.0;
+    for (size_t i = 0; i < n; ++i) sq += (double)v[i] * v[i];
+    return (float)std::sqrt(sq);
+  };
+  for (size_t l = 0; l < L; ++l) {
+    LayerWeights& w = m->layers[l];
+    const float* const* t = tensors + 4 + 12 * l;
+    const float* b = bounds.data() + 8 * l;
+    if (int r = pairs(w.w_qkv, 3 * C * C, b[0], &w.q_qkv)) return r;
+    if (int r = pairs(w.w_proj, C * C, b[2], &w.q_proj)) return r;
+    if (int r = pairs(w.w_fc, C * F, b[4], &w.q_fc)) return r;
+    if (int r = pairs(w.w_proj2, C * F, b[6], &w.q_proj2)) return r;
+    // a normalised row has a norm of at most sqrt(C), so one output of the product behind it is at most its weight row's norm
+    // times the norm of the scaled and shifted row; attention outputs are convex combinations of value rows, |gelu(y)| <= |y|
+    const float root = std::sqrt((float)C);
+    const float row1 = root * largest(t[0], C) + norm(t[1], C), row2 = root * largest(t[6], C) + norm(t[7], C);
+    w.x_norm1 = pair_scale(root * largest(t[0], C) + largest(t[1], C));
+    w.x_attn = pair_scale(b[1] * row1 + largest(t[3] + 2 * C, C));
+    w.x_norm2 = pair_scale(root * largest(t[6], C) + largest(t[7], C));
+    w.x_h = pair_scale(b[5] * row2 + largest(t[9], F));
+  }
+  return PG_OK;
+}
 
 static int build_model(const pg_gpt2_config& cfg, const float* const* tensors, const uint64_t* lens, uint64_t n,
                        const pg_backend_config* backend, pg_model** out) {
@@ -289,23 +358,8 @@ static int build_model(const pg_gpt2_config& cfg, const float* const* tensors, c
       if (int r = tile(w.w_proj2, C, F, &w.t_proj2)) return r;
     }
     if (int r = tile(m->head_w, V, C, &m->t_wte)) return r;
-    if (C % 4 == 0 && F % 4 == 0) {
-      const size_t per_lo = (size_t)3 * C * C + (size_t)C * C + 2 * (size_t)C * F;
-      PG_CUDA_TRY(cudaMalloc(&m->lo_arena, per_lo * cfg.n_layer * sizeof(float)));
-      float* q = m->lo_arena;
-      auto lo = [&](const float* src, size_t n, float** dst) -> int {
-        *dst = q;
-        PG_CUDA_TRY(launch_tf32_lo(src, q, n, 0));
-        q += n;
-        return PG_OK;
-      };
-      for (auto& w : m->layers) {
-        if (int r = lo(w.w_qkv, (size_t)3 * C * C, &w.l_qkv)) return r;
-        if (int r = lo(w.w_proj, (size_t)C * C, &w.l_proj)) return r;
-        if (int r = lo(w.w_fc, (size_t)C * F, &w.l_fc)) return r;
-        if (int r = lo(w.w_proj2, (size_t)C * F, &w.l_proj2)) return r;
-      }
-    }
+    if (be.math_mode != PG_MATH_TF32)
+      if (int r = make_pair_weights(m.get(), tensors)) return r;
     PG_CUDA_TRY(cudaDeviceSynchronize());
   }
   *out = m.release();
@@ -875,9 +929,9 @@ struct PrefillPlan {
 static int grow_prefill_workspace(pg_cache* c, size_t rows) {
   if (rows <= c->pre_rows) return PG_OK;
   const pg_model* m = c->model;
-  for (void* p : {(void*)c->px, (void*)c->pnorm, (void*)c->pqkv, (void*)c->pattn, (void*)c->ph, (void*)c->plo, (void*)c->prow})
+  for (void* p : {(void*)c->px, (void*)c->pnorm, (void*)c->pqkv, (void*)c->pattn, (void*)c->ph, (void*)c->prow})
     if (p) cudaFree(p);
-  c->px = c->pnorm = c->pqkv = c->pattn = c->ph = c->plo = nullptr;
+  c->px = c->pnorm = c->pqkv = c->pattn = c->ph = nullptr;
   c->prow = nullptr;
   c->pre_rows = 0;
   const size_t C = m->c(), F = m->f();
@@ -886,7 +940,6 @@ static int grow_prefill_workspace(pg_cache* c, size_t rows) {
   PG_CUDA_TRY(cudaMalloc(&c->pqkv, rows * 3 * C * sizeof(float)));
   PG_CUDA_TRY(cudaMalloc(&c->pattn, rows * C * sizeof(float)));
   PG_CUDA_TRY(cudaMalloc(&c->ph, rows * F * sizeof(float)));
-  if (m->lo_arena) PG_CUDA_TRY(cudaMalloc(&c->plo, rows * (size_t)(C + F) * sizeof(float)));
   PG_CUDA_TRY(cudaMalloc(&c->prow, (rows * 3 + 2 * (size_t)c->max_batch + 2) * sizeof(int)));
   c->pre_rows = rows;
   return PG_OK;
@@ -897,7 +950,6 @@ static int grow_prefill_workspace(pg_cache* c, size_t rows) {
 // the paged cache. block_forward, rust.rs:1053-1134.
 struct BlockWorkspace {
   float *x, *norm, *qkv, *attn, *h;
-  float* lo;  // FP32-grade tensor-core prefill: lo parts of the GEMM inputs, [rows, C] then [rows, F], or nullptr
   const int *d_slot, *d_pos, *d_seq_start;
   int* d_error;  // error word of the tensor-core kernels (may be nullptr: then they are not used)
 };
@@ -906,25 +958,30 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
                       cudaStream_t s) {
   const int C = m->c(), F = m->f(), rows = plan.rows;
   const float eps = m->cfg.layer_norm_epsilon;
-  const bool x3_mode = m->backend.math_mode == PG_MATH_TF32X3 || m->backend.math_mode == PG_MATH_BF16;
-  // The FP32-grade tensor-core GEMM reads x and x - hi(x); whoever produces x (LayerNorm, attention, the GELU
-  // epilogue of the MLP's first GEMM) writes the lo part along with it, so no separate pass over x is needed.
-  const bool x3_rows = x3_mode && ws.lo && ws.d_error && rows >= 128 && m->lo_arena && m->head_dim() == 64 &&
-                       C % 4 == 0 && C <= 4096 && tc_gemm_supported(rows, C, C) && tc_gemm_supported(rows, C, F);
-  float* lo_c = x3_rows ? ws.lo : nullptr;                    // [rows, C]: LayerNorm or attention output
-  float* lo_f = x3_rows ? ws.lo + (size_t)rows * C : nullptr;  // [rows, F]: MLP hidden
-  auto gemm = [&](const float* w, const float* w_lo, const float* bias, const float* x, const float* x_lo, float* out,
-                  float* out_lo, int n_out, int k, int epi, const float* resid) -> cudaError_t {
+  // FP32-grade products on the tensor cores read FP16 pairs; whoever produces an input (LayerNorm, attention, the GELU
+  // epilogue of the MLP's first product) writes pairs instead of FP32, into the same buffer: [rows, k] hi, then lo.
+  const bool pairs = m->pair_arena && ws.d_error && rows >= 128 && m->head_dim() == 64 && C <= 4096;
+  auto pair_of = [&](float* buf, int k, float scale) {
+    PairOut p;
+    if (pairs) {
+      p.hi = reinterpret_cast<uint16_t*>(buf);
+      p.lo = p.hi + (size_t)rows * k;
+      p.scale = scale;
+    }
+    return p;
+  };
+  auto gemm = [&](const float* w, const PairWeights& q, const float* bias, const float* x, const PairOut& xp, float* out,
+                  const PairOut& outp, int n_out, int k, int epi, const float* resid) -> cudaError_t {
     LinearArgs a{};
     a.w = w; a.bias = bias; a.x = x; a.out = out; a.resid = resid; a.eps = eps;
     a.m = rows; a.n = n_out; a.k = k;
-    if (x3_rows && w_lo && x_lo) {
-      // FP32-grade product on the tensor cores: x.w + x.w_lo + x_lo.w as three TF32 MMAs per k step
-      TcGemmArgs t{};
-      t.x = x; t.x_lo = x_lo; t.w = w; t.w_lo = w_lo; t.bias = bias; t.resid = resid; t.out = out; t.out_lo = out_lo;
+    if (pairs) {
+      PairGemmArgs t{};
+      t.x_hi = xp.hi; t.x_lo = xp.lo; t.w_hi = q.hi; t.w_lo = q.lo; t.inv_x = 1.f / xp.scale; t.inv_w = 1.f / q.scale;
+      t.bias = bias; t.resid = resid; t.out = outp.hi ? nullptr : out; t.out_hi = outp.hi; t.out_lo = outp.lo; t.out_scale = outp.scale;
       t.error_flag = ws.d_error;
       t.m = rows; t.n = n_out; t.k = k; t.epilogue = epi;
-      return launch_tc_gemm_tf32x3_rows(t, s);
+      return launch_tc_gemm_pair(t, s);
     }
     if (m->backend.math_mode == PG_MATH_TF32 && ws.d_error && rows >= 128 && tc_gemm_supported(rows, n_out, k)) {
       // single TF32 pass on the tensor cores: the fast prefill variant with its own looser bound
@@ -938,27 +995,26 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
   static const bool no_tc_attn = getenv("PG_NO_TC_ATTN") != nullptr;
   for (int l = 0; l < m->layers_n(); ++l) {
     const LayerWeights& w = m->layers[l];
-    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln1_g, w.ln1_b, eps, ws.norm, rows, C, false, s, lo_c));
-    PG_CUDA_TRY(gemm(w.w_qkv, w.l_qkv, w.b_qkv, ws.norm, lo_c, ws.qkv, nullptr, 3 * C, C, EPI_NONE, nullptr));
+    const PairOut n1 = pair_of(ws.norm, C, w.x_norm1), at = pair_of(ws.attn, C, w.x_attn), n2 = pair_of(ws.norm, C, w.x_norm2),
+                  hp = pair_of(ws.h, F, w.x_h), none;
+    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln1_g, w.ln1_b, eps, ws.norm, rows, C, false, s, n1));
+    PG_CUDA_TRY(gemm(w.w_qkv, w.q_qkv, w.b_qkv, ws.norm, n1, ws.qkv, none, 3 * C, C, EPI_NONE, nullptr));
     if (cache)
       PG_CUDA_TRY(launch_kv_scatter(ws.qkv, ws.d_slot, ws.d_pos, cache->layer_pool(l), cache->tables[0].d_table, cache->kv,
                                     rows, s));
     PrefillAttnArgs pa{};
-    pa.qkv = ws.qkv; pa.out = ws.attn; pa.seq_start = ws.d_seq_start;
+    pa.qkv = ws.qkv; pa.out = ws.attn; pa.pair = at; pa.seq_start = ws.d_seq_start;
     pa.n_head = m->heads(); pa.head_dim = m->head_dim(); pa.batch = plan.batch; pa.max_len = plan.max_len;
-    if (m->backend.math_mode == PG_MATH_TF32 && ws.d_error && !no_tc_attn && prefill_attention_tc_supported(pa)) {
+    if (m->backend.math_mode == PG_MATH_TF32 && ws.d_error && !no_tc_attn && prefill_attention_tc_supported(pa))
       PG_CUDA_TRY(launch_prefill_attention_tc(pa, rows, ws.d_error, s));
-    } else if (x3_rows && !no_tc_attn && prefill_attention_tc_supported(pa)) {
-      pa.out_lo = lo_c;
+    else if (pairs && !no_tc_attn && prefill_attention_tc_supported(pa))
       PG_CUDA_TRY(launch_prefill_attention_x3(pa, rows, ws.d_error, s));
-    } else {
-      pa.out_lo = lo_c;
+    else
       PG_CUDA_TRY(launch_prefill_attention(pa, s));
-    }
-    PG_CUDA_TRY(gemm(w.w_proj, w.l_proj, w.b_proj, ws.attn, lo_c, ws.x, nullptr, C, C, EPI_RESID, ws.x));
-    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln2_g, w.ln2_b, eps, ws.norm, rows, C, false, s, lo_c));
-    PG_CUDA_TRY(gemm(w.w_fc, w.l_fc, w.b_fc, ws.norm, lo_c, ws.h, lo_f, F, C, EPI_GELU, nullptr));
-    PG_CUDA_TRY(gemm(w.w_proj2, w.l_proj2, w.b_proj2, ws.h, lo_f, ws.x, nullptr, C, F, EPI_RESID, ws.x));
+    PG_CUDA_TRY(gemm(w.w_proj, w.q_proj, w.b_proj, ws.attn, at, ws.x, none, C, C, EPI_RESID, ws.x));
+    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln2_g, w.ln2_b, eps, ws.norm, rows, C, false, s, n2));
+    PG_CUDA_TRY(gemm(w.w_fc, w.q_fc, w.b_fc, ws.norm, n2, ws.h, hp, F, C, EPI_GELU, nullptr));
+    PG_CUDA_TRY(gemm(w.w_proj2, w.q_proj2, w.b_proj2, ws.h, hp, ws.x, none, C, F, EPI_RESID, ws.x));
   }
   return PG_OK;
 }
@@ -1191,7 +1247,7 @@ static int do_prefill(const pg_model* m, pg_cache* c, const int32_t* ids, const 
   PG_CUDA_TRY(cudaMemcpyAsync(d_start, plan.seq_start.data(), (batch + 1) * sizeof(int), cudaMemcpyHostToDevice, s));
   PG_CUDA_TRY(cudaMemcpyAsync(d_last, plan.last_rows.data(), batch * sizeof(int), cudaMemcpyHostToDevice, s));
   PG_CUDA_TRY(launch_embed(m->wte, m->wpe, d_ids, d_pos, c->px, plan.rows, m->c(), false, s));
-  BlockWorkspace ws{c->px, c->pnorm, c->pqkv, c->pattn, c->ph, c->plo, d_slot, d_pos, d_start, c->d_error};
+  BlockWorkspace ws{c->px, c->pnorm, c->pqkv, c->pattn, c->ph, d_slot, d_pos, d_start, c->d_error};
   if (int r = run_blocks(m, ws, plan, c, s)) return r;
   // last position of each prompt -> ln_f -> lm_head (the reference computes logits for every
   // prompt token and keeps the last, rust.rs:920-926; only the last is observable)
@@ -1367,7 +1423,7 @@ static int do_forward(const pg_model* m, const int32_t* ids, int t, float* logit
   hm[2 * R + 1] = t;
   PG_CUDA_TRY(cudaMemcpyAsync(ws.meta, hm.data(), hm.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   PG_CUDA_TRY(launch_embed(m->wte, m->wpe, ws.meta, ws.meta + R, ws.x, t, (int)C, false, s));
-  BlockWorkspace bw{ws.x, ws.norm, ws.qkv, ws.attn, ws.h, nullptr, nullptr, ws.meta + R, ws.meta + 2 * R, nullptr};
+  BlockWorkspace bw{ws.x, ws.norm, ws.qkv, ws.attn, ws.h, nullptr, ws.meta + R, ws.meta + 2 * R, nullptr};
   if (int r = run_blocks(m, bw, plan, nullptr, s)) return r;
   const float* hidden = last_only ? ws.x + (R - 1) * C : ws.x;
   PG_CUDA_TRY(launch_layernorm_rows(hidden, m->lnf_g, m->lnf_b, m->cfg.layer_norm_epsilon, ws.norm, (int)out_rows, (int)C, false, s));

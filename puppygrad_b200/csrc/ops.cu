@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <string>
@@ -54,6 +55,15 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const size_t xs = (size_t)m * k, ws = (size_t)n * k, os = (size_t)m * n;
+  float x_scale = 1.f, w_scale = 1.f;  // of the FP16 pairs
+  if (x3_rows) {
+    float top = 0.f;
+    for (size_t i = 0; i < xs; ++i) top = std::max(top, std::fabs(x[i]));
+    x_scale = pair_scale(top);
+    top = 0.f;
+    for (size_t i = 0; i < ws; ++i) top = std::max(top, std::fabs(w[i]));
+    w_scale = pair_scale(top);
+  }
   DeviceBuf dx, dw, dwt, db, dr, dout, dhi, dlo, derr, dflush, dtrace, dpart, dbar, dwlo;
 #ifdef PG_DEV_TRACE
   const bool want_trace = getenv("PG_TRACE") != nullptr;  // developer aid: phase time stamps of the kernel, printed below
@@ -80,11 +90,15 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
       a.x = dx.as<float>();
       return launch_tc_gemm_tf32(a, st);
     }
-    if (x3_rows) {  // the lo parts of the activations are made per call, as the prefill does; those of the weights once
-      cudaError_t e = launch_tf32_lo(dx.as<float>(), dlo.as<float>(), xs, st);
+    if (x3_rows) {  // the pairs of the activations are made per call, those of the weights once
+      uint16_t *xp = dlo.as<uint16_t>(), *wp = dwlo.as<uint16_t>();
+      cudaError_t e = launch_make_pairs(dx.as<float>(), xp, xp + xs, xs, x_scale, st);
       if (e != cudaSuccess) return e;
-      a.x = dx.as<float>(); a.x_lo = dlo.as<float>(); a.w_lo = dwlo.as<float>();
-      return launch_tc_gemm_tf32x3_rows(a, st);
+      PairGemmArgs p{};
+      p.x_hi = xp; p.x_lo = xp + xs; p.w_hi = wp; p.w_lo = wp + ws; p.inv_x = 1.f / x_scale; p.inv_w = 1.f / w_scale;
+      p.bias = a.bias; p.resid = a.resid; p.out = a.out; p.error_flag = a.error_flag;
+      p.m = m; p.n = n; p.k = k; p.epilogue = epilogue;
+      return launch_tc_gemm_pair(p, st);
     }
     cudaError_t e = launch_split_tf32(dx.as<float>(), dhi.as<float>(), dlo.as<float>(), xs, false, st);
     if (e != cudaSuccess) return e;
@@ -122,7 +136,7 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
     }
     PG_OP_TRY(cudaMalloc(&dlo.p, xs * 4));
     PG_OP_TRY(cudaMalloc(&dwlo.p, ws * 4));
-    PG_OP_TRY(launch_tf32_lo(dw.as<float>(), dwlo.as<float>(), ws, s));
+    PG_OP_TRY(launch_make_pairs(dw.as<float>(), dwlo.as<uint16_t>(), dwlo.as<uint16_t>() + ws, ws, w_scale, s));
   } else if (math_mode == PG_MATH_TF32X3) {
     splits = tc_gemm_x3_splits(n, k, sms);
     PG_OP_TRY(cudaMalloc(&dhi.p, xs * 4));

@@ -23,13 +23,20 @@ namespace pg {
                                     __FILE__ + ":" + std::to_string(__LINE__) + " (" #expr ")"); \
   } while (0)
 
+// A weight matrix as FP16 pairs (gemm_pair.cu), [out, in] row-major; lo nullptr: all zero.
+struct PairWeights {
+  const uint16_t *hi = nullptr, *lo = nullptr;
+  float scale = 1.f;
+};
+
 struct LayerWeights {
   float *ln1_g, *ln1_b, *w_qkv, *b_qkv, *w_proj, *b_proj, *ln2_g, *ln2_b, *w_fc, *b_fc, *w_proj2, *b_proj2;
   // copies in the tiled layout of the tensor-core decode kernel (nullptr in fp32 mode)
   float *t_qkv = nullptr, *t_proj = nullptr, *t_fc = nullptr, *t_proj2 = nullptr;
-  // lo parts (w - hi(w), hi = the upper 19 bits a TF32 tensor core reads) of the four matrices, [out, in] row-major:
-  // second operand of the FP32-grade prefill GEMM (nullptr in fp32 mode)
-  float *l_qkv = nullptr, *l_proj = nullptr, *l_fc = nullptr, *l_proj2 = nullptr;
+  // FP16 pairs of the four matrices for FP32-grade products of prompt rows (tf32x3 and bf16 modes), and the scales of the pairs
+  // that their inputs are kept as: LayerNorm and attention outputs, hidden units
+  PairWeights q_qkv, q_proj, q_fc, q_proj2;
+  float x_norm1 = 1.f, x_attn = 1.f, x_norm2 = 1.f, x_h = 1.f;
   // packed copies for the single-kernel decode step (BF16 or row-quantised int8 weights), [out, in] rows, and,
   // for int8, one scale per output row
   void *p_qkv = nullptr, *p_proj = nullptr, *p_fc = nullptr, *p_proj2 = nullptr;
@@ -97,7 +104,7 @@ struct pg_model {
   float* tiled_arena = nullptr;  // second copy of the dense matrices, tiled for TMA (tensor-core modes)
   size_t tiled_floats = 0;
   float* t_wte = nullptr;
-  float* lo_arena = nullptr;
+  uint16_t* pair_arena = nullptr;  // FP16 pairs of the dense matrices (FP32-grade products of prompt rows)
   size_t arena_floats = 0;
   int stream_weight_type = STREAM_W_F32;  // what the single-kernel decode step streams
   unsigned char* packed_arena = nullptr;  // BF16 / int8 copies of the dense matrices and of wte
@@ -173,7 +180,7 @@ struct pg_cache {
   int *h_ids = nullptr, *h_out = nullptr;  // pinned staging
   // prefill workspace (grow-only)
   size_t pre_rows = 0;
-  float *px = nullptr, *pnorm = nullptr, *pqkv = nullptr, *pattn = nullptr, *ph = nullptr, *plo = nullptr;
+  float *px = nullptr, *pnorm = nullptr, *pqkv = nullptr, *pattn = nullptr, *ph = nullptr;
   int* prow = nullptr;  // [4][pre_rows]: ids, pos, slot, (batch+1 seq_start / last rows)
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (batch, splits) -> decode-step graph
   std::map<std::pair<int, int>, uint64_t> graphs_launches;  // kernel nodes in each graph
