@@ -250,36 +250,41 @@ __global__ void __launch_bounds__(192, 1)
 }
 
 // ------------------------------------------------------------------ decode rows
-template <int BN, int SPLITS>
+template <int BN>
 struct RowsSmem {
-  static constexpr int STAGES = 6;
+  static constexpr int STAGES = BN == 64 ? 4 : 5;
   static constexpr int A_BYTES = TILE_M * KB * 2, B_BYTES = BN * KB * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // both multiples of 1024
-  static constexpr int RECV_BYTES = TILE_M * BN * 4;     // partial sums of this block's rows from every block of the cluster
-  static constexpr size_t BYTES = (size_t)STAGES * STAGE_BYTES + RECV_BYTES + 1024 + 256;
+  static constexpr size_t BYTES = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
+  static_assert(TILE_M * BN * 4 <= STAGES * STAGE_BYTES, "the partial sums reuse the ring");
+  static_assert(2 * (BYTES + 1024) <= 228 * 1024, "two blocks on an SM");
 };
 
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+__device__ __forceinline__ float4 cluster_load4(uint32_t addr, uint32_t rank) {
   uint32_t r;
-  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r) : "memory");
+  return v;
 }
-__device__ __forceinline__ void cluster_store(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-template <int BN, int SPLITS>
-__global__ void __launch_bounds__(192, 1)
+// A block multiplies 128 weight rows with the m <= BN input rows over its share of k, leaves the partial sums in its shared
+// memory (where the operands were), and the blocks of the cluster each add and store an equal part of the tile, in split order.
+//
+// Bound by the weight stream, so the grid is made to fill the chip (launch_rows_bn), and a block takes less than half of an SM's
+// shared memory: the next kernel's blocks find room beside the running ones and have their first weights loaded when
+// the dependency is released.
+template <int BN>
+__global__ void __launch_bounds__(192, 2)
     tc_gemm_bf16_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, Bf16GemmArgs a,
                              int out_kind) {
-  using S = RowsSmem<BN, SPLITS>;
+  using S = RowsSmem<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* recv = reinterpret_cast<float*>(base + (size_t)S::STAGES * S::STAGE_BYTES);  // [SPLITS][BN][TILE_M / SPLITS]
-  uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(recv) + S::RECV_BYTES);
+  float* part = reinterpret_cast<float*>(base);  // [BN][TILE_M], once the products are done
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + (size_t)S::STAGES * S::STAGE_BYTES);
   uint64_t* empty = full + S::STAGES;
   uint64_t* d_full = empty + S::STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_full + 1);
@@ -287,8 +292,8 @@ __global__ void __launch_bounds__(192, 1)
   constexpr uint32_t COLS = BN < 32 ? 32 : BN;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * TILE_M, split = blockIdx.y;
-  const int nkb_all = (a.k + KB - 1) / KB, kb0 = nkb_all * split / SPLITS, nkb = nkb_all * (split + 1) / SPLITS - kb0;
+  const int n0 = blockIdx.x * TILE_M, split = blockIdx.y, splits = gridDim.y;
+  const int nkb_all = (a.k + KB - 1) / KB, kb0 = nkb_all * split / splits, nkb = nkb_all * (split + 1) / splits - kb0;
   const int head = blockIdx.z, x0 = head * a.x_head;
   const int wrow = ((head * (int)gridDim.x + (int)blockIdx.x) * nkb_all + kb0) * TILE_M;  // first row of this block's run of weight tiles
 
@@ -304,8 +309,6 @@ __global__ void __launch_bounds__(192, 1)
   if (warp == 1) tmem_alloc(tmem_slot, COLS);
   tc_fence_before();
   __syncthreads();
-  // nobody writes into a peer's receive buffer before every block of the cluster runs
-  cluster_barrier();
   tc_fence_after();
   const uint32_t tmem_d = *tmem_slot;
   pdl_launch();
@@ -321,74 +324,104 @@ __global__ void __launch_bounds__(192, 1)
       for (int i = 0; i < ahead; ++i)
         tma_load_2d(base + (size_t)i * S::STAGE_BYTES + S::A_BYTES, &map_x, x0 + (kb0 + i) * KB, 0, &full[i]);
       bool ok = true;
-      for (int i = ahead; i < nkb; ++i) {
-        const int s = i % S::STAGES;
-        ok = mbar_wait(&empty[s], ((i / S::STAGES) - 1) & 1, failed, a.error_flag, 11);
+      RingCursor c;  // of the stage that block i goes to
+      for (int i = 0; i < ahead; ++i) c.next(S::STAGES);
+      for (int i = ahead; i < nkb; ++i, c.next(S::STAGES)) {
+        ok = mbar_wait(&empty[c.stage], c.parity ^ 1, failed, a.error_flag, 11);
         if (!ok) break;
-        mbar_expect_tx(&full[s], S::STAGE_BYTES);
-        tma_load_2d(base + (size_t)s * S::STAGE_BYTES, &map_w, 0, wrow + i * TILE_M, &full[s]);
-        tma_load_2d(base + (size_t)s * S::STAGE_BYTES + S::A_BYTES, &map_x, x0 + (kb0 + i) * KB, 0, &full[s]);
+        mbar_expect_tx(&full[c.stage], S::STAGE_BYTES);
+        tma_load_2d(base + (size_t)c.stage * S::STAGE_BYTES, &map_w, 0, wrow + i * TILE_M, &full[c.stage]);
+        tma_load_2d(base + (size_t)c.stage * S::STAGE_BYTES + S::A_BYTES, &map_x, x0 + (kb0 + i) * KB, 0, &full[c.stage]);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc = umma_idesc_bf16(TILE_M, BN);
       bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
-        const int s = i % S::STAGES;
-        ok = mbar_wait(&full[s], (i / S::STAGES) & 1, failed, a.error_flag, 12);
+      RingCursor c;
+      for (int i = 0; i < nkb; ++i, c.next(S::STAGES)) {
+        ok = mbar_wait(&full[c.stage], c.parity, failed, a.error_flag, 12);
         if (!ok) break;
         tc_fence_after();
-        const uint64_t da = umma_desc_sw128(base + (size_t)s * S::STAGE_BYTES);
-        const uint64_t db = umma_desc_sw128(base + (size_t)s * S::STAGE_BYTES + S::A_BYTES);
+        const uint64_t da = umma_desc_sw128(base + (size_t)c.stage * S::STAGE_BYTES);
+        const uint64_t db = umma_desc_sw128(base + (size_t)c.stage * S::STAGE_BYTES + S::A_BYTES);
 #pragma unroll
         for (int k = 0; k < KB / 16; ++k) umma_bf16_ss(tmem_d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i | k) != 0);
-        umma_commit(&empty[s]);
+        umma_commit(&empty[c.stage]);
       }
       if (ok) umma_commit(d_full);
     }
   } else {
-    // row r of the tile is finished by block r / RP of the cluster: this thread sends its partial sums there
     const int r = (warp & 3) * 32 + lane;
-    constexpr int RP = TILE_M / SPLITS;
     bool ok = mbar_wait(d_full, 0, failed, a.error_flag, 13);
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
-      const uint32_t dst = cluster_addr(smem_u32(recv), (uint32_t)(r / RP)) + (uint32_t)((split * BN) * RP + (r % RP)) * 4u;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 16) {
+      for (int c0 = 0; c0 < BN && c0 < a.m; c0 += 16) {
         float v[16];
         tmem_ld16(tmem_d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) cluster_store(dst + (uint32_t)((c0 + j) * RP) * 4u, v[j]);
+        for (int j = 0; j < 16; ++j) part[(c0 + j) * TILE_M + r] = v[j];
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  cluster_barrier();  // every partial sum has arrived; no peer touches this block's memory after it
-  pdl_wait();         // nothing may be overwritten before the previous kernel has ended
-  if (warp >= 2 && !*failed) {
-    constexpr int RP = TILE_M / SPLITS;
-    const int t = threadIdx.x - 64;
-    for (int i = t; i < RP * BN; i += 128) {
-      const int j = i / RP, rl = i % RP, feat = n0 + split * RP + rl;
-      if (j < a.m && feat < a.n) {
-        float s = 0.f;
-#pragma unroll
-        for (int sp = 0; sp < SPLITS; ++sp) s += recv[(size_t)(sp * BN + j) * RP + rl];  // in split order
-        const bool split = a.act_from > 0 && feat >= a.act_from;
-        if (out_kind == OUT_BF16_ACT || split) {
-          float z = 0.f;
-          activate_pair(a.act, s, z);
+  if (splits > 1) {  // every partial sum of the tile is in place
+    cluster_arrive();
+    cluster_wait();
+  }
+  pdl_wait();  // nothing may be overwritten before the previous kernel has ended
+  if (!*failed) {
+    const uint32_t part_addr = smem_u32(part);
+    const bool vec = a.ldo % 4 == 0 && a.out_head % 4 == 0 &&  // four results in one store
+                     ((out_kind == OUT_F32 ? reinterpret_cast<uintptr_t>(a.out) : reinterpret_cast<uintptr_t>(a.out_h)) & 15) == 0;
+    const int pieces = a.m * (TILE_M / 4), first = pieces * split / splits, last = pieces * (split + 1) / splits;
+    for (int i = first + (int)threadIdx.x; i < last; i += 192) {
+      const int j = i / (TILE_M / 4), f0 = n0 + (i % (TILE_M / 4)) * 4;
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (splits == 1) {
+        sum = reinterpret_cast<const float4*>(part)[i];
+      } else {
+        for (int q = 0; q < splits; ++q) {
+          const float4 v = cluster_load4(part_addr + (uint32_t)i * 16u, (uint32_t)q);
+          sum.x += v.x;
+          sum.y += v.y;
+          sum.z += v.z;
+          sum.w += v.w;
         }
-        const size_t at = (size_t)j * a.ldo + (size_t)head * a.out_head + feat;
-        if (split) static_cast<__nv_bfloat16*>(a.out_act)[(size_t)j * a.ldo_act + feat - a.act_from] = __float2bfloat16_rn(s);
-        else if (out_kind == OUT_F32) a.out[at] = s;
-        else static_cast<__nv_bfloat16*>(a.out_h)[at] = __float2bfloat16_rn(s);
+      }
+      const size_t at = (size_t)j * a.ldo + (size_t)head * a.out_head + f0;
+      if (vec && f0 + 3 < a.n && (a.act_from <= 0 || f0 + 3 < a.act_from)) {
+        if (out_kind == OUT_BF16_ACT) {
+          activate_pair(a.act, sum.x, sum.y);
+          activate_pair(a.act, sum.z, sum.w);
+        }
+        if (out_kind == OUT_F32) store4(a.out + at, sum);
+        else store4(static_cast<__nv_bfloat16*>(a.out_h) + at, sum);
+        continue;
+      }
+      float y[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int feat = f0 + e;
+        if (feat >= a.n) break;
+        float v = y[e];
+        const bool act_part = a.act_from > 0 && feat >= a.act_from;
+        if (out_kind == OUT_BF16_ACT || act_part) {
+          float z = 0.f;
+          activate_pair(a.act, v, z);
+        }
+        if (act_part) static_cast<__nv_bfloat16*>(a.out_act)[(size_t)j * a.ldo_act + feat - a.act_from] = __float2bfloat16_rn(v);
+        else if (out_kind == OUT_F32) a.out[at + e] = v;
+        else static_cast<__nv_bfloat16*>(a.out_h)[at + e] = __float2bfloat16_rn(v);
       }
     }
+  }
+  if (splits > 1) {  // no block's memory goes away while another reads it
+    cluster_arrive();
+    cluster_wait();
   }
   tc_fence_before();
   __syncthreads();
@@ -435,46 +468,36 @@ cudaError_t launch_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
   return launch_kernel(tc_gemm_bf16_kernel<BN>, dim3(std::min(tiles, sm_count())), dim3(192), smem, s, pdl, mx, mw, mo, a, kind, tma_out);
 }
 
-template <int BN, int SPLITS>
-cudaError_t launch_rows(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
+template <int BN>
+cudaError_t launch_rows_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
+  // As many parts of k as give every SM a block, each of at least two k blocks, at most a portable cluster's eight. A decode step
+  // of 64 sequences of width 2048 (in products of 49, 16, 64 and 16 row tiles) with 4 / 6 / 8 parts at most, ms of 24 steps and
+  // prompts: Dirurax 27.8 / 27.3 / 27.0, Sanesun 25.3 / 24.7 / 24.5. Powers of two up to four, blocks of 176 KB, peers' sums
+  // pushed into a buffer of their own: 28.3 and 26.1. Alone, 16.8 MB (n 2048, k 4096) take 10.8 us, 33.6 MB 15.
+  const int row_tiles = (a.n + TILE_M - 1) / TILE_M, heads = std::max(a.heads, 1), nkb = (a.k + KB - 1) / KB;
+  const int splits = std::max(1, std::min({8, sm_count() / (row_tiles * heads), nkb / 2}));
   CUtensorMap mx, mw;
-  const uint64_t heads = std::max(a.heads, 1), tiles = heads * ((a.n + TILE_M - 1) / TILE_M) * (a.k / KB);
-  if (!make_map_bf16(&mx, a.x, a.m, a.heads ? a.ldx : a.k, BN) || !make_map_bf16(&mw, a.w_tiled, tiles * TILE_M, KB, TILE_M)) return cudaErrorInvalidValue;
-  auto kernel = tc_gemm_bf16_rows_kernel<BN, SPLITS>;
-  const size_t smem = RowsSmem<BN, SPLITS>::BYTES;
+  if (!make_map_bf16(&mx, a.x, a.m, a.heads ? a.ldx : a.k, BN) || !make_map_bf16(&mw, a.w_tiled, (uint64_t)heads * row_tiles * (a.k / KB) * TILE_M, KB, TILE_M))
+    return cudaErrorInvalidValue;
+  auto kernel = tc_gemm_bf16_rows_kernel<BN>;
+  const size_t smem = RowsSmem<BN>::BYTES;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((a.n + TILE_M - 1) / TILE_M, SPLITS, (unsigned)heads);
+  cfg.gridDim = dim3(row_tiles, splits, heads);
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = SPLITS;
+  attr[0].val.clusterDim.y = splits;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, mx, mw, a, out_kind_of(a));
-}
-
-template <int BN>
-cudaError_t launch_rows_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
-  // As many parts of k as fill the chip once, each at least two k blocks; clusters of eight only where a few of them are
-  // needed: sixteen do not run at the same time (measured, 2048 output columns: 19 us in eight parts, 12 us in four).
-  const int tiles = (a.n + TILE_M - 1) / TILE_M * std::max(a.heads, 1), nkb = (a.k + KB - 1) / KB;
-  const int max_splits = tiles <= 8 ? 8 : 4;
-  int splits = 1;
-  while (splits < max_splits && tiles * splits * 2 <= sm_count() && splits * 4 <= nkb) splits *= 2;
-  switch (splits) {
-    case 1: return launch_rows<BN, 1>(a, pdl, s);
-    case 2: return launch_rows<BN, 2>(a, pdl, s);
-    case 4: return launch_rows<BN, 4>(a, pdl, s);
-    default: return launch_rows<BN, 8>(a, pdl, s);
-  }
 }
 
 }  // namespace
