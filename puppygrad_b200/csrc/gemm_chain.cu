@@ -6,23 +6,24 @@
 // times the streaming time of its weights. Here one CTA per SM stays resident for a whole list of
 // phases (GEMM, ROWS, ELEM, ATTN, EMBED, FINAL; see kernels.cuh), separated by grid barriers:
 //
-//   warp 0      weight producer: TMA loads of 32 KB weight units (two 128 x 32 blocks of the tiled
-//               weight copy) into a ring of shared-memory stages. Weights do not depend on
-//               activations, so this warp never waits for a phase to begin: while the other warps
+//   warp 0      weight producer: TMA loads of weight units (one 128 x 64 block of FP16 pairs, 32 KB, or 16 KB of
+//               hi parts where the weights are BF16; gemm_pair.cu) into a ring of shared-memory stages. Weights do not
+//               depend on activations, so this warp never waits for a phase to begin: while the other warps
 //               reduce, normalise, attend or wait at the grid barrier it already fetches the next
 //               GEMM's units.
-//   warps 4-7   splitters: FP32 weight tile -> TF32 hi/lo pair in tensor memory (tcgen05.st); they
-//               run ahead as far as tensor memory stages are free.
 //   warp 2      activation producer: after the phase's inputs exist (grid barrier), TMA loads of
-//               the 64-token x 32 hi and lo tiles.
-//   warps 1, 3  MMA issuers, one per k block of a unit, a 64-column accumulator in tensor memory each:
-//               per 8-wide k slice three tcgen05.mma of N = 64 into it (w_hi . x_hi, w_lo . x_hi,
-//               w_hi . x_lo). One accumulator for the three products leaves tensor memory for three
-//               stages of split weights (two stages and separate columns for w_hi . x_lo measured
-//               1% slower: a stage comes back only when its MMAs have completed).
-//   warps 8-15  workers: drain the accumulators into per-CTA partial tiles (global memory, L2
+//               the 64-value hi and lo tiles of 16, 32 or 64 tokens (the smallest that holds the batch).
+//   warps 1, 3  MMA issuers, two of a unit's four 16-value k slices each, into accumulators of their own: per
+//               slice one MMA of the hi weights with the hi and lo tokens side by side (the hi.hi sums and the
+//               hi.lo sums next to each other in tensor memory) and one of the lo weights with the hi tokens.
+//   warps 4-11  workers: drain the accumulators into per-CTA partial tiles (global memory, L2
 //               resident), take part in the grid barrier, run the reduce phases, the attention
 //               phases (one warp per sequence-head pair), the embedding and the end-of-step phase.
+//
+// Weights arrive as pairs, so nothing splits them on the way (FP32 tiles, split by four warps into three TF32 products, took 24
+// MMAs per 64 values of k; this takes 12, or 4 with BF16 weights) and BF16 weights are half the bytes. A step of GPT-2 medium
+// with 64 sequences 1.39 -> 1.25 ms, of XL with 32 at 512 positions 5.67 -> 5.1 ms; what bounds it is the chain of phases: a grid
+// barrier each, L2 round trips behind it, and the keys and values of the attention phases.
 //
 // Every GEMM's units (row tile major, k minor) are cut into equal contiguous shares, one per CTA,
 // so all SMs stream the same number of bytes whatever the matrix shape. Partials are added in k
@@ -31,40 +32,34 @@
 // Every wait is bounded. On expiry the CTA raises the error word; every role then falls through
 // its remaining loops without touching memory, tensor memory is freed and the kernel ends.
 #include "kernels.cuh"
+#include "pair.cuh"
 #include "tc_common.cuh"
 
 namespace pg {
 namespace {
 
-constexpr int CH_THREADS = 512;
-// The pipelines move units of CH_UB consecutive k blocks (128 weight rows x 32 floats each): a wait
-// on an mbarrier or a tcgen05.commit costs the single MMA-issuing thread as much as several MMAs,
-// so fewer, larger hand-overs keep the tensor pipe busier.
-constexpr int CH_UB = 2;
-constexpr int CH_W_STAGES = 3;    // weight units in flight per SM (32 KB each)
-constexpr int CH_X_STAGES = 3;    // units whose activation tiles (shared memory) and split weights (tensor memory) are staged
+constexpr int CH_THREADS = 384;
+constexpr int CH_K = 64;                        // values of k per unit: one 128-byte swizzle row of FP16
+constexpr int CH_BLOCK = TILE_M * CH_K * 2;     // bytes of a unit's hi (or lo) weights
+constexpr int CH_W_RING = 6 * CH_BLOCK;         // three units of pairs or six of hi parts in flight per SM
+constexpr int CH_X_STAGES = 8;                  // units whose activation tiles are staged, and barriers of the ring
 constexpr int CH_BN = 64;
-constexpr int CH_W_BYTES = CH_UB * TILE_M * BK * 4;
-constexpr int CH_ACT_BYTES = CH_UB * 2 * CH_BN * BK * 4;  // per block: x_hi tile then x_lo tile
+constexpr int CH_ACT_BYTES = 2 * CH_BN * CH_K * 2;  // x_hi tile, then x_lo tile
 constexpr int CH_MAX_SEG = 4;     // row tiles one CTA's share may touch
 constexpr int CH_WORKERS = 256;
-// tensor memory: two accumulators of CH_BN columns, then CH_X_STAGES stages of w_hi | w_lo for the unit's two k blocks
-constexpr uint32_t CH_D_COLS = 64, CH_A_COL0 = 128, CH_TMEM_COLS = 512;
-static_assert(CH_D_COLS == CH_BN && CH_A_COL0 == 2 * CH_D_COLS && CH_A_COL0 + CH_X_STAGES * 64 * CH_UB <= CH_TMEM_COLS, "tensor memory columns");
-// Attention phases stage key / value rows in the (then idle) activation ring plus an extra region:
+constexpr uint32_t CH_D_COLS = 128, CH_TMEM_COLS = 256;  // an issuer's accumulators: hi.hi sums of the tokens, then their small terms
+static_assert(CH_D_COLS == 2 * CH_BN && 2 * CH_D_COLS <= CH_TMEM_COLS, "tensor memory columns");
+// Attention phases stage key / value rows in the (then idle) activation ring:
 // each of the eight worker warps has AT_SLOTS slots, each holding AT_ROWS key rows and the AT_ROWS
 // value rows of the same positions (one mbarrier per slot: one wait per block of keys).
 constexpr int AT_ROWS = 16;
 constexpr int AT_SLOTS = 2;
 constexpr int AT_SLOT_BYTES = 2 * AT_ROWS * 64 * 4;
-constexpr int AT_EXTRA_BYTES = 8 * AT_SLOTS * AT_SLOT_BYTES - CH_X_STAGES * CH_ACT_BYTES;
 constexpr int AT_SCRATCH_FLOATS = 4 * 64;  // per group of four warps: one 64-float query per warp
-static_assert(AT_EXTRA_BYTES >= 0, "the activation ring is part of the attention staging area");
+static_assert(8 * AT_SLOTS * AT_SLOT_BYTES <= CH_X_STAGES * CH_ACT_BYTES, "attention stages in the activation ring");
 // 227 KB, the most a CTA can have: the dynamic shared memory must start 1024-byte aligned (checked at run time)
-constexpr size_t CH_SMEM = (size_t)CH_W_STAGES * CH_W_BYTES + (size_t)CH_X_STAGES * CH_ACT_BYTES + AT_EXTRA_BYTES +
-                           2 * AT_SCRATCH_FLOATS * 4 + 1024;
+constexpr size_t CH_SMEM = (size_t)CH_W_RING + (size_t)CH_X_STAGES * CH_ACT_BYTES + 2 * AT_SCRATCH_FLOATS * 4 + 1024;
 static_assert(CH_SMEM <= 232448, "shared memory of one CTA");
-static_assert(CH_UB == 2, "one MMA issuer per k block of a unit");
 static_assert(sizeof(ChainPhase) % 8 == 0 && 384 + 2 * sizeof(ChainPhase) <= 1024, "two phase descriptors behind the barriers");
 constexpr size_t CH_PART_TILE = (size_t)CH_BN * TILE_M;  // floats of one partial tile: [token][row]
 
@@ -73,7 +68,7 @@ struct ChRange {
   int g0, g1, nkb, per;
 };
 __device__ __host__ inline ChRange chain_range(int n, int k, int cta, int grid, bool whole_tiles = false) {
-  const int tiles = (n + TILE_M - 1) / TILE_M, nkb = k / (BK * CH_UB);  // units per row tile
+  const int tiles = (n + TILE_M - 1) / TILE_M, nkb = k / CH_K;  // units per row tile
   const int total = tiles * nkb;
   int per = (total + grid - 1) / grid;
   // one block more per CTA when that makes shares line up with row tiles: fewer partial tiles to
@@ -169,18 +164,6 @@ __device__ __forceinline__ void chain_trace(const ChainArgs& a, int slot) {
   }
 }
 
-// Developer aid, compiled in only with -DPG_DEV_TRACE (and then active only when the trace buffer exists): clock64()
-// stamps of the first 48 weight units of CTA 0 in the whole-tile GEMM (the lm_head), eight events per unit, behind the
-// per-CTA slots of the buffer: 0 weight copy issued, 1 splitters saw the weights, 2 ... the free tensor-memory stage,
-// 3 split weights stored, 4 activation copy issued, 5 issuer saw the unit ready, 6 its MMAs committed, 7 issuer began
-// to wait. Slots 20-22 of every CTA: globaltimer at the start and at the end of its lm_head work, and its SM.
-#ifdef PG_DEV_TRACE
-__device__ __forceinline__ void unit_trace(const ChainArgs& a, bool on, int u, int e) {
-  if (on && a.trace && u < 48) a.trace[(size_t)gridDim.x * 32 + (size_t)u * 8 + e] = (unsigned long long)clock64();
-}
-#else
-__device__ __forceinline__ void unit_trace(const ChainArgs&, bool, int, int) {}
-#endif
 __device__ __forceinline__ const ChainPhase& phase_at(const ChainArgs& a, int p) {
   return a.phases_dev ? a.phases_dev[p] : a.ph[p];
 }
@@ -278,7 +261,7 @@ __device__ __forceinline__ float warp_sum_f(float v) {
 }
 
 // ROWS phase: x[j, :] += bias + sum of partials, then optional LayerNorm of the updated row written
-// as a TF32 hi/lo pair. One CTA per token; wt = worker thread 0..255; n % 4 == 0, n <= 4096.
+// as FP16 pairs. One CTA per token; wt = worker thread 0..255; n % 4 == 0, n <= 4096.
 __device__ __forceinline__ void chain_rows_phase(const ChainArgs& a, const ChainPhase& ph, int j, int wt, float* red, bool embed) {
   const int n = ph.n, n4 = n >> 2;
   const ChRange r = chain_range_ph(ph, 0);
@@ -331,24 +314,17 @@ __device__ __forceinline__ void chain_rows_phase(const ChainArgs& a, const Chain
   workers_sync();
   const float var = (((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]))) / (float)n;
   const float inv_std = 1.0f / sqrtf(var + a.eps);
-  float4* hi4 = reinterpret_cast<float4*>(ph.out_hi + (size_t)j * n);
-  float4* lo4 = reinterpret_cast<float4*>(ph.out_lo + (size_t)j * n);
+  uint16_t *hi = ph.out_hi + (size_t)j * n, *lo = ph.out_lo + (size_t)j * n;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int u = wt + i * CH_WORKERS;
     if (u < n4) {
       const float4 g = __ldg(reinterpret_cast<const float4*>(ph.ln_g) + u);
       const float4 b = __ldg(reinterpret_cast<const float4*>(ph.ln_b) + u);
-      const float y[4] = {(v[i].x - mean) * inv_std * g.x + b.x, (v[i].y - mean) * inv_std * g.y + b.y,
-                          (v[i].z - mean) * inv_std * g.z + b.z, (v[i].w - mean) * inv_std * g.w + b.w};
-      float h[4], l[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        h[e] = tf32_hi(y[e]);
-        l[e] = y[e] - h[e];
-      }
-      hi4[u] = make_float4(h[0], h[1], h[2], h[3]);
-      lo4[u] = make_float4(l[0], l[1], l[2], l[3]);
+      store_pair4(hi + 4 * u, lo + 4 * u,
+                  make_float4((v[i].x - mean) * inv_std * g.x + b.x, (v[i].y - mean) * inv_std * g.y + b.y,
+                              (v[i].z - mean) * inv_std * g.z + b.z, (v[i].w - mean) * inv_std * g.w + b.w),
+                  ph.out_scale);
     }
   }
   workers_sync();  // `red` is reused by the next phase
@@ -419,26 +395,12 @@ __device__ __forceinline__ void chain_elem_phase(const ChainArgs& a, const Chain
     const size_t o = (size_t)j * n + f;
     if (vec) {
       if (ph.out) *reinterpret_cast<float4*>(ph.out + o) = make_float4(y[0], y[1], y[2], y[3]);
-      if (ph.out_hi) {
-        float h[4], l[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          h[e] = tf32_hi(y[e]);
-          l[e] = y[e] - h[e];
-        }
-        *reinterpret_cast<float4*>(ph.out_hi + o) = make_float4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<float4*>(ph.out_lo + o) = make_float4(l[0], l[1], l[2], l[3]);
-      }
+      if (ph.out_hi) store_pair4(ph.out_hi + o, ph.out_lo + o, make_float4(y[0], y[1], y[2], y[3]), ph.out_scale);
     } else {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         if (f + e < n) {
           if (ph.out) ph.out[o + e] = y[e];
-          if (ph.out_hi) {
-            const float h = tf32_hi(y[e]);
-            ph.out_hi[o + e] = h;
-            ph.out_lo[o + e] = y[e] - h;
-          }
         }
       }
     }
@@ -766,17 +728,10 @@ __device__ __forceinline__ void chain_attn_phase(const ChainArgs& a, const Chain
     }
     if (lane < 16 && ok && part == 0) {
       const float inv = 1.0f / ls;
-      const float y[4] = {fmaf(pn, vn.x, acc.x) * inv, fmaf(pn, vn.y, acc.y) * inv, fmaf(pn, vn.z, acc.z) * inv,
-                          fmaf(pn, vn.w, acc.w) * inv};
-      float hi[4], lo[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        hi[e] = tf32_hi(y[e]);
-        lo[e] = y[e] - hi[e];
-      }
       const size_t idx = (size_t)b * C + h * D + lane * 4;
-      *reinterpret_cast<float4*>(ph.out_hi + idx) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<float4*>(ph.out_lo + idx) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      store_pair4(ph.out_hi + idx, ph.out_lo + idx,
+                  make_float4(fmaf(pn, vn.x, acc.x) * inv, fmaf(pn, vn.y, acc.y) * inv, fmaf(pn, vn.z, acc.z) * inv, fmaf(pn, vn.w, acc.w) * inv),
+                  ph.out_scale);
     }
     if (lane < 16 && part == 0) {  // append the new K and V rows
       const int off = t & (pt - 1);
@@ -791,7 +746,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
     chain_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi0,
                  const __grid_constant__ CUtensorMap map_lo0, const __grid_constant__ CUtensorMap map_hi1,
                  const __grid_constant__ CUtensorMap map_lo1, const __grid_constant__ CUtensorMap map_hi2,
-                 const __grid_constant__ CUtensorMap map_lo2, const __grid_constant__ ChainArgs a) {
+                 const __grid_constant__ CUtensorMap map_lo2, const __grid_constant__ ChainArgs a, int bn) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* base = smem_raw;
   if ((smem_u32(base) & 1023u) != 0) {  // swizzled TMA tiles need it; every thread takes the same way out
@@ -799,16 +754,14 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
     return;
   }
   uint8_t* w_ring = base;
-  uint8_t* act_ring = base + (size_t)CH_W_STAGES * CH_W_BYTES;
-  // attention staging = the activation ring and the region after it; then the attention scratch
-  float* at_scratch = reinterpret_cast<float*>(act_ring + (size_t)CH_X_STAGES * CH_ACT_BYTES + AT_EXTRA_BYTES);
-  uint64_t* w_full = reinterpret_cast<uint64_t*>(at_scratch + 2 * AT_SCRATCH_FLOATS);
-  uint64_t* w_empty = w_full + CH_W_STAGES;
-  uint64_t* ready = w_empty + CH_W_STAGES;  // split weights in tensor memory AND activation tiles in shared memory
-  uint64_t* done = ready + CH_X_STAGES;     // the MMAs that read them have completed
+  uint8_t* act_ring = base + CH_W_RING;
+  // attention staging = the activation ring; then the attention scratch
+  float* at_scratch = reinterpret_cast<float*>(act_ring + (size_t)CH_X_STAGES * CH_ACT_BYTES);
+  uint64_t* ready = reinterpret_cast<uint64_t*>(at_scratch + 2 * AT_SCRATCH_FLOATS);  // a unit's weights and activation tiles are there
+  uint64_t* done = ready + CH_X_STAGES;  // the MMAs that read them have completed
   uint64_t* d_full = done + CH_X_STAGES;
-  uint64_t* d_empty = d_full + 2;
-  uint64_t* go = d_empty + 2;
+  uint64_t* d_empty = d_full + 1;
+  uint64_t* go = d_empty + 1;
   uint64_t* kv_full = go + 1;  // [8 worker warps][AT_SLOTS]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(kv_full + 8 * AT_SLOTS);
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -816,24 +769,18 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
   float* red = reinterpret_cast<float*>(tmem_slot + 4);  // 8 floats
   // the descriptor of the current and of the next phase, copied here ahead of the barrier before the phase: what a
   // phase needs first is then a shared-memory read away instead of a chain of L2 reads
-  ChainPhase* ph_s = reinterpret_cast<ChainPhase*>(reinterpret_cast<uint8_t*>(w_full) + 384);
+  ChainPhase* ph_s = reinterpret_cast<ChainPhase*>(reinterpret_cast<uint8_t*>(ready) + 384);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cta = (int)blockIdx.x, grid = (int)gridDim.x;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < CH_W_STAGES; ++s) {
-      mbar_init(&w_full[s], 1);
-      mbar_init(&w_empty[s], 4);
-    }
     for (int s = 0; s < CH_X_STAGES; ++s) {
-      mbar_init(&ready[s], 5);  // four splitter warps + the activation producer's expect_tx arrival
-      mbar_init(&done[s], 2);  // both MMA issuers commit
+      mbar_init(&ready[s], 2);  // both producers' expect_tx arrivals
+      mbar_init(&done[s], 2);   // both MMA issuers commit
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&d_full[s], 2);  // both MMA issuers commit ([0] is used; accumulators are not double-buffered)
-      mbar_init(&d_empty[s], 8);
-    }
+    mbar_init(d_full, 2);  // both MMA issuers commit
+    mbar_init(d_empty, 8);
     mbar_init(go, 1);
     for (int s = 0; s < 8 * AT_SLOTS; ++s) mbar_init(&kv_full[s], 1);
     *failed = 0;
@@ -845,12 +792,11 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // Registers follow the work: the producer / issuer warps (one busy lane each) and the splitters
-  // give registers back, the worker warps, whose reduce and attention code wants many loads in
-  // flight, take them (per warp group of four warps; 128 * (40 + 128) + 256 * 168 = 64 K).
-
-  if (warp < 4) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+  const int block_bytes = a.exact ? CH_BLOCK : 2 * CH_BLOCK, w_stages = CH_W_RING / block_bytes;
+  const int act_bytes = 2 * bn * CH_K * 2;  // of a unit; its x_lo tile lies right behind the x_hi tile
+  // Units are numbered through all phases. Unit u waits at ready[u % 8] and done[u % 8]; its weights lie in stage u % w_stages of
+  // their ring, which the weight producer may refill once unit u - w_stages is done: w_stages <= 8, so that the barrier it looks at
+  // cannot be a round further.
   if (warp == 0) {
     // ---------------------------------------------------------------- weight producer
     if (lane == 0) {
@@ -858,37 +804,39 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
       uint64_t evict_first;
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(evict_first));
       const bool hint = (a.tune_fence & 8) == 0;
-      uint32_t wi = 0;
+      const int block_rows = block_bytes / (CH_K * 2);
+      uint32_t u = 0, ws = 0;
       bool ok = true;
       for (int p = 0; p < a.n_phases && ok; ++p) {
         if (phase_at(a, p).kind != CH_GEMM) continue;
         const ChRange r = chain_range_ph(phase_at(a, p), cta);
         const uint32_t b0 = phase_at(a, p).w_block0;
-        const bool tr = cta == 0 && phase_at(a, p).whole_tiles;
-        for (int g = r.g0; g < r.g1 && ok; ++g, ++wi) {
-          const uint32_t s = wi % CH_W_STAGES;
-          if (wi >= CH_W_STAGES) ok = mbar_wait(&w_empty[s], ((wi / CH_W_STAGES) - 1) & 1, failed, a.error_flag, 21);
+        for (int g = r.g0; g < r.g1 && ok; ++g, ++u) {
+          if (u >= (uint32_t)w_stages) {
+            const uint32_t old = u - w_stages;
+            ok = mbar_wait(&done[old % CH_X_STAGES], (old / CH_X_STAGES) & 1, failed, a.error_flag, 21);
+          }
           if (!ok) break;
-          unit_trace(a, tr, g - r.g0, 0);
-          // one unit = CH_UB consecutive 16 KB blocks of the tiled arena = one box of CH_UB * 128 rows
-          mbar_expect_tx(&w_full[s], CH_W_BYTES);
-          if (hint)
-            tma_load_2d_hint(w_ring + (size_t)s * CH_W_BYTES, &map_w, 0, (int)((b0 + (uint32_t)g * CH_UB) * TILE_M), &w_full[s], evict_first);
-          else
-            tma_load_2d(w_ring + (size_t)s * CH_W_BYTES, &map_w, 0, (int)((b0 + (uint32_t)g * CH_UB) * TILE_M), &w_full[s]);
+          uint64_t* bar = &ready[u % CH_X_STAGES];
+          uint8_t* dst = w_ring + (size_t)ws * block_bytes;
+          const int y = (int)(b0 + (uint32_t)g) * block_rows;
+          mbar_expect_tx(bar, block_bytes);
+          if (hint) tma_load_2d_hint(dst, &map_w, 0, y, bar, evict_first);
+          else tma_load_2d(dst, &map_w, 0, y, bar);
+          if (++ws == (uint32_t)w_stages) ws = 0;
         }
       }
     }
   } else if (warp == 1 || warp == 3) {
     // ---------------------------------------------------------------- MMA issuers
-    // Issuing one tcgen05.mma costs its thread ~60 clocks whatever the tile, so two threads share the
-    // work: the issuer of warp 1 takes k block 0 of every unit, the one of warp 3 k block 1, each
-    // into an accumulator of its own; the drain adds the two.
+    // Issuing one tcgen05.mma costs its thread ~60 clocks whatever the tile, so two threads share the work; the drain adds
+    // their accumulators.
     if (lane == 0) {
       const int b = warp == 1 ? 0 : 1;
-      const uint32_t idesc1 = umma_idesc_tf32(TILE_M, CH_BN);
+      const uint32_t idesc_both = umma_idesc_f16(TILE_M, 2 * bn), idesc = umma_idesc_f16(TILE_M, bn);
       const uint32_t dcol = tmem_base + (uint32_t)b * CH_D_COLS;
-      uint32_t wi = 0, si = 0;
+      const bool exact = a.exact != 0;
+      uint32_t u = 0, ws = 0, si = 0;
       bool ok = true;
       for (int p = 0; p < a.n_phases && ok; ++p) {
         if (phase_at(a, p).kind != CH_GEMM) continue;
@@ -899,26 +847,20 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
           if (si >= 1) ok = mbar_wait(d_empty, (si - 1) & 1, failed, a.error_flag, 22);  // the previous row tile is drained
           if (!ok) break;
           tc_fence_after();
-          for (int gb = g; gb < gend && ok; ++gb, ++wi) {
-            const uint32_t xs = wi % CH_X_STAGES;
-            const bool tr = cta == 0 && b == 0 && phase_at(a, p).whole_tiles;
-            unit_trace(a, tr, gb - r.g0, 7);
-            ok = mbar_wait(&ready[xs], (wi / CH_X_STAGES) & 1, failed, a.error_flag, 23);
+          for (int gb = g; gb < gend && ok; ++gb, ++u) {
+            const uint32_t xs = u % CH_X_STAGES;
+            ok = mbar_wait(&ready[xs], (u / CH_X_STAGES) & 1, failed, a.error_flag, 23);
             if (!ok) break;
-            unit_trace(a, tr, gb - r.g0, 5);
             tc_fence_after();
-            // block b of the unit: x_hi rows then x_lo rows in shared memory, w_hi | w_lo columns in tensor memory
-            const uint64_t dx = umma_desc_sw128(act_ring + (size_t)xs * CH_ACT_BYTES + (size_t)b * (CH_ACT_BYTES / CH_UB));
-            const uint64_t dxl = umma_desc_sw128(act_ring + (size_t)xs * CH_ACT_BYTES + (size_t)b * (CH_ACT_BYTES / CH_UB) + CH_BN * BK * 4);
-            const uint32_t ahi = tmem_base + CH_A_COL0 + xs * (64 * CH_UB) + b * 64, alo = ahi + 32;
+            const uint64_t dx = umma_desc_sw128(act_ring + (size_t)xs * CH_ACT_BYTES) + b * 4;
+            const uint64_t dw = umma_desc_sw128(w_ring + (size_t)ws * block_bytes) + b * 4;
 #pragma unroll
-            for (int k = 0; k < BK / 8; ++k) {
-              umma_tf32_ts(dcol, ahi + k * 8, dx + (uint64_t)(k * 2), idesc1, (gb != g || k != 0) ? 1u : 0u);
-              umma_tf32_ts(dcol, alo + k * 8, dx + (uint64_t)(k * 2), idesc1, 1u);
-              umma_tf32_ts(dcol, ahi + k * 8, dxl + (uint64_t)(k * 2), idesc1, 1u);
+            for (int k = 0; k < 2; ++k) {  // slices 2 b and 2 b + 1: 32 bytes of a row each
+              umma_bf16_ss(dcol, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), idesc_both, (gb != g || k != 0) ? 1u : 0u);
+              if (!exact) umma_bf16_ss(dcol + bn, dw + (uint64_t)(CH_BLOCK / 16 + k * 2), dx + (uint64_t)(k * 2), idesc, 1u);
             }
             umma_commit(&done[xs]);
-            unit_trace(a, tr, gb - r.g0, 6);
+            if (++ws == (uint32_t)w_stages) ws = 0;
           }
           if (ok) umma_commit(d_full);
           ++si;
@@ -931,7 +873,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_hi0) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&map_lo0) : "memory");
-      uint32_t wi = 0, gp = 0;
+      uint32_t u = 0, gp = 0;
       bool ok = true;
       for (int p = 0; p < a.n_phases && ok; ++p) {
         if (phase_at(a, p).kind != CH_GEMM) continue;
@@ -943,77 +885,21 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
         ++gp;
         if (!ok) break;
         asm volatile("fence.proxy.async;" ::: "memory");
-        for (int g = r.g0; g < r.g1 && ok; ++g, ++wi) {
-          const uint32_t s = wi % CH_X_STAGES;
-          if (wi >= CH_X_STAGES) ok = mbar_wait(&done[s], ((wi / CH_X_STAGES) - 1) & 1, failed, a.error_flag, 26);
+        for (int g = r.g0; g < r.g1 && ok; ++g, ++u) {
+          const uint32_t s = u % CH_X_STAGES;
+          if (u >= CH_X_STAGES) ok = mbar_wait(&done[s], ((u / CH_X_STAGES) - 1) & 1, failed, a.error_flag, 26);
           if (!ok) break;
-          unit_trace(a, cta == 0 && phase_at(a, p).whole_tiles, g - r.g0, 4);
-          const int kb = (g % r.nkb) * CH_UB;
+          const int k0 = (g % r.nkb) * CH_K;
           uint8_t* dst = act_ring + (size_t)s * CH_ACT_BYTES;
-          mbar_expect_tx(&ready[s], CH_ACT_BYTES);
-#pragma unroll
-          for (int b = 0; b < CH_UB; ++b) {
-            tma_load_2d(dst + (size_t)b * (CH_ACT_BYTES / CH_UB), mh, (kb + b) * BK, 0, &ready[s]);
-            tma_load_2d(dst + (size_t)b * (CH_ACT_BYTES / CH_UB) + CH_BN * BK * 4, ml, (kb + b) * BK, 0, &ready[s]);
-          }
+          mbar_expect_tx(&ready[s], act_bytes);
+          tma_load_2d(dst, mh, k0, 0, &ready[s]);
+          tma_load_2d(dst + act_bytes / 2, ml, k0, 0, &ready[s]);
         }
-      }
-    }
-  }
-  } else if (warp < 8) {
-    // ---------------------------------------------------------------- splitters
-    const int q = warp & 3;
-    const int row = q * 32 + lane;  // row of the weight tile == tensor-memory lane
-    const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-    uint32_t wi = 0;
-    bool ok = true;
-    for (int p = 0; p < a.n_phases && ok; ++p) {
-      if (phase_at(a, p).kind != CH_GEMM) continue;
-      const ChRange r = chain_range_ph(phase_at(a, p), cta);
-      for (int g = r.g0; g < r.g1 && ok; ++g, ++wi) {
-        const uint32_t s = wi % CH_W_STAGES, xs = wi % CH_X_STAGES;
-        const bool tr = cta == 0 && warp == 4 && lane == 0 && phase_at(a, p).whole_tiles;
-        ok = warp_wait(&w_full[s], (wi / CH_W_STAGES) & 1, failed, a.error_flag, 27);
-        if (!ok) break;
-        unit_trace(a, tr, g - r.g0, 1);
-        // the tensor-memory stage is free once the MMAs of the unit that used it last have completed
-        if (wi >= CH_X_STAGES) ok = warp_wait(&done[xs], ((wi / CH_X_STAGES) - 1) & 1, failed, a.error_flag, 28);
-        if (!ok) break;
-        unit_trace(a, tr, g - r.g0, 2);
-        tc_fence_after();
-#pragma unroll
-        for (int b = 0; b < CH_UB; ++b) {
-          const float4* rowp = reinterpret_cast<const float4*>(w_ring + (size_t)s * CH_W_BYTES + (size_t)b * (TILE_M * BK * 4) +
-                                                               (size_t)row * 128);
-          uint32_t hi[32], lo[32];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 v = rowp[j ^ (row & 7)];  // undo the 128-byte swizzle: conflict-free per quarter warp
-            const float f[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float h = tf32_hi(f[e]);
-              hi[j * 4 + e] = __float_as_uint(h);
-              lo[j * 4 + e] = __float_as_uint(f[e] - h);
-            }
-          }
-          const uint32_t col = tmem_base + CH_A_COL0 + xs * (64 * CH_UB) + b * 64 + lane_addr;
-          tmem_st32(col, hi);
-          tmem_st32(col + 32, lo);
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&w_empty[s]);  // the unit is in registers / tensor memory: the stage may be refilled
-        tmem_wait_st();
-        unit_trace(a, tr, g - r.g0, 3);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ready[xs]);
       }
     }
   } else {
     // ---------------------------------------------------------------- workers
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
-    const int wt = (int)threadIdx.x - 256;
+    const int wt = (int)threadIdx.x - 128;
     const int ww = wt >> 5;
     const int q = ww & 3, half = ww >> 2;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
@@ -1032,15 +918,21 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
     bool at_prepared = false;
     at_cur.item = at_cur.blk = at_cur.nblk = at_cur.t = at_cur.b = at_cur.h = at_cur.pg0 = at_cur.pg1 = 0;
     at_cur.issued = 0;
-    // Sums of token columns [c0, c0 + 16) of this thread's row: two accumulators (k block 0 and 1 of every unit);
-    // the two loads are in flight together
-    auto ld_acc = [&](int c0, float* y) {
-      uint32_t v[16], u[16];
-      tmem_ld16_issue(tmem_base + lane_addr + (uint32_t)c0, v);
-      tmem_ld16_issue(tmem_base + CH_D_COLS + lane_addr + (uint32_t)c0, u);
+    // Sums of token columns [c0, c0 + 16) of this thread's row: hi.hi products and small terms of both issuers, scales undone
+    // (two exact multiplications); the four loads are in flight together
+    auto ld_acc = [&](const ChainPhase& gp, int c0, float* y) {
+      uint32_t h0[16], l0[16], h1[16], l1[16];
+      const uint32_t at = tmem_base + lane_addr + (uint32_t)c0;
+      tmem_ld16_issue(at, h0);
+      tmem_ld16_issue(at + (uint32_t)bn, l0);
+      tmem_ld16_issue(at + CH_D_COLS, h1);
+      tmem_ld16_issue(at + CH_D_COLS + (uint32_t)bn, l1);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 16; ++j) y[j] = __uint_as_float(v[j]) + __uint_as_float(u[j]);
+      for (int j = 0; j < 16; ++j) {
+        const float hh = __uint_as_float(h0[j]) + __uint_as_float(h1[j]), small = __uint_as_float(l0[j]) + __uint_as_float(l1[j]);
+        y[j] = fmaf(small, PAIR_LO_INV, hh) * gp.inv_x * gp.inv_w;
+      }
     };
     constexpr int PH_WORDS = (int)(sizeof(ChainPhase) / 4);
     const bool ph_staged = !(a.tune_fence & 4);
@@ -1078,7 +970,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
 #pragma unroll
             for (int cc = 0; cc < 32; cc += 16) {
               const int c0 = half * 32 + cc;
-              ld_acc(c0, &y[cc]);
+              if (c0 < bn) ld_acc(ph, c0, &y[cc]);
             }
             tc_fence_before();
             __syncwarp();
@@ -1104,8 +996,9 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
 #pragma unroll
             for (int cc = 0; cc < 32; cc += 16) {
               const int c0 = half * 32 + cc;
+              if (c0 >= bn) break;
               float y[16];
-              ld_acc(c0, y);
+              ld_acc(ph, c0, y);
 #pragma unroll
               for (int j = 0; j < 16; ++j)
                 if (c0 + j < a.m) dst[(size_t)(c0 + j) * TILE_M] = y[j];
@@ -1201,7 +1094,7 @@ void chain_prepare_phases(ChainPhase* phases, int n_phases, int grid) {
     ChainPhase& ph = phases[p];
     ph.r_nkb = ph.r_per = 0;
     ph.r_magic_per = ph.r_magic_nkb = 0;
-    if (ph.kind == CH_FINAL || ph.k < BK * CH_UB || ph.n < 1) continue;
+    if (ph.kind == CH_FINAL || ph.k < CH_K || ph.n < 1) continue;
     const ChRange r = chain_range(ph.n, ph.k, 0, grid, ph.kind == CH_GEMM && ph.whole_tiles);
     ph.r_nkb = r.nkb;
     ph.r_per = r.per;
@@ -1229,7 +1122,7 @@ bool chain_supported(const ChainArgs& a, int grid, const ChainPhase* host_phases
       if (phs[p - 1].kind != CH_ELEM && !(phs[p - 1].kind == CH_GEMM && phs[p - 1].whole_tiles)) return false;
       continue;
     }
-    if (ph.k < BK * CH_UB || ph.k % (BK * CH_UB) != 0 || ph.n < 1) return false;
+    if (ph.k < CH_K || ph.k % CH_K != 0 || ph.n < 1) return false;
     if (ph.kind == CH_EMBED) {
       if (ph.n % 4 != 0 || ph.n > 4 * 4 * CH_WORKERS || !ph.x || !ph.ln_g || !ph.ln_b || !ph.out_hi || !ph.out_lo) return false;
       if (!a.wte || !a.wpe || !a.ids || !a.pos) return false;
@@ -1242,14 +1135,15 @@ bool chain_supported(const ChainArgs& a, int grid, const ChainPhase* host_phases
     if (!whole && ph.kind == CH_GEMM && (ph.best || ph.out)) return false;
     if (ph.kind == CH_GEMM) {
       if (ph.act < 0 || ph.act > 2 || !a.act_hi[ph.act] || !a.act_lo[ph.act] || a.act_k[ph.act] != ph.k) return false;
-      const unsigned long long rows = ((unsigned long long)ph.w_block0 + (unsigned long long)((ph.n + TILE_M - 1) / TILE_M) * r.nkb * CH_UB) * TILE_M;
-      if (rows > 0x7fffffffull || rows * BK > a.arena_floats) return false;
+      const unsigned long long rows =
+          ((unsigned long long)ph.w_block0 + (unsigned long long)((ph.n + TILE_M - 1) / TILE_M) * r.nkb) * (a.exact ? 1 : 2) * TILE_M;
+      if (rows > 0x7fffffffull || rows * CH_K > a.arena_halves) return false;
     } else if (ph.kind == CH_ROWS) {
       if (ph.n % 4 != 0 || ph.n > 4 * 4 * CH_WORKERS || !ph.x) return false;
       if (ph.ln_g && (!ph.ln_b || !ph.out_hi || !ph.out_lo)) return false;
       if (p == 0 || phs[p - 1].kind != CH_GEMM || phs[p - 1].n != ph.n || phs[p - 1].k != ph.k) return false;
     } else if (ph.kind == CH_ELEM) {
-      if (ph.out_hi && !ph.out_lo) return false;
+      if (ph.out_hi && (!ph.out_lo || ph.n % 4 != 0)) return false;
       if (p == 0 || phs[p - 1].kind != CH_GEMM || phs[p - 1].n != ph.n || phs[p - 1].k != ph.k) return false;
     } else {
       return false;
@@ -1263,16 +1157,17 @@ cudaError_t launch_chain(const ChainArgs& a, int grid, cudaStream_t s) {
   if (!a.phases_dev && !chain_supported(a, grid)) return cudaErrorInvalidValue;
   CUtensorMap maps[7];
   memset(maps, 0, sizeof(maps));
-  if (!make_map(&maps[0], a.arena, a.arena_floats / BK, BK, CH_UB * TILE_M)) return cudaErrorInvalidValue;
+  const int bn = a.m <= 16 ? 16 : a.m <= 32 ? 32 : CH_BN;
+  if (!make_map_f16(&maps[0], a.arena, a.arena_halves / CH_K, CH_K, (a.exact ? 1 : 2) * TILE_M)) return cudaErrorInvalidValue;
   for (int i = 0; i < 3; ++i) {
     if (!a.act_hi[i]) continue;
-    if (!make_map(&maps[1 + 2 * i], a.act_hi[i], (uint64_t)a.m, (uint64_t)a.act_k[i], CH_BN) ||
-        !make_map(&maps[2 + 2 * i], a.act_lo[i], (uint64_t)a.m, (uint64_t)a.act_k[i], CH_BN))
+    if (!make_map_f16(&maps[1 + 2 * i], a.act_hi[i], (uint64_t)a.m, (uint64_t)a.act_k[i], bn) ||
+        !make_map_f16(&maps[2 + 2 * i], a.act_lo[i], (uint64_t)a.m, (uint64_t)a.act_k[i], bn))
       return cudaErrorInvalidValue;
   }
   ChainArgs args = a;
   if (!args.phases_dev) chain_prepare_phases(args.ph, args.n_phases, grid);
-  void* params[8] = {&maps[0], &maps[1], &maps[2], &maps[3], &maps[4], &maps[5], &maps[6], &args};
+  void* params[9] = {&maps[0], &maps[1], &maps[2], &maps[3], &maps[4], &maps[5], &maps[6], &args, const_cast<int*>(&bn)};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(CH_THREADS);

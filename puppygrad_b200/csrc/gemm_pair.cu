@@ -25,11 +25,6 @@ namespace {
 constexpr int PK = 64;   // FP16 elements per k block: one 128-byte swizzle row
 constexpr int PBN = 128; // columns of an output tile
 
-// Instruction descriptor for kind::f16 with FP16 operands: FP32 accumulate, both K-major.
-__device__ __forceinline__ uint32_t umma_idesc_f16(int m, int n) {
-  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
 // EXACT_W: the weights are BF16 values, their lo parts zero and not read.
 template <bool EXACT_W>
 struct PairSmem {
@@ -40,6 +35,9 @@ struct PairSmem {
   static constexpr size_t BYTES = (size_t)STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 
+// The weights lie in blocks of 128 rows x 64 values, hi tile and then (unless EXACT_W) lo tile, k block after k block, row tile after
+// row tile (launch_tile_pairs): one box per block, and the same copy serves the decode step (gemm_chain.cu).
+//
 // Persistent over 128 x 128 output tiles (column tiles of one row panel are neighbours, so the activation panel is reused
 // from L2). Warp 0 loads by TMA, one thread of warp 1 issues the MMAs, warps 2..5 drain. Tensor memory holds two buffers of
 // two accumulators, so that a tile is drained while the next one is multiplied: the tensor core adds with truncation, a bias
@@ -53,7 +51,7 @@ struct PairSmem {
 template <bool EXACT_W>
 __global__ void __launch_bounds__(192, 1)
     tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_constant__ CUtensorMap map_xl,
-                        const __grid_constant__ CUtensorMap map_wh, const __grid_constant__ CUtensorMap map_wl, PairGemmArgs a) {
+                        const __grid_constant__ CUtensorMap map_w, PairGemmArgs a) {
   using S = PairSmem<EXACT_W>;
   constexpr int TILE = S::TILE_BYTES;
   extern __shared__ uint8_t smem_raw[];
@@ -106,8 +104,7 @@ __global__ void __launch_bounds__(192, 1)
           mbar_expect_tx(bar, S::STAGE_BYTES);
           tma_load_2d(st, &map_xh, kb * PK, m0, bar);
           tma_load_2d(st + TILE, &map_xl, kb * PK, m0, bar);
-          tma_load_2d(st + 2 * TILE, &map_wh, kb * PK, n0, bar);
-          if (!EXACT_W) tma_load_2d(st + 3 * TILE, &map_wl, kb * PK, n0, bar);
+          tma_load_2d(st + 2 * TILE, &map_w, 0, ((n0 / TILE_M) * nkb + kb) * ((EXACT_W ? 1 : 2) * TILE_M), bar);
         }
       }
     }
@@ -219,14 +216,23 @@ __global__ void __launch_bounds__(192, 1)
 
 __global__ void __launch_bounds__(256) make_pairs_kernel(const float4* __restrict__ x, uint16_t* hi, uint16_t* lo, size_t n4, float scale) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x)
-    if (lo) {
-      store_pair4(hi + 4 * i, lo + 4 * i, x[i], scale);
-    } else {
-      uint2 h, l;
-      split_pair2(x[i].x, x[i].y, scale, h.x, l.x);
-      split_pair2(x[i].z, x[i].w, scale, h.y, l.y);
-      *reinterpret_cast<uint2*>(hi + 4 * i) = h;
-    }
+    store_pair4(hi + 4 * i, lo + 4 * i, x[i], scale);
+}
+
+// One warp per 64-value piece of a weight row (rows up to the next multiple of 128 and k up to one of 64: zeros).
+__global__ void __launch_bounds__(256) tile_pairs_kernel(const float* __restrict__ w, uint16_t* dst, int n, int k, int exact, float scale) {
+  const int nkb = (k + PK - 1) / PK, lane = threadIdx.x & 31;
+  const long long pieces = (long long)((n + TILE_M - 1) / TILE_M) * TILE_M * nkb;
+  for (long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); i < pieces; i += (long long)gridDim.x * 8) {
+    const int row = (int)(i / nkb), kb = (int)(i - (long long)row * nkb), col = kb * PK + lane * 2;
+    const float a = row < n && col < k ? w[(size_t)row * k + col] : 0.f, b = row < n && col + 1 < k ? w[(size_t)row * k + col + 1] : 0.f;
+    uint32_t hi, lo;
+    split_pair2(a, b, scale, hi, lo);
+    const long long block = (long long)(row / TILE_M) * nkb + kb;
+    uint32_t* at = reinterpret_cast<uint32_t*>(dst + (block * (exact ? 1 : 2) * TILE_M + row % TILE_M) * PK) + lane;
+    at[0] = hi;
+    if (!exact) at[TILE_M * PK / 2] = lo;
+  }
 }
 
 // Per matrix [rows, cols]: the largest |w| and the largest Euclidean norm of a row at or after `norm_from`, as bit patterns
@@ -253,18 +259,6 @@ __global__ void __launch_bounds__(256) matrix_bounds_kernel(const float* __restr
   }
 }
 
-// 2-D FP16 tensor [rows, k] (k contiguous, k % 8 == 0), boxes of 64 elements x 128 rows, 128-byte swizzle, zeros outside
-bool make_map_f16(CUtensorMap* map, const uint16_t* ptr, uint64_t rows, uint64_t k) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {k, rows};
-  cuuint64_t strides[1] = {k * 2};
-  cuuint32_t box[2] = {PK, TILE_M};
-  cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 int sm_count() {
   static const int n = [] {
     int dev = 0, v = 148;
@@ -277,12 +271,13 @@ int sm_count() {
 
 template <bool EXACT_W>
 cudaError_t launch_pair(const PairGemmArgs& a, cudaStream_t s) {
-  CUtensorMap xh, xl, wh, wl;
-  if (!make_map_f16(&xh, a.x_hi, a.m, a.k) || !make_map_f16(&xl, a.x_lo, a.m, a.k) || !make_map_f16(&wh, a.w_hi, a.n, a.k) ||
-      !make_map_f16(&wl, EXACT_W ? a.w_hi : a.w_lo, a.n, a.k))
+  CUtensorMap xh, xl, w;
+  const uint64_t w_rows = pair_tiled_halves(a.n, a.k, EXACT_W) / PK;
+  if (!make_map_f16(&xh, a.x_hi, a.m, a.k, TILE_M) || !make_map_f16(&xl, a.x_lo, a.m, a.k, TILE_M) ||
+      w_rows > 0x7fffffffull || !make_map_f16(&w, a.w, w_rows, PK, (EXACT_W ? 1 : 2) * TILE_M))
     return cudaErrorInvalidValue;
   const int tiles = ((a.n + PBN - 1) / PBN) * ((a.m + TILE_M - 1) / TILE_M);
-  tc_gemm_pair_kernel<EXACT_W><<<std::min(tiles, sm_count()), 192, PairSmem<EXACT_W>::BYTES, s>>>(xh, xl, wh, wl, a);
+  tc_gemm_pair_kernel<EXACT_W><<<std::min(tiles, sm_count()), 192, PairSmem<EXACT_W>::BYTES, s>>>(xh, xl, w, a);
   return cudaGetLastError();
 }
 
@@ -294,6 +289,15 @@ float pair_scale(float bound) {
   if (!(bound > 0.f) || !std::isfinite(bound)) return 1.f;
   const int e = 14 - std::ilogb(bound);  // bound * 2^e in [2^14, 2^15)
   return std::ldexp(1.f, std::max(-120, std::min(120, e)));
+}
+
+size_t pair_tiled_halves(int n, int k, bool exact) {
+  return (size_t)((n + TILE_M - 1) / TILE_M) * ((k + PK - 1) / PK) * TILE_M * PK * (exact ? 1 : 2);
+}
+
+cudaError_t launch_tile_pairs(const float* w, uint16_t* dst, int n, int k, bool exact, float scale, cudaStream_t s) {
+  tile_pairs_kernel<<<148 * 8, 256, 0, s>>>(w, dst, n, k, exact ? 1 : 0, scale);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_make_pairs(const float* x, uint16_t* hi, uint16_t* lo, size_t n, float scale, cudaStream_t s) {
@@ -316,9 +320,9 @@ cudaError_t init_pair_gemm_attributes() {
 
 cudaError_t launch_tc_gemm_pair(const PairGemmArgs& a, cudaStream_t s) {
   if (a.m <= 0 || a.n <= 0) return cudaSuccess;
-  if (!pair_gemm_supported(a.k) || !a.x_hi || !a.x_lo || !a.w_hi || (!a.out && !a.out_hi)) return cudaErrorInvalidValue;
+  if (!pair_gemm_supported(a.k) || !a.x_hi || !a.x_lo || !a.w || (!a.out && !a.out_hi)) return cudaErrorInvalidValue;
   if (a.out_hi && (a.n % 2 != 0 || !a.out_lo || a.epilogue == EPI_RESID || (a.epilogue != EPI_GELU && a.k > 56 * PK))) return cudaErrorInvalidValue;
-  return a.w_lo ? launch_pair<false>(a, s) : launch_pair<true>(a, s);
+  return a.w_exact ? launch_pair<true>(a, s) : launch_pair<false>(a, s);
 }
 
 }  // namespace pg

@@ -144,7 +144,8 @@ cudaError_t launch_tc_gemm_tf32(const TcGemmArgs& a, cudaStream_t s);
 // FP32-grade product of FP16 pairs, any m (prefill; gemm_pair.cu): out[m, n] = x[m, k] . w[n, k]^T (+bias)(+GELU | +resid).
 struct PairGemmArgs {
   const uint16_t *x_hi, *x_lo;  // [m, k]
-  const uint16_t *w_hi, *w_lo;  // [n, k]; w_lo nullptr: all zero (BF16 weights)
+  const uint16_t* w;            // [n, k], laid out by launch_tile_pairs
+  bool w_exact;                 // BF16 weights: no lo tiles
   float inv_x, inv_w;           // reciprocals of the two scales
   const float* bias;            // [n] or nullptr
   const float* resid;           // [m, n], EPI_RESID (may alias out)
@@ -157,9 +158,11 @@ struct PairGemmArgs {
 bool pair_gemm_supported(int k);
 cudaError_t launch_tc_gemm_pair(const PairGemmArgs& a, cudaStream_t s);
 cudaError_t init_pair_gemm_attributes();
-// Scale for values that stay below `bound`; pairs of n values (n % 4 == 0; lo nullptr: only hi parts); {largest |w|, largest norm of a row from
-// `norm_from` on} as bit patterns into out[2], which starts at zero.
+// Scale for values that stay below `bound`; pairs of n values (n % 4 == 0); a weight matrix [n, k] as tiles of pairs (`exact`: only
+// the hi tiles); {largest |w|, largest norm of a row from `norm_from` on} as bit patterns into out[2], which starts at zero.
 float pair_scale(float bound);
+size_t pair_tiled_halves(int n, int k, bool exact);
+cudaError_t launch_tile_pairs(const float* w, uint16_t* dst, int n, int k, bool exact, float scale, cudaStream_t s);
 cudaError_t launch_make_pairs(const float* x, uint16_t* hi, uint16_t* lo, size_t n, float scale, cudaStream_t s);
 cudaError_t launch_matrix_bounds(const float* w, int rows, int cols, int norm_from, unsigned* out, cudaStream_t s);
 // three TF32 passes (FP32-grade), m <= 64 (decode)
@@ -167,39 +170,40 @@ int tc_gemm_x3_splits(int n, int k, int num_sms);
 cudaError_t launch_tc_gemm_x3(const TcGemmArgs& a, int splits, bool pdl, cudaStream_t s);
 cudaError_t launch_finalize(const FinalizeArgs& a, bool pdl, cudaStream_t s);
 
-// A chain of dependent decode linears (m <= 64 tokens, three TF32 products each) as ONE persistent
+// A chain of dependent decode linears (m <= 64 tokens, products of FP16 pairs) as ONE persistent
 // cooperative kernel (gemm_chain.cu), one CTA per SM. The weights of every GEMM phase are one
-// contiguous run of 16 KB blocks of the tiled arena, cut into equal shares per CTA whatever the
+// contiguous run of blocks of the arena of pair tiles (launch_tile_pairs), cut into equal shares per CTA whatever the
 // matrix shape; a CTA's share may cross row tiles, and it writes one partial accumulator per tile
 // it touched. The phase after a GEMM adds the partials in k order and applies the bias with either
-// a residual update (+ LayerNorm, written as a TF32 hi/lo pair) or an element-wise epilogue (GELU,
-// hi/lo pair and/or plain FP32). Phases are separated by a bounded grid barrier that only the
+// a residual update (+ LayerNorm, written as FP16 pairs) or an element-wise epilogue (GELU,
+// pairs and/or plain FP32). Phases are separated by a bounded grid barrier that only the
 // worker warps take part in: the weight stream of later phases keeps running through it.
 enum ChainKind { CH_GEMM = 0, CH_ROWS = 1, CH_ELEM = 2, CH_ATTN = 3, CH_EMBED = 4, CH_FINAL = 5 };
 enum ChainAct { CH_ACT_NORM = 0, CH_ACT_ATTN = 1, CH_ACT_H = 2 };
 struct ChainPhase {
   int kind;
   int n, k;           // GEMM: output features and reduction length; ROWS / ELEM / ATTN: those of the GEMM being reduced
-  int act;            // GEMM: which hi/lo activation pair is the input (ChainAct)
-  unsigned w_block0;  // GEMM: index of the first 16 KB block of this matrix inside the tiled arena
+  int act;            // GEMM: which pair of activations is the input (ChainAct)
+  unsigned w_block0;  // GEMM: index of the first 128 x 64 block of this matrix inside the arena
+  float inv_x, inv_w; // GEMM: reciprocals of the scales of its activations and weights
+  float out_scale;    // phases with out_hi: scale of the pairs
   int gelu;           // ELEM: tanh-GELU after the bias
   const float* bias;  // ROWS / ELEM: [n] or nullptr
   float* x;           // ROWS: residual stream [m, n], updated in place
   const float* ln_g;  // ROWS: LayerNorm over the updated row (nullptr: none) ...
   const float* ln_b;
   float* out;         // ELEM: plain FP32 result [m, n] or nullptr
-  float* out_hi;      // ROWS: LayerNorm result, ELEM / ATTN: result, as a TF32 hi/lo pair (or nullptr)
-  float* out_lo;
+  uint16_t* out_hi;   // ROWS: LayerNorm result, ELEM / ATTN: result, as FP16 pairs (or nullptr)
+  uint16_t* out_lo;
   float* kv_pool;     // ATTN: this layer's page pool (n, k, bias: those of the QKV GEMM right before it)
   unsigned long long* best;  // ELEM, whole-tile GEMM: optional row arg-max accumulator [m] (packed value | index, see CH_FINAL)
   // derived by chain_prepare_phases (share arithmetic of the phase's GEMM for the launch grid, so that no thread
-  // divides when a phase starts): 32 KB weight units per row tile, units per CTA, multiply-high reciprocals of both
+  // divides when a phase starts): weight units (one block each) per row tile, units per CTA, multiply-high reciprocals of both
   int r_nkb, r_per;
   unsigned r_magic_per, r_magic_nkb;
   // GEMM without a reduce phase behind it (the lm_head): every CTA takes whole row tiles, so an accumulator holds
   // finished sums, and the drain stores them to `out` (or nowhere) and folds them into `best`; no bias, no partial tiles
   int whole_tiles;
-  int reserved_;
 };
 constexpr int CHAIN_MAX_PHASES = 10;
 struct ChainArgs {
@@ -224,10 +228,11 @@ struct ChainArgs {
   unsigned long long* best;  // [m], holds chain_argmax_init() between launches
   int m;               // tokens (rows of every activation matrix), <= 64
   float eps;
-  const float* arena;  // tiled weight arena (all matrices of the model)
-  size_t arena_floats;
-  const float* act_hi[3];  // activation pairs by ChainAct: [m, k] each
-  const float* act_lo[3];
+  const uint16_t* arena;  // tiles of pairs, all matrices of the model
+  size_t arena_halves;
+  int exact;              // BF16 weights: hi tiles only
+  const uint16_t* act_hi[3];  // activation pairs by ChainAct: [m, k] each
+  const uint16_t* act_lo[3];
   int act_k[3];
   float* partials;     // chain_partial_floats(grid) floats
   unsigned* barrier;   // one word, zero before the first launch (the kernel leaves it zero)

@@ -57,7 +57,7 @@ pg_cache::~pg_cache() {
 #endif
 #ifdef PG_DEV_TRACE
   if (d_chain_trace) {
-    std::vector<unsigned long long> t((size_t)chain_ctas * 32 + 512);
+    std::vector<unsigned long long> t((size_t)chain_ctas * 32);
     if (cudaMemcpy(t.data(), d_chain_trace, t.size() * 8, cudaMemcpyDeviceToHost) == cudaSuccess) {
       unsigned long long t0 = ~0ULL;
       for (int i = 0; i < chain_ctas; ++i) t0 = std::min(t0, t[(size_t)i * 32 + 31]);
@@ -69,16 +69,10 @@ pg_cache::~pg_cache() {
         }
         fprintf(stderr, "chain trace phase %d: work done %6llu..%6llu ns, barrier passed %6llu..%6llu ns\n", sl, wlo, whi, lo, hi);
       }
-      // the lm_head of the last step: per CTA its SM and the time its share took; then CTA 0's units (see unit_trace)
+      // the lm_head of the last step: per CTA its SM and the time its share took
       for (int i = 0; i < chain_ctas; ++i) {
         const unsigned long long* r = t.data() + (size_t)i * 32;
         fprintf(stderr, "chain trace lm_head cta %3d sm %3llu work %7lld ns\n", i, r[22], (long long)(r[21] - r[20]));
-      }
-      const unsigned long long* u = t.data() + (size_t)chain_ctas * 32;
-      for (int i = 0; i < 48; ++i) {
-        fprintf(stderr, "chain trace unit %2d:", i);
-        for (int e = 0; e < 8; ++e) fprintf(stderr, " %7lld", u[i * 8 + e] ? (long long)(u[i * 8 + e] - u[0]) : -1LL);
-        fprintf(stderr, "\n");
       }
     }
   }
@@ -144,16 +138,19 @@ static size_t align_up(size_t n, size_t a) { return (n + a - 1) / a * a; }
 // FP16 pairs of the dense matrices, and the scales of their inputs: what the values of each can reach at most, from the
 // weights alone. `tensors`: the host tensors of the model.
 static int make_pair_weights(pg_model* m, const float* const* tensors) {
-  const size_t C = m->c(), F = m->f(), L = m->layers.size();
+  const size_t C = m->c(), F = m->f(), V = m->v(), L = m->layers.size();
   if (!pair_gemm_supported((int)C) || !pair_gemm_supported((int)F)) return PG_OK;
   const bool exact = m->backend.math_mode == PG_MATH_BF16;  // BF16 values fit the hi part
-  const size_t per_layer = 4 * C * C + 2 * C * F;
-  PG_CUDA_TRY(cudaMalloc(&m->pair_arena, per_layer * L * (exact ? 1 : 2) * sizeof(uint16_t)));
+  auto halves = [&](size_t n, size_t k) { return pair_tiled_halves((int)n, (int)k, exact); };
+  m->pair_exact = exact;
+  m->pair_halves = L * (halves(3 * C, C) + halves(C, C) + halves(F, C) + halves(C, F)) + halves(V, C);
+  PG_CUDA_TRY(cudaMalloc(&m->pair_arena, m->pair_halves * sizeof(uint16_t)));
   unsigned* d_bounds = nullptr;
-  PG_CUDA_TRY(cudaMalloc(&d_bounds, L * 8 * sizeof(unsigned)));
-  std::vector<float> bounds(L * 8);
+  const size_t n_bounds = L * 8 + 2;
+  PG_CUDA_TRY(cudaMalloc(&d_bounds, n_bounds * sizeof(unsigned)));
+  std::vector<float> bounds(n_bounds);
   int rc = [&]() -> int {
-    PG_CUDA_TRY(cudaMemsetAsync(d_bounds, 0, L * 8 * sizeof(unsigned), 0));
+    PG_CUDA_TRY(cudaMemsetAsync(d_bounds, 0, n_bounds * sizeof(unsigned), 0));
     for (size_t l = 0; l < L; ++l) {
       const LayerWeights& w = m->layers[l];
       unsigned* b = d_bounds + 8 * l;
@@ -162,20 +159,18 @@ static int make_pair_weights(pg_model* m, const float* const* tensors) {
       PG_CUDA_TRY(launch_matrix_bounds(w.w_fc, (int)F, (int)C, 0, b + 4, 0));
       PG_CUDA_TRY(launch_matrix_bounds(w.w_proj2, (int)C, (int)F, 0, b + 6, 0));
     }
-    PG_CUDA_TRY(cudaMemcpy(bounds.data(), d_bounds, L * 8 * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    PG_CUDA_TRY(launch_matrix_bounds(m->head_w, (int)V, (int)C, 0, d_bounds + 8 * L, 0));
+    PG_CUDA_TRY(cudaMemcpy(bounds.data(), d_bounds, n_bounds * sizeof(unsigned), cudaMemcpyDeviceToHost));
     return PG_OK;
   }();
   cudaFree(d_bounds);
   if (rc != PG_OK) return rc;
   uint16_t* at = m->pair_arena;
-  auto pairs = [&](const float* w, size_t n, float top, PairWeights* out) -> int {
+  auto pairs = [&](const float* w, size_t n, size_t k, float top, PairWeights* out) -> int {
     out->scale = pair_scale(top);
-    uint16_t *hi = at, *lo = at + n;
-    if (exact) lo = nullptr;
-    PG_CUDA_TRY(launch_make_pairs(w, hi, lo, n, out->scale, 0));
-    out->hi = hi;
-    out->lo = lo;
-    at += exact ? n : 2 * n;
+    out->w = at;
+    PG_CUDA_TRY(launch_tile_pairs(w, at, (int)n, (int)k, exact, out->scale, 0));
+    at += halves(n, k);
     return PG_OK;
   };
   auto largest = [](const float* v, size_t n) {
@@ -192,10 +187,10 @@ static int make_pair_weights(pg_model* m, const float* const* tensors) {
     LayerWeights& w = m->layers[l];
     const float* const* t = tensors + 4 + 12 * l;
     const float* b = bounds.data() + 8 * l;
-    if (int r = pairs(w.w_qkv, 3 * C * C, b[0], &w.q_qkv)) return r;
-    if (int r = pairs(w.w_proj, C * C, b[2], &w.q_proj)) return r;
-    if (int r = pairs(w.w_fc, C * F, b[4], &w.q_fc)) return r;
-    if (int r = pairs(w.w_proj2, C * F, b[6], &w.q_proj2)) return r;
+    if (int r = pairs(w.w_qkv, 3 * C, C, b[0], &w.q_qkv)) return r;
+    if (int r = pairs(w.w_proj, C, C, b[2], &w.q_proj)) return r;
+    if (int r = pairs(w.w_fc, F, C, b[4], &w.q_fc)) return r;
+    if (int r = pairs(w.w_proj2, C, F, b[6], &w.q_proj2)) return r;
     // a normalised row has a norm of at most sqrt(C), so one output of the product behind it is at most its weight row's norm
     // times the norm of the scaled and shifted row; attention outputs are convex combinations of value rows, |gelu(y)| <= |y|
     const float root = std::sqrt((float)C);
@@ -205,7 +200,8 @@ static int make_pair_weights(pg_model* m, const float* const* tensors) {
     w.x_norm2 = pair_scale(root * largest(t[6], C) + largest(t[7], C));
     w.x_h = pair_scale(b[5] * row2 + largest(t[9], F));
   }
-  return PG_OK;
+  m->x_normf = pair_scale(std::sqrt((float)C) * largest(tensors[2], C) + largest(tensors[3], C));
+  return pairs(m->head_w, V, C, bounds[8 * L], &m->q_wte);
 }
 
 static int build_model(const pg_gpt2_config& cfg, const float* const* tensors, const uint64_t* lens, uint64_t n,
@@ -358,8 +354,7 @@ static int build_model(const pg_gpt2_config& cfg, const float* const* tensors, c
       if (int r = tile(w.w_proj2, C, F, &w.t_proj2)) return r;
     }
     if (int r = tile(m->head_w, V, C, &m->t_wte)) return r;
-    if (be.math_mode != PG_MATH_TF32)
-      if (int r = make_pair_weights(m.get(), tensors)) return r;
+    if (int r = make_pair_weights(m.get(), tensors)) return r;
     PG_CUDA_TRY(cudaDeviceSynchronize());
   }
   *out = m.release();
@@ -442,13 +437,14 @@ static int cache_new(const pg_model* m, int max_batch, pg_cache** out) {
   PG_CUDA_TRY(cudaMalloc(&c->attn_part, B * H * MAX_SPLITS * (D + 2) * sizeof(float)));
   PG_CUDA_TRY(cudaMalloc(&c->attn_counters, B * H * sizeof(unsigned)));
   PG_CUDA_TRY(cudaMemsetAsync(c->attn_counters, 0, B * H * sizeof(unsigned), c->stream));
+  c->chain_min_batch = m->pair_exact ? 5 : 9;
   if (const char* e = getenv("PG_CHAIN_MIN_BATCH")) c->chain_min_batch = std::max(1, std::min(65, atoi(e)));
   if (max_batch >= c->chain_min_batch && C % 32 == 0 && F % 32 == 0) {
     const int bmax = std::min(max_batch, 64);
     PG_CUDA_TRY(cudaMalloc(&c->norm_lo, (size_t)bmax * C * sizeof(float)));
     PG_CUDA_TRY(cudaMalloc(&c->attn_lo, (size_t)bmax * C * sizeof(float)));
     PG_CUDA_TRY(cudaMalloc(&c->h_lo, (size_t)bmax * F * sizeof(float)));
-    if (m->t_wte && !env_flag("PG_NO_CHAIN") && chain_grid(m->num_sms) > 0) {
+    if (m->pair_arena && !env_flag("PG_NO_CHAIN") && chain_grid(m->num_sms) > 0) {
       c->chain_ctas = chain_grid(m->num_sms);
       PG_CUDA_TRY(cudaMalloc(&c->chain_partials, chain_partial_floats(c->chain_ctas) * sizeof(float)));
       PG_CUDA_TRY(cudaMalloc(&c->d_chain_barrier, sizeof(unsigned)));
@@ -460,8 +456,8 @@ static int cache_new(const pg_model* m, int max_batch, pg_cache** out) {
       }
 #ifdef PG_DEV_TRACE
       if (env_flag("PG_CHAIN_TRACE")) {
-        PG_CUDA_TRY(cudaMalloc(&c->d_chain_trace, ((size_t)c->chain_ctas * 32 + 512) * sizeof(unsigned long long)));
-        PG_CUDA_TRY(cudaMemsetAsync(c->d_chain_trace, 0, ((size_t)c->chain_ctas * 32 + 512) * sizeof(unsigned long long), c->stream));
+        PG_CUDA_TRY(cudaMalloc(&c->d_chain_trace, (size_t)c->chain_ctas * 32 * sizeof(unsigned long long)));
+        PG_CUDA_TRY(cudaMemsetAsync(c->d_chain_trace, 0, (size_t)c->chain_ctas * 32 * sizeof(unsigned long long), c->stream));
       }
 #endif
     }
@@ -541,14 +537,16 @@ static int choose_splits(const pg_cache* c, int batch, int max_len) {
 
 // Arguments of the chain kernel for `batch` sequences starting at slot 64 * chunk (steps of more than 64
 // sequences run as one launch per 64: the activation buffers are reused, what belongs to a slot is offset).
+static uint16_t* halves_of(float* buf) { return reinterpret_cast<uint16_t*>(buf); }
 static ChainArgs chain_base_args(const pg_cache* c, int batch, int chunk = 0) {
   const pg_model* m = c->model;
   const size_t s0 = (size_t)chunk * 64;
   ChainArgs base{};
-  base.m = batch; base.eps = m->cfg.layer_norm_epsilon; base.arena = m->tiled_arena; base.arena_floats = m->tiled_floats;
-  base.act_hi[CH_ACT_NORM] = c->norm; base.act_lo[CH_ACT_NORM] = c->norm_lo; base.act_k[CH_ACT_NORM] = m->c();
-  base.act_hi[CH_ACT_ATTN] = c->attn; base.act_lo[CH_ACT_ATTN] = c->attn_lo; base.act_k[CH_ACT_ATTN] = m->c();
-  base.act_hi[CH_ACT_H] = c->hbuf; base.act_lo[CH_ACT_H] = c->h_lo; base.act_k[CH_ACT_H] = m->f();
+  base.m = batch; base.eps = m->cfg.layer_norm_epsilon; base.arena = m->pair_arena; base.arena_halves = m->pair_halves;
+  base.exact = m->pair_exact;
+  base.act_hi[CH_ACT_NORM] = halves_of(c->norm); base.act_lo[CH_ACT_NORM] = halves_of(c->norm_lo); base.act_k[CH_ACT_NORM] = m->c();
+  base.act_hi[CH_ACT_ATTN] = halves_of(c->attn); base.act_lo[CH_ACT_ATTN] = halves_of(c->attn_lo); base.act_k[CH_ACT_ATTN] = m->c();
+  base.act_hi[CH_ACT_H] = halves_of(c->hbuf); base.act_lo[CH_ACT_H] = halves_of(c->h_lo); base.act_k[CH_ACT_H] = m->f();
   base.partials = c->chain_partials; base.barrier = c->d_chain_barrier; base.error_flag = c->d_error;
   base.trace = c->d_chain_trace;
   base.kv = c->kv; base.page_table = c->tables[0].d_table + s0 * c->kv.pages_per_seq; base.pos = c->d_pos + s0;
@@ -575,61 +573,62 @@ static int ensure_chain_program(pg_cache* c, int batch, int chunk = 0) {
   std::vector<ChainPhase> ph;
   std::vector<int> bucket;
   int cur_b = B_OTHER;  // bucket of the phases being appended
-  auto block0 = [&](const float* t) { return (unsigned)((size_t)(t - m->tiled_arena) / 4096); };
-  auto gemm = [&](const float* t, int n_out, int k, int act) {
+  auto gemm = [&](const PairWeights& w, float x_scale, int n_out, int k, int act) {
     ChainPhase p{};
-    p.kind = CH_GEMM; p.n = n_out; p.k = k; p.act = act; p.w_block0 = block0(t);
+    p.kind = CH_GEMM; p.n = n_out; p.k = k; p.act = act;
+    p.w_block0 = (unsigned)((size_t)(w.w - m->pair_arena) / pair_tiled_halves(1, 1, m->pair_exact));
+    p.inv_x = 1.f / x_scale; p.inv_w = 1.f / w.scale;
     ph.push_back(p);
     bucket.push_back(cur_b);
   };
-  auto rows = [&](int n_out, int k, const float* bias, const float* g, const float* b) {
+  auto rows = [&](int n_out, int k, const float* bias, const float* g, const float* b, float scale) {
     ChainPhase p{};
     p.kind = CH_ROWS; p.n = n_out; p.k = k; p.bias = bias; p.x = c->x; p.ln_g = g; p.ln_b = b;
-    p.out_hi = c->norm; p.out_lo = c->norm_lo;
+    p.out_hi = halves_of(c->norm); p.out_lo = halves_of(c->norm_lo); p.out_scale = scale;
     ph.push_back(p);
     bucket.push_back(B_LAYER_NORM);  // partial sums + bias + residual + LayerNorm
   };
-  auto elem = [&](int n_out, int k, const float* bias, int gelu, float* out, float* ohi, float* olo) {
+  auto elem = [&](int n_out, int k, const float* bias, int gelu, float* out, uint16_t* ohi, uint16_t* olo, float scale) {
     ChainPhase p{};
-    p.kind = CH_ELEM; p.n = n_out; p.k = k; p.bias = bias; p.gelu = gelu; p.out = out; p.out_hi = ohi; p.out_lo = olo;
+    p.kind = CH_ELEM; p.n = n_out; p.k = k; p.bias = bias; p.gelu = gelu; p.out = out; p.out_hi = ohi; p.out_lo = olo; p.out_scale = scale;
     ph.push_back(p);
     bucket.push_back(cur_b);  // belongs to the GEMM it finishes
   };
   {
     ChainPhase p{};  // token + position embedding and the first LayerNorm
     p.kind = CH_EMBED; p.n = C; p.k = C; p.x = c->x; p.ln_g = m->layers[0].ln1_g; p.ln_b = m->layers[0].ln1_b;
-    p.out_hi = c->norm; p.out_lo = c->norm_lo;
+    p.out_hi = halves_of(c->norm); p.out_lo = halves_of(c->norm_lo); p.out_scale = m->layers[0].x_norm1;
     ph.push_back(p);
     bucket.push_back(B_LAYER_NORM);
   }
   for (int l = 0; l < L; ++l) {
     const LayerWeights& w = m->layers[l];
     cur_b = B_QKV;
-    gemm(w.t_qkv, 3 * C, C, CH_ACT_NORM);
+    gemm(w.q_qkv, w.x_norm1, 3 * C, C, CH_ACT_NORM);
     ChainPhase at{};  // reduces the QKV partials itself
     at.kind = CH_ATTN; at.n = 3 * C; at.k = C; at.bias = w.b_qkv; at.kv_pool = c->layer_pool(l);
-    at.out_hi = c->attn; at.out_lo = c->attn_lo;
+    at.out_hi = halves_of(c->attn); at.out_lo = halves_of(c->attn_lo); at.out_scale = w.x_attn;
     ph.push_back(at);
     bucket.push_back(B_ATTN);
     cur_b = B_ATTN_PROJ;
-    gemm(w.t_proj, C, C, CH_ACT_ATTN);
-    rows(C, C, w.b_proj, w.ln2_g, w.ln2_b);
+    gemm(w.q_proj, w.x_attn, C, C, CH_ACT_ATTN);
+    rows(C, C, w.b_proj, w.ln2_g, w.ln2_b, w.x_norm2);
     cur_b = B_MLP_FC;
-    gemm(w.t_fc, F, C, CH_ACT_NORM);
-    elem(F, C, w.b_fc, 1, nullptr, c->hbuf, c->h_lo);
+    gemm(w.q_fc, w.x_norm2, F, C, CH_ACT_NORM);
+    elem(F, C, w.b_fc, 1, nullptr, halves_of(c->hbuf), halves_of(c->h_lo), w.x_h);
     cur_b = B_MLP_PROJ;
-    gemm(w.t_proj2, C, F, CH_ACT_H);
-    if (l + 1 < L) rows(C, F, w.b_proj2, m->layers[l + 1].ln1_g, m->layers[l + 1].ln1_b);
-    else rows(C, F, w.b_proj2, m->lnf_g, m->lnf_b);
+    gemm(w.q_proj2, w.x_h, C, F, CH_ACT_H);
+    if (l + 1 < L) rows(C, F, w.b_proj2, m->layers[l + 1].ln1_g, m->layers[l + 1].ln1_b, m->layers[l + 1].x_norm1);
+    else rows(C, F, w.b_proj2, m->lnf_g, m->lnf_b, m->x_normf);
   }
   cur_b = B_LOGITS;
-  gemm(m->t_wte, V, C, CH_ACT_NORM);
+  gemm(m->q_wte, m->x_normf, V, C, CH_ACT_NORM);
   // The lm_head in whole row tiles per CTA: its drain stores the logits and finds the row arg-max, and there is no
   // reduce phase (measured on GPT-2 medium, 64 sequences: 38 + 37 us for GEMM + reduce with equal shares).
   // PG_CHAIN_LM_HEAD_REDUCE=1 brings the equal shares and the reduce phase back.
   static const bool lm_head_reduce = getenv("PG_CHAIN_LM_HEAD_REDUCE") && atoi(getenv("PG_CHAIN_LM_HEAD_REDUCE")) != 0;
   if (lm_head_reduce) {
-    elem(V, C, nullptr, 0, c->logits + (size_t)chunk * 64 * V, nullptr, nullptr);
+    elem(V, C, nullptr, 0, c->logits + (size_t)chunk * 64 * V, nullptr, nullptr, 1.f);
   } else {
     ph.back().whole_tiles = 1;
     ph.back().out = c->logits + (size_t)chunk * 64 * V;
@@ -676,9 +675,12 @@ static cudaError_t enqueue_decode_step(pg_cache* c, int batch, int splits, cudaS
                                        StepProfiler* prof = nullptr) {
   if (c->model->layered) return layered_enqueue_decode(c, batch, splits, s, launches, prof);
   // FP32 weights: the single-kernel step wins up to 4 sequences (measured on B200: 279 against 306 us for one GPT-2
-  // small sequence, 1014 against 1168 us for four GPT-2 medium ones; at eight it loses, 1806 against 1548 us);
-  // packed weights (BF16, int8) are only read by that kernel
-  const bool stream_wanted = c->model->stream_weight_type != STREAM_W_F32 || batch <= 4 || c->model->backend.persistent_step == 1;
+  // small sequence, 1014 against 1168 us for four GPT-2 medium ones; at eight it loses, 1806 against 1548 us).
+  // BF16: up to 4 too, where the chain kernel takes over (GPT-2 medium, us: 868 against 930 at four sequences, 1285
+  // against 964 at six, 1346 against 973 at eight; small 386 / 471, 587 / 478, 597 / 491). int8 rows are only read here.
+  auto chained = c->chain_programs.find(batch <= 64 ? chain_program_key(batch, 0) : -1);
+  const bool chain_takes = batch > 4 && c->model->pair_exact && chained != c->chain_programs.end() && chained->second.dev;
+  const bool stream_wanted = (c->model->stream_weight_type != STREAM_W_F32 && !chain_takes) || batch <= 4 || c->model->backend.persistent_step == 1;
   if (!prof && c->stream_grid > 0 && stream_wanted &&
       decode_stream_supported(batch, c->model->c(), c->model->f(), c->model->v(), c->model->head_dim(),
                               c->model->positions(), c->kv.page_tokens, c->model->stream_weight_type, c->stream_grid)) {
@@ -960,7 +962,7 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
   const float eps = m->cfg.layer_norm_epsilon;
   // FP32-grade products on the tensor cores read FP16 pairs; whoever produces an input (LayerNorm, attention, the GELU
   // epilogue of the MLP's first product) writes pairs instead of FP32, into the same buffer: [rows, k] hi, then lo.
-  const bool pairs = m->pair_arena && ws.d_error && rows >= 128 && m->head_dim() == 64 && C <= 4096;
+  const bool pairs = m->pair_arena && m->backend.math_mode != PG_MATH_TF32 && ws.d_error && rows >= 128 && m->head_dim() == 64 && C <= 4096;
   auto pair_of = [&](float* buf, int k, float scale) {
     PairOut p;
     if (pairs) {
@@ -977,7 +979,7 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
     a.m = rows; a.n = n_out; a.k = k;
     if (pairs) {
       PairGemmArgs t{};
-      t.x_hi = xp.hi; t.x_lo = xp.lo; t.w_hi = q.hi; t.w_lo = q.lo; t.inv_x = 1.f / xp.scale; t.inv_w = 1.f / q.scale;
+      t.x_hi = xp.hi; t.x_lo = xp.lo; t.w = q.w; t.w_exact = m->pair_exact; t.inv_x = 1.f / xp.scale; t.inv_w = 1.f / q.scale;
       t.bias = bias; t.resid = resid; t.out = outp.hi ? nullptr : out; t.out_hi = outp.hi; t.out_lo = outp.lo; t.out_scale = outp.scale;
       t.error_flag = ws.d_error;
       t.m = rows; t.n = n_out; t.k = k; t.epilogue = epi;

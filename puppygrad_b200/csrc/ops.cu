@@ -56,7 +56,7 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const size_t xs = (size_t)m * k, ws = (size_t)n * k, os = (size_t)m * n;
   float x_scale = 1.f, w_scale = 1.f;  // of the FP16 pairs
-  if (x3_rows) {
+  if (math_mode == PG_MATH_TF32X3) {
     float top = 0.f;
     for (size_t i = 0; i < xs; ++i) top = std::max(top, std::fabs(x[i]));
     x_scale = pair_scale(top);
@@ -95,20 +95,22 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
       cudaError_t e = launch_make_pairs(dx.as<float>(), xp, xp + xs, xs, x_scale, st);
       if (e != cudaSuccess) return e;
       PairGemmArgs p{};
-      p.x_hi = xp; p.x_lo = xp + xs; p.w_hi = wp; p.w_lo = wp + ws; p.inv_x = 1.f / x_scale; p.inv_w = 1.f / w_scale;
+      p.x_hi = xp; p.x_lo = xp + xs; p.w = wp; p.inv_x = 1.f / x_scale; p.inv_w = 1.f / w_scale;
       p.bias = a.bias; p.resid = a.resid; p.out = a.out; p.error_flag = a.error_flag;
       p.m = m; p.n = n; p.k = k; p.epilogue = epilogue;
       return launch_tc_gemm_pair(p, st);
     }
-    cudaError_t e = launch_split_tf32(dx.as<float>(), dhi.as<float>(), dlo.as<float>(), xs, false, st);
-    if (e != cudaSuccess) return e;
     if (chain_ctas > 0) {
+      cudaError_t e = launch_make_pairs(dx.as<float>(), dhi.as<uint16_t>(), dlo.as<uint16_t>(), xs, x_scale, st);
+      if (e != cudaSuccess) return e;
       if (epilogue == EPI_RESID) {
         e = cudaMemcpyAsync(dout.p, dr.p, os * 4, cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) return e;
       }
       return launch_chain(chain, chain_ctas, st);
     }
+    cudaError_t e = launch_split_tf32(dx.as<float>(), dhi.as<float>(), dlo.as<float>(), xs, false, st);
+    if (e != cudaSuccess) return e;
     a.x = dhi.as<float>(); a.x_lo = dlo.as<float>(); a.w = dwt.as<float>();
     a.trace = dtrace.as<unsigned long long>();
     return launch_tc_gemm_x3(a, splits, false, st);
@@ -135,8 +137,8 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
       goto done;
     }
     PG_OP_TRY(cudaMalloc(&dlo.p, xs * 4));
-    PG_OP_TRY(cudaMalloc(&dwlo.p, ws * 4));
-    PG_OP_TRY(launch_make_pairs(dw.as<float>(), dwlo.as<uint16_t>(), dwlo.as<uint16_t>() + ws, ws, w_scale, s));
+    PG_OP_TRY(cudaMalloc(&dwlo.p, pair_tiled_halves(n, k, false) * 2));
+    PG_OP_TRY(launch_tile_pairs(dw.as<float>(), dwlo.as<uint16_t>(), n, k, false, w_scale, s));
   } else if (math_mode == PG_MATH_TF32X3) {
     splits = tc_gemm_x3_splits(n, k, sms);
     PG_OP_TRY(cudaMalloc(&dhi.p, xs * 4));
@@ -147,12 +149,15 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
       const int g = chain_grid(sms);
       chain.n_phases = 2;
       chain.ph[0].kind = CH_GEMM; chain.ph[0].n = n; chain.ph[0].k = k; chain.ph[0].act = CH_ACT_NORM;
-      chain.ph[0].w_block0 = 0;
+      chain.ph[0].w_block0 = 0; chain.ph[0].inv_x = 1.f / x_scale; chain.ph[0].inv_w = 1.f / w_scale;
       chain.ph[1].kind = epilogue == EPI_RESID ? CH_ROWS : CH_ELEM;
       chain.ph[1].n = n; chain.ph[1].k = k; chain.ph[1].bias = db.as<float>();
       chain.ph[1].gelu = epilogue == EPI_GELU; chain.ph[1].x = dout.as<float>(); chain.ph[1].out = dout.as<float>();
-      chain.m = m; chain.eps = 1e-5f; chain.arena = dwt.as<float>(); chain.arena_floats = tc_tiled_weight_floats(n, k);
-      chain.act_hi[0] = dhi.as<float>(); chain.act_lo[0] = dlo.as<float>(); chain.act_k[0] = k;
+      chain.m = m; chain.eps = 1e-5f; chain.arena_halves = pair_tiled_halves(n, k, false);
+      PG_OP_TRY(cudaMalloc(&dwlo.p, chain.arena_halves * 2));
+      PG_OP_TRY(launch_tile_pairs(dw.as<float>(), dwlo.as<uint16_t>(), n, k, false, w_scale, s));
+      chain.arena = dwlo.as<uint16_t>();
+      chain.act_hi[0] = dhi.as<uint16_t>(); chain.act_lo[0] = dlo.as<uint16_t>(); chain.act_k[0] = k;
       chain.error_flag = derr.as<int>();
       PG_OP_TRY(cudaMalloc(&dpart.p, chain_partial_floats(g) * 4));
       PG_OP_TRY(cudaMalloc(&dbar.p, 4));

@@ -23,9 +23,9 @@ namespace pg {
                                     __FILE__ + ":" + std::to_string(__LINE__) + " (" #expr ")"); \
   } while (0)
 
-// A weight matrix as FP16 pairs (gemm_pair.cu), [out, in] row-major; lo nullptr: all zero.
+// A weight matrix [out, in] as tiles of FP16 pairs (gemm_pair.cu).
 struct PairWeights {
-  const uint16_t *hi = nullptr, *lo = nullptr;
+  const uint16_t* w = nullptr;
   float scale = 1.f;
 };
 
@@ -33,8 +33,8 @@ struct LayerWeights {
   float *ln1_g, *ln1_b, *w_qkv, *b_qkv, *w_proj, *b_proj, *ln2_g, *ln2_b, *w_fc, *b_fc, *w_proj2, *b_proj2;
   // copies in the tiled layout of the tensor-core decode kernel (nullptr in fp32 mode)
   float *t_qkv = nullptr, *t_proj = nullptr, *t_fc = nullptr, *t_proj2 = nullptr;
-  // FP16 pairs of the four matrices for FP32-grade products of prompt rows (tf32x3 and bf16 modes), and the scales of the pairs
-  // that their inputs are kept as: LayerNorm and attention outputs, hidden units
+  // FP16 pairs of the four matrices for FP32-grade products on the tensor cores, and the scales of the pairs that their inputs
+  // are kept as: LayerNorm and attention outputs, hidden units
   PairWeights q_qkv, q_proj, q_fc, q_proj2;
   float x_norm1 = 1.f, x_attn = 1.f, x_norm2 = 1.f, x_h = 1.f;
   // packed copies for the single-kernel decode step (BF16 or row-quantised int8 weights), [out, in] rows, and,
@@ -104,7 +104,11 @@ struct pg_model {
   float* tiled_arena = nullptr;  // second copy of the dense matrices, tiled for TMA (tensor-core modes)
   size_t tiled_floats = 0;
   float* t_wte = nullptr;
-  uint16_t* pair_arena = nullptr;  // FP16 pairs of the dense matrices (FP32-grade products of prompt rows)
+  uint16_t* pair_arena = nullptr;  // FP16 pairs of the dense matrices (FP32-grade products)
+  size_t pair_halves = 0;
+  bool pair_exact = false;         // BF16 weights: no lo tiles
+  PairWeights q_wte;
+  float x_normf = 1.f;             // scale of the lm_head's input
   size_t arena_floats = 0;
   int stream_weight_type = STREAM_W_F32;  // what the single-kernel decode step streams
   unsigned char* packed_arena = nullptr;  // BF16 / int8 copies of the dense matrices and of wte
@@ -149,7 +153,7 @@ struct pg_cache {
   unsigned* attn_counters = nullptr;
   float* topk_vals = nullptr;
   int* topk_idx = nullptr;
-  // tensor-core decode path (9..64 sequences): TF32 hi/lo pairs of the GEMM inputs, split-K scratch
+  // tensor-core decode path: pairs of the GEMM inputs (FP16 for the chain kernel, else TF32), split-K scratch
   float *norm_lo = nullptr, *attn_lo = nullptr, *h_lo = nullptr;
   int* d_error = nullptr;
   // persistent chain kernel of the tensor-core decode path: partial tiles, grid-barrier word
@@ -158,8 +162,9 @@ struct pg_cache {
   unsigned long long* d_chain_best = nullptr;  // row arg-max accumulators of the lm_head phase
   unsigned long long* d_chain_trace = nullptr;  // developer aid: only allocated in builds with -DPG_DEV_TRACE
   int chain_ctas = 0;
-  int chain_min_batch = 9;  // smallest batch whose decode step runs as the chain kernel in the tensor-core modes (measured on
-                            // B200, GPT-2 medium, 8 sequences: 1.34 ms as the chain kernel, 1.09 ms as one kernel per operation)
+  // Smallest batch whose decode step runs as the chain kernel: 9 in the FP32-grade modes (8 sequences as the chain kernel / as one
+  // kernel per operation, us: GPT-2 small 511 / 493, medium 1026 / 1052), 5 with BF16 weights (enqueue_decode_step).
+  int chain_min_batch = 9;
   struct ChainProgram {  // whole-step phase list of the persistent chain kernel for one batch size
     ChainPhase* dev = nullptr;            // in device memory (nullptr: this batch size is not supported)
     ChainPhase* dev_argmax_only = nullptr;  // the same list whose lm_head reduce phase keeps the row arg-max but stores no logits

@@ -103,6 +103,11 @@ __device__ __forceinline__ uint32_t umma_idesc_bf16(int m, int n, bool b_mn = fa
   return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// ... and with FP16 operands, both K-major.
+__device__ __forceinline__ uint32_t umma_idesc_f16(int m, int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
 __device__ __forceinline__ void umma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile(
@@ -279,18 +284,23 @@ bool make_map(CUtensorMap* map, const float* ptr, uint64_t rows, uint64_t k, uin
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// 2-D BF16 tensor [rows, k] (k contiguous, k % 8 == 0), box = 64 elements x box_rows, 128-byte swizzle,
+// 2-D tensor [rows, k] of 16-bit floats (k contiguous, k % 8 == 0), box = 64 elements x box_rows, 128-byte swizzle,
 // out-of-range rows and columns read as zero.
-bool make_map_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t k, uint32_t box_rows) {
+bool make_map_16(CUtensorMap* map, CUtensorMapDataType type, const void* ptr, uint64_t rows, uint64_t k, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {k, rows};
   cuuint64_t strides[1] = {k * 2};
   cuuint32_t box[2] = {64, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return fn(map, type, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool make_map_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t k, uint32_t box_rows) {
+  return make_map_16(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, rows, k, box_rows);
+}
+bool make_map_f16(CUtensorMap* map, const uint16_t* ptr, uint64_t rows, uint64_t k, uint32_t box_rows) {
+  return make_map_16(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ptr, rows, k, box_rows);
 }
 
 }  // namespace

@@ -98,6 +98,14 @@ def test_linear_tf32x3_prefill_sized_matches_oracle(oracle, m, n, k, epilogue):
     np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
 
 
+# The token tiles of 16, 32 and 64 at their edges, one k block and a share that crosses row tiles, rows off the 128-row tile.
+@pytest.mark.parametrize("m,n,k", [(1, 130, 64), (16, 2, 3584), (17, 4097, 128), (32, 1000, 1024), (33, 129, 64), (64, 50257, 128)])
+@pytest.mark.parametrize("spread", [0.0, 3.0])
+def test_linear_pairs_of_decode_rows_against_float64(m, n, k, spread):
+    """As test_linear_pairs_against_float64, for the persistent kernel of the decode steps: sums of at most 3584 products."""
+    test_linear_pairs_against_float64(m, n, k, spread)
+
+
 @pytest.mark.parametrize("m,n,k", [(16, 1600, 1600), (64, 6400, 1600), (33, 1600, 6400), (40, 1000, 256)])
 @pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
 def test_linear_tf32x3_one_launch_per_gemm_kernel_matches_oracle(oracle, monkeypatch, m, n, k, epilogue):

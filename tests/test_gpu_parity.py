@@ -881,6 +881,30 @@ def test_narrow_weight_modes_exclude_each_other():
 
 
 # ------------------------------------------------------------------ GPT-2 small prefill, 8 x 1024 (second benchmark config)
+@pytest.mark.parametrize("batch", [5, 8, 16, 17, 33])
+def test_bf16_steps_of_more_than_four_sequences(oracle, batch):
+    """The persistent tensor-core step with the hi parts of the weights alone, at the edges of its token tiles: one launch, the
+    oracle's logits on the rounded weights within the FP32 tolerance (the weights are exact, activations keep 22 bits)."""
+    cfg = synthetic.preset("midi")
+    w = synthetic.perturbed_weights(cfg, 57)
+    g = pg.Gpt2Model(cfg, w, pg.Gpt2CudaConfig(math_mode="bf16"))
+    o = oracle.Model(cfg, synthetic.bf16_rounded_weights(w), threads=4)
+    prompts = [synthetic.uniform_prompt(1300 + i, 3 + (5 * i) % 29, cfg["vocab_size"]) for i in range(batch)]
+    cache = g.new_kv_cache(max_batch=batch)
+    _, cur = g.prefill_batch(prompts, cache)
+    ocaches = [o.new_kv_cache() for _ in prompts]
+    for p, c in zip(prompts, ocaches):
+        o.prefill(p, c)
+    for _ in range(3):
+        n0 = cache.kernel_launches()
+        logits, am, _, _ = g.forward_one_batch(cur, cache, want_logits=True)
+        assert cache.kernel_launches() - n0 == 1
+        ol = np.stack([o.forward_one(int(cur[i]), ocaches[i]) for i in range(batch)])
+        assert_logits_close(logits, ol)
+        assert list(am) == [oracle.argmax_logits(l) for l in ol]
+        cur = am.copy()
+
+
 @pytest.mark.parametrize("math_mode,span_bound", [("fp32", None), ("tf32x3", None), ("tf32", 5e-3), ("bf16", 3e-2)])
 def test_gpt2_small_prefill_8x1024_against_golden(math_mode, span_bound):
     """Eight prompts of 1024 tokens through the batched prefill, final-position logits against the oracle's
