@@ -151,11 +151,10 @@ struct pg_cache {
   int part_stride = 0;
   float* attn_part = nullptr;
   unsigned* attn_counters = nullptr;
-  float* topk_vals = nullptr;
-  int* topk_idx = nullptr;
   // tensor-core decode path: pairs of the GEMM inputs (FP16 for the chain kernel, else TF32), split-K scratch
   float *norm_lo = nullptr, *attn_lo = nullptr, *h_lo = nullptr;
-  int* d_error = nullptr;
+  int* d_results = nullptr;  // what a call copies to the host, in one piece: error word, arg-max of the slots, top-k values, their ids
+  int* d_error = nullptr;    // inside d_results, as is d_argmax
   // persistent chain kernel of the tensor-core decode path: partial tiles, grid-barrier word
   float* chain_partials = nullptr;
   unsigned* d_chain_barrier = nullptr;
