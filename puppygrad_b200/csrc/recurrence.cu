@@ -2,6 +2,7 @@
 // [dim, vdim] FP32 state of every head is read, advanced and written back, with the gates before it and the head norm and
 // output gate after it in the same kernel. Everything that enters the recurrence is FP32.
 #include <algorithm>
+#include <climits>
 
 #include "recurrence.cuh"
 
@@ -9,279 +10,442 @@ namespace pg {
 namespace {
 
 // ------------------------------------------------------------------ one token per sequence
+// Bound by the state, read and written once, and by the instructions around it. A block takes one head of a sequence after
+// another, as many blocks as are resident at a time: while the sums, gates and norms of one state are worked out, the next state
+// (into words that the copying thread reads itself) and what goes with it come into shared memory.
+// 64 sequences, us (one block per item, loads at the start of each): 16 heads of 64 x 128 26.3 -> 23.3 (2.9 TB/s of state), 32 of
+// 64 x 64 34.0 -> 31.6; one sequence, 8 heads of 64 x 128 6.2 -> 4.8.
 constexpr int STEP_THREADS = 256;
 
-template <int NR>
-__global__ void __launch_bounds__(STEP_THREADS) recurrence_step_kernel(RecurrenceStepArgs a, int y_bf16) {
+__device__ __forceinline__ void async_copy4(float4* to_shared, const float* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to_shared)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void async_copy1(float* to_shared, const float* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(to_shared)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void async_copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Four neighbouring values as two packed pairs.
+struct Quad {
+  unsigned long long a, b;
+};
+__device__ __forceinline__ Quad quad(float4 v) { return Quad{pack2(v.x, v.y), pack2(v.z, v.w)}; }
+__device__ __forceinline__ float4 unquad(Quad q) {
+  float4 v;
+  unpack2(q.a, v.x, v.y);
+  unpack2(q.b, v.z, v.w);
+  return v;
+}
+__device__ __forceinline__ Quad fma_quad(float x, Quad y, Quad z) {
+  const unsigned long long x2 = pack2(x, x);
+  return Quad{fma2(x2, y.a, z.a), fma2(x2, y.b, z.b)};
+}
+
+__device__ __host__ inline int pad4(int n) { return (n + 3) & ~3; }
+// Floats of one step's inputs in shared memory: key, query, removal rate, value, gate and low-rank columns.
+__device__ __host__ inline int step_input_floats(const RecurrenceLayer& l) { return 3 * pad4(l.dim) + 2 * l.dvp + pad4(l.rank); }
+inline size_t step_floats(const RecurrenceLayer& l, int buffers) {
+  return (size_t)buffers * step_input_floats(l) + 5 * pad4(l.dim) + 2 * l.dvp + std::max(STEP_THREADS, pad4(l.dim)) +
+         (size_t)(STEP_THREADS / (l.dvp / 4)) * l.dvp;
+}
+
+// An item per block, without the limit on registers that goes with several, or several; STEP_FULL: and every thread owns NR rows
+// and four columns of the state, so that nothing is asked per row.
+enum { STEP_ONE = 0, STEP_MANY = 1, STEP_FULL = 2 };
+constexpr int step_blocks(int nr) { return nr <= 4 ? 4 : nr <= 8 ? 3 : 2; }  // on an SM
+
+template <int NR, int MODE>
+__global__ void __launch_bounds__(STEP_THREADS, MODE != STEP_ONE ? step_blocks(NR) : 1) recurrence_step_kernel(RecurrenceStepArgs a, int y_bf16, int ahead_at) {
+  constexpr bool MANY = MODE != STEP_ONE, FULL = MODE == STEP_FULL;
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[33];
   const RecurrenceLayer& l = a.l;
   const int dk = l.dim, dv = l.vdim, dvp = l.dvp, K = l.heads * dk;
-  const int head = blockIdx.x, seq = blockIdx.y, tid = threadIdx.x;
+  const int tid = threadIdx.x, head = blockIdx.x % l.heads, seq_step = gridDim.x / l.heads;  // the head of all its items
   const bool delta = l.kind == KIND_DELTA;
-  const int dka = (dk + 3) & ~3, rka = (l.rank + 3) & ~3;  // rows of shared memory start on 16-byte boundaries
-  float* ks = sm;            // [dk] key
-  float* ws = ks + dka;      // decay
-  float* qs = ws + dka;      // query (r)
-  float* us = qs + dka;      // unit key
-  float* bs = us + dka;      // a * u
-  float* ts = bs + dka;      // [rank]
-  float* vs = ts + rka;      // [dvp]
-  float* ds = vs + dvp;      // [dvp] u^T S
-  float* os = ds + dvp;      // [dvp]
-  float* zs = os + dvp;      // [max(256, dk)] partial sums of the decay projection
+  const int dka = pad4(dk), in_floats = step_input_floats(l);  // rows of shared memory start on 16-byte boundaries
+  float4* rp = reinterpret_cast<float4*>(sm + (MANY ? 2 : 1) * in_floats);  // [dk] of a row of the state: decay, key, query, a * u
+  float* us = reinterpret_cast<float*>(rp + dka);  // [dk] unit key
+  float* ds = us + dka;            // [dvp] u^T S
+  float* os = ds + dvp;            // [dvp]
+  float* zs = os + dvp;            // [max(256, dk)] partial sums of the decay projection
   float* part = zs + (dk > STEP_THREADS ? dka : STEP_THREADS);  // [KG][dvp]
   const int dv4 = dvp / 4, KG = STEP_THREADS / dv4;
   const int c4 = tid % dv4, kg = tid / dv4;
-  const bool active = kg < KG;
+  const bool active = FULL || kg < KG;
+  const int own = FULL ? INT_MAX : dk;  // rows below are there
+  float4* ahead = reinterpret_cast<float4*>(sm + ahead_at) + tid;  // [NR][STEP_THREADS], this thread's column
+  auto fetch = [&](int seq, float* in) {
+    const float* p = a.p + (size_t)seq * a.ldp;
+    for (int c = tid; c < dk; c += STEP_THREADS) {
+      async_copy1(in + c, p + l.off_k + head * dk + c);
+      async_copy1(in + dka + c, p + l.off_q + head * dk + c);
+      if (delta) async_copy1(in + 2 * dka + c, p + l.off_a + head * dk + c);
+    }
+    for (int c = tid; c < dv; c += STEP_THREADS) {
+      async_copy1(in + 3 * dka + c, p + l.off_v + head * dv + c);
+      async_copy1(in + 3 * dka + dvp + c, p + l.off_g + head * dv + c);
+    }
+    for (int r = tid; r < l.rank; r += STEP_THREADS) async_copy1(in + 3 * dka + 2 * dvp + r, p + l.off_t + r);
+  };
 
+  for (int c = dv + tid; c < dvp; c += STEP_THREADS) {  // padding of the value rows
+    sm[3 * dka + c] = 0.f;
+    if (MANY) sm[in_floats + 3 * dka + c] = 0.f;
+  }
   grid_dep_launch();
   grid_dep_wait();
-  const float* p = a.p + (size_t)seq * a.ldp;
-  const bool fresh = a.pos[seq] == 0;
-  float* S = a.state + ((size_t)seq * l.heads + head) * dk * dvp;
-  constexpr int NRR = NR > 0 ? NR : 1;
-  float4 st[NRR];
-  if (NR > 0) {  // the state's loads overlap the gate arithmetic below
+  const int first = blockIdx.x / l.heads;
+  fetch(first, sm);
+  bool fresh = a.pos[first] == 0;
+  int flip = 0;
+  for (int seq = first; seq < a.batch; seq += seq_step, flip ^= 1) {
+    const int next = MANY ? seq + seq_step : a.batch;
+    const float *ks = sm + flip * in_floats, *qs = ks + dka, *as = qs + dka, *vs = as + dka, *gs = vs + dvp;
+    float* ts = sm + flip * in_floats + 3 * dka + 2 * dvp;
+    float* S = a.state + ((size_t)seq * l.heads + head) * dk * dvp + (size_t)kg * dvp + c4 * 4;  // this thread's first row
+    const size_t pitch = (size_t)KG * dvp;
+    constexpr int NRR = NR > 0 ? NR : 1;
+    Quad st[NRR];
 #pragma unroll
-    for (int i = 0; i < NRR; ++i) {
-      const int r = kg + i * KG;
-      st[i] = (active && !fresh && r < dk) ? load4(S + (size_t)r * dvp + c4 * 4) : make_float4(0, 0, 0, 0);
+    for (int i = 0; i < NRR; ++i) st[i] = Quad{0, 0};
+    const bool stored = active && !fresh;
+    if (NR > 0 && stored && (!MANY || seq == first)) {  // the first state's loads overlap the gate arithmetic below
+#pragma unroll
+      for (int i = 0; i < NRR; ++i)
+        if (kg + i * KG < own) st[i] = quad(load4(S + i * pitch));
     }
-  }
-  for (int r = tid; r < l.rank; r += STEP_THREADS) ts[r] = delta ? tanhf(p[l.off_t + r]) : p[l.off_t + r];
-  float kk = 0.f;
-  for (int c = tid; c < dk; c += STEP_THREADS) {
-    ks[c] = p[l.off_k + head * dk + c];
-    qs[c] = p[l.off_q + head * dk + c];
-    kk += ks[c] * ks[c];
-  }
-  for (int c = tid; c < dvp; c += STEP_THREADS) vs[c] = c < dv ? p[l.off_v + head * dv + c] : 0.f;
-  kk = block_sum(kk, red);  // also orders the shared-memory writes above
-  const float inv_norm = 1.f / sqrtf(kk + UNIT_EPS);
-  // second half of the decay projection: RG threads share a channel, so that its weights arrive in one round trip or two
-  const int RG = dk >= STEP_THREADS ? 1 : STEP_THREADS / dk;
-  for (int i = tid; i < RG * dk; i += STEP_THREADS) {
-    const int c = i % dk, g = i / dk;
-    const float* __restrict__ w2 = l.w2 + head * dk + c;
-    float z = 0.f;
-#pragma unroll 16
-    for (int r = g; r < l.rank; r += RG) z = fmaf(w2[(size_t)r * K], ts[r], z);
-    zs[i] = z;
-  }
-  __syncthreads();
-  for (int c = tid; c < dk; c += STEP_THREADS) {
-    const int ch = head * dk + c;
-    float z = l.b2[ch];
-    for (int g = 0; g < RG; ++g) z += zs[g * dk + c];
-    ws[c] = decay_of(l.kind, z, l.inv_tau);
-    if (delta) {
-      const float u = ks[c] * inv_norm;
-      us[c] = u;
-      bs[c] = sigmoid_f(p[l.off_a + ch] + l.a_bias[ch]) * u;
+    async_copies_done();
+    if (NR > 0 && MANY && stored && seq != first) {
+#pragma unroll
+      for (int i = 0; i < NRR; ++i)
+        if (kg + i * KG < own) st[i] = quad(ahead[i * STEP_THREADS]);
     }
-  }
-  __syncthreads();
-  if (delta) {
-    float4 d = make_float4(0, 0, 0, 0);
-    if (active && !fresh) {
-      for (int i = 0; i < (NR > 0 ? NRR : (dk + KG - 1) / KG); ++i) {
-        const int r = kg + i * KG;
-        if (r >= dk) break;
-        const float4 s = NR > 0 ? st[NR > 0 ? i : 0] : load4(S + (size_t)r * dvp + c4 * 4);
-        const float u = us[r];
-        d.x = fmaf(u, s.x, d.x); d.y = fmaf(u, s.y, d.y); d.z = fmaf(u, s.z, d.z); d.w = fmaf(u, s.w, d.w);
+    if (delta)
+      for (int r = tid; r < l.rank; r += STEP_THREADS) ts[r] = tanhf(ts[r]);  // this thread's copies
+    float kk = 0.f;
+    for (int c = tid; c < dk; c += STEP_THREADS) kk += ks[c] * ks[c];
+    kk = block_sum(kk, red);  // also orders the copies, and the last item's reads of the other buffer before the next ones
+    if (next < a.batch) {
+      fetch(next, sm + (flip ^ 1) * in_floats);
+      if (NR > 0 && active) {
+        const float* from = S + (size_t)seq_step * l.heads * dk * dvp;
+#pragma unroll
+        for (int i = 0; i < NRR; ++i)
+          if (kg + i * KG < own) async_copy4(ahead + i * STEP_THREADS, from + i * pitch);
       }
     }
-    if (active) store4(part + (size_t)kg * dvp + c4 * 4, d);
-    __syncthreads();
-    for (int c = tid; c < dvp; c += STEP_THREADS) {
-      float s = 0.f;
-      for (int g = 0; g < KG; ++g) s += part[(size_t)g * dvp + c];
-      ds[c] = s;
+    const int next_pos = next < a.batch ? a.pos[next] : 0;
+    const float inv_norm = 1.f / sqrtf(kk + UNIT_EPS);
+    // second half of the decay projection: RG threads share a channel, so that its weights arrive in one round trip or two
+    const int RG = dk >= STEP_THREADS ? 1 : STEP_THREADS / dk;
+    for (int i = tid; i < RG * dk; i += STEP_THREADS) {
+      const int c = i % dk, g = i / dk;
+      const float* __restrict__ w2 = l.w2 + head * dk + c;
+      float z = 0.f;
+#pragma unroll 16
+      for (int r = g; r < l.rank; r += RG) z = fmaf(w2[(size_t)r * K], ts[r], z);
+      zs[i] = z;
     }
     __syncthreads();
-  }
-  float4 o = make_float4(0, 0, 0, 0);
-  if (active) {
-    const float4 v = load4(vs + c4 * 4);
-    const float4 d = delta ? load4(ds + c4 * 4) : make_float4(0, 0, 0, 0);
-    for (int i = 0; i < (NR > 0 ? NRR : (dk + KG - 1) / KG); ++i) {
-      const int r = kg + i * KG;
-      if (r >= dk) break;
-      float4 s = NR > 0 ? st[NR > 0 ? i : 0] : (fresh ? make_float4(0, 0, 0, 0) : load4(S + (size_t)r * dvp + c4 * 4));
-      const float w = ws[r], k = ks[r], q = qs[r], b = delta ? bs[r] : 0.f;
-      s.x = fmaf(w, s.x, fmaf(k, v.x, -b * d.x));
-      s.y = fmaf(w, s.y, fmaf(k, v.y, -b * d.y));
-      s.z = fmaf(w, s.z, fmaf(k, v.z, -b * d.z));
-      s.w = fmaf(w, s.w, fmaf(k, v.w, -b * d.w));
-      store4(S + (size_t)r * dvp + c4 * 4, s);
-      o.x = fmaf(q, s.x, o.x); o.y = fmaf(q, s.y, o.y); o.z = fmaf(q, s.z, o.z); o.w = fmaf(q, s.w, o.w);
+    for (int c = tid; c < dk; c += STEP_THREADS) {
+      const int ch = head * dk + c;
+      float z = l.b2[ch];
+      for (int g = 0; g < RG; ++g) z += zs[g * dk + c];
+      float b = 0.f;
+      if (delta) {
+        const float u = ks[c] * inv_norm;
+        us[c] = u;
+        b = sigmoid_f(as[c] + l.a_bias[ch]) * u;
+      }
+      rp[c] = make_float4(decay_of(l.kind, z, l.inv_tau), ks[c], qs[c], b);
     }
-    store4(part + (size_t)kg * dvp + c4 * 4, o);
-  }
-  __syncthreads();
-  float sq = 0.f;
-  for (int c = tid; c < dv; c += STEP_THREADS) {
-    float s = 0.f;
-    for (int g = 0; g < KG; ++g) s += part[(size_t)g * dvp + c];
-    s *= l.q_scale;
-    os[c] = s;
-    sq += s * s;
-  }
-  sq = block_sum(sq, red);
-  const float rinv = 1.f / sqrtf(sq / (float)dv + l.eps);
-  for (int c = tid; c < dv; c += STEP_THREADS) {
-    const float g = p[l.off_g + head * dv + c];
-    const float gate = delta ? sigmoid_f(g) : silu_f(g);
-    const float y = os[c] * rinv * l.norm[delta ? head * dv + c : c] * gate * l.out_scale;
-    const size_t i = (size_t)seq * a.ldy + head * dv + c;
-    if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[i] = __float2bfloat16_rn(y);
-    else static_cast<float*>(a.y)[i] = y;
+    __syncthreads();
+    const int count = NR > 0 ? NRR : (dk + KG - 1) / KG;
+    if (delta) {
+      Quad d = {0, 0};
+      if (stored) {
+#pragma unroll
+        for (int i = 0; i < count; ++i) {
+          const int r = kg + i * KG;
+          if (r >= own) break;
+          d = fma_quad(us[r], NR > 0 ? st[NR > 0 ? i : 0] : quad(load4(S + i * pitch)), d);
+        }
+      }
+      if (active) store4(part + (size_t)kg * dvp + c4 * 4, unquad(d));
+      __syncthreads();
+      for (int c = tid; c < dvp; c += STEP_THREADS) {
+        float sum = 0.f;
+#pragma unroll 8
+        for (int g = 0; g < KG; ++g) sum += part[(size_t)g * dvp + c];
+        ds[c] = sum;
+      }
+      __syncthreads();
+    }
+    if (active) {
+      const Quad v = quad(load4(vs + c4 * 4)), d = delta ? quad(load4(ds + c4 * 4)) : Quad{0, 0}, zero = {0, 0};
+      Quad o = {0, 0};
+#pragma unroll
+      for (int i = 0; i < count; ++i) {
+        const int r = kg + i * KG;
+        if (r >= own) break;
+        const float4 row = rp[r];
+        Quad x = NR > 0 ? st[NR > 0 ? i : 0] : fresh ? Quad{0, 0} : quad(load4(S + i * pitch));
+        x = fma_quad(row.x, x, fma_quad(row.y, v, delta ? fma_quad(-row.w, d, zero) : zero));
+        store4(S + i * pitch, unquad(x));
+        o = fma_quad(row.z, x, o);
+      }
+      store4(part + (size_t)kg * dvp + c4 * 4, unquad(o));
+    }
+    __syncthreads();
+    float sq = 0.f;
+    for (int c = tid; c < dv; c += STEP_THREADS) {
+      float sum = 0.f;
+#pragma unroll 8
+      for (int g = 0; g < KG; ++g) sum += part[(size_t)g * dvp + c];
+      sum *= l.q_scale;
+      os[c] = sum;
+      sq += sum * sum;
+    }
+    sq = block_sum(sq, red);
+    const float rinv = 1.f / sqrtf(sq / (float)dv + l.eps);
+    for (int c = tid; c < dv; c += STEP_THREADS) {
+      const float gate = delta ? sigmoid_f(gs[c]) : silu_f(gs[c]);
+      const float y = os[c] * rinv * l.norm[delta ? head * dv + c : c] * gate * l.out_scale;
+      const size_t at = (size_t)seq * a.ldy + head * dv + c;
+      if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[at] = __float2bfloat16_rn(y);
+      else static_cast<float*>(a.y)[at] = y;
+    }
+    fresh = next_pos == 0;
   }
 }
 
 // ------------------------------------------------------------------ channel delta rule
-// Block = one head of one sequence. A thread owns four columns of NR rows of the state (NR = 0: it is read twice instead). The
-// unit lengths of k and q are factors of sums, so that the rows go on as they leave the convolutions.
+// Block = one head of a sequence, then of another, as in recurrence_step_kernel. A thread owns four columns of NR rows of the
+// state (NR = 0: it is read twice instead). The unit lengths of k and q are factors of sums, so that the rows go on as they leave
+// the convolutions.
+// 64 sequences, 16 heads of 128 x 128: 46 -> 41 us (3.2 TB/s; DRAM 22% busy and half of the issue slots taken in the former kernel).
 constexpr int CH_THREADS = 512, CH_WARPS = CH_THREADS / 32;
 
-template <int NR>
-__global__ void __launch_bounds__(CH_THREADS, NR > 0 && NR <= 8 ? 2 : 1) channel_step_kernel(RecurrenceStepArgs a, int y_bf16) {
+// Floats of one step's inputs in shared memory: `taps` rows of key, query and value inputs, decay and gate columns, write strength.
+__device__ __host__ inline int channel_input_floats(const RecurrenceLayer& l) { return l.taps * (2 * l.dim + l.vdim) + l.dim + l.vdim + 1; }
+inline size_t channel_floats(const RecurrenceLayer& l, int buffers) {
+  return 4 * (size_t)pad4(l.dim) + l.dvp + (size_t)(CH_THREADS / (l.dvp / 4)) * l.dvp + (size_t)buffers * channel_input_floats(l);
+}
+constexpr int channel_blocks(int nr) { return nr > 0 && nr <= 8 ? 2 : 1; }
+
+template <int NR, int MODE>
+__global__ void __launch_bounds__(CH_THREADS, channel_blocks(NR)) channel_step_kernel(RecurrenceStepArgs a, int y_bf16, int ahead_at) {
+  constexpr bool MANY = MODE != STEP_ONE, FULL = MODE == STEP_FULL;
   extern __shared__ __align__(16) float sm[];
-  __shared__ float red[CH_WARPS], lengths[2];
+  __shared__ float red[CH_WARPS], lengths[3];  // of key and query; write strength
   const RecurrenceLayer& l = a.l;
-  const int dk = l.dim, dv = l.vdim, dvp = l.dvp, dka = (dk + 3) & ~3, rep = l.heads / l.kv_heads;
-  const int head = blockIdx.x, seq = blockIdx.y, kv = head / rep, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float* ks = sm;         // [dk] key
-  float* qs = ks + dka;   // query
-  float* ws = qs + dka;   // decay
-  float* vs = ws + dka;   // [dvp] value, then what is written
-  float* part = vs + dvp; // [KG][dvp]
+  const int dk = l.dim, dv = l.vdim, dvp = l.dvp, dka = pad4(dk), rep = l.heads / l.kv_heads;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, head = blockIdx.x % l.heads, seq_step = gridDim.x / l.heads, kv = head / rep;
   const int dv4 = dvp / 4, KG = CH_THREADS / dv4, c4 = tid % dv4, kg = tid / dv4;
-  const bool active = kg < KG;
-  float* S = a.state + ((size_t)seq * l.heads + head) * dk * dvp;
+  const bool active = FULL || kg < KG;
+  const int own = FULL ? INT_MAX : dk;   // rows below are there
+  float* rp = sm;                        // [dk][4] of a row of the state: decay, key, query, unused
+  float* vs = rp + 4 * dka;              // [dvp] value, then what is written
+  float* part = vs + dvp;                // [KG][dvp]
+  float* inputs = part + (size_t)KG * dvp;
+  const int rows = 2 * dk + dv, in_floats = channel_input_floats(l);
+  float4* ahead = reinterpret_cast<float4*>(sm + ahead_at) + tid;  // [NR][CH_THREADS], this thread's column
+  // column j of an input row: key, query, value
+  auto column = [&](int j) { return j < dk ? l.off_k + kv * dk + j : j < 2 * dk ? l.off_q + kv * dk + j - dk : l.off_v + head * dv + j - 2 * dk; };
+  auto fetch = [&](int seq, int slot, float* in) {
+    const float *p = a.p + (size_t)seq * a.ldp, *z = a.z + (size_t)seq * a.ldz, *taps = a.taps + (size_t)seq * l.taps * l.channels;
+    for (int j = tid; j < rows; j += CH_THREADS) {
+      const int col = column(j);
+      async_copy1(in + j, p + col);
+      const float* past = taps + (size_t)slot * l.channels + col - l.off_q;
+      for (int back = 1, at = slot; back < l.taps; ++back) {
+        past += at == 0 ? (l.taps - 1) * l.channels : -l.channels;
+        at = at == 0 ? l.taps - 1 : at - 1;
+        async_copy1(in + back * rows + j, past);
+      }
+    }
+    in += l.taps * rows;
+    for (int j = tid; j < dk + dv + 1; j += CH_THREADS)
+      async_copy1(in + j, j < dk ? z + head * dk + j : j < dk + dv ? z + l.heads * dk + head * dv + j - dk : p + l.off_b + head);
+  };
 
   grid_dep_launch();
   grid_dep_wait();
-  constexpr int NRR = NR > 0 ? NR : 1;
-  float4 st[NRR];
-  if (NR > 0) {  // the state's loads overlap everything up to its first use
+  const int first = blockIdx.x / l.heads;
+  int pos = a.pos[first], slot = pos % l.taps, flip = 0;
+  fetch(first, slot, inputs);
+  int next_pos = MANY && first + seq_step < a.batch ? a.pos[first + seq_step] : 0;
+  for (int seq = first; seq < a.batch; seq += seq_step, flip ^= 1) {
+    const int next = MANY ? seq + seq_step : a.batch;
+    const float *in = inputs + flip * in_floats, *zs = in + l.taps * rows;  // [dk] decay, [dv] gate, write strength
+    float* S = a.state + ((size_t)seq * l.heads + head) * dk * dvp + (size_t)kg * dvp + c4 * 4;  // this thread's first row
+    const size_t pitch = (size_t)KG * dvp;
+    const bool fresh = pos == 0, stored = active && !fresh;
+    constexpr int NRR = NR > 0 ? NR : 1;
+    Quad st[NRR];
 #pragma unroll
-    for (int i = 0; i < NRR; ++i) {
-      const int r = kg + i * KG;
-      st[i] = active && r < dk ? load4(S + (size_t)r * dvp + c4 * 4) : make_float4(0, 0, 0, 0);
-    }
-  }
-  const float* p = a.p + (size_t)seq * a.ldp;
-  const float* z = a.z + (size_t)seq * a.ldz;
-  const int pos = a.pos[seq], slot = pos % l.taps;
-  const bool fresh = pos == 0;
-  float* taps = a.taps + (size_t)seq * l.taps * l.channels;
-  for (int i = tid; i < 3 * dk + dvp; i += CH_THREADS) {
-    if (i < dk) {  // decay
-      ws[i] = channel_decay(l, head, head * dk + i, z[head * dk + i]);
-      continue;
-    }
-    const int j = i - dk;
-    const bool is_k = j < dk, is_q = !is_k && j < 2 * dk;
-    const int c = is_k ? j : is_q ? j - dk : j - 2 * dk;
-    if (!is_k && !is_q && c >= dv) {
-      vs[c] = 0.f;
-      continue;
-    }
-    const int col = is_k ? l.off_k + kv * dk + c : is_q ? l.off_q + kv * dk + c : l.off_v + head * dv + c, ch = col - l.off_q;
-    const float now = p[col];
-    float x = 0.f;
-    for (int back = l.taps - 1; back > 0; --back) {
-      const int at = slot - back < 0 ? slot - back + l.taps : slot - back;
-      const float past = taps[(size_t)at * l.channels + ch];
-      if (pos >= back) x = fmaf(l.conv[(size_t)(l.taps - 1 - back) * l.channels + ch], past, x);
-    }
-    x = silu_f(fmaf(l.conv[(size_t)(l.taps - 1) * l.channels + ch], now, x));
-    (is_k ? ks : is_q ? qs : vs)[c] = x;
-    // the input is cached where no token that still matters lies; one block per group caches the shared q and k
-    if (head % rep == 0 || (!is_k && !is_q)) taps[(size_t)slot * l.channels + ch] = now;
-  }
-  const float beta = sigmoid_f(p[l.off_b + head]);
-  __syncthreads();
-  if (warp >= CH_WARPS - 2) {  // squared lengths
-    const float* x = warp == CH_WARPS - 1 ? qs : ks;
-    float s = 0.f;
-    for (int c = lane; c < dk; c += 32) s += x[c] * x[c];
-    s = lane_sum(s);
-    if (lane == 0) lengths[warp - (CH_WARPS - 2)] = 1.f / sqrtf(s + UNIT_EPS);
-  }
-  auto state = [&](int i, int r) { return fresh ? make_float4(0, 0, 0, 0) : NR > 0 ? st[i] : load4(S + (size_t)r * dvp + c4 * 4); };
-  const int count = NR > 0 ? NRR : (dk + KG - 1) / KG;
-  float4 d = make_float4(0, 0, 0, 0);
-  if (active) {
+    for (int i = 0; i < NRR; ++i) st[i] = Quad{0, 0};
+    if (NR > 0 && stored && (!MANY || seq == first)) {  // the first state's loads overlap everything up to its first use
 #pragma unroll
-    for (int i = 0; i < count; ++i) {
-      const int r = kg + i * KG;
-      if (r < dk) {
-        const float4 s = state(NR > 0 ? i : 0, r);
-        const float u = ws[r] * ks[r];
-        d.x = fmaf(u, s.x, d.x); d.y = fmaf(u, s.y, d.y); d.z = fmaf(u, s.z, d.z); d.w = fmaf(u, s.w, d.w);
+      for (int i = 0; i < NRR; ++i)
+        if (kg + i * KG < own) st[i] = quad(load4(S + i * pitch));
+    }
+    async_copies_done();
+    if (NR > 0 && MANY && stored && seq != first) {
+#pragma unroll
+      for (int i = 0; i < NRR; ++i)
+        if (kg + i * KG < own) st[i] = quad(ahead[i * CH_THREADS]);
+    }
+    float* taps = a.taps + ((size_t)seq * l.taps + slot) * l.channels;
+    for (int c = dv + tid; c < dvp; c += CH_THREADS) vs[c] = 0.f;
+    for (int j = tid; j < rows; j += CH_THREADS) {  // this thread's copies
+      const int ch = column(j) - l.off_q;
+      const float now = in[j];
+      float x = 0.f;
+      for (int back = l.taps - 1; back > 0; --back)
+        if (pos >= back) x = fmaf(l.conv[(size_t)(l.taps - 1 - back) * l.channels + ch], in[back * rows + j], x);
+      x = silu_f(fmaf(l.conv[(size_t)(l.taps - 1) * l.channels + ch], now, x));
+      (j < dk ? rp + 4 * j + 1 : j < 2 * dk ? rp + 4 * (j - dk) + 2 : vs + j - 2 * dk)[0] = x;
+      // the input is cached where no token that still matters lies; one block per group caches the shared q and k
+      if (head % rep == 0 || j >= 2 * dk) taps[ch] = now;
+    }
+    __syncthreads();  // also the copies of the other threads, and the last item's reads of the other buffer before the next ones
+    pos = next_pos;
+    slot = pos % l.taps;
+    if (next < a.batch) {
+      fetch(next, slot, inputs + (flip ^ 1) * in_floats);
+      if (NR > 0 && active) {
+        const float* from = S + (size_t)seq_step * l.heads * dk * dvp;
+#pragma unroll
+        for (int i = 0; i < NRR; ++i)
+          if (kg + i * KG < own) async_copy4(ahead + i * CH_THREADS, from + i * pitch);
       }
+      next_pos = next + seq_step < a.batch ? a.pos[next + seq_step] : 0;
     }
-    store4(part + (size_t)kg * dvp + c4 * 4, d);
-  }
-  __syncthreads();
-  const float ki = lengths[0], qi = lengths[1];
-  for (int c = tid; c < dvp; c += CH_THREADS) {
-    float s = 0.f;
-    for (int g = 0; g < KG; ++g) s += part[(size_t)g * dvp + c];
-    vs[c] = beta * ki * (vs[c] - ki * s);
-  }
-  __syncthreads();
-  if (active) {
-    const float4 v = load4(vs + c4 * 4);
-    float4 o = make_float4(0, 0, 0, 0);
+    for (int c = tid; c < dk; c += CH_THREADS) rp[4 * c] = channel_decay(l, head, head * dk + c, zs[c]);
+    if (warp >= CH_WARPS - 2) {  // squared lengths
+      const int at = warp == CH_WARPS - 1 ? 2 : 1;
+      float sum = 0.f;
+      for (int c = lane; c < dk; c += 32) sum += rp[4 * c + at] * rp[4 * c + at];
+      sum = lane_sum(sum);
+      if (lane == 0) lengths[at - 1] = 1.f / sqrtf(sum + UNIT_EPS);
+    } else if (warp == CH_WARPS - 3 && lane == 0) {
+      lengths[2] = sigmoid_f(zs[dk + dv]);
+    }
+    __syncthreads();
+    const int count = NR > 0 ? NRR : (dk + KG - 1) / KG;
+    const float4* rows4 = reinterpret_cast<const float4*>(rp);
+    if (active) {
+      Quad d = {0, 0};
+      if (stored) {
 #pragma unroll
-    for (int i = 0; i < count; ++i) {
-      const int r = kg + i * KG;
-      if (r < dk) {
-        float4 s = state(NR > 0 ? i : 0, r);
-        const float w = ws[r], k = ks[r], q = qs[r];
-        s.x = fmaf(w, s.x, k * v.x); s.y = fmaf(w, s.y, k * v.y); s.z = fmaf(w, s.z, k * v.z); s.w = fmaf(w, s.w, k * v.w);
-        store4(S + (size_t)r * dvp + c4 * 4, s);
-        o.x = fmaf(q, s.x, o.x); o.y = fmaf(q, s.y, o.y); o.z = fmaf(q, s.z, o.z); o.w = fmaf(q, s.w, o.w);
+        for (int i = 0; i < count; ++i) {
+          const int r = kg + i * KG;
+          if (r >= own) break;
+          const float4 row = rows4[r];
+          d = fma_quad(row.x * row.y, NR > 0 ? st[NR > 0 ? i : 0] : quad(load4(S + i * pitch)), d);
+        }
       }
+      store4(part + (size_t)kg * dvp + c4 * 4, unquad(d));
     }
-    store4(part + (size_t)kg * dvp + c4 * 4, o);
-  }
-  __syncthreads();
-  float out = 0.f;  // one column per thread: dv <= CH_THREADS
-  if (tid < dv) {
-    for (int g = 0; g < KG; ++g) out += part[(size_t)g * dvp + tid];
-    out *= qi * l.q_scale;
-  }
-  const float sq = lane_sum(out * out);
-  if (lane == 0) red[warp] = sq;
-  __syncthreads();
-  if (tid < dv) {
-    float total = 0.f;
+    __syncthreads();
+    const float ki = lengths[0], qi = lengths[1], beta = lengths[2];
+    for (int c = tid; c < dvp; c += CH_THREADS) {
+      float sum = 0.f;
+#pragma unroll 8
+      for (int g = 0; g < KG; ++g) sum += part[(size_t)g * dvp + c];
+      vs[c] = beta * ki * (vs[c] - ki * sum);
+    }
+    __syncthreads();
+    if (active) {
+      const Quad v = quad(load4(vs + c4 * 4)), zero = {0, 0};
+      Quad o = {0, 0};
 #pragma unroll
-    for (int i = 0; i < CH_WARPS; ++i) total += red[i];
-    const float y = out / sqrtf(total / (float)dv + l.eps) * l.norm[tid] * sigmoid_f(z[l.heads * dk + head * dv + tid]) * l.out_scale;
-    const size_t at = (size_t)seq * a.ldy + head * dv + tid;
-    if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[at] = __float2bfloat16_rn(y);
-    else static_cast<float*>(a.y)[at] = y;
+      for (int i = 0; i < count; ++i) {
+        const int r = kg + i * KG;
+        if (r >= own) break;
+        const float4 row = rows4[r];
+        Quad x = NR > 0 ? st[NR > 0 ? i : 0] : fresh ? Quad{0, 0} : quad(load4(S + i * pitch));
+        x = fma_quad(row.x, x, fma_quad(row.y, v, zero));
+        store4(S + i * pitch, unquad(x));
+        o = fma_quad(row.z, x, o);
+      }
+      store4(part + (size_t)kg * dvp + c4 * 4, unquad(o));
+    }
+    __syncthreads();
+    float out = 0.f;  // one column per thread: dv <= CH_THREADS
+    if (tid < dv) {
+#pragma unroll 8
+      for (int g = 0; g < KG; ++g) out += part[(size_t)g * dvp + tid];
+      out *= qi * l.q_scale;
+    }
+    const float sq = lane_sum(out * out);
+    if (lane == 0) red[warp] = sq;
+    __syncthreads();
+    if (tid < dv) {
+      float total = 0.f;
+#pragma unroll
+      for (int i = 0; i < CH_WARPS; ++i) total += red[i];
+      const float y = out / sqrtf(total / (float)dv + l.eps) * l.norm[tid] * sigmoid_f(zs[dk + tid]) * l.out_scale;
+      const size_t at = (size_t)seq * a.ldy + head * dv + tid;
+      if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[at] = __float2bfloat16_rn(y);
+      else static_cast<float*>(a.y)[at] = y;
+    }
   }
+}
+
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 148;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) v = 148;
+    return v;
+  }();
+  return n;
+}
+
+// As many blocks as are resident at `per_sm` an SM, where there are more items than that and the kernel keeps the state in
+// registers (NR > 0): a multiple of the heads then, since a block stays with one head. Else a block per item.
+typedef void (*StepKernel)(RecurrenceStepArgs, int, int);
+template <int NR, int THREADS>
+cudaError_t launch_step(StepKernel one, StepKernel some, StepKernel full, const RecurrenceStepArgs& a, int per_sm, int yb, bool pdl, cudaStream_t s) {
+  const RecurrenceLayer& l = a.l;
+  auto floats = [&](int buffers) { return l.kind == KIND_CHANNEL ? channel_floats(l, buffers) : step_floats(l, buffers); };
+  const int items = l.heads * a.batch, resident = per_sm * sm_count() / l.heads * l.heads;
+  const size_t smem = floats(1) * sizeof(float), ahead = (floats(2) + 3) / 4 * 16, bytes = ahead + (size_t)NR * THREADS * 16;
+  const bool single = NR == 0 || resident == 0 || items <= resident || bytes > (size_t)227 * 1024 / per_sm - 1024;
+  const StepKernel many = l.dim == NR * (THREADS / (l.dvp / 4)) && THREADS % (l.dvp / 4) == 0 ? full : some;
+  if (!single || smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(single ? one : many, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(single ? smem : bytes));
+    if (e != cudaSuccess) return e;
+  }
+  if (single) return launch_kernel(one, dim3(items), dim3(THREADS), smem, s, pdl, a, yb, 0);
+  return launch_kernel(many, dim3(resident), dim3(THREADS), bytes, s, pdl, a, yb, (int)(ahead / sizeof(float)));
+}
+
+template <int NR>
+cudaError_t launch_channel(const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {
+  constexpr int SOME = NR == 0 ? STEP_ONE : STEP_MANY, FULL = NR == 0 ? STEP_ONE : STEP_FULL;
+  return launch_step<NR, CH_THREADS>(channel_step_kernel<NR, STEP_ONE>, channel_step_kernel<NR, SOME>, channel_step_kernel<NR, FULL>, a,
+                                     channel_blocks(NR), yb, pdl, s);
+}
+template <int NR>
+cudaError_t launch_gated(const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {
+  constexpr int SOME = NR == 0 ? STEP_ONE : STEP_MANY, FULL = NR == 0 ? STEP_ONE : STEP_FULL;
+  return launch_step<NR, STEP_THREADS>(recurrence_step_kernel<NR, STEP_ONE>, recurrence_step_kernel<NR, SOME>, recurrence_step_kernel<NR, FULL>, a,
+                                       step_blocks(NR), yb, pdl, s);
 }
 
 cudaError_t launch_channel_step(const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {
   const RecurrenceLayer& l = a.l;
   const int kg = CH_THREADS / (l.dvp / 4), nr = (l.dim + kg - 1) / kg;
   if (l.dvp > CH_THREADS) return cudaErrorInvalidValue;
-  const size_t smem = ((size_t)3 * ((l.dim + 3) & ~3) + l.dvp + (size_t)kg * l.dvp) * sizeof(float);
-  const dim3 grid(l.heads, a.batch), block(CH_THREADS);
-  if (nr <= 2) return launch_kernel(channel_step_kernel<2>, grid, block, smem, s, pdl, a, yb);
-  if (nr <= 4) return launch_kernel(channel_step_kernel<4>, grid, block, smem, s, pdl, a, yb);
-  if (nr <= 8) return launch_kernel(channel_step_kernel<8>, grid, block, smem, s, pdl, a, yb);
-  if (nr <= 16) return launch_kernel(channel_step_kernel<16>, grid, block, smem, s, pdl, a, yb);
-  return launch_kernel(channel_step_kernel<0>, grid, block, smem, s, pdl, a, yb);
+  if (nr <= 2) return launch_channel<2>(a, yb, pdl, s);
+  if (nr <= 4) return launch_channel<4>(a, yb, pdl, s);
+  if (nr <= 8) return launch_channel<8>(a, yb, pdl, s);
+  if (nr <= 16) return launch_channel<16>(a, yb, pdl, s);
+  return launch_channel<0>(a, yb, pdl, s);
 }
 
 }  // namespace
@@ -293,13 +457,11 @@ cudaError_t launch_recurrence_step(const RecurrenceStepArgs& a, bool y_bf16, boo
   if (l.kind == KIND_CHANNEL) return launch_channel_step(a, y_bf16 ? 1 : 0, pdl, s);
   const int dv4 = l.dvp / 4, kg = STEP_THREADS / dv4, nr = (l.dim + kg - 1) / kg;
   if (dv4 > STEP_THREADS) return cudaErrorInvalidValue;
-  const size_t smem = ((size_t)5 * ((l.dim + 3) & ~3) + ((l.rank + 3) & ~3) + 3 * (size_t)l.dvp + std::max(STEP_THREADS, (l.dim + 3) & ~3) + (size_t)kg * l.dvp) * sizeof(float);
-  const dim3 grid(l.heads, a.batch), block(STEP_THREADS);
   const int yb = y_bf16 ? 1 : 0;
-  if (nr <= 4) return launch_kernel(recurrence_step_kernel<4>, grid, block, smem, s, pdl, a, yb);
-  if (nr <= 8) return launch_kernel(recurrence_step_kernel<8>, grid, block, smem, s, pdl, a, yb);
-  if (nr <= 16) return launch_kernel(recurrence_step_kernel<16>, grid, block, smem, s, pdl, a, yb);
-  return launch_kernel(recurrence_step_kernel<0>, grid, block, smem, s, pdl, a, yb);
+  if (nr <= 4) return launch_gated<4>(a, yb, pdl, s);
+  if (nr <= 8) return launch_gated<8>(a, yb, pdl, s);
+  if (nr <= 16) return launch_gated<16>(a, yb, pdl, s);
+  return launch_gated<0>(a, yb, pdl, s);
 }
 
 }  // namespace pg

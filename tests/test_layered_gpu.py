@@ -12,7 +12,7 @@ import puppygrad_b200 as pg
 from puppygrad_b200 import trace
 from tests import layered_cases as cases
 from tests import layered_oracle as lo
-from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, row_errors, run_portions
+from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, many_sequences, row_errors, run_portions
 
 pytestmark = pytest.mark.gpu
 
@@ -49,6 +49,23 @@ ALONE = {
     "feed-forward": lo.config(67, 48, [lo.gla(1, 4, 4, ff=136)]),
     "eps": lo.config(67, 48, [lo.gla(2, 8, 8), lo.pair(2, 1, 8, 8, 9, 2, 8, ff=16)], eps=0.3),
 }
+
+
+# More (sequence, head) states than blocks are resident at a time, so that a block takes several and copies the next one ahead: heads
+# that divide the number of resident blocks and ones that do not, four to sixteen rows of the state per thread, odd sizes.
+MANY = {
+    "gla-16": lo.config(61, 48, [lo.gla(16, 16, 24)]),
+    "gla-11-odd": lo.config(61, 50, [lo.gla(11, 7, 9)]),
+    "gla-10-wide": lo.config(61, 48, [lo.gla(10, 64, 128)]),
+    "gla-5-wider": lo.config(61, 48, [lo.gla(5, 128, 128)]),
+    "delta-13": lo.config(61, 48, [lo.pair(1, 1, 8, 8, 5, 13, 64, left_scale=0.0)]),
+    "delta-8-wide": lo.config(61, 48, [lo.pair(1, 1, 8, 8, 5, 8, 96, left_scale=0.0)]),
+}
+
+
+@pytest.mark.parametrize("name", MANY)
+def test_steps_of_many_sequences(name):
+    many_sequences(Case(MANY[name], 7, rank=9))
 
 
 @pytest.mark.parametrize("mode", MODES)

@@ -9,7 +9,7 @@ import puppygrad_b200 as pg
 from puppygrad_b200 import trace
 from tests import layered_cases as cases
 from tests import sanesun_oracle as so
-from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, row_errors, run_portions
+from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, many_sequences, row_errors, run_portions
 
 pytestmark = pytest.mark.gpu
 
@@ -70,6 +70,13 @@ ALONE = {
     "latent-1000": so.latent(3, 128, 256, 1000, 48),
     "feed-forward": so.delta(1, 1, 4, 4, 2, ff=136),
 }
+
+
+# More states than blocks are resident at a time (see test_layered_gpu.py): two to sixteen rows of the state per thread.
+@pytest.mark.parametrize("layer", [so.delta(6, 2, 16, 24, 4), so.delta(7, 7, 7, 9, 3), so.delta(6, 3, 128, 128, 4), so.delta(3, 1, 128, 256, 3),
+                                   so.delta(5, 5, 72, 40, 1)])
+def test_steps_of_many_sequences(layer):
+    many_sequences(Case(so.config(61, 50, [layer]), 7, rank=9))
 
 
 @pytest.mark.parametrize("mode", MODES)
