@@ -74,6 +74,9 @@ __device__ __host__ inline ChRange chain_range(int n, int k, int cta, int grid, 
   // one block more per CTA when that makes shares line up with row tiles: fewer partial tiles to
   // write and to add, at the price of a few idle SMs
   if (nkb % per != 0 && nkb % (per + 1) == 0) per += 1;
+  // a share is two units at least: half the partial tiles to write, acknowledge and add outweigh a unit's 0.3 us (the attention's
+  // output projection of GPT-2 medium, 64 sequences: 1392 -> 1382 us per step; 8 965 -> 954; small, 16 sequences 499 -> 493)
+  if (per == 1 && nkb % 2 == 0) per = 2;
   if (whole_tiles) per = nkb * ((tiles + grid - 1) / grid);
   ChRange r;
   r.nkb = nkb;
