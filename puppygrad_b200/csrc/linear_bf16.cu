@@ -42,7 +42,7 @@ __device__ __forceinline__ float group_sum(float v, float* red, int warp, int la
 template <int MT>
 __global__ void __launch_bounds__(RL_THREADS, 1) rows_linear_kernel(RowsLinearArgs a, int kp_shift, int kpad) {
   extern __shared__ __align__(16) float xs[];  // [MT][kpad] in act_slot order
-  __shared__ float part[RL_WARPS][RL_ROWS * MT];
+  __shared__ float part[2][RL_WARPS][RL_ROWS * MT];  // by turns, so that a round needs one barrier
   __shared__ float red[RL_WARPS];
   __shared__ float best_v[RL_WARPS * RL_ROWS * MT];
   __shared__ int best_i[RL_WARPS * RL_ROWS * MT];
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(RL_THREADS, 1) rows_linear_kernel(RowsLinearAr
 #pragma unroll
     for (int i = 0; i < RL_ROWS * MT; ++i) acc[i] = 0.f;
     for (int st = s0; st < s1; st += RL_PRE) {
-      if (st != s0 || round > 0) request(unit, st);
+      if (st != s0) request(unit, st);
 #pragma unroll
       for (int j = 0; j < RL_PRE; ++j) {
         if (st + j < s1) {
@@ -159,16 +159,18 @@ __global__ void __launch_bounds__(RL_THREADS, 1) rows_linear_kernel(RowsLinearAr
         }
       }
     }
+    // the next round's first weights are on their way while this one is added up
+    if ((round + 1) * upc * (int)gridDim.x + (int)blockIdx.x < units) request(unit + upc * (int)gridDim.x, s0);
 #pragma unroll
     for (int i = 0; i < RL_ROWS * MT; ++i) {
       acc[i] = lane_sum(acc[i]);
-      if (lane == 0) part[warp][i] = acc[i];
+      if (lane == 0) part[round & 1][warp][i] = acc[i];
     }
     __syncthreads();
     for (int i = tid; i < upc * RL_ROWS * MT; i += RL_THREADS) {
       const int uu = i / (RL_ROWS * MT), e = i % (RL_ROWS * MT), r = e / MT, m = e % MT;
       float v = 0.f;
-      for (int q = 0; q < kparts; ++q) v += part[uu * kparts + q][e];
+      for (int q = 0; q < kparts; ++q) v += part[round & 1][uu * kparts + q][e];
       const int row = ((round * upc + uu) * (int)gridDim.x + (int)blockIdx.x) * RL_ROWS + r;
       if (row < a.n && m < a.m) {
         if (row >= a.act_from) a.out_act[(size_t)m * a.ldo_act + row - a.act_from] = activate(a.act, v);
@@ -179,7 +181,6 @@ __global__ void __launch_bounds__(RL_THREADS, 1) rows_linear_kernel(RowsLinearAr
         }
       }
     }
-    __syncthreads();
   }
   if (!a.part_val) return;
   // i % MT is the activation row of thread i in every round (RL_THREADS is a multiple of MT)
