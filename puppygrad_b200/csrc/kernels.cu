@@ -690,6 +690,8 @@ template <int VEC>
 __global__ void kv_scatter_kernel(const float* __restrict__ qkv, const int* __restrict__ row_slot,
                                   const int* __restrict__ row_pos, float* __restrict__ pool,
                                   const int* __restrict__ page_table, KvLayout kv, int rows) {
+  pdl_launch();
+  pdl_wait();
   const int c = kv.n_head * kv.head_dim;
   const int per_row = 2 * c / VEC;
   const size_t total = (size_t)rows * per_row;
@@ -960,6 +962,8 @@ __global__ void __launch_bounds__(128) prefill_attention_kernel(PrefillAttnArgs 
   const int h = blockIdx.x, qb = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
   const int c = a.n_head * D;
+  pdl_launch();
+  pdl_wait();
   const int r0 = a.seq_start[b], len = a.seq_start[b + 1] - r0;
   const int q0 = qb * PA_Q;
   if (q0 >= len) return;
@@ -1515,10 +1519,10 @@ cudaError_t launch_decode_attention(const DecodeAttnArgs& a, bool pdl, cudaStrea
   return launch(kern, dim3(a.kv.n_head, a.batch, 1), dim3(ATT_THREADS), smem, s, pdl, a);
 }
 
-cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, cudaStream_t s) {
+cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, bool pdl, cudaStream_t s) {
   if (a.head_dim == 64) {
     dim3 grid(a.n_head, (a.max_len + PA_Q - 1) / PA_Q, a.batch);
-    prefill_attention_kernel<64><<<grid, 128, PA_SMEM, s>>>(a);
+    return launch(prefill_attention_kernel<64>, grid, dim3(128), PA_SMEM, s, pdl, a);
   } else {
     if (a.head_dim > 128) return cudaErrorInvalidValue;
     dim3 grid(a.n_head, (a.max_len + 63) / 64, a.batch);
@@ -1528,15 +1532,13 @@ cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, cudaStream_t s) {
 }
 
 cudaError_t launch_kv_scatter(const float* qkv, const int* row_slot, const int* row_pos, float* kv_pool,
-                              const int* page_table, KvLayout kv, int rows, cudaStream_t s) {
+                              const int* page_table, KvLayout kv, int rows, bool pdl, cudaStream_t s) {
   const int vec = kv.head_dim % 4 == 0 ? 4 : 1;
   const size_t total = (size_t)rows * (2 * kv.n_head * kv.head_dim / vec);
   const unsigned blocks = std::max(1u, (unsigned)std::min<size_t>((total + 255) / 256, (size_t)148 * 16));
   if (vec == 4)
-    kv_scatter_kernel<4><<<blocks, 256, 0, s>>>(qkv, row_slot, row_pos, kv_pool, page_table, kv, rows);
-  else
-    kv_scatter_kernel<1><<<blocks, 256, 0, s>>>(qkv, row_slot, row_pos, kv_pool, page_table, kv, rows);
-  return cudaGetLastError();
+    return launch(kv_scatter_kernel<4>, dim3(blocks), dim3(256), 0, s, pdl, qkv, row_slot, row_pos, kv_pool, page_table, kv, rows);
+  return launch(kv_scatter_kernel<1>, dim3(blocks), dim3(256), 0, s, pdl, qkv, row_slot, row_pos, kv_pool, page_table, kv, rows);
 }
 
 cudaError_t launch_kv_gather(const float* kv_pool, const int* page_table, KvLayout kv, int slot, int seq_len,

@@ -77,7 +77,7 @@ struct PrefillAttnArgs {
   const int* seq_start;  // [batch + 1] row offsets
   int n_head, head_dim, batch, max_len;
 };
-cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, cudaStream_t s);
+cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, bool pdl, cudaStream_t s);
 // The same attention with TF32 products on the tensor cores (head_dim 64; used by the TF32 prefill mode).
 // rows = rows of the QKV matrix; error_flag receives a code when a bounded wait runs out.
 bool prefill_attention_tc_supported(const PrefillAttnArgs& a);
@@ -87,7 +87,7 @@ cudaError_t launch_prefill_attention_x3(const PrefillAttnArgs& a, int rows, int*
 cudaError_t init_attn_tc_attributes();
 // Copies K,V of every prompt row into the paged cache.
 cudaError_t launch_kv_scatter(const float* qkv, const int* row_slot, const int* row_pos, float* kv_pool,
-                              const int* page_table, KvLayout kv, int rows, cudaStream_t s);
+                              const int* page_table, KvLayout kv, int rows, bool pdl, cudaStream_t s);
 // Reads one slot's K,V of one layer back in [head][n_positions][head_dim] order.
 cudaError_t launch_kv_gather(const float* kv_pool, const int* page_table, KvLayout kv, int slot, int seq_len,
                              int n_positions, float* keys, float* values, cudaStream_t s);

@@ -330,7 +330,7 @@ static int build_model(const pg_gpt2_config& cfg, const float* const* tensors, c
     PG_CUDA_TRY(cudaDeviceSynchronize());
   }
   // BF16 mode: everything that is not the single-kernel step multiplies the rounded FP32 values, on the tensor
-  // cores as three TF32 products where the FP32-grade mode would
+  // cores as pairs of FP16 numbers where the FP32-grade mode would
   const bool tc_modes = be.math_mode != PG_MATH_FP32;
   if (tc_modes && C % 32 == 0 && F % 32 == 0) {
     const int V = (int)cfg.vocab_size;
@@ -962,6 +962,9 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
   // FP32-grade products on the tensor cores read FP16 pairs; whoever produces an input (LayerNorm, attention, the GELU
   // epilogue of the MLP's first product) writes pairs instead of FP32, into the same buffer: [rows, k] hi, then lo.
   const bool pairs = m->pair_arena && m->backend.math_mode != PG_MATH_TF32 && ws.d_error && rows >= 128 && m->head_dim() == 64 && C <= 4096;
+  // A prompt of a few rows is a chain of launches of 2 to 10 us: the next one's blocks come up, and its first weights, while the last
+  // one ends (11 rows of GPT-2 small: 897 -> 785 us). Larger ones gain nothing.
+  const bool pdl = m->use_pdl && rows <= 16;
   auto pair_of = [&](float* buf, int k, float scale) {
     PairOut p;
     if (pairs) {
@@ -991,18 +994,18 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
       t.m = rows; t.n = n_out; t.k = k; t.epilogue = epi;
       return launch_tc_gemm_tf32(t, s);
     }
-    return launch_linear_rows(a, epi, false, s);
+    return launch_linear_rows(a, epi, pdl, s);
   };
   static const bool no_tc_attn = getenv("PG_NO_TC_ATTN") != nullptr;
   for (int l = 0; l < m->layers_n(); ++l) {
     const LayerWeights& w = m->layers[l];
     const PairOut n1 = pair_of(ws.norm, C, w.x_norm1), at = pair_of(ws.attn, C, w.x_attn), n2 = pair_of(ws.norm, C, w.x_norm2),
                   hp = pair_of(ws.h, F, w.x_h), none;
-    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln1_g, w.ln1_b, eps, ws.norm, rows, C, false, s, n1));
+    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln1_g, w.ln1_b, eps, ws.norm, rows, C, pdl, s, n1));
     PG_CUDA_TRY(gemm(w.w_qkv, w.q_qkv, w.b_qkv, ws.norm, n1, ws.qkv, none, 3 * C, C, EPI_NONE, nullptr));
     if (cache)
       PG_CUDA_TRY(launch_kv_scatter(ws.qkv, ws.d_slot, ws.d_pos, cache->layer_pool(l), cache->tables[0].d_table, cache->kv,
-                                    rows, s));
+                                    rows, pdl, s));
     PrefillAttnArgs pa{};
     pa.qkv = ws.qkv; pa.out = ws.attn; pa.pair = at; pa.seq_start = ws.d_seq_start;
     pa.n_head = m->heads(); pa.head_dim = m->head_dim(); pa.batch = plan.batch; pa.max_len = plan.max_len;
@@ -1011,9 +1014,9 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
     else if (pairs && !no_tc_attn && prefill_attention_tc_supported(pa))
       PG_CUDA_TRY(launch_prefill_attention_x3(pa, rows, ws.d_error, s));
     else
-      PG_CUDA_TRY(launch_prefill_attention(pa, s));
+      PG_CUDA_TRY(launch_prefill_attention(pa, pdl, s));
     PG_CUDA_TRY(gemm(w.w_proj, w.q_proj, w.b_proj, ws.attn, at, ws.x, none, C, C, EPI_RESID, ws.x));
-    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln2_g, w.ln2_b, eps, ws.norm, rows, C, false, s, n2));
+    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln2_g, w.ln2_b, eps, ws.norm, rows, C, pdl, s, n2));
     PG_CUDA_TRY(gemm(w.w_fc, w.q_fc, w.b_fc, ws.norm, n2, ws.h, hp, F, C, EPI_GELU, nullptr));
     PG_CUDA_TRY(gemm(w.w_proj2, w.q_proj2, w.b_proj2, ws.h, hp, ws.x, none, C, F, EPI_RESID, ws.x));
   }
