@@ -473,7 +473,7 @@ def run_ours(args):
             "config": {"workload": f"gpt2-{MODEL} fp32, {total} sequences in total ({B} per GPU, sequence i on GPU i mod {world}), "
                                    f"{PROMPT_LEN}-token prompts, greedy decode; step = one decode step of every sequence "
                                    f"({total} tokens)",
-                       "linears": ("fp32 weights and activations; products as 3xTF32 on tcgen05 tensor cores, "
+                       "linears": ("fp32 weights and activations; products as pairs of FP16 numbers on tcgen05 tensor cores, "
                                    "FP32 accumulate" if args.math == "tf32x3" and B > 8 else "fp32 CUDA-core FMA"),
                        "step_kernels": ("ONE persistent kernel per step: embedding, all layers, lm_head, arg-max, "
                                         "token feedback" if launches == K else f"{launches // K} kernels per step in a CUDA graph"),
@@ -520,8 +520,8 @@ def main():
     ap.add_argument("--seqs", type=int, default=TOTAL_SEQS,
                     help="sequences in total (default 64, the benchmark workload; smaller for profiler captures)")
     ap.add_argument("--math", default="tf32x3", choices=["fp32", "tf32x3"],
-                    help="arithmetic of decode linears of 9..64 sequences per GPU: fp32 = CUDA-core FMA, tf32x3 = three TF32 "
-                         "tensor-core products with FP32 accumulation (FP32-grade, token-exact against the oracle)")
+                    help="arithmetic of decode linears of 9..64 sequences per GPU: fp32 = CUDA-core FMA, tf32x3 = three FP16 "
+                         "tensor-core products of hi and lo parts with FP32 accumulation (FP32-grade, token-exact against the oracle)")
     ap.add_argument("--no-xl", action="store_true", help="skip the GPT-2 XL sampling line under `also`")
     ap.add_argument("--no-also", action="store_true", help="skip every line under `also` but the weak-scaling one")
     ap.add_argument("--skip-extras", action="store_true",

@@ -55,15 +55,14 @@ typedef struct {
 typedef enum {
   PG_MATH_FP32 = 0,   /* FP32 FMA everywhere */
   PG_MATH_TF32X3 = 1, /* FP32-grade products on the tensor cores as three MMAs over hi and lo parts of both
-                         operands (x.w + x.w_lo + x_lo.w) with FP32 accumulation: TF32 parts in the decode linears of
-                         9..64 sequences, FP16 parts of scaled values (22 bits together, no larger error) in prefill
-                         GEMMs of at least 128 rows; passes the same token-exact and
+                         operands (x.w + x.w_lo + x_lo.w) with FP32 accumulation, FP16 parts of scaled values (22 bits
+                         together): the decode linears of 9..64 sequences and prefill GEMMs of at least 128 rows; passes the same token-exact and
                          1e-3 / 1e-4 logit tests as PG_MATH_FP32. Everything else as PG_MATH_FP32 */
   PG_MATH_TF32 = 2,   /* as TF32X3 for decode; prefill GEMMs of at least 128 rows and prefill attention
                          (head_dim 64) as single TF32 passes: a speed mode, bound 5e-3 of the logit span */
   PG_MATH_BF16 = 3    /* BF16 WEIGHTS, FP32 activations and sums: the four dense matrices of every block and the
                          tied embedding are rounded to BF16 (nearest even) at load; what the model computes is
-                         the FP32 path of the reference on those rounded weights. Decode steps of at most 8
+                         the FP32 path of the reference on those rounded weights. Decode steps of at most 4
                          sequences stream the 2-byte copies; prefill and larger batches multiply the rounded
                          values as PG_MATH_TF32X3 does. No reference counterpart (it rejects every dtype but F32,
                          src/models/safetensors.rs:126-130) */
