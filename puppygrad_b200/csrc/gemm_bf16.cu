@@ -470,16 +470,15 @@ cudaError_t launch_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
 
 template <int BN>
 cudaError_t launch_rows_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
-  // As many parts of k as give every SM a block, each of at least two k blocks, at most a portable cluster's eight. A decode step
-  // of 64 sequences of width 2048 (in products of 49, 16, 64 and 16 row tiles) with 4 / 6 / 8 parts at most, ms of 24 steps and
-  // prompts: Dirurax 27.8 / 27.3 / 27.0, Sanesun 25.3 / 24.7 / 24.5. Powers of two up to four, blocks of 176 KB, peers' sums
-  // pushed into a buffer of their own: 28.3 and 26.1. Alone, 16.8 MB (n 2048, k 4096) take 10.8 us, 33.6 MB 15.
-  // Up to four parts also where that gives an SM two blocks, because one block's ring does not keep enough bytes in flight (us,
-  // one / two blocks per SM: 115 row tiles of k 2048 20.3 / 17.1, 88 20.4 / 14.9, 64 13.0 / 10.7; more than four parts lose: 49 row
-  // tiles in three / six 10.5 / 15.5). Dirurax 26.8 -> 26.3, Sanesun 24.3 -> 23.5.
-  const int row_tiles = (a.n + TILE_M - 1) / TILE_M, heads = std::max(a.heads, 1), nkb = (a.k + KB - 1) / KB;
-  const int one = sm_count() / (row_tiles * heads), two = 2 * sm_count() / (row_tiles * heads);  // parts at one and two blocks per SM
-  const int splits = std::max(1, std::min({8, std::max(one, std::min(two, 4)), nkb / 2}));
+  // Parts of k: a power of two that gives every SM at most one block, each part of at least two k blocks; eight only where the matrix
+  // has eight row tiles or fewer. The parts are where a sum is rounded, and so which way BF16 results behind it fall: up to eight parts, or
+  // four where that gives an SM two blocks, are faster (steps of 64 sequences of width 2048 with their prompts, 24 of them: Dirurax
+  // 25.9 instead of 27.3 ms, Sanesun 23.1 instead of 24.8), but 0.4% off in what a model says. Blocks of 176 KB with the sums pushed into
+  // a buffer of their peers: 30.2 and 27.5 ms.
+  const int row_tiles = (a.n + TILE_M - 1) / TILE_M, heads = std::max(a.heads, 1), nkb = (a.k + KB - 1) / KB, tiles = row_tiles * heads;
+  const int most = tiles <= 8 ? 8 : 4;
+  int splits = 1;
+  while (splits < most && tiles * splits * 2 <= sm_count() && splits * 4 <= nkb) splits *= 2;
   CUtensorMap mx, mw;
   if (!make_map_bf16(&mx, a.x, a.m, a.heads ? a.ldx : a.k, BN) || !make_map_bf16(&mw, a.w_tiled, (uint64_t)heads * row_tiles * (a.k / KB) * TILE_M, KB, TILE_M))
     return cudaErrorInvalidValue;

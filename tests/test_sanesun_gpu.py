@@ -417,6 +417,32 @@ def test_profiles_and_sizes(mixed):
     assert model.state_bytes_per_sequence() == want
 
 
+# ------------------------------------------------------------------ the parts of k that a product of decode rows is summed in
+@pytest.mark.parametrize("vocab,parts", [(1024, 8), (1025, 4), (37 * 128, 4), (37 * 128 + 1, 2), (74 * 128, 2), (74 * 128 + 1, 1)])
+def test_parts_of_a_sum(vocab, parts):
+    """The output matrix (k = 4096) of 9 and 40 sequences whose final rows are ones. A row of it adds 1, 2^30 and -2^30: 0 within one part,
+    whose FP32 sum loses the 1, and 1 where the 1 lies in another part. First, last and middle parts by turns."""
+    k, size = 4096, 4096 // parts
+    where, want = [], []
+    for v in range(vocab):
+        base = v // 2 % parts * size
+        apart = v % 2 and parts > 1
+        where.append((base if not apart else (base + size) % k, base + size - 40, base + size - 1))
+        want.append(1.0 if apart else 0.0)
+
+    def edit(w):
+        for name in w:
+            w[name][:] = 0.0 if name in ("l0.mix.o", "head") else 1.0 if name in ("embed", "final.norm") else w[name]
+        for value, at in zip((1.0, 2.0 ** 30, -2.0 ** 30), np.array(where).T):
+            w["head"][np.arange(vocab), at] = value
+
+    model = Case(so.config(vocab, k, [so.delta(1, 1, 4, 4, 2)]), 5, edit=edit).model("bf16")
+    for n in (9, 40):
+        cache = model.new_kv_cache(n)
+        rows = [model.prefill_batch([[7]] * n, cache, want_logits=True)[0], model.forward_one_batch([7] * n, cache, want_logits=True)[0]]
+        np.testing.assert_array_equal(np.concatenate(rows), np.tile(want, (2 * n, 1)))
+
+
 # ------------------------------------------------------------------ sizes past one tile of every product
 @pytest.fixture(scope="module")
 def wide():
