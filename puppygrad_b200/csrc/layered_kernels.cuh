@@ -133,6 +133,7 @@ struct RecurrenceStepArgs {  // one new token for slots 0..batch-1
   int batch;
 };
 cudaError_t launch_recurrence_step(const RecurrenceStepArgs& a, bool y_bf16, bool pdl, cudaStream_t s);
+cudaError_t init_recurrence_step_attributes();
 struct RecurrenceScanArgs {  // whole portions of `nseq` sequences
   RecurrenceLayer l;
   const float* p;        // [rows, ldp]

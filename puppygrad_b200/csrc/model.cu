@@ -20,6 +20,7 @@
 #include "design.h"
 #include "kernels.cuh"
 #include "layered.h"
+#include "layered_kernels.cuh"
 #include "runtime.h"
 #include "sampler.h"
 
@@ -127,6 +128,7 @@ int ensure_device(int device) {
     PG_CUDA_TRY(init_tc_kernel_attributes());
     PG_CUDA_TRY(init_pair_gemm_attributes());
     PG_CUDA_TRY(init_attn_tc_attributes());
+    PG_CUDA_TRY(init_recurrence_step_attributes());
     g_device_inited[device] = true;
   }
   return PG_OK;

@@ -405,50 +405,67 @@ int sm_count() {
   return n;
 }
 
-// As many blocks as are resident at `per_sm` an SM, where there are more items than that and the kernel keeps the state in
-// registers (NR > 0): a multiple of the heads then, since a block stays with one head. Else a block per item.
+// Shared memory of a block where `per_sm` of them share an SM (of 228 KB, 1 KB of it taken with every block).
+constexpr size_t step_smem_limit(int per_sm) { return (size_t)227 * 1024 / per_sm - 1024; }
+
+// The instances that hold NR rows of the state per thread.
 typedef void (*StepKernel)(RecurrenceStepArgs, int, int);
-template <int NR, int THREADS>
-cudaError_t launch_step(StepKernel one, StepKernel some, StepKernel full, const RecurrenceStepArgs& a, int per_sm, int yb, bool pdl, cudaStream_t s) {
-  const RecurrenceLayer& l = a.l;
-  auto floats = [&](int buffers) { return l.kind == KIND_CHANNEL ? channel_floats(l, buffers) : step_floats(l, buffers); };
-  const int items = l.heads * a.batch, resident = per_sm * sm_count() / l.heads * l.heads;
-  const size_t smem = floats(1) * sizeof(float), ahead = (floats(2) + 3) / 4 * 16, bytes = ahead + (size_t)NR * THREADS * 16;
-  const bool single = NR == 0 || resident == 0 || items <= resident || bytes > (size_t)227 * 1024 / per_sm - 1024;
-  const StepKernel many = l.dim == NR * (THREADS / (l.dvp / 4)) && THREADS % (l.dvp / 4) == 0 ? full : some;
-  if (!single || smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(single ? one : many, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(single ? smem : bytes));
-    if (e != cudaSuccess) return e;
-  }
-  if (single) return launch_kernel(one, dim3(items), dim3(THREADS), smem, s, pdl, a, yb, 0);
-  return launch_kernel(many, dim3(resident), dim3(THREADS), bytes, s, pdl, a, yb, (int)(ahead / sizeof(float)));
+struct StepKernels {
+  StepKernel one, some, full;
+  int nr, threads, per_sm;
+};
+template <int NR>
+StepKernels channel_kernels() {
+  constexpr int SOME = NR == 0 ? STEP_ONE : STEP_MANY, FULL = NR == 0 ? STEP_ONE : STEP_FULL;
+  return {channel_step_kernel<NR, STEP_ONE>, channel_step_kernel<NR, SOME>, channel_step_kernel<NR, FULL>, NR, CH_THREADS, channel_blocks(NR)};
+}
+template <int NR>
+StepKernels gated_kernels() {
+  constexpr int SOME = NR == 0 ? STEP_ONE : STEP_MANY, FULL = NR == 0 ? STEP_ONE : STEP_FULL;
+  return {recurrence_step_kernel<NR, STEP_ONE>, recurrence_step_kernel<NR, SOME>, recurrence_step_kernel<NR, FULL>, NR, STEP_THREADS, step_blocks(NR)};
 }
 
-template <int NR>
-cudaError_t launch_channel(const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {
-  constexpr int SOME = NR == 0 ? STEP_ONE : STEP_MANY, FULL = NR == 0 ? STEP_ONE : STEP_FULL;
-  return launch_step<NR, CH_THREADS>(channel_step_kernel<NR, STEP_ONE>, channel_step_kernel<NR, SOME>, channel_step_kernel<NR, FULL>, a,
-                                     channel_blocks(NR), yb, pdl, s);
-}
-template <int NR>
-cudaError_t launch_gated(const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {
-  constexpr int SOME = NR == 0 ? STEP_ONE : STEP_MANY, FULL = NR == 0 ? STEP_ONE : STEP_FULL;
-  return launch_step<NR, STEP_THREADS>(recurrence_step_kernel<NR, STEP_ONE>, recurrence_step_kernel<NR, SOME>, recurrence_step_kernel<NR, FULL>, a,
-                                       step_blocks(NR), yb, pdl, s);
+// As many blocks as are resident at `per_sm` an SM, where there are more items than that and the kernel keeps the state in
+// registers (nr > 0): a multiple of the heads then, since a block stays with one head. Else a block per item. Whole steps, us, a block
+// per item and several, from the first number of sequences past residency on: Dirurax of width 2048 (592 blocks of the delta rule, 432 of
+// the gated one) 19 627 / 607, 27 663 / 632, 28 689 / 602, 64 966 / 795; of width 1024 38 466 / 446, 64 550 / 465; Sanesun of width
+// 2048 (288 blocks) 19 572 / 557, 32 592 / 587, 37 629 / 644, 64 750 / 732.
+cudaError_t launch_step(const StepKernels& k, const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {
+  const RecurrenceLayer& l = a.l;
+  auto floats = [&](int buffers) { return l.kind == KIND_CHANNEL ? channel_floats(l, buffers) : step_floats(l, buffers); };
+  const int items = l.heads * a.batch, resident = k.per_sm * sm_count() / l.heads * l.heads;
+  const size_t smem = floats(1) * sizeof(float), ahead = (floats(2) + 3) / 4 * 16, bytes = ahead + (size_t)k.nr * k.threads * 16;
+  if (k.nr == 0 || resident == 0 || items <= resident || bytes > step_smem_limit(k.per_sm))
+    return launch_kernel(k.one, dim3(items), dim3(k.threads), smem, s, pdl, a, yb, 0);
+  const bool full = l.dim == k.nr * (k.threads / (l.dvp / 4)) && k.threads % (l.dvp / 4) == 0;
+  return launch_kernel(full ? k.full : k.some, dim3(resident), dim3(k.threads), bytes, s, pdl, a, yb, (int)(ahead / sizeof(float)));
 }
 
 cudaError_t launch_channel_step(const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {
   const RecurrenceLayer& l = a.l;
   const int kg = CH_THREADS / (l.dvp / 4), nr = (l.dim + kg - 1) / kg;
   if (l.dvp > CH_THREADS) return cudaErrorInvalidValue;
-  if (nr <= 2) return launch_channel<2>(a, yb, pdl, s);
-  if (nr <= 4) return launch_channel<4>(a, yb, pdl, s);
-  if (nr <= 8) return launch_channel<8>(a, yb, pdl, s);
-  if (nr <= 16) return launch_channel<16>(a, yb, pdl, s);
-  return launch_channel<0>(a, yb, pdl, s);
+  if (nr <= 2) return launch_step(channel_kernels<2>(), a, yb, pdl, s);
+  if (nr <= 4) return launch_step(channel_kernels<4>(), a, yb, pdl, s);
+  if (nr <= 8) return launch_step(channel_kernels<8>(), a, yb, pdl, s);
+  if (nr <= 16) return launch_step(channel_kernels<16>(), a, yb, pdl, s);
+  return launch_step(channel_kernels<0>(), a, yb, pdl, s);
 }
 
 }  // namespace
+
+// The limits on shared memory belong to the kernels, which layers, models and threads share: they are set once, to the most that a
+// layer of any size asks for.
+cudaError_t init_recurrence_step_attributes() {
+  for (const StepKernels& k : {channel_kernels<2>(), channel_kernels<4>(), channel_kernels<8>(), channel_kernels<16>(), channel_kernels<0>(),
+                               gated_kernels<4>(), gated_kernels<8>(), gated_kernels<16>(), gated_kernels<0>()}) {
+    cudaError_t e = cudaFuncSetAttribute(k.one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem_limit(1));
+    if (e == cudaSuccess && k.nr > 0) e = cudaFuncSetAttribute(k.some, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem_limit(k.per_sm));
+    if (e == cudaSuccess && k.nr > 0) e = cudaFuncSetAttribute(k.full, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)step_smem_limit(k.per_sm));
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
 
 size_t recurrence_state_floats(const RecurrenceLayer& l) { return (size_t)l.heads * l.dim * l.dvp; }
 
@@ -458,10 +475,10 @@ cudaError_t launch_recurrence_step(const RecurrenceStepArgs& a, bool y_bf16, boo
   const int dv4 = l.dvp / 4, kg = STEP_THREADS / dv4, nr = (l.dim + kg - 1) / kg;
   if (dv4 > STEP_THREADS) return cudaErrorInvalidValue;
   const int yb = y_bf16 ? 1 : 0;
-  if (nr <= 4) return launch_gated<4>(a, yb, pdl, s);
-  if (nr <= 8) return launch_gated<8>(a, yb, pdl, s);
-  if (nr <= 16) return launch_gated<16>(a, yb, pdl, s);
-  return launch_gated<0>(a, yb, pdl, s);
+  if (nr <= 4) return launch_step(gated_kernels<4>(), a, yb, pdl, s);
+  if (nr <= 8) return launch_step(gated_kernels<8>(), a, yb, pdl, s);
+  if (nr <= 16) return launch_step(gated_kernels<16>(), a, yb, pdl, s);
+  return launch_step(gated_kernels<0>(), a, yb, pdl, s);
 }
 
 }  // namespace pg

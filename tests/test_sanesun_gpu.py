@@ -1,6 +1,7 @@
 """GPU tests of the Sanesun design against its plain FP64 restatement (sanesun_oracle.py): each mechanism alone, prompts
 against decoding, portions, batches, reuse of pages and slots, edges of windows and pages, generation."""
 import io
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -77,6 +78,40 @@ ALONE = {
                                    so.delta(5, 5, 72, 40, 1)])
 def test_steps_of_many_sequences(layer):
     many_sequences(Case(so.config(61, 50, [layer]), 7, rank=9))
+
+
+# One kernel with two sizes of shared memory in one model: heads of 128 x 128 behind four and behind three taps.
+def test_steps_of_many_sequences_through_layers_of_different_sizes():
+    many_sequences(Case(so.config(61, 50, [so.delta(6, 3, 128, 128, 4), so.delta(6, 3, 128, 128, 3)]), 7, rank=9))
+
+
+def test_threads_that_step_layers_of_different_sizes():
+    """The same two sizes in two models, each stepped by a thread of its own, launch by launch."""
+    n, steps, runs = 61, 40, []
+    for taps in (4, 3):
+        case = Case(so.config(61, 50, [so.delta(6, 3, 128, 128, taps)]), 7, rank=9)
+        model = case.model("fp32", use_graphs=False)
+        runs.append((model, model.new_kv_cache(max_batch=n), [case.ids(steps, seed=i) for i in range(n)]))
+
+    def step(model, cache, ids):
+        cache.clear()
+        return np.stack([model.forward_one_batch([x[t] for x in ids], cache, want_logits=True)[0] for t in range(steps)])
+
+    alone = [step(*run) for run in runs]
+    with ThreadPoolExecutor(2) as pool:
+        together = list(pool.map(lambda run: step(*run), runs))
+    for a, b in zip(alone, together):
+        np.testing.assert_array_equal(a, b)
+
+
+# A block's inputs to within a few bytes of 48 KB (38 taps), and the most that a layer can have (64 taps, heads of 256 x 256).
+@pytest.mark.parametrize("layer", [so.delta(2, 1, 16, 224, 38), so.delta(1, 1, 256, 256, 64)])
+def test_steps_with_many_taps(layer):
+    case = Case(so.config(61, 50, [layer]), 7, rank=9)
+    ids = case.ids(80)
+    model = case.model("fp32")
+    rows = run_portions(model, model.new_kv_cache(1), 0, [ids[:70]] + [[t] for t in ids[70:]])
+    assert_rows(rows, case.want(ids), "fp32")
 
 
 @pytest.mark.parametrize("mode", MODES)
