@@ -239,7 +239,8 @@ template <int MT>
 cudaError_t launch_q8_smem(const int8_t* q, const float* scales, const float* bias, const float* x, float* out, int m,
                            int n, int k, int sms, cudaStream_t s) {
   const size_t smem = (size_t)MT * k * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(linear_q8_smem_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit belongs to the kernel, which threads share: always the same one
+  cudaError_t e = cudaFuncSetAttribute(linear_q8_smem_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Q8_MAX_SMEM);
   if (e != cudaSuccess) return e;
   const int blocks = std::max(1, std::min((n + 63) / 64, sms));  // 32 warps of two rows each
   linear_q8_smem_kernel<MT><<<blocks, 1024, smem, s>>>(q, scales, bias, x, out, m, n, k);
