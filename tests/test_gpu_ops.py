@@ -63,24 +63,35 @@ def test_linear_tf32x3_matches_oracle(oracle, m, n, k, epilogue):
     np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
 
 
+def hi_part(a):
+    """Rounded to the 11 significant bits of an FP16 number."""
+    m, e = np.frexp(a)
+    return np.ldexp(np.round(m * 2048), e - 11)
+
+
 # Row and column counts off the 128 x 128 tile (65, 129; n 1, 2, 130), k that ends inside a block of 64 (32, 96), the first
 # length that is summed in two chunks (57 blocks); columns of very different size and rows that are all zero.
 @pytest.mark.parametrize("m,n,k", [(65, 130, 32), (129, 2, 96), (128, 1, 64), (257, 129, 512), (130, 40, 57 * 64)])
 @pytest.mark.parametrize("spread", [0.0, 3.0])
 def test_linear_pairs_against_float64(m, n, k, spread):
     """Products of FP16 pairs. Each operand is held to 2^-22 of its size (three terms of that) where it is not below 2^-28
-    of the matrix' largest value (there: 2^-50 of that value), and sums of at most 3584 products are truncated once per 16 of
-    them: 2^-23 of the sum of absolute products each time. Chunks and the rest of the epilogue: another 2^-22."""
+    of the matrix' largest value (there: 2^-50 of that value); chunks and the rest of the epilogue: another 2^-22. Sums of at most
+    3584 products are truncated once per 16 of them: 2^-23 of the partial sum each time, which for products of random sign is
+    within six times the root of their squares. Without the lo parts of one operand a product is further off than that."""
     rng = np.random.default_rng(m * 17 + n * 3 + k)
     x = rng.standard_normal((m, k)) * np.exp(spread * rng.standard_normal(k))
     w = rng.standard_normal((n, k)) * np.exp(-spread * rng.standard_normal(k)) * 1e-3
-    x[m // 2] = 0
+    if m > 1:
+        x[m // 2] = 0
     x, w = x.astype(np.float32), w.astype(np.float32)
     got, _ = ops.linear(x, w, math_mode="tf32x3")
     x, w = x.astype(np.float64), w.astype(np.float64)
-    size = np.abs(x) @ np.abs(w).T
+    size, root = np.abs(x) @ np.abs(w).T, np.sqrt((x * x) @ (w * w).T)
     floor = 2.0 ** -50 * (np.abs(x).max() * np.abs(w).sum(1)[None, :] + np.abs(w).max() * np.abs(x).sum(1)[:, None])
-    assert (np.abs(got - x @ w.T) <= (4 * 2.0 ** -22 + min(k, 3584) / 16 * 2.0 ** -23) * size + floor).all()
+    bound = 4 * 2.0 ** -22 * size + min(k, 3584) / 16 * 2.0 ** -23 * np.minimum(size, 6 * root) + floor
+    assert (np.abs(got - x @ w.T) <= bound).all()
+    for without in (hi_part(x) @ w.T, x @ hi_part(w).T):
+        assert (np.abs(without - x @ w.T) > bound).any()
 
 
 @pytest.mark.parametrize("m,n,k", [(128, 1600, 1600), (512, 4800, 1600), (300, 1600, 6400), (1000, 777, 256)])
