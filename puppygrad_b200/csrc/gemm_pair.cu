@@ -9,10 +9,15 @@
 // the bytes per value of the FP32 words that three TF32 products read. The scales put a bound of |v| at 2^14..2^15, so nothing
 // overflows: the largest |w| of a matrix, and for activations what a LayerNorm, a convex combination of value rows or a
 // product of a LayerNorm's row can reach (pair_scale, set when the weights are loaded). Everything within 2^-28 of the bound
-// keeps its 22 bits; below that the error stays under 2^-50 of the bound.
+// keeps its 22 bits; below that the error stays under 2^-50 of the bound. Whether that takes anything from a model is found out
+// when it is loaded: how well pairs hold the rows of its weights (launch_pair_fit), and whether a bound is out of proportion to
+// what the other columns can reach (PAIR_SPREAD). A model that fails either, or has weights that are not finite, goes without pairs.
+// Splitting FP32 into FP16 parts with a scaled rest: Ootomo and Yokota, "Recovering single precision accuracy from Tensor Cores
+// while surpassing the FP32 theoretical peak performance", 2022.
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 
 #include "kernels.cuh"
@@ -25,7 +30,7 @@ namespace {
 constexpr int PK = 64;   // FP16 elements per k block: one 128-byte swizzle row
 constexpr int PBN = 128; // columns of an output tile
 
-// EXACT_W: the weights are BF16 values, their lo parts zero and not read.
+// EXACT_W: the weights are BF16 values that their hi parts hold, the lo parts are not read (PAIR_FIT_HI).
 template <bool EXACT_W>
 struct PairSmem {
   static constexpr int TILE_BYTES = TILE_M * PK * 2;  // 16 KB; 128 rows of weights are a tile too
@@ -235,27 +240,54 @@ __global__ void __launch_bounds__(256) tile_pairs_kernel(const float* __restrict
   }
 }
 
-// Per matrix [rows, cols]: the largest |w| and the largest Euclidean norm of a row at or after `norm_from`, as bit patterns
-// that order like the non-negative numbers they are. One warp per row.
-__global__ void __launch_bounds__(256) matrix_bounds_kernel(const float* __restrict__ w, int rows, int cols, int norm_from, unsigned* out) {
+// The largest |w| of a matrix [rows, cols], as a bit pattern that orders like the non-negative number it is, and the Euclidean norms
+// of its rows (unless null). Values that are not finite do not count. One warp per row.
+__global__ void __launch_bounds__(256) matrix_bounds_kernel(const float* __restrict__ w, int rows, int cols, unsigned* largest, float* norms) {
   const int lane = threadIdx.x & 31;
-  float top = 0.f, norm = 0.f;
+  float top = 0.f;
   for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {
-    float sq = 0.f;
+    double sq = 0.0;
     for (int i = lane; i < cols; i += 32) {
       const float v = fabsf(w[(size_t)r * cols + i]);
+      if (!isfinite(v)) continue;
       top = fmaxf(top, v);
-      sq = fmaf(v, v, sq);
+      sq = fma((double)v, (double)v, sq);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if (r >= norm_from) norm = fmaxf(norm, sqrtf(sq));
+    if (norms && lane == 0) norms[r] = __double2float_ru(sqrt(sq));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if (lane == 0) {
-    atomicMax(out, __float_as_uint(top));
-    atomicMax(out + 1, __float_as_uint(norm));
+  if (lane == 0) atomicMax(largest, __float_as_uint(top));
+}
+
+// How well FP16 holds the rows of w * scale: the largest share of a row's squared length that is lost by hi parts alone and by
+// pairs, as bit patterns (NaN, of a row with values that are not finite, comes out above all numbers). One warp per row.
+__global__ void __launch_bounds__(256) pair_fit_kernel(const float* __restrict__ w, int rows, int cols, float scale, unsigned* out) {
+  const int lane = threadIdx.x & 31;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {
+    double sq = 0.0, hi_off = 0.0, pair_off = 0.0;
+    for (int i = lane; i < cols; i += 32) {
+      const float v = w[(size_t)r * cols + i];
+      uint32_t hi, lo;
+      split_pair2(v, 0.f, scale, hi, lo);
+      const double x = (double)v * scale, left = x - __half2float(__ushort_as_half((unsigned short)hi)),
+                   rest = left - (double)__half2float(__ushort_as_half((unsigned short)lo)) * PAIR_LO_INV;
+      sq = fma(x, x, sq);
+      hi_off = fma(left, left, hi_off);
+      pair_off = fma(rest, rest, pair_off);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      hi_off += __shfl_xor_sync(0xffffffffu, hi_off, o);
+      pair_off += __shfl_xor_sync(0xffffffffu, pair_off, o);
+    }
+    if (lane == 0 && sq != 0.0) {
+      atomicMax(out, __float_as_uint((float)(hi_off / sq)) & 0x7fffffffu);
+      atomicMax(out + 1, __float_as_uint((float)(pair_off / sq)) & 0x7fffffffu);
+    }
   }
 }
 
@@ -285,10 +317,10 @@ cudaError_t launch_pair(const PairGemmArgs& a, cudaStream_t s) {
 
 bool pair_gemm_supported(int k) { return k > 0 && k % 32 == 0 && encode_fn() != nullptr; }
 
-float pair_scale(float bound) {
-  if (!(bound > 0.f) || !std::isfinite(bound)) return 1.f;
-  const int e = 14 - std::ilogb(bound);  // bound * 2^e in [2^14, 2^15)
-  return std::ldexp(1.f, std::max(-120, std::min(120, e)));
+float pair_scale(double bound) {
+  if (!(bound > 0.0)) return 1.f;
+  const int e = 14 - std::ilogb(std::min(bound, (double)FLT_MAX));  // bound * 2^e in [2^14, 2^15); no FP32 value is above FLT_MAX
+  return std::ldexp(1.f, std::min(120, e));
 }
 
 size_t pair_tiled_halves(int n, int k, bool exact) {
@@ -307,8 +339,13 @@ cudaError_t launch_make_pairs(const float* x, uint16_t* hi, uint16_t* lo, size_t
   return cudaGetLastError();
 }
 
-cudaError_t launch_matrix_bounds(const float* w, int rows, int cols, int norm_from, unsigned* out, cudaStream_t s) {
-  matrix_bounds_kernel<<<std::max(1, std::min((rows + 7) / 8, 148 * 8)), 256, 0, s>>>(w, rows, cols, norm_from, out);
+cudaError_t launch_matrix_bounds(const float* w, int rows, int cols, unsigned* largest, float* norms, cudaStream_t s) {
+  matrix_bounds_kernel<<<std::max(1, std::min((rows + 7) / 8, 148 * 8)), 256, 0, s>>>(w, rows, cols, largest, norms);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pair_fit(const float* w, int rows, int cols, float scale, unsigned* out, cudaStream_t s) {
+  pair_fit_kernel<<<std::max(1, std::min((rows + 7) / 8, 148 * 8)), 256, 0, s>>>(w, rows, cols, scale, out);
   return cudaGetLastError();
 }
 

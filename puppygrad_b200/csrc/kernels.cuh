@@ -159,12 +159,20 @@ bool pair_gemm_supported(int k);
 cudaError_t launch_tc_gemm_pair(const PairGemmArgs& a, cudaStream_t s);
 cudaError_t init_pair_gemm_attributes();
 // Scale for values that stay below `bound`; pairs of n values (n % 4 == 0); a weight matrix [n, k] as tiles of pairs (`exact`: only
-// the hi tiles); {largest |w|, largest norm of a row from `norm_from` on} as bit patterns into out[2], which starts at zero.
-float pair_scale(float bound);
+// the hi tiles); the largest |w| of a matrix as a bit pattern (maximum with what is there) and the norms of its rows (or null).
+float pair_scale(double bound);
 size_t pair_tiled_halves(int n, int k, bool exact);
 cudaError_t launch_tile_pairs(const float* w, uint16_t* dst, int n, int k, bool exact, float scale, cudaStream_t s);
 cudaError_t launch_make_pairs(const float* x, uint16_t* hi, uint16_t* lo, size_t n, float scale, cudaStream_t s);
-cudaError_t launch_matrix_bounds(const float* w, int rows, int cols, int norm_from, unsigned* out, cudaStream_t s);
+cudaError_t launch_matrix_bounds(const float* w, int rows, int cols, unsigned* largest, float* norms, cudaStream_t s);
+// Largest share of a row's squared length that is lost {by hi parts alone, by pairs}, as bit patterns into out[2] (maximum with what is
+// there). Pairs take FP32's place where they keep 22 bits of every row, hi parts alone where what is missing is below FP32's own
+// rounding. Neither comparison holds for NaN.
+constexpr float PAIR_FIT = 0x1p-44f, PAIR_FIT_HI = 0x1p-50f;
+// The most that the inputs of a product can reach over what half of their columns can. At that, a value 2^10 below what its own column
+// can reach (sums of random sign stay a factor of about sqrt(k) below, means of many keys or a GELU another one) still keeps 22 bits.
+constexpr double PAIR_SPREAD = 0x1p18;
+cudaError_t launch_pair_fit(const float* w, int rows, int cols, float scale, unsigned* out, cudaStream_t s);
 // three TF32 passes (FP32-grade), m <= 64 (decode)
 int tc_gemm_x3_splits(int n, int k, int num_sms);
 cudaError_t launch_tc_gemm_x3(const TcGemmArgs& a, int splits, bool pdl, cudaStream_t s);

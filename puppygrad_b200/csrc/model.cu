@@ -137,72 +137,95 @@ int ensure_device(int device) {
 static size_t align_up(size_t n, size_t a) { return (n + a - 1) / a * a; }
 
 // FP16 pairs of the dense matrices, and the scales of their inputs: what the values of each can reach at most, from the
-// weights alone. `tensors`: the host tensors of the model.
+// weights alone. `tensors`: the host tensors of the model. A model for which pairs are not FP32-grade is left without them.
 static int make_pair_weights(pg_model* m, const float* const* tensors) {
   const size_t C = m->c(), F = m->f(), V = m->v(), L = m->layers.size();
   if (!pair_gemm_supported((int)C) || !pair_gemm_supported((int)F)) return PG_OK;
-  const bool exact = m->backend.math_mode == PG_MATH_BF16;  // BF16 values fit the hi part
-  auto halves = [&](size_t n, size_t k) { return pair_tiled_halves((int)n, (int)k, exact); };
-  m->pair_exact = exact;
-  m->pair_halves = L * (halves(3 * C, C) + halves(C, C) + halves(F, C) + halves(C, F)) + halves(V, C);
-  PG_CUDA_TRY(cudaMalloc(&m->pair_arena, m->pair_halves * sizeof(uint16_t)));
-  unsigned* d_bounds = nullptr;
-  const size_t n_bounds = L * 8 + 2;
-  PG_CUDA_TRY(cudaMalloc(&d_bounds, n_bounds * sizeof(unsigned)));
-  std::vector<float> bounds(n_bounds);
+  struct Matrix {
+    const float* w;
+    size_t n, k;
+    PairWeights* out;
+  };
+  std::vector<Matrix> all;
+  for (LayerWeights& w : m->layers) {
+    all.push_back({w.w_qkv, 3 * C, C, &w.q_qkv});
+    all.push_back({w.w_proj, C, C, &w.q_proj});
+    all.push_back({w.w_fc, F, C, &w.q_fc});
+    all.push_back({w.w_proj2, C, F, &w.q_proj2});
+  }
+  all.push_back({m->head_w, V, C, &m->q_wte});
+  // the largest value of each, what halves and pairs lose of a row at most, then per layer the norms of the rows of w_qkv and w_fc
+  const size_t words = all.size() + 2, per_layer = 3 * C + F;
+  std::vector<float> found(words + L * per_layer);
+  const float *lost = found.data() + all.size(), *norms = found.data() + words;
+  float* d_found = nullptr;
+  PG_CUDA_TRY(cudaMalloc(&d_found, found.size() * sizeof(float)));
   int rc = [&]() -> int {
-    PG_CUDA_TRY(cudaMemsetAsync(d_bounds, 0, n_bounds * sizeof(unsigned), 0));
-    for (size_t l = 0; l < L; ++l) {
-      const LayerWeights& w = m->layers[l];
-      unsigned* b = d_bounds + 8 * l;
-      PG_CUDA_TRY(launch_matrix_bounds(w.w_qkv, (int)(3 * C), (int)C, (int)(2 * C), b, 0));  // norms of the value rows
-      PG_CUDA_TRY(launch_matrix_bounds(w.w_proj, (int)C, (int)C, 0, b + 2, 0));
-      PG_CUDA_TRY(launch_matrix_bounds(w.w_fc, (int)F, (int)C, 0, b + 4, 0));
-      PG_CUDA_TRY(launch_matrix_bounds(w.w_proj2, (int)C, (int)F, 0, b + 6, 0));
+    unsigned* top = reinterpret_cast<unsigned*>(d_found);
+    PG_CUDA_TRY(cudaMemsetAsync(d_found, 0, words * sizeof(float), 0));
+    for (size_t i = 0; i < all.size(); ++i) {
+      float* at = d_found + words + i / 4 * per_layer;
+      PG_CUDA_TRY(launch_matrix_bounds(all[i].w, (int)all[i].n, (int)all[i].k, top + i,
+                                       i + 1 == all.size() ? nullptr : i % 4 == 0 ? at : i % 4 == 2 ? at + 3 * C : nullptr, 0));
     }
-    PG_CUDA_TRY(launch_matrix_bounds(m->head_w, (int)V, (int)C, 0, d_bounds + 8 * L, 0));
-    PG_CUDA_TRY(cudaMemcpy(bounds.data(), d_bounds, n_bounds * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    PG_CUDA_TRY(cudaMemcpy(found.data(), d_found, found.size() * sizeof(float), cudaMemcpyDeviceToHost));
+    for (size_t i = 0; i < all.size(); ++i) {
+      all[i].out->scale = pair_scale(found[i]);
+      PG_CUDA_TRY(launch_pair_fit(all[i].w, (int)all[i].n, (int)all[i].k, all[i].out->scale, top + all.size(), 0));
+    }
+    PG_CUDA_TRY(cudaMemcpy(found.data() + all.size(), d_found + all.size(), 2 * sizeof(float), cudaMemcpyDeviceToHost));
     return PG_OK;
   }();
-  cudaFree(d_bounds);
+  cudaFree(d_found);
   if (rc != PG_OK) return rc;
-  uint16_t* at = m->pair_arena;
-  auto pairs = [&](const float* w, size_t n, size_t k, float top, PairWeights* out) -> int {
-    out->scale = pair_scale(top);
-    out->w = at;
-    PG_CUDA_TRY(launch_tile_pairs(w, at, (int)n, (int)k, exact, out->scale, 0));
-    at += halves(n, k);
-    return PG_OK;
+  bool held = lost[1] <= PAIR_FIT;
+  auto input_scale = [&](std::vector<double> reach) {  // what each column of the inputs of a product can reach
+    const double most = *std::max_element(reach.begin(), reach.end());
+    std::nth_element(reach.begin(), reach.begin() + reach.size() / 2, reach.end());
+    held = held && most <= PAIR_SPREAD * reach[reach.size() / 2];
+    return pair_scale(most);
   };
-  auto largest = [](const float* v, size_t n) {
-    float top = 0.f;
-    for (size_t i = 0; i < n; ++i) top = std::max(top, std::fabs(v[i]));
-    return top;
+  // a normalised row has a norm of at most sqrt(C) ...
+  const double root = std::sqrt((double)C);
+  auto normed = [&](const float* gain, const float* shift) {
+    std::vector<double> reach(C);
+    for (size_t i = 0; i < C; ++i) reach[i] = root * std::fabs(gain[i]) + std::fabs(shift[i]);
+    return input_scale(reach);
   };
-  auto norm = [](const float* v, size_t n) {
-    double sq = 0.0;
-    for (size_t i = 0; i < n; ++i) sq += (double)v[i] * v[i];
-    return (float)std::sqrt(sq);
+  // ... so one output of the product behind it is at most its weight row's norm times the norm of the scaled and shifted row;
+  // attention outputs are convex combinations of value rows, |gelu(y)| <= |y|
+  auto multiplied = [&](const float* gain, const float* shift, const float* row_norms, const float* bias, size_t n) {
+    double most = 0.0, sq = 0.0;
+    for (size_t i = 0; i < C; ++i) {
+      most = std::max(most, (double)std::fabs(gain[i]));
+      sq += (double)shift[i] * shift[i];
+    }
+    std::vector<double> reach(n);
+    for (size_t i = 0; i < n; ++i) reach[i] = row_norms[i] * (root * most + std::sqrt(sq)) + std::fabs(bias[i]);
+    return input_scale(reach);
   };
   for (size_t l = 0; l < L; ++l) {
     LayerWeights& w = m->layers[l];
     const float* const* t = tensors + 4 + 12 * l;
-    const float* b = bounds.data() + 8 * l;
-    if (int r = pairs(w.w_qkv, 3 * C, C, b[0], &w.q_qkv)) return r;
-    if (int r = pairs(w.w_proj, C, C, b[2], &w.q_proj)) return r;
-    if (int r = pairs(w.w_fc, F, C, b[4], &w.q_fc)) return r;
-    if (int r = pairs(w.w_proj2, C, F, b[6], &w.q_proj2)) return r;
-    // a normalised row has a norm of at most sqrt(C), so one output of the product behind it is at most its weight row's norm
-    // times the norm of the scaled and shifted row; attention outputs are convex combinations of value rows, |gelu(y)| <= |y|
-    const float root = std::sqrt((float)C);
-    const float row1 = root * largest(t[0], C) + norm(t[1], C), row2 = root * largest(t[6], C) + norm(t[7], C);
-    w.x_norm1 = pair_scale(root * largest(t[0], C) + largest(t[1], C));
-    w.x_attn = pair_scale(b[1] * row1 + largest(t[3] + 2 * C, C));
-    w.x_norm2 = pair_scale(root * largest(t[6], C) + largest(t[7], C));
-    w.x_h = pair_scale(b[5] * row2 + largest(t[9], F));
+    const float* at = norms + l * per_layer;
+    w.x_norm1 = normed(t[0], t[1]);
+    w.x_attn = multiplied(t[0], t[1], at + 2 * C, t[3] + 2 * C, C);
+    w.x_norm2 = normed(t[6], t[7]);
+    w.x_h = multiplied(t[6], t[7], at + 3 * C, t[9], F);
   }
-  m->x_normf = pair_scale(std::sqrt((float)C) * largest(tensors[2], C) + largest(tensors[3], C));
-  return pairs(m->head_w, V, C, bounds[8 * L], &m->q_wte);
+  m->x_normf = normed(tensors[2], tensors[3]);
+  if (!held) return PG_OK;
+  const bool exact = m->backend.math_mode == PG_MATH_BF16 && lost[0] <= PAIR_FIT_HI;
+  m->pair_exact = exact;
+  for (const Matrix& x : all) m->pair_halves += pair_tiled_halves((int)x.n, (int)x.k, exact);
+  PG_CUDA_TRY(cudaMalloc(&m->pair_arena, m->pair_halves * sizeof(uint16_t)));
+  uint16_t* at = m->pair_arena;
+  for (const Matrix& x : all) {
+    x.out->w = at;
+    PG_CUDA_TRY(launch_tile_pairs(x.w, at, (int)x.n, (int)x.k, exact, x.out->scale, 0));
+    at += pair_tiled_halves((int)x.n, (int)x.k, exact);
+  }
+  return PG_OK;
 }
 
 static int build_model(const pg_gpt2_config& cfg, const float* const* tensors, const uint64_t* lens, uint64_t n,

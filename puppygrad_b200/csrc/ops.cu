@@ -57,27 +57,30 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
   const size_t xs = (size_t)m * k, ws = (size_t)n * k, os = (size_t)m * n;
   float x_scale = 1.f, w_scale = 1.f;  // of the FP16 pairs
   if (math_mode == PG_MATH_TF32X3) {
-    float top = 0.f;
-    for (size_t i = 0; i < xs; ++i) top = std::max(top, std::fabs(x[i]));
-    x_scale = pair_scale(top);
-    top = 0.f;
-    for (size_t i = 0; i < ws; ++i) top = std::max(top, std::fabs(w[i]));
-    w_scale = pair_scale(top);
+    auto scale_of = [](const float* v, size_t n) {
+      float top = 0.f;
+      for (size_t i = 0; i < n; ++i)
+        if (std::isfinite(v[i])) top = std::max(top, std::fabs(v[i]));
+      return pair_scale(top);
+    };
+    x_scale = scale_of(x, xs);
+    w_scale = scale_of(w, ws);
   }
-  DeviceBuf dx, dw, dwt, db, dr, dout, dhi, dlo, derr, dflush, dtrace, dpart, dbar, dwlo;
+  DeviceBuf dx, dw, dwt, db, dr, dout, dhi, dlo, derr, dflush, dtrace, dpart, dbar, dwlo, dfit;
 #ifdef PG_DEV_TRACE
   const bool want_trace = getenv("PG_TRACE") != nullptr;  // developer aid: phase time stamps of the kernel, printed below
 #else
   constexpr bool want_trace = false;
 #endif
-  // tf32x3 runs on the persistent chain kernel (one GEMM phase + its reduce phase) unless PG_NO_CHAIN is set
+  // tf32x3 of at most 64 rows runs on the persistent chain kernel (one GEMM phase + its reduce phase) unless PG_NO_CHAIN is set
   int chain_ctas = 0;
   ChainArgs chain{};
   cudaStream_t s = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int splits = 1;
+  bool pairs = false;  // FP16 pairs hold both operands
   auto run = [&](cudaStream_t st) -> cudaError_t {
-    if (math_mode == PG_MATH_FP32) {
+    if (math_mode == PG_MATH_FP32 || (x3_rows && !pairs)) {
       LinearArgs a{};
       a.w = dw.as<float>(); a.bias = db.as<float>(); a.x = dx.as<float>(); a.out = dout.as<float>();
       a.resid = dr.as<float>(); a.m = m; a.n = n; a.k = k;
@@ -131,6 +134,16 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
     PG_OP_TRY(cudaMalloc(&dr.p, os * 4));
     PG_OP_TRY(cudaMemcpyAsync(dr.p, resid, os * 4, cudaMemcpyHostToDevice, s));
   }
+  if (math_mode == PG_MATH_TF32X3) {
+    float lost[2];
+    PG_OP_TRY(cudaMalloc(&dfit.p, sizeof(lost)));
+    PG_OP_TRY(cudaMemsetAsync(dfit.p, 0, sizeof(lost), s));
+    PG_OP_TRY(launch_pair_fit(dx.as<float>(), m, k, x_scale, dfit.as<unsigned>(), s));
+    PG_OP_TRY(launch_pair_fit(dw.as<float>(), n, k, w_scale, dfit.as<unsigned>(), s));
+    PG_OP_TRY(cudaMemcpyAsync(lost, dfit.p, sizeof(lost), cudaMemcpyDeviceToHost, s));
+    PG_OP_TRY(cudaStreamSynchronize(s));
+    pairs = lost[1] <= PAIR_FIT;
+  }
   if (x3_rows) {
     if (xs % 4 || ws % 4) {
       rc = set_error(PG_INVALID_INPUT, "tf32x3 with more than 64 rows needs m * k and n * k to be multiples of 4");
@@ -145,7 +158,7 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
     PG_OP_TRY(cudaMalloc(&dlo.p, xs * 4));
     PG_OP_TRY(cudaMalloc(&dwt.p, tc_tiled_weight_floats(n, k) * 4));
     PG_OP_TRY(launch_tile_weights(dw.as<float>(), dwt.as<float>(), n, k, s));
-    if (!getenv("PG_NO_CHAIN") && chain_grid(sms) > 0) {
+    if (pairs && !getenv("PG_NO_CHAIN") && chain_grid(sms) > 0) {
       const int g = chain_grid(sms);
       chain.n_phases = 2;
       chain.ph[0].kind = CH_GEMM; chain.ph[0].n = n; chain.ph[0].k = k; chain.ph[0].act = CH_ACT_NORM;

@@ -94,6 +94,23 @@ def test_linear_pairs_against_float64(m, n, k, spread):
         assert (np.abs(without - x @ w.T) > bound).any()
 
 
+# Rows far below the matrix' largest value, in the input, the weights or both: pairs do not hold them, other kernels run.
+@pytest.mark.parametrize("m,n,k", [(33, 70, 128), (130, 70, 128)])
+@pytest.mark.parametrize("rows", ["x", "w", "xw"])
+def test_linear_of_rows_that_pairs_do_not_hold(m, n, k, rows):
+    """Every row of the result to FP32 grade: three TF32 products hold an operand to 2^-21 of its size and truncate a sum three times
+    per 8 products."""
+    rng = np.random.default_rng(m)
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    if "x" in rows:
+        x[5:9] *= np.float32(2.0 ** -40)
+    if "w" in rows:
+        w[60:] *= np.float32(2.0 ** -40)
+    got, _ = ops.linear(x, w, math_mode="tf32x3")
+    x, w = x.astype(np.float64), w.astype(np.float64)
+    assert (np.abs(got - x @ w.T) <= (4 * 2.0 ** -21 + 3 * k / 8 * 2.0 ** -23) * (np.abs(x) @ np.abs(w).T)).all()
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 1600, 1600), (512, 4800, 1600), (300, 1600, 6400), (1000, 777, 256)])
 @pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
 def test_linear_tf32x3_prefill_sized_matches_oracle(oracle, m, n, k, epilogue):

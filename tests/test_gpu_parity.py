@@ -11,6 +11,7 @@ import pytest
 
 import puppygrad_b200 as pg
 from puppygrad_b200 import synthetic
+from tests.f64_model import forward_f64
 
 pytestmark = pytest.mark.gpu
 
@@ -880,7 +881,6 @@ def test_narrow_weight_modes_exclude_each_other():
         pg.Gpt2Model(cfg, w, pg.Gpt2CudaConfig(math_mode="bf16", quantized_weights=True))
 
 
-# ------------------------------------------------------------------ GPT-2 small prefill, 8 x 1024 (second benchmark config)
 @pytest.mark.parametrize("batch", [5, 8, 16, 17, 33])
 def test_bf16_steps_of_more_than_four_sequences(oracle, batch):
     """The persistent tensor-core step with the hi parts of the weights alone, at the edges of its token tiles: one launch, the
@@ -905,6 +905,81 @@ def test_bf16_steps_of_more_than_four_sequences(oracle, batch):
         cur = am.copy()
 
 
+# ------------------------------------------------------------------ scales of FP16 pairs
+def _edge_weights(cfg, kind):
+    """Weights whose activations come near, or stay far below, what the weights bound them by."""
+    w, c = synthetic.perturbed_weights(cfg, 61), cfg["n_embd"]
+    for l in range(cfg["n_layer"]):
+        p = f"h.{l}."
+        if kind == "gain":
+            w[p + "ln_1.weight"][7] = w[p + "ln_2.weight"][11] = 300.0
+        elif kind == "shift":
+            w[p + "ln_1.bias"][:] += 20.0
+            w[p + "ln_2.bias"][3] = -500.0
+        elif kind == "value":
+            w[p + "attn.c_attn.weight"][:, 2 * c + 5] *= 500.0
+            w[p + "attn.c_attn.bias"][2 * c + 9] = 300.0
+        elif kind == "outlier":
+            for name in ("attn.c_attn", "attn.c_proj", "mlp.c_fc", "mlp.c_proj"):
+                w[p + name + ".weight"][13, 17] = 60.0
+        else:  # one entry of a row holds all of its length, and a value row and a hidden unit see nothing else
+            for name, col in (("attn.c_attn", 2 * c + 5), ("mlp.c_fc", 21)):
+                w[p + name + ".weight"][:, col] = 0.0
+                w[p + name + ".weight"][3, col] = 2.0
+            w[p + "ln_1.weight"][3] = w[p + "ln_2.weight"][3] = 2.0
+    if kind == "one entry":
+        w["wte.weight"][:, 3] = 900.0
+    if kind in ("gain", "shift"):
+        w["ln_f.weight"][5], w["ln_f.bias"][6] = 200.0, 100.0
+    return w
+
+
+@pytest.mark.parametrize("math_mode", ["tf32x3", "bf16"])
+@pytest.mark.parametrize("kind", ["gain", "shift", "value", "outlier", "one entry"])
+def test_scales_of_pairs_at_their_edge(kind, math_mode):
+    """Products of FP16 pairs, in a prompt of more than 128 rows and in steps of nine sequences, where a LayerNorm's gain or shift, a
+    value row or a weight is out of line and where the scales' bounds are reached. Against 64 bits, and no more than 32 times as far
+    from them as the FP32 kernels: at k = 1024 a sum is truncated 64 times, by 2^-24 of it on average and always towards zero, where
+    a thread of those rounds some 16 partial sums, by 2^-25 on average and either way (4 of them add up). TF32 products: up to 15."""
+    cfg = synthetic.preset("midi")
+    assert_pairs_close(cfg, _edge_weights(cfg, kind), math_mode)
+
+
+def assert_pairs_close(cfg, w, math_mode):
+    w64 = synthetic.bf16_rounded_weights(w) if math_mode == "bf16" else w
+    prompts = [synthetic.uniform_prompt(1500 + i, 14 + 2 * i, cfg["vocab_size"]) for i in range(9)]
+    got = {}
+    for mode in ("fp32", math_mode):
+        m = pg.Gpt2Model(cfg, w64, pg.Gpt2CudaConfig(math_mode=mode))
+        cache = m.new_kv_cache(max_batch=9)
+        rows = [m.prefill_batch(prompts, cache, want_logits=True)[0]]
+        for t in (5, 6):
+            rows.append(m.forward_one_batch([100 * t + i for i in range(9)], cache, want_logits=True)[0])
+        got[mode] = np.array(rows, np.float64)
+    want = np.array([[forward_f64(cfg, w64, list(p) + [100 * t + i for t in (5, 6)][:n])[-1] for i, p in enumerate(prompts)] for n in range(3)])
+    off = {mode: np.linalg.norm(rows - want, axis=-1) / np.linalg.norm(want, axis=-1) for mode, rows in got.items()}
+    assert np.isfinite(got[math_mode]).all()
+    assert off[math_mode].max() <= 32 * max(off["fp32"].max(), 2.0 ** -24), off
+
+
+@pytest.mark.parametrize("math_mode", ["tf32x3", "bf16"])
+@pytest.mark.parametrize("name,outlier", [("c_proj", 2.0 ** 10), ("c_proj", 2.0 ** 20), ("c_proj", 2.0 ** 30), ("c_fc", 2.0 ** 10), ("c_fc", 2.0 ** 30)])
+def test_weights_that_pairs_do_not_hold(name, outlier, math_mode):
+    """One weight of a matrix so far above the others that the hi parts alone, or pairs, do not hold the other rows (c_proj), or the other
+    hidden units (c_fc). It meets a column of zeros, so that the others decide the logits. Bound as above."""
+    cfg = synthetic.preset("midi")
+    w = synthetic.perturbed_weights(cfg, 63)
+    for l in range(cfg["n_layer"]):
+        p = f"h.{l}."
+        if name == "c_fc":
+            w[p + "ln_2.weight"][3] = w[p + "ln_2.bias"][3] = 0.0
+        else:
+            w[p + "mlp.c_fc.weight"][:, 3] = w[p + "mlp.c_fc.bias"][3] = 0.0
+        w[p + "mlp." + name + ".weight"][3, 21] = outlier
+    assert_pairs_close(cfg, w, math_mode)
+
+
+# ------------------------------------------------------------------ GPT-2 small prefill, 8 x 1024 (second benchmark config)
 @pytest.mark.parametrize("math_mode,span_bound", [("fp32", None), ("tf32x3", None), ("tf32", 5e-3), ("bf16", 3e-2)])
 def test_gpt2_small_prefill_8x1024_against_golden(math_mode, span_bound):
     """Eight prompts of 1024 tokens through the batched prefill, final-position logits against the oracle's
