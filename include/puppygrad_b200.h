@@ -79,9 +79,11 @@ typedef struct {
   int32_t persistent_step; /* decode steps of at most 8 sequences (head_dim 64, n_positions <= 1024) can run as ONE
                               persistent cooperative kernel whose weight stream runs ahead of the dependent
                               operations and whose CTAs exchange activations as tagged words instead of meeting
-                              at grid barriers. 0 = where it measured faster than one kernel per operation in a
-                              CUDA graph (up to 4 sequences with FP32 weights; always with BF16 / int8 weights,
-                              which only that kernel reads), 1 = whenever the shapes allow, 2 = never */
+                              at grid barriers. 0 = where it measured faster than the alternatives: up to 4 sequences
+                              with FP32 weights (then one kernel per operation in a CUDA graph) and with BF16 weights
+                              (then the persistent step of larger batches, which reads them too), always with int8
+                              weights. 1 = whenever the shapes allow, 2 = never: one kernel per operation up to 8
+                              sequences */
   int32_t quantized_weights; /* Gpt2RustConfig::quantized_weights (src/models/gpt2/options.rs:62-104): 1 = the four
                                 dense matrices of every block and the lm_head as row-wise int8 (QuantizedRows,
                                 src/models/cpu.rs:26-56; quantize_weights, rust.rs:1354-1376); the embedding lookup

@@ -461,7 +461,7 @@ static int cache_new(const pg_model* m, int max_batch, pg_cache** out) {
   PG_CUDA_TRY(cudaMalloc(&c->attn_part, B * H * MAX_SPLITS * (D + 2) * sizeof(float)));
   PG_CUDA_TRY(cudaMalloc(&c->attn_counters, B * H * sizeof(unsigned)));
   PG_CUDA_TRY(cudaMemsetAsync(c->attn_counters, 0, B * H * sizeof(unsigned), c->stream));
-  c->chain_min_batch = m->pair_exact ? 5 : 9;
+  c->chain_min_batch = m->pair_exact && m->backend.persistent_step != 2 ? 5 : 9;
   if (const char* e = getenv("PG_CHAIN_MIN_BATCH")) c->chain_min_batch = std::max(1, std::min(65, atoi(e)));
   if (max_batch >= c->chain_min_batch && C % 32 == 0 && F % 32 == 0) {
     const int bmax = std::min(max_batch, 64);
@@ -1557,8 +1557,8 @@ uint64_t pg_model_weight_bytes_per_step(const pg_model* model) {
   const pg_gpt2_config& c = model->cfg;
   // every block matrix, bias and LayerNorm vector once; the tied embedding once as lm_head;
   // ln_f; one wte row and one wpe row are negligible and not counted. With BF16 / int8 weights the
-  // matrices and the lm_head count at their narrow size (what decode steps of at most 8 sequences read),
-  // int8 with one FP32 scale per row
+  // matrices and the lm_head count at their narrow size (what decode steps read: of any number of sequences with BF16
+  // weights, of at most 8 with int8 ones), int8 with one FP32 scale per row
   const uint64_t dense = c.n_embd * 3 * c.n_embd + c.n_embd * c.n_embd + 2 * c.n_embd * c.n_inner;
   const uint64_t dense_rows = 3 * c.n_embd + c.n_embd + c.n_inner + c.n_embd;
   const uint64_t vectors = 3 * c.n_embd + c.n_embd + c.n_inner + c.n_embd + 4 * c.n_embd;

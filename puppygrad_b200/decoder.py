@@ -31,7 +31,7 @@ class CudaConfig:
     use_graphs: bool = True
     attn_splits: int = 0
     # one cooperative kernel per decode step of <= 8 sequences: None = where it is the faster path, True = whenever
-    # the shapes allow, False = never (a CUDA graph of one kernel per operation)
+    # the shapes allow, False = never (a CUDA graph of one kernel per operation, also where another persistent step exists)
     persistent_step: Optional[bool] = None
     max_context: int = 0  # models without a position limit: the most tokens a sequence may hold (0: the library's default)
     quantized_weights: bool = False  # Gpt2RustConfig::quantized_weights: row-wise int8 dense matrices and lm_head

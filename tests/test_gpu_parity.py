@@ -875,6 +875,25 @@ def test_bf16_weights_model_is_fp32_math_on_rounded_weights(oracle, batch):
         cur = am.copy()
 
 
+@pytest.mark.parametrize("batch", [5, 8])
+def test_persistent_step_chooses_the_kernels_of_bf16_steps(batch):
+    """One kernel per operation where it is False, one kernel for the step (either of the two) where it is not; logits agree."""
+    cfg = synthetic.preset("midi")
+    w = synthetic.perturbed_weights(cfg, 58)
+    prompts = [synthetic.uniform_prompt(1400 + i, 7 + i, cfg["vocab_size"]) for i in range(batch)]
+    got = {}
+    for persistent in (None, True, False):
+        m = pg.Gpt2Model(cfg, w, pg.Gpt2CudaConfig(math_mode="bf16", persistent_step=persistent))
+        cache = m.new_kv_cache(max_batch=batch)
+        m.prefill_batch(prompts, cache)
+        n0 = cache.kernel_launches()
+        got[persistent] = m.forward_one_batch(range(batch), cache, want_logits=True)[0]
+        n = cache.kernel_launches() - n0
+        assert n > cfg["n_layer"] if persistent is False else n == 1, (persistent, n)
+    assert_logits_close(got[None], got[False])
+    assert_logits_close(got[True], got[False])
+
+
 def test_narrow_weight_modes_exclude_each_other():
     cfg, w = tiny()
     with pytest.raises(pg.Gpt2Error, match="exclude each other"):
