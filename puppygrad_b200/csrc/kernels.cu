@@ -1489,12 +1489,13 @@ cudaError_t launch_layernorm_rows_split(const float* x, const float* g, const fl
   return launch(layernorm_rows_split_kernel, dim3(rows), dim3(128), 0, s, pdl, x, g, b, eps, hi, lo, rows, c);
 }
 
-// The decode kernels stream the weights once per 8 rows. GPT-2 small's products on them and on the tiles: 9 rows
-// 14.3 / 10.3 / 18.5 and 14.4 / 11.5 / 18.4 us, 16 rows 15.8 / 11.3 / 21.3 and 14.4 / 11.7 / 18.4 us, 64 rows 42 / 28 / 65 and
-// 18.5 / 12.3 / 24.4 us (n 2304, k 768 / n 768, k 768 / n 768, k 3072); a whole prefill of 11 rows 917 and 990 us. The tiles win
-// earlier where the weights are many: lm_head of 12 rows 150 and 82 us.
+// The decode kernels stream the weights once per 8 rows and start before the kernel in front of them has ended; the tiles read them
+// once. Whole steps on decode kernels and on tiles, us: 13 / 16 sequences of GPT-2 small 666 / 681 and 725 / 731, of medium 1515 / 1577 and
+// 1783 / 1798; with 17, a third round, 937 (20 sequences) and 739, 2136 and 1818. Prompts of 13 and 16 rows: small 757 / 778 and 869 / 869,
+// medium 1575 / 1635 and 2030 / 2033. The lm_head alone, the rest of the step on decode kernels: medium 1426 / 1449 / 1512 / 1524 / 1611 and
+// 1459 / 1474 / 1502 / 1515 / 1577 for 9 / 10 / 12 / 13 / 16 sequences.
 cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s) {
-  if (a.m <= 8 || a.k % 4 != 0 || (a.m <= 12 && a.n <= 16384)) return launch_linear_decode(a, epilogue, pdl, s, nullptr);
+  if (a.m <= (a.n <= 16384 ? 16 : 10) || a.k % 4 != 0) return launch_linear_decode(a, epilogue, pdl, s, nullptr);
   return launch_gemm_f32_tiles(a, epilogue, s);
 }
 

@@ -34,9 +34,9 @@ def test_linear_fp32_matches_oracle(oracle, m, n, k, epilogue):
     np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
 
 
-# Tiles of 32 and 64 rows by 64 columns, k in blocks of 32 shared out over up to 8 CTAs: edges of all of these, a last share
-# without any block (k 1600: 50 blocks in shares of 7), k that ends inside a block.
-@pytest.mark.parametrize("m,n,k", [(9, 1, 4), (31, 63, 36), (32, 64, 64), (33, 65, 516), (128, 130, 1600), (129, 64, 512),
+# Tiles of 32 and 64 rows by 64 columns, k in blocks of 32 shared out over up to 8 CTAs: edges of all of these, last shares
+# without any block (k 516: 17 blocks in shares of 3), a last share of one (k 1600: 50 in shares of 7), k that ends inside a block.
+@pytest.mark.parametrize("m,n,k", [(17, 1, 4), (11, 16385, 36), (31, 63, 36), (32, 64, 64), (33, 65, 516), (128, 130, 1600), (129, 64, 512),
                                    (65, 777, 100), (200, 2304, 768)])
 @pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
 def test_linear_fp32_tiles_match_oracle(oracle, m, n, k, epilogue):
