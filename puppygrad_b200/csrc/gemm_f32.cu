@@ -38,7 +38,7 @@ __global__ void __launch_bounds__((F32Tile<BM, BN, TM, TN>::THREADS)) gemm_f32_k
   constexpr int BK = T::BK, STRIDE = T::STRIDE, TX = T::TX, TY = T::TY, THREADS = T::THREADS;
   extern __shared__ __align__(16) float ring[];
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-  const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM, rank = blockIdx.z;
+  const int tiles_n = (a.n + BN - 1) / BN, n0 = (int)blockIdx.x % tiles_n * BN, m0 = (int)blockIdx.x / tiles_n * BM, rank = blockIdx.z;
   // this CTA's share of k, in whole blocks of BK
   const int blocks = (a.k + BK - 1) / BK, per = (blocks + splits - 1) / splits;
   const int first = rank * per, count = max(0, min(blocks, first + per) - first);
@@ -142,7 +142,7 @@ template <int BM, int BN, int TM, int TN>
 cudaError_t launch_tile(const LinearArgs& a, int epi, int splits, cudaStream_t s) {
   using T = F32Tile<BM, BN, TM, TN>;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((a.n + BN - 1) / BN, (a.m + BM - 1) / BM, splits);
+  cfg.gridDim = dim3((unsigned)((a.n + BN - 1) / BN) * (unsigned)((a.m + BM - 1) / BM), 1, splits);  // rows alone may be more than y holds
   cfg.blockDim = dim3(T::THREADS);
   cfg.dynamicSmemBytes = T::SMEM;
   cfg.stream = s;

@@ -49,6 +49,13 @@ def test_linear_fp32_tiles_match_oracle(oracle, m, n, k, epilogue):
     np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
 
 
+def test_linear_fp32_of_more_rows_than_a_grid_dimension_holds():
+    """One row more than 65535 tiles of 64."""
+    m = 65535 * 64 + 1
+    x, w = np.arange(4 * m, dtype=np.float32).reshape(m, 4) % 97, np.float32([[1, 2, 3, 4]])
+    np.testing.assert_array_equal(ops.linear(x, w)[0], x @ w.T)  # whole numbers below 2^24
+
+
 @pytest.mark.parametrize("m,n,k", [(9, 4800, 1600), (16, 1600, 1600), (64, 6400, 1600), (33, 1600, 6400),
                                    (64, 50257, 1024), (40, 1000, 256)])
 @pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
