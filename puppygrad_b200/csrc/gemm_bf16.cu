@@ -273,9 +273,8 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // A block multiplies 128 weight rows with the m <= BN input rows over its share of k, leaves the partial sums in its shared
 // memory (where the operands were), and the blocks of the cluster each add and store an equal part of the tile, in split order.
 //
-// Bound by the weight stream, so the grid is made to fill the chip (launch_rows_bn), and a block takes less than half of an SM's
-// shared memory: the next kernel's blocks find room beside the running ones and have their first weights loaded when
-// the dependency is released.
+// Bound by the weight stream. A block takes less than half of an SM's shared memory: the next kernel's blocks find room beside the
+// running ones and have their first weights loaded when the dependency is released.
 template <int BN>
 __global__ void __launch_bounds__(192, 2)
     tc_gemm_bf16_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, Bf16GemmArgs a,

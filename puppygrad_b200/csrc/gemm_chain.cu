@@ -21,7 +21,7 @@
 //               phases (one warp per sequence-head pair), the embedding and the end-of-step phase.
 //
 // Weights arrive as pairs, so nothing splits them on the way (FP32 tiles, split by four warps into three TF32 products, took 24
-// MMAs per 64 values of k; this takes 12, or 4 with BF16 weights) and BF16 weights are half the bytes. A step of GPT-2 medium
+// MMAs per 64 values of k; this takes 8, or 4 with BF16 weights) and BF16 weights are half the bytes. A step of GPT-2 medium
 // with 64 sequences 1.39 -> 1.25 ms, of XL with 32 at 512 positions 5.67 -> 5.1 ms; what bounds it is the chain of phases: a grid
 // barrier each, L2 round trips behind it, and the keys and values of the attention phases.
 //

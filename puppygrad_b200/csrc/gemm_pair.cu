@@ -49,10 +49,10 @@ struct PairSmem {
 // that grows with the MMAs into one accumulator, so the hi.hi products have one of their own and the small terms another.
 // hi_x times the hi and the lo weight tile, which lie next to each other, is one MMA of N = 256 into both.
 //
-// Bound by operand bytes: a k block of 64 moves 64 KB from L2 to shared memory and 80 KB from there into the tensor core
-// for 768 clocks of tensor work. Mean of a layer's four products, useful TFLOP/s (a third of the FP16 rate is 530):
-// 8192 rows of GPT-2 small 343 (three TF32 products of FP32 words: 184), 16384 rows of GPT-2 XL 448 (207). Relative error
-// against 64 bits of 16384 x 4800 x 1600: 1.9e-6.
+// Bound by the tensor pipe where k is long: 82% of its active cycles at 8192 x 4800 x 1600; 66% at 8192 x 2304 x 768, where L2 (38%)
+// and shared memory (28% of its reads, 23% of its writes) are no nearer their limits. Mean of a layer's four products, useful
+// TFLOP/s (a third of the FP16 rate is 530): 8192 rows of GPT-2 small 343 (three TF32 products of FP32 words: 184), 16384 rows of
+// GPT-2 XL 448 (207). Relative error against 64 bits of 16384 x 4800 x 1600: 1.9e-6.
 template <bool EXACT_W>
 __global__ void __launch_bounds__(192, 1)
     tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_constant__ CUtensorMap map_xl,

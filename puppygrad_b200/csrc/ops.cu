@@ -177,8 +177,8 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
       PG_OP_TRY(cudaMemsetAsync(dbar.p, 0, 4, s));
       chain.partials = dpart.as<float>(); chain.barrier = dbar.as<unsigned>();
       if (want_trace) {
-        PG_OP_TRY(cudaMalloc(&dtrace.p, (size_t)g * 256 + 4096));
-        PG_OP_TRY(cudaMemset(dtrace.p, 0, (size_t)g * 256 + 4096));
+        PG_OP_TRY(cudaMalloc(&dtrace.p, (size_t)g * 256));
+        PG_OP_TRY(cudaMemset(dtrace.p, 0, (size_t)g * 256));
         chain.trace = dtrace.as<unsigned long long>();
       }
       if (chain_supported(chain, g)) chain_ctas = g;
@@ -218,7 +218,7 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
   }
   if (want_trace && dtrace.p && chain_ctas > 0) {
     // tuning aid: when worker thread 0 of each CTA left each phase, relative to the earliest start
-    std::vector<unsigned long long> t((size_t)chain_ctas * 32 + 512);
+    std::vector<unsigned long long> t((size_t)chain_ctas * 32);
     PG_OP_TRY(cudaMemcpy(t.data(), dtrace.p, t.size() * 8, cudaMemcpyDeviceToHost));
     unsigned long long t0 = ~0ULL;
     for (int i = 0; i < chain_ctas; ++i) t0 = std::min(t0, t[(size_t)i * 32 + 31]);
@@ -229,12 +229,6 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
         lo = std::min(lo, v); hi = std::max(hi, v); wlo = std::min(wlo, w); whi = std::max(whi, w);
       }
       fprintf(stderr, "chain trace phase %d: work done %6llu..%6llu ns, barrier passed %6llu..%6llu ns\n", sl, wlo, whi, lo, hi);
-    }
-    const char* cn[6] = {"split wait w_full", "split wait tmem", "mma wait ready", "(unused)", "mma issue", "mma wait d_empty"};
-    for (int sl = 0; sl < 6; ++sl) {
-      double mean = 0;
-      for (int i = 0; i < chain_ctas; ++i) mean += (double)t[(size_t)i * 32 + 20 + sl];
-      fprintf(stderr, "chain trace %-18s mean %8.0f cycles per CTA\n", cn[sl], mean / chain_ctas);
     }
   } else if (want_trace && dtrace.p) {
     // tuning aid: phase timestamps of the last launch, relative to the earliest CTA start

@@ -161,8 +161,9 @@ struct pg_cache {
   unsigned long long* d_chain_best = nullptr;  // row arg-max accumulators of the lm_head phase
   unsigned long long* d_chain_trace = nullptr;  // developer aid: only allocated in builds with -DPG_DEV_TRACE
   int chain_ctas = 0;
-  // Smallest batch whose decode step runs as the chain kernel: 9 in the FP32-grade modes (8 sequences as the chain kernel / as one
-  // kernel per operation, us: GPT-2 small 511 / 493, medium 1026 / 1052), 5 with BF16 weights (enqueue_decode_step).
+  // Smallest batch whose decode step runs as the chain kernel: 9 in the FP32-grade modes, where up to 8 sequences are promised FP32
+  // multiply-adds (as the chain kernel / as one kernel per operation 8 would take, us: GPT-2 small 506 / 488, medium 1018 / 1064, XL
+  // 2816 / 3717), 5 with BF16 weights (enqueue_decode_step).
   int chain_min_batch = 9;
   struct ChainProgram {  // whole-step phase list of the persistent chain kernel for one batch size
     ChainPhase* dev = nullptr;            // in device memory (nullptr: this batch size is not supported)

@@ -196,7 +196,7 @@ def test_token_by_token_prefill_equals_batched_prefill(midi):
                                              (33, "tf32x3"), (64, "tf32x3"), (70, "tf32x3"), (130, "tf32x3")])
 def test_ragged_batches_match_single_sequences(midi, oracle, batch, math_mode):
     cfg, w, g, o = midi
-    if math_mode != "fp32":  # linears as three TF32 tensor-core products with FP32 accumulation
+    if math_mode != "fp32":  # linears as three tensor-core products with FP32 accumulation
         g = pg.Gpt2Model(cfg, w, pg.Gpt2CudaConfig(math_mode=math_mode))
     prompts = [synthetic.uniform_prompt(100 + i, 3 + 7 * i % 40 + i, cfg["vocab_size"]) for i in range(batch)]
     cache = g.new_kv_cache(max_batch=batch)
