@@ -70,16 +70,19 @@ __device__ __forceinline__ float norm_step_square(float4 v, float mean, int c, i
   return q;
 }
 
-// (v - mean) * rstd * g [+ b], zero past width (g and b are padded to the row pitch).
-__device__ __forceinline__ float4 norm_step_apply(float4 v, float mean, float rstd, const float* g, const float* b, int c,
-                                                  int width) {
-  const float4 gg = load4(g + c), bb = b ? load4(b + c) : make_float4(0, 0, 0, 0);
+// (v - mean) * rstd * g + b, zero past width.
+__device__ __forceinline__ float4 norm_step_scale(float4 v, float mean, float rstd, float4 gg, float4 bb, int c, int width) {
   float4 o;
   o.x = (v.x - mean) * rstd * gg.x + bb.x;
   o.y = (v.y - mean) * rstd * gg.y + bb.y;
   o.z = (v.z - mean) * rstd * gg.z + bb.z;
   o.w = (v.w - mean) * rstd * gg.w + bb.w;
   return mask4(o, c, width);
+}
+// The same with g and b (or none) in memory, padded to the row pitch.
+__device__ __forceinline__ float4 norm_step_apply(float4 v, float mean, float rstd, const float* g, const float* b, int c,
+                                                  int width) {
+  return norm_step_scale(v, mean, rstd, load4(g + c), b ? load4(b + c) : make_float4(0, 0, 0, 0), c, width);
 }
 
 }  // namespace

@@ -84,14 +84,13 @@ def assert_stream(tokens, want, gaps, n_prompt, bound):
     assert len(tokens) == len(want)
 
 
-def many_sequences(case):
-    """Two decode steps of 61 sequences of different lengths."""
-    n = 61
-    model = case.model("fp32")
+def many_sequences(case, n=61, mode="fp32"):
+    """Two decode steps of n sequences of different lengths."""
+    model = case.model(mode)
     cache = model.new_kv_cache(max_batch=n)
     ids, at = [case.ids(8, seed=i) for i in range(n)], [2 + i % 4 for i in range(n)]
     model.extend(range(n), [x[:t] for x, t in zip(ids, at)], cache)
     for _ in range(2):
         got = model.forward_one_batch([x[t] for x, t in zip(ids, at)], cache, want_logits=True)[0]
         at = [t + 1 for t in at]
-        assert_rows(got, np.stack([case.want(x[:t])[-1] for x, t in zip(ids, at)]), "fp32")
+        assert_rows(got, np.stack([case.want(x[:t])[-1] for x, t in zip(ids, at)]), mode)

@@ -68,6 +68,12 @@ def test_steps_of_many_sequences(name):
     many_sequences(Case(MANY[name], 7, rank=9))
 
 
+# Rows whose norms stay in registers and longer ones, by the number of sequences (1, 2 and 4 rows of a block's warps; a block per row).
+@pytest.mark.parametrize("width, n", [(1020, 1), (1028, 1), (2052, 1), (1020, 2), (2052, 2), (1020, 3), (1028, 3), (1020, 9), (1028, 9), (2052, 9)])
+def test_norms_of_wide_rows(width, n):
+    many_sequences(Case(lo.config(61, width, [lo.gla(2, 8, 12, ff=64)]), 5, rank=3), n, "bf16")
+
+
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("name", ALONE)
 def test_mechanism_alone(name, mode):
