@@ -250,13 +250,15 @@ __global__ void __launch_bounds__(192, 1)
 }
 
 // ------------------------------------------------------------------ decode rows
-template <int BN>
+// A ring of stages of ROWS weight rows and BN input rows. The ring is smaller than half an SM's shared memory: the next kernel's blocks
+// find room beside the running ones and have their first weights loaded when the dependency is released.
+template <int BN, int ROWS>
 struct RowsSmem {
-  static constexpr int STAGES = BN == 64 ? 4 : 5;
-  static constexpr int A_BYTES = TILE_M * KB * 2, B_BYTES = BN * KB * 2;
+  static constexpr int A_BYTES = ROWS * KB * 2, B_BYTES = BN * KB * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // both multiples of 1024
+  static constexpr int STAGES = ROWS == 64 ? (BN == 64 ? 6 : BN == 32 ? 8 : 9) : BN == 64 ? 4 : 5;
   static constexpr size_t BYTES = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
-  static_assert(TILE_M * BN * 4 <= STAGES * STAGE_BYTES, "the partial sums reuse the ring");
+  static_assert(ROWS * BN * 4 <= STAGES * STAGE_BYTES, "the partial sums reuse the ring");
   static_assert(2 * (BYTES + 1024) <= 228 * 1024, "two blocks on an SM");
 };
 
@@ -270,19 +272,19 @@ __device__ __forceinline__ float4 cluster_load4(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// A block multiplies 128 weight rows with the m <= BN input rows over its share of k, leaves the partial sums in its shared
+// A block multiplies ROWS weight rows with the m <= BN input rows over its share of k, leaves the partial sums in its shared
 // memory (where the operands were), and the blocks of the cluster each add and store an equal part of the tile, in split order.
 //
-// Bound by the weight stream. A block takes less than half of an SM's shared memory: the next kernel's blocks find room beside the
-// running ones and have their first weights loaded when the dependency is released.
-template <int BN>
+// Bound by the weight stream: 64 rows, inside a step, us (and TB/s) with ROWS 128 and with 64: 2048 x 8192 in four parts 16.5 -> 14.3 (2.3),
+// 14656 x 2048 in one 20.4 -> 16.3 (3.7), 9536 x 2048 21.6 -> 16.2 (2.4); 32000 x 2048, which has 250 blocks of 128, 25.6 (5.1).
+template <int BN, int ROWS>
 __global__ void __launch_bounds__(192, 2)
     tc_gemm_bf16_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, Bf16GemmArgs a,
                              int out_kind) {
-  using S = RowsSmem<BN>;
+  using S = RowsSmem<BN, ROWS>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* part = reinterpret_cast<float*>(base);  // [BN][TILE_M], once the products are done
+  float* part = reinterpret_cast<float*>(base);  // [BN][ROWS], once the products are done
   uint64_t* full = reinterpret_cast<uint64_t*>(base + (size_t)S::STAGES * S::STAGE_BYTES);
   uint64_t* empty = full + S::STAGES;
   uint64_t* d_full = empty + S::STAGES;
@@ -291,10 +293,12 @@ __global__ void __launch_bounds__(192, 2)
   constexpr uint32_t COLS = BN < 32 ? 32 : BN;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * TILE_M, split = blockIdx.y, splits = gridDim.y;
+  const int n0 = blockIdx.x * ROWS, split = blockIdx.y, splits = gridDim.y;
   const int nkb_all = (a.k + KB - 1) / KB, kb0 = nkb_all * split / splits, nkb = nkb_all * (split + 1) / splits - kb0;
   const int head = blockIdx.z, x0 = head * a.x_head;
-  const int wrow = ((head * (int)gridDim.x + (int)blockIdx.x) * nkb_all + kb0) * TILE_M;  // first row of this block's run of weight tiles
+  // first row of this block's part of the weight tiles, which have TILE_M rows
+  const int row_tiles = ((int)gridDim.x * ROWS + TILE_M - 1) / TILE_M;
+  const int wrow = ((head * row_tiles + n0 / TILE_M) * nkb_all + kb0) * TILE_M + n0 % TILE_M;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) {
@@ -335,7 +339,7 @@ __global__ void __launch_bounds__(192, 2)
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16(TILE_M, BN);
+      const uint32_t idesc = umma_idesc_bf16(ROWS, BN);
       bool ok = true;
       RingCursor c;
       for (int i = 0; i < nkb; ++i, c.next(S::STAGES)) {
@@ -351,7 +355,8 @@ __global__ void __launch_bounds__(192, 2)
       if (ok) umma_commit(d_full);
     }
   } else {
-    const int r = (warp & 3) * 32 + lane;
+    // Rows of an accumulator of 128 lie in the 128 lanes of tensor memory, those of 64 in the first sixteen of every 32.
+    const int r = ROWS == 128 ? (warp & 3) * 32 + lane : (warp & 3) * 16 + lane;
     bool ok = mbar_wait(d_full, 0, failed, a.error_flag, 13);
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
@@ -361,7 +366,8 @@ __global__ void __launch_bounds__(192, 2)
         float v[16];
         tmem_ld16(tmem_d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) part[(c0 + j) * TILE_M + r] = v[j];
+        for (int j = 0; j < 16; ++j)
+          if (ROWS == 128 || lane < 16) part[(c0 + j) * ROWS + r] = v[j];
       }
     }
   }
@@ -376,9 +382,9 @@ __global__ void __launch_bounds__(192, 2)
     const uint32_t part_addr = smem_u32(part);
     const bool vec = a.ldo % 4 == 0 && a.out_head % 4 == 0 &&  // four results in one store
                      ((out_kind == OUT_F32 ? reinterpret_cast<uintptr_t>(a.out) : reinterpret_cast<uintptr_t>(a.out_h)) & 15) == 0;
-    const int pieces = a.m * (TILE_M / 4), first = pieces * split / splits, last = pieces * (split + 1) / splits;
+    const int pieces = a.m * (ROWS / 4), first = pieces * split / splits, last = pieces * (split + 1) / splits;
     for (int i = first + (int)threadIdx.x; i < last; i += 192) {
-      const int j = i / (TILE_M / 4), f0 = n0 + (i % (TILE_M / 4)) * 4;
+      const int j = i / (ROWS / 4), f0 = n0 + (i % (ROWS / 4)) * 4;
       float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
       if (splits == 1) {
         sum = reinterpret_cast<const float4*>(part)[i];
@@ -467,26 +473,17 @@ cudaError_t launch_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
   return launch_kernel(tc_gemm_bf16_kernel<BN>, dim3(std::min(tiles, sm_count())), dim3(192), smem, s, pdl, mx, mw, mo, a, kind, tma_out);
 }
 
-template <int BN>
-cudaError_t launch_rows_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
-  // Parts of k: a power of two that gives every SM at most one block, each part of at least two k blocks; eight only where the matrix
-  // has eight row tiles or fewer. The parts are where a sum is rounded, and so which way BF16 results behind it fall: up to eight parts, or
-  // four where that gives an SM two blocks, are faster (steps of 64 sequences of width 2048 with their prompts, 24 of them: Dirurax
-  // 25.9 instead of 27.3 ms, Sanesun 23.1 instead of 24.8), but 0.4% off in what a model says. Blocks of 176 KB with the sums pushed into
-  // a buffer of their peers: 30.2 and 27.5 ms.
-  const int row_tiles = (a.n + TILE_M - 1) / TILE_M, heads = std::max(a.heads, 1), nkb = (a.k + KB - 1) / KB, tiles = row_tiles * heads;
-  const int most = tiles <= 8 ? 8 : 4;
-  int splits = 1;
-  while (splits < most && tiles * splits * 2 <= sm_count() && splits * 4 <= nkb) splits *= 2;
+template <int BN, int ROWS>
+cudaError_t launch_rows_tile(const Bf16GemmArgs& a, int row_tiles, int heads, int splits, bool pdl, cudaStream_t s) {
   CUtensorMap mx, mw;
-  if (!make_map_bf16(&mx, a.x, a.m, a.heads ? a.ldx : a.k, BN) || !make_map_bf16(&mw, a.w_tiled, (uint64_t)heads * row_tiles * (a.k / KB) * TILE_M, KB, TILE_M))
+  if (!make_map_bf16(&mx, a.x, a.m, a.heads ? a.ldx : a.k, BN) || !make_map_bf16(&mw, a.w_tiled, (uint64_t)heads * row_tiles * (a.k / KB) * TILE_M, KB, ROWS))
     return cudaErrorInvalidValue;
-  auto kernel = tc_gemm_bf16_rows_kernel<BN>;
-  const size_t smem = RowsSmem<BN>::BYTES;
+  auto kernel = tc_gemm_bf16_rows_kernel<BN, ROWS>;
+  const size_t smem = RowsSmem<BN, ROWS>::BYTES;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(row_tiles, splits, heads);
+  cfg.gridDim = dim3((a.n + ROWS - 1) / ROWS, splits, heads);
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -500,6 +497,22 @@ cudaError_t launch_rows_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, mx, mw, a, out_kind_of(a));
+}
+
+template <int BN>
+cudaError_t launch_rows_bn(const Bf16GemmArgs& a, bool pdl, cudaStream_t s) {
+  // Parts of k: a power of two that gives every SM at most one block of 128 weight rows, each part of at least two k blocks; eight only
+  // where the matrix has eight row tiles or fewer. The parts are where a sum is rounded, and so which way BF16 results behind it fall:
+  // other parts were up to 0.4% off in what a model says.
+  const int row_tiles = (a.n + TILE_M - 1) / TILE_M, heads = std::max(a.heads, 1), nkb = (a.k + KB - 1) / KB, tiles = row_tiles * heads;
+  const int most = tiles <= 8 ? 8 : 4;
+  int splits = 1;
+  while (splits < most && tiles * splits * 2 <= sm_count() && splits * 4 <= nkb) splits *= 2;
+  // Half tiles, the same sums in twice the blocks, where whole ones leave SMs without a second block: steps of 64 sequences of width 2048 with
+  // their prompts, 24 of them, Dirurax 26.9 -> 25.5 ms, Sanesun 24.7 -> 23.1 (with four stages instead of six 26.3 and 23.9); 12 sequences of
+  // width 1024 the same within the spread.
+  return tiles * splits <= sm_count() ? launch_rows_tile<BN, 64>(a, row_tiles, heads, splits, pdl, s)
+                                      : launch_rows_tile<BN, 128>(a, row_tiles, heads, splits, pdl, s);
 }
 
 }  // namespace

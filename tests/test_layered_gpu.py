@@ -68,6 +68,14 @@ def test_steps_of_many_sequences(name):
     many_sequences(Case(MANY[name], 7, rank=9))
 
 
+# Products of 9 to 64 rows take tiles of 64 weight rows: one row, whole and half tiles, and a row or two beside them; two tiles of 128 to a tile
+# of the weights' layout; input rows at the edges of 16, 32 and 64; k in one part and in several.
+@pytest.mark.parametrize("vocab", [63, 64, 65, 127, 129, 193])
+@pytest.mark.parametrize("width, n", [(48, 9), (48, 16), (192, 17), (192, 33), (600, 61)])
+def test_products_of_half_tiles(vocab, width, n):
+    many_sequences(Case(lo.config(vocab, width, [lo.gla(2, 8, 12, ff=72)]), 5, rank=3), n, "bf16")
+
+
 # Rows whose norms stay in registers and longer ones, by the number of sequences (1, 2 and 4 rows of a block's warps; a block per row).
 @pytest.mark.parametrize("width, n", [(1020, 1), (1028, 1), (2052, 1), (1020, 2), (2052, 2), (1020, 3), (1028, 3), (1020, 9), (1028, 9), (2052, 9)])
 def test_norms_of_wide_rows(width, n):
