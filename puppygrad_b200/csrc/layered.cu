@@ -822,7 +822,10 @@ cudaError_t layered_enqueue_decode(pg_cache* c, int batch, int splits, cudaStrea
   bool rows_path = m->bf16 && batch <= MAX_ROWS_LINEAR && rows_linear_supported(batch, m->max_y, false, 0) &&
                    rows_linear_supported(batch, m->head.kp, true, 0) && (m->max_mid == 0 || rows_linear_supported(batch, m->max_mid_k, true, 0)) &&
                    (m->max_ff == 0 || rows_linear_supported(batch, m->max_ff, false, 0));
-  const bool pdl = pm->use_pdl && (rows_path || m->bf16);
+  // Programmatic launches, but for the step's first: kernels read what earlier steps and prompts left behind (states, pages, positions)
+  // before their own dependency wait.
+  bool pdl = false;
+  const bool chain = pm->use_pdl && (rows_path || m->bf16);
   const bool y_bf16 = m->bf16 && !rows_path;
   void* y = rows_path ? (void*)r.y32 : r.y;
   cudaError_t e;
@@ -858,10 +861,13 @@ cudaError_t layered_enqueue_decode(pg_cache* c, int batch, int splits, cudaStrea
       na.h32 = rows32;
       if ((e = launch_norm_step(na, batch, true, pdl, s)) != cudaSuccess) return e;
       ++n;
+      pdl = chain;
       a.x = rows32;
       a.ldx = a.kx = w.kp;
     }
-    return launch_rows_linear(a, pdl, s, grid);
+    e = launch_rows_linear(a, pdl, s, grid);
+    pdl = chain;
+    return e;
   };
   auto rows_linear = [&](const Matrix& w, const float* x, const NormStepArgs* norm, float* out, int ldo, int n_out, const ActArgs* act, float* pv, int* pi,
                          int* grid) -> cudaError_t {
@@ -890,6 +896,7 @@ cudaError_t layered_enqueue_decode(pg_cache* c, int batch, int splits, cudaStrea
     float2* at = r.angles;
     for (const Rotation& rot : m->rotations) {
       PG_L(B_OTHER, launch_angles(c->d_pos, rot.freq, at, batch, rot.dims / 2, pdl, s));
+      pdl = chain;
       at += (size_t)batch * (rot.dims / 2);
     }
   }
@@ -967,6 +974,7 @@ cudaError_t layered_enqueue_decode(pg_cache* c, int batch, int splits, cudaStrea
       PG_L(B_QKV, run_rows(a, l.in, nullptr, 0, 0, &na, r.h32, nullptr));
     } else {
       PG_L(B_LAYER_NORM, launch_norm_step(step_norm(l.norm1), batch, m->bf16, pdl, s));
+      pdl = chain;
       PG_L(B_QKV, in_product(m, l, r.h, r.p, r.y, batch, c->d_error, pdl, s, &n));
     }
     advanced();
