@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_decode_kernel(LinearArgs a
 // ------------------------------------------------------------------ decode linear, activations in shared memory
 // The same operator as one persistent CTA of 16 warps per SM: with several input rows the kernel above
 // re-reads the activations from L1 once per input row and 16 weights, and starts a CTA (and, fused, a
-// LayerNorm) per four weight rows. Here a CTA stages the input rows once ([MT][k] floats, LayerNorm applied
-// in place when asked for) and its warps then walk units of (four weight rows, one of `kparts` parts of
+// LayerNorm) per four weight rows. Here a CTA stages the input rows once ([MT][k] floats; a LayerNorm, where asked
+// for, by one warp per row, which holds it in registers up to k = 1024) and its warps then walk units of (four weight rows, one of `kparts` parts of
 // k): 128-bit streaming loads of the weights, activations from shared memory (consecutive lanes,
 // consecutive 16-byte units: no bank conflict), one folding warp reduction per unit. With kparts = 1 the
 // lanes that hold the sums finish the rows; otherwise the parts of a row group, which are neighbouring
@@ -303,14 +303,19 @@ constexpr int LR_THREADS = 512;
 constexpr int LR_WARPS = LR_THREADS / 32;
 constexpr int LR_ROWS = 4;
 constexpr size_t LR_MAX_SMEM = 208 * 1024;  // [MT][k] floats
+// Rows of one launch: eight, or sixteen where it makes their LayerNorm. 11 rows of GPT-2 small behind a norm, us, in a prompt: norm and
+// linear_decode_kernel, which reads the weights once per eight rows, 11.2 (2304 x 768) and 14.1 (3072 x 768), this one about 8.5; without a norm that
+// kernel is the faster one (whole FP32 steps of 9 and 16 sequences 639 and 676 us, with this one for all products 677 and 740).
+constexpr int LR_NORM_ROWS = 16, LR_PLAIN_ROWS = 8;
 constexpr int LR_ONE_ROW_MIN_N = 16384;      // one input row takes this kernel only for the lm_head
 
 template <int MT, int EPI>
 __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearArgs a, int kp_shift) {
   extern __shared__ float4 dyn_smem4[];
-  float4* xs4 = dyn_smem4;  // [MT][k / 4]
+  float4* xs4 = dyn_smem4;  // [MT][k / 4]; above eight rows [a.m][k / 4]
   constexpr int NV = LR_ROWS * MT;
-  constexpr int SH = (NV == 32) ? 0 : (NV == 16) ? 1 : (NV == 8) ? 2 : 3;  // 5 - log2(NV)
+  constexpr int SH = (NV >= 32) ? 0 : (NV == 16) ? 1 : (NV == 8) ? 2 : 3;  // 5 - log2(NV)
+  constexpr int FOLDS = NV > 32 ? NV / 32 : 1, FV = NV / FOLDS;             // sums are folded over a warp's lanes 32 at a time
   __shared__ float part[LR_WARPS][NV];
   __shared__ float best_v[LR_WARPS][NV];
   __shared__ int best_i[LR_WARPS][NV];
@@ -325,63 +330,101 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
   const int g_first = (int)blockIdx.x * gpc + wg, g_stride = (int)gridDim.x * gpc;
 
   pdl_launch();
-  // weights do not depend on the previous kernel: the warp's first loads go out before the dependency wait
+  // weights do not depend on the previous kernel: the warp's first loads go out before the dependency wait, what follows is asked for as
+  // far as L2
   float4 wpre[LR_ROWS];
 #pragma unroll
-  for (int r = 0; r < LR_ROWS; ++r)
-    wpre[r] = (g_first < groups && c_beg + lane < c_end)
-                  ? ldg_stream(w4 + (size_t)min(g_first * LR_ROWS + r, a.n - 1) * k4 + c_beg + lane)
-                  : make_float4(0, 0, 0, 0);
+  for (int r = 0; r < LR_ROWS; ++r) {
+    const float4* row = w4 + (size_t)min(g_first * LR_ROWS + r, a.n - 1) * k4;
+    wpre[r] = (g_first < groups && c_beg + lane < c_end) ? ldg_stream(row + c_beg + lane) : make_float4(0, 0, 0, 0);
+    if (MT > 8 && g_first < groups)
+      for (int c = c_beg + 32 + lane * 8; c < c_end; c += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c));
+  }
   pdl_wait();
 
-  {
-    const float4* x4 = reinterpret_cast<const float4*>(a.x);
-    for (int idx = tid; idx < MT * k4; idx += LR_THREADS) {
-      const int r = idx / k4;
-      xs4[idx] = r < a.m ? x4[idx] : make_float4(0, 0, 0, 0);
-    }
+  const float4* x4 = reinterpret_cast<const float4*>(a.x);
+  constexpr int LN_HELD = 8;  // 16-byte pieces of a row per lane that fit the registers
+  const bool ln_held = a.ln_g && k4 <= 32 * LN_HELD;
+  const int have = a.m * k4, fill = MT > 8 ? have : MT * k4;
+  if (!ln_held) {
+    for (int idx = tid; idx < have; idx += LR_THREADS)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(xs4 + idx)), "l"(x4 + idx) : "memory");
+    for (int idx = have + tid; idx < fill; idx += LR_THREADS) xs4[idx] = make_float4(0, 0, 0, 0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
   }
-  __syncthreads();
   if (a.ln_g) {  // LayerNorm of each row, by one warp (layer_norm_in_place, src/models/cpu.rs:119-143, tree sums)
     const float4* g4 = reinterpret_cast<const float4*>(a.ln_g);
     const float4* b4 = reinterpret_cast<const float4*>(a.ln_b);
-    for (int r = warp; r < a.m && r < MT; r += LR_WARPS) {
-      float4* row = xs4 + (size_t)r * k4;
-      float sum = 0.f;
-      for (int c = lane; c < k4; c += 32) {
-        const float4 v = row[c];
-        sum += (v.x + v.y) + (v.z + v.w);
+    auto square = [](float4 v, float mean) {
+      const float d0 = v.x - mean, d1 = v.y - mean, d2 = v.z - mean, d3 = v.w - mean;
+      return (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
+    };
+    auto scaled = [](float4 v, float mean, float inv_std, float4 g, float4 b) {
+      return make_float4((v.x - mean) * inv_std * g.x + b.x, (v.y - mean) * inv_std * g.y + b.y, (v.z - mean) * inv_std * g.z + b.z,
+                         (v.w - mean) * inv_std * g.w + b.w);
+    };
+    if (ln_held) {
+      static_assert(MT <= LR_WARPS, "a warp per row");
+      if (warp < a.m) {
+        float4 v[LN_HELD], g[LN_HELD], b[LN_HELD];
+        float sum = 0.f, q = 0.f;
+#pragma unroll
+        for (int i = 0; i < LN_HELD; ++i) {
+          const int c = lane + 32 * i;
+          v[i] = c < k4 ? x4[(size_t)warp * k4 + c] : make_float4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < LN_HELD; ++i) {
+          const int c = lane + 32 * i;
+          g[i] = c < k4 ? g4[c] : make_float4(0, 0, 0, 0);
+          b[i] = c < k4 ? b4[c] : make_float4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < LN_HELD; ++i) sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        const float mean = warp_sum(sum) / (float)a.k;
+#pragma unroll
+        for (int i = 0; i < LN_HELD; ++i)
+          if (lane + 32 * i < k4) q += square(v[i], mean);
+        const float inv_std = 1.0f / sqrtf(warp_sum(q) / (float)a.k + a.eps);
+#pragma unroll
+        for (int i = 0; i < LN_HELD; ++i) {
+          const int c = lane + 32 * i;
+          if (c < k4) xs4[(size_t)warp * k4 + c] = scaled(v[i], mean, inv_std, g[i], b[i]);
+        }
       }
-      const float mean = warp_sum(sum) / (float)a.k;
-      float q = 0.f;
-      for (int c = lane; c < k4; c += 32) {
-        const float4 v = row[c];
-        const float d0 = v.x - mean, d1 = v.y - mean, d2 = v.z - mean, d3 = v.w - mean;
-        q += (d0 * d0 + d1 * d1) + (d2 * d2 + d3 * d3);
-      }
-      const float inv_std = 1.0f / sqrtf(warp_sum(q) / (float)a.k + a.eps);
-      for (int c = lane; c < k4; c += 32) {
-        const float4 g = g4[c], b = b4[c];
-        float4 v = row[c];
-        v.x = (v.x - mean) * inv_std * g.x + b.x;
-        v.y = (v.y - mean) * inv_std * g.y + b.y;
-        v.z = (v.z - mean) * inv_std * g.z + b.z;
-        v.w = (v.w - mean) * inv_std * g.w + b.w;
-        row[c] = v;
+      for (int idx = have + tid; idx < fill; idx += LR_THREADS) xs4[idx] = make_float4(0, 0, 0, 0);
+    } else {
+      for (int r = warp; r < a.m && r < MT; r += LR_WARPS) {
+        float4* row = xs4 + (size_t)r * k4;
+        float sum = 0.f, q = 0.f;
+        for (int c = lane; c < k4; c += 32) {
+          const float4 v = row[c];
+          sum += (v.x + v.y) + (v.z + v.w);
+        }
+        const float mean = warp_sum(sum) / (float)a.k;
+        for (int c = lane; c < k4; c += 32) q += square(row[c], mean);
+        const float inv_std = 1.0f / sqrtf(warp_sum(q) / (float)a.k + a.eps);
+        for (int c = lane; c < k4; c += 32) row[c] = scaled(row[c], mean, inv_std, g4[c], b4[c]);
       }
     }
     __syncthreads();
   }
 
-  // after the warp reduction the lanes with (lane & (2^SH - 1)) == 0 hold sum number lane >> SH = r * MT + m
+  // after the warp reduction the lanes with (lane & (2^SH - 1)) == 0 hold sum number lane >> SH = r * MT + m (of every fold)
   const bool holder = (lane & ((1 << SH) - 1)) == 0;
   // who finishes a sum: with kparts = 1 the holder lanes of the warp, else thread t < gpc * NV for (group slot, sum)
   const bool finisher = kparts == 1 ? holder : tid < gpc * NV;
-  const int fs = kparts == 1 ? (lane >> SH) : tid % NV;  // sum number
+  const int own = kparts == 1 ? FOLDS : 1;               // sums a finisher has
+  const int fs = kparts == 1 ? (lane >> SH) : tid % NV;  // number of its first one; the next is FV on
   const int fslot = kparts == 1 ? wg : tid / NV;         // group slot
-  const int fr = fs / MT, fm = fs % MT;
-  float run_best = -INFINITY;  // lm_head arg-max partial of this finisher's (row in group, input row) pair
-  int run_idx = INT_MAX;
+  float run_best[FOLDS];  // lm_head arg-max partial of this finisher's (row in group, input row) pairs
+  int run_idx[FOLDS];
+#pragma unroll
+  for (int h = 0; h < FOLDS; ++h) {
+    run_best[h] = -INFINITY;
+    run_idx[h] = INT_MAX;
+  }
 
   // every warp of the CTA makes the same number of rounds (the CTA barrier inside needs all of them)
   const int rounds = (groups - (int)blockIdx.x * gpc + g_stride - 1) / g_stride;
@@ -390,12 +433,22 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
     const bool live = g < groups;
     const int row0 = g * LR_ROWS;
     // what the epilogue needs from memory, asked for before the loop
-    const int orow = ((int)blockIdx.x * gpc + fslot + it * g_stride) * LR_ROWS + fr;
-    const bool fin = finisher && orow < a.n && fm < a.m && ((int)blockIdx.x * gpc + fslot + it * g_stride) < groups;
-    float bias_v = 0.f, resid_v = 0.f;
-    if (fin) {
-      if (a.bias) bias_v = a.bias[orow];
-      if (EPI == EPI_RESID) resid_v = a.resid[(size_t)fm * a.n + orow];
+    const int fgroup = (int)blockIdx.x * gpc + fslot + it * g_stride;
+    auto sum_of = [&](int h, int* orow, int* fm) {  // whether this thread finishes its sum h, and of which weight row and input row
+      const int i = fs + h * FV;
+      *orow = fgroup * LR_ROWS + i / MT;
+      *fm = i % MT;
+      return finisher && h < own && fgroup < groups && *orow < a.n && *fm < a.m;
+    };
+    float bias_v[FOLDS], resid_v[FOLDS];
+#pragma unroll
+    for (int h = 0; h < FOLDS; ++h) {
+      int orow, fm;
+      bias_v[h] = resid_v[h] = 0.f;
+      if (sum_of(h, &orow, &fm)) {
+        if (a.bias) bias_v[h] = a.bias[orow];
+        if (EPI == EPI_RESID) resid_v[h] = a.resid[(size_t)fm * a.n + orow];
+      }
     }
     float acc[NV];
 #pragma unroll
@@ -407,7 +460,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
       auto accumulate = [&](const float4 (&w)[LR_ROWS], int c) {
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-          const float4 xv = xs4[(size_t)m * k4 + c];
+          const float4 xv = xs4[(size_t)(MT > 8 ? min(m, a.m - 1) : m) * k4 + c];  // sums past the last row go nowhere
 #pragma unroll
           for (int r = 0; r < LR_ROWS; ++r) acc[r * MT + m] = dot4(w[r], xv, acc[r * MT + m]);
         }
@@ -417,7 +470,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
         if (c < c_end) accumulate(wpre, c);
         c += 32;
       }
-      constexpr int UNR = MT >= 4 ? 2 : 4;  // iterations whose loads are in flight together (registers permitting)
+      constexpr int UNR = MT > 8 ? 1 : MT >= 4 ? 2 : 4;  // iterations whose loads are in flight together (registers permitting)
 #pragma unroll(UNR)
       for (; c < c_end; c += 32) {
         float4 w[LR_ROWS];
@@ -425,25 +478,32 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
         for (int r = 0; r < LR_ROWS; ++r) w[r] = ldg_stream(wrow[r] + c);
         accumulate(w, c);
       }
-      WarpMultiReduce<NV, 16>::run(acc, lane);
+#pragma unroll
+      for (int h = 0; h < FOLDS; ++h) WarpMultiReduce<FV, 16>::run(acc + h * FV, lane);
     }
-    float total = acc[0];
     if (kparts > 1) {
-      if (holder) part[warp][lane >> SH] = acc[0];
+      if (holder) {
+#pragma unroll
+        for (int h = 0; h < FOLDS; ++h) part[warp][(lane >> SH) + h * FV] = acc[h * FV];
+      }
       __syncthreads();
-      if (fin) {
+    }
+#pragma unroll
+    for (int h = 0; h < FOLDS; ++h) {
+      int orow, fm;
+      if (!sum_of(h, &orow, &fm)) continue;
+      float total = acc[h * FV];
+      if (kparts > 1) {
         total = 0.f;
         for (int q = 0; q < kparts; ++q) total += part[(fslot << kp_shift) + q][fs];  // in part order
       }
-    }
-    if (fin) {
-      float v = a.bias ? bias_v + total : total;
+      float v = a.bias ? bias_v[h] + total : total;
       if (EPI == EPI_GELU) v = gelu_ref(v);
-      if (EPI == EPI_RESID) v = resid_v + v;
+      if (EPI == EPI_RESID) v = resid_v[h] + v;
       a.out[(size_t)fm * a.n + orow] = v;
-      if (a.part_val && v > run_best) {
-        run_best = v;
-        run_idx = orow;
+      if (a.part_val && v > run_best[h]) {
+        run_best[h] = v;
+        run_idx[h] = orow;
       }
     }
     if (kparts > 1) __syncthreads();  // `part` is rewritten in the next round
@@ -453,12 +513,15 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
     // finishers: kparts = 1: holder lanes of every warp, sum number lane >> SH; else threads t < gpc * NV
     if (kparts == 1) {
       if (holder) {
-        best_v[warp][lane >> SH] = run_best;
-        best_i[warp][lane >> SH] = run_idx;
+#pragma unroll
+        for (int h = 0; h < FOLDS; ++h) {
+          best_v[warp][(lane >> SH) + h * FV] = run_best[h];
+          best_i[warp][(lane >> SH) + h * FV] = run_idx[h];
+        }
       }
     } else if (tid < gpc * NV) {
-      best_v[tid / NV][tid % NV] = run_best;
-      best_i[tid / NV][tid % NV] = run_idx;
+      best_v[tid / NV][tid % NV] = run_best[0];
+      best_i[tid / NV][tid % NV] = run_idx[0];
     }
     __syncthreads();
     if (tid < MT && tid < a.m) {
@@ -1094,6 +1157,74 @@ __global__ void __launch_bounds__(128) prefill_attention_kernel(PrefillAttnArgs 
   }
 }
 
+// Prompts of at most PS_KEYS tokens, head_dim 64: a block takes `per_block` queries of one head of one sequence, a warp one of them at
+// a time, with all keys and values they see in shared memory, and writes its own positions' keys and values to the cache (where there is one)
+// on the way. Bound by latency: 11 tokens, 12 heads 4.9 us; tiles of 64 queries and keys, and a kernel that fills the cache, 14.1 and 2.4.
+constexpr int PS_KEYS = 64, PS_PITCH = 68, PS_THREADS = 256;
+__global__ void __launch_bounds__(PS_THREADS) prefill_attention_small_kernel(PrefillAttnArgs a, int per_block) {
+  constexpr int D = 64, D4 = D / 4, WARPS = PS_THREADS / 32;
+  __shared__ float4 ks[PS_KEYS * PS_PITCH / 4], vs[PS_KEYS * D4], qs[WARPS][D4];
+  const int h = blockIdx.x, q0 = blockIdx.y * per_block, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c4 = a.n_head * D4;
+  pdl_launch();
+  pdl_wait();
+  const int r0 = a.seq_start[b], len = a.seq_start[b + 1] - r0, q1 = min(q0 + per_block, len);
+  if (q0 >= len) return;
+  const float4* rows = reinterpret_cast<const float4*>(a.qkv) + (size_t)r0 * 3 * c4 + h * D4;
+  for (int i = tid; i < q1 * D4; i += PS_THREADS) {
+    const int r = i / D4, d = i % D4;
+    const float4 k = rows[(size_t)r * 3 * c4 + c4 + d], v = rows[(size_t)r * 3 * c4 + 2 * c4 + d];
+    ks[r * (PS_PITCH / 4) + d] = k;
+    vs[i] = v;
+    if (a.kv_pool && r >= q0) {
+      const int page = a.page_table[(size_t)a.row_slot[r0 + r] * a.kv.pages_per_seq + r / a.kv.page_tokens], off = r % a.kv.page_tokens;
+      reinterpret_cast<float4*>(a.kv_pool + kv_row_offset(a.kv, page, 0, h, off))[d] = k;
+      reinterpret_cast<float4*>(a.kv_pool + kv_row_offset(a.kv, page, 1, h, off))[d] = v;
+    }
+  }
+  __syncthreads();
+  for (int q = q0 + warp; q < q1; q += WARPS) {
+    __syncwarp();
+    if (lane < D4) qs[warp][lane] = rows[(size_t)q * 3 * c4 + lane];
+    __syncwarp();
+    float s[2];  // keys lane and lane + 32
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int k = lane + 32 * j;
+      s[j] = -INFINITY;
+      if (k <= q) {
+        float t = 0.f;
+#pragma unroll
+        for (int d = 0; d < D4; ++d) t = dot4(qs[warp][d], ks[k * (PS_PITCH / 4) + d], t);
+        s[j] = t * 0.125f;  // 1 / sqrt(64)
+      }
+    }
+    const float mx = warp_max(fmaxf(s[0], s[1])), ref = mx == -INFINITY ? 0.f : mx;
+    const float p0 = expf(s[0] - ref), p1 = expf(s[1] - ref);
+    const float inv = 1.f / warp_sum(p0 + p1);
+    const int d = lane & 15, odd = lane >> 4;  // values: sixteen lanes per row, even and odd keys apart
+    float4 acc = make_float4(0, 0, 0, 0);
+    for (int k2 = 0; k2 <= q; k2 += 2) {
+      const int k = k2 + odd;
+      const float p = __shfl_sync(FULL, k2 < 32 ? p0 : p1, k & 31);
+      if (k <= q) {
+        const float4 v = vs[k * D4 + d];
+        acc.x = fmaf(p, v.x, acc.x); acc.y = fmaf(p, v.y, acc.y); acc.z = fmaf(p, v.z, acc.z); acc.w = fmaf(p, v.w, acc.w);
+      }
+    }
+    acc.x += __shfl_xor_sync(FULL, acc.x, 16);
+    acc.y += __shfl_xor_sync(FULL, acc.y, 16);
+    acc.z += __shfl_xor_sync(FULL, acc.z, 16);
+    acc.w += __shfl_xor_sync(FULL, acc.w, 16);
+    if (lane < D4) {
+      const size_t at = ((size_t)(r0 + q) * c4 + h * D4 + lane) * 4;
+      const float4 y = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+      if (a.pair.hi) store_pair4(a.pair.hi + at, a.pair.lo + at, y, a.pair.scale);
+      else *reinterpret_cast<float4*>(a.out + at) = y;
+    }
+  }
+}
+
 // Any head_dim <= 128: one thread per query, two passes over the keys.
 __global__ void prefill_attention_generic_kernel(PrefillAttnArgs a) {
   const int h = blockIdx.x, b = blockIdx.z;
@@ -1425,15 +1556,26 @@ int linear_decode_grid(int n, int sms) {
 // 758 / 789 / 921 / 1091 us with the shared-memory kernel); PG_LR_MIN_MT overrides it for tuning
 static int g_lr_min_mt = [] { const char* e = getenv("PG_LR_MIN_MT"); return e ? atoi(e) : 2; }();
 
+// Shared memory of linear_rows_smem_kernel: rows of zeros fill a tile of at most eight, no room is spent on them above.
+static size_t linear_rows_smem(int m, int k) {
+  const int rows = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : m <= 8 ? 8 : m;
+  return (size_t)rows * k * sizeof(float);
+}
+static bool linear_rows_in_smem(int m, int k, bool norm) { return m <= (norm ? LR_NORM_ROWS : LR_PLAIN_ROWS) && linear_rows_smem(m, k) <= LR_MAX_SMEM; }
+
+bool linear_decode_fuses_norm(int m, int k) {
+  return k % 4 == 0 && k <= 2048 && (m <= 8 || linear_rows_in_smem(m, k, true));
+}
+
 cudaError_t launch_linear_decode(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s, int* grid_out) {
-  if (a.k % 4 != 0 || (a.ln_g && (a.m > 8 || a.k > 2048)) || (a.part_val && a.m > 8)) {
+  if (a.k % 4 != 0 || (a.ln_g && !linear_decode_fuses_norm(a.m, a.k)) || (a.part_val && a.m > 8)) {
     if (a.ln_g || a.part_val) return cudaErrorInvalidValue;  // callers un-fuse these cases
     size_t total = (size_t)a.m * a.n;
     if (grid_out) *grid_out = 0;
     return launch(linear_generic_kernel, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, s, pdl, a, epilogue);
   }
-  int mt = a.m <= 1 ? 1 : a.m <= 2 ? 2 : a.m <= 4 ? 4 : 8;
-  if (a.m <= 8 && (mt >= g_lr_min_mt || a.n >= LR_ONE_ROW_MIN_N) && (size_t)mt * a.k * sizeof(float) <= LR_MAX_SMEM) {
+  const int mt = a.m <= 1 ? 1 : a.m <= 2 ? 2 : a.m <= 4 ? 4 : 8;
+  if (linear_rows_in_smem(a.m, a.k, a.ln_g != nullptr) && (mt >= g_lr_min_mt || a.n >= LR_ONE_ROW_MIN_N)) {
     // activations staged in shared memory, one persistent CTA per SM; k is shared out over the warps of a
     // CTA when the matrix has too few rows to give every warp of the chip a row group
     const int groups = (a.n + LR_ROWS - 1) / LR_ROWS, k4 = a.k / 4;
@@ -1442,7 +1584,7 @@ cudaError_t launch_linear_decode(const LinearArgs& a, int epilogue, bool pdl, cu
     const int gpc = LR_WARPS >> kp_shift;
     const int grid = std::max(1, std::min(num_sms(), (groups + gpc - 1) / gpc));
     if (grid_out) *grid_out = grid;
-    const size_t smem = (size_t)mt * a.k * sizeof(float);
+    const size_t smem = linear_rows_smem(a.m, a.k);
 #define PG_LR(MT_)                                                                                                        \
   switch (epilogue) {                                                                                                      \
     case EPI_GELU: return launch(linear_rows_smem_kernel<MT_, EPI_GELU>, dim3(grid), dim3(LR_THREADS), smem, s, pdl, a, kp_shift);   \
@@ -1452,8 +1594,11 @@ cudaError_t launch_linear_decode(const LinearArgs& a, int epilogue, bool pdl, cu
     if (mt == 1) { PG_LR(1) }
     if (mt == 2) { PG_LR(2) }
     if (mt == 4) { PG_LR(4) }
-    PG_LR(8)
+    if (a.m <= 8) { PG_LR(8) }
 #undef PG_LR
+    if (epilogue == EPI_RESID) return cudaErrorInvalidValue;  // no residual sum follows a LayerNorm's product
+    return epilogue == EPI_GELU ? launch(linear_rows_smem_kernel<16, EPI_GELU>, dim3(grid), dim3(LR_THREADS), smem, s, pdl, a, kp_shift)
+                                : launch(linear_rows_smem_kernel<16, EPI_NONE>, dim3(grid), dim3(LR_THREADS), smem, s, pdl, a, kp_shift);
   }
   int grid = linear_decode_grid(a.n, num_sms());
   if (grid_out) *grid_out = grid;
@@ -1495,7 +1640,7 @@ cudaError_t launch_layernorm_rows_split(const float* x, const float* g, const fl
 // medium 1575 / 1635 and 2030 / 2033. The lm_head alone, the rest of the step on decode kernels: medium 1426 / 1449 / 1512 / 1524 / 1611 and
 // 1459 / 1474 / 1502 / 1515 / 1577 for 9 / 10 / 12 / 13 / 16 sequences.
 cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s) {
-  if (a.m <= (a.n <= 16384 ? 16 : 10) || a.k % 4 != 0) return launch_linear_decode(a, epilogue, pdl, s, nullptr);
+  if (a.m <= (a.n <= 16384 ? 16 : 10) || a.k % 4 != 0 || a.ln_g) return launch_linear_decode(a, epilogue, pdl, s, nullptr);
   return launch_gemm_f32_tiles(a, epilogue, s);
 }
 
@@ -1520,7 +1665,15 @@ cudaError_t launch_decode_attention(const DecodeAttnArgs& a, bool pdl, cudaStrea
   return launch(kern, dim3(a.kv.n_head, a.batch, 1), dim3(ATT_THREADS), smem, s, pdl, a);
 }
 
+bool prefill_attention_stores_kv(const PrefillAttnArgs& a) { return a.head_dim == 64 && a.max_len <= PS_KEYS; }
+
 cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, bool pdl, cudaStream_t s) {
+  if (prefill_attention_stores_kv(a)) {
+    // eight queries per block, a warp each, while that leaves an SM at most four blocks; else a block per head and sequence
+    const long long fine = (long long)a.n_head * a.batch * ((a.max_len + 7) / 8);
+    const int per_block = fine <= 4ll * num_sms() ? 8 : PS_KEYS;
+    return launch(prefill_attention_small_kernel, dim3(a.n_head, (a.max_len + per_block - 1) / per_block, a.batch), dim3(PS_THREADS), 0, s, pdl, a, per_block);
+  }
   if (a.head_dim == 64) {
     dim3 grid(a.n_head, (a.max_len + PA_Q - 1) / PA_Q, a.batch);
     return launch(prefill_attention_kernel<64>, grid, dim3(128), PA_SMEM, s, pdl, a);
@@ -1575,6 +1728,8 @@ cudaError_t init_kernel_attributes() {
   PG_SET((linear_rows_smem_kernel<MT_, EPI_RESID>), LR_MAX_SMEM)
   PG_SET_LR(1) PG_SET_LR(2) PG_SET_LR(4) PG_SET_LR(8)
 #undef PG_SET_LR
+  PG_SET((linear_rows_smem_kernel<16, EPI_NONE>), LR_MAX_SMEM)
+  PG_SET((linear_rows_smem_kernel<16, EPI_GELU>), LR_MAX_SMEM)
   PG_SET(decode_attention_kernel<64>, 64 * 1024)
   PG_SET(prefill_attention_kernel<64>, PA_SMEM)
   PG_SET(decode_attention_generic_kernel, 64 * 1024)

@@ -29,11 +29,13 @@ struct LinearArgs {
 };
 
 // Decode-time linear for a few activation rows (m <= 64): streams W once per 8 rows of x with
-// 128-bit loads, optional fused LayerNorm prologue (m <= 8, k <= 2048) and bias/GELU/residual
+// 128-bit loads, optional fused LayerNorm prologue (linear_decode_fuses_norm) and bias/GELU/residual
 // epilogue. `pdl` launches with programmatic dependent launch. Returns the grid size used in
 // *grid_out (the stride of part_val / part_idx).
 cudaError_t launch_linear_decode(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s, int* grid_out);
 int linear_decode_grid(int n, int num_sms);
+// Whether it makes the LayerNorm of m rows of k itself.
+bool linear_decode_fuses_norm(int m, int k);
 
 // out[r, :] = wte[ids[r]] + wpe[pos[r]]
 cudaError_t launch_embed(const float* wte, const float* wpe, const int* ids, const int* pos, float* out,
@@ -50,7 +52,7 @@ cudaError_t launch_layernorm_rows(const float* x, const float* g, const float* b
 // General FP32 GEMM out[m,n] = x[m,k] . w[n,k]^T (+bias)(+GELU | +resid), CUDA-core FMA (gemm_f32.cu); k % 4 == 0.
 cudaError_t launch_gemm_f32_tiles(const LinearArgs& a, int epilogue, cudaStream_t s);
 cudaError_t init_gemm_f32_attributes();
-// The faster of the two FP32 products for any number of rows (no LayerNorm prologue, no arg-max partials).
+// The faster of the two FP32 products for any number of rows (no arg-max partials; LayerNorm prologue: at most 16 rows).
 cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s);
 // dst[o, i] = src[i, o]
 cudaError_t launch_transpose(const float* src, float* dst, int in_f, int out_f, cudaStream_t s);
@@ -76,7 +78,13 @@ struct PrefillAttnArgs {
   PairOut pair;          // optional (head_dim 64; not the single TF32 pass): receives the result instead of out
   const int* seq_start;  // [batch + 1] row offsets
   int n_head, head_dim, batch, max_len;
+  // where prefill_attention_stores_kv: the cache that receives the rows' keys and values, or no pool
+  float* kv_pool;
+  const int *page_table, *row_slot;  // row_slot [rows]; positions count from a sequence's first row
+  KvLayout kv;
 };
+// Whether launch_prefill_attention writes keys and values to the cache too.
+bool prefill_attention_stores_kv(const PrefillAttnArgs& a);
 cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, bool pdl, cudaStream_t s);
 // The same attention with TF32 products on the tensor cores (head_dim 64; used by the TF32 prefill mode).
 // rows = rows of the QKV matrix; error_flag receives a code when a bounded wait runs out.

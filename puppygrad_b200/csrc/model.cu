@@ -988,7 +988,7 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
   // epilogue of the MLP's first product) writes pairs instead of FP32, into the same buffer: [rows, k] hi, then lo.
   const bool pairs = m->pair_arena && m->backend.math_mode != PG_MATH_TF32 && ws.d_error && rows >= 128 && m->head_dim() == 64 && C <= 4096;
   // A prompt of a few rows is a chain of launches of 2 to 10 us: the next one's blocks come up, and its first weights, while the last
-  // one ends (11 rows of GPT-2 small: 879 -> 749 us, 16: 902 -> 778). From 17 rows on the products are tiles (launch_linear_rows), which
+  // one ends (11 rows of GPT-2 small: 879 -> 749 us, 16: 902 -> 778; 585 and 614 with the norms made by the products). From 17 rows on the products are tiles (launch_linear_rows), which
   // start when everything in front of them has ended.
   const bool pdl = m->use_pdl && rows <= 16;
   auto pair_of = [&](float* buf, int k, float scale) {
@@ -1001,8 +1001,9 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
     return p;
   };
   auto gemm = [&](const float* w, const PairWeights& q, const float* bias, const float* x, const PairOut& xp, float* out,
-                  const PairOut& outp, int n_out, int k, int epi, const float* resid) -> cudaError_t {
+                  const PairOut& outp, int n_out, int k, int epi, const float* resid, const float* ln_g = nullptr, const float* ln_b = nullptr) -> cudaError_t {
     LinearArgs a{};
+    a.ln_g = ln_g; a.ln_b = ln_b;
     a.w = w; a.bias = bias; a.x = x; a.out = out; a.resid = resid; a.eps = eps;
     a.m = rows; a.n = n_out; a.k = k;
     if (pairs) {
@@ -1023,27 +1024,30 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
     return launch_linear_rows(a, epi, pdl, s);
   };
   static const bool no_tc_attn = getenv("PG_NO_TC_ATTN") != nullptr;
+  const bool fuse_norm = rows <= 16 && linear_decode_fuses_norm(rows, C);  // the products of a few rows make their normed rows themselves
   for (int l = 0; l < m->layers_n(); ++l) {
     const LayerWeights& w = m->layers[l];
     const PairOut n1 = pair_of(ws.norm, C, w.x_norm1), at = pair_of(ws.attn, C, w.x_attn), n2 = pair_of(ws.norm, C, w.x_norm2),
                   hp = pair_of(ws.h, F, w.x_h), none;
-    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln1_g, w.ln1_b, eps, ws.norm, rows, C, pdl, s, n1));
-    PG_CUDA_TRY(gemm(w.w_qkv, w.q_qkv, w.b_qkv, ws.norm, n1, ws.qkv, none, 3 * C, C, EPI_NONE, nullptr));
-    if (cache)
-      PG_CUDA_TRY(launch_kv_scatter(ws.qkv, ws.d_slot, ws.d_pos, cache->layer_pool(l), cache->tables[0].d_table, cache->kv,
-                                    rows, pdl, s));
+    if (!fuse_norm) PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln1_g, w.ln1_b, eps, ws.norm, rows, C, pdl, s, n1));
+    PG_CUDA_TRY(gemm(w.w_qkv, w.q_qkv, w.b_qkv, fuse_norm ? ws.x : ws.norm, n1, ws.qkv, none, 3 * C, C, EPI_NONE, nullptr,
+                     fuse_norm ? w.ln1_g : nullptr, w.ln1_b));
     PrefillAttnArgs pa{};
     pa.qkv = ws.qkv; pa.out = ws.attn; pa.pair = at; pa.seq_start = ws.d_seq_start;
     pa.n_head = m->heads(); pa.head_dim = m->head_dim(); pa.batch = plan.batch; pa.max_len = plan.max_len;
-    if (m->backend.math_mode == PG_MATH_TF32 && ws.d_error && !no_tc_attn && prefill_attention_tc_supported(pa))
-      PG_CUDA_TRY(launch_prefill_attention_tc(pa, rows, ws.d_error, s));
-    else if (pairs && !no_tc_attn && prefill_attention_tc_supported(pa))
-      PG_CUDA_TRY(launch_prefill_attention_x3(pa, rows, ws.d_error, s));
-    else
-      PG_CUDA_TRY(launch_prefill_attention(pa, pdl, s));
+    const bool tc = !no_tc_attn && ws.d_error && prefill_attention_tc_supported(pa), tf32 = tc && m->backend.math_mode == PG_MATH_TF32, x3 = tc && pairs;
+    if (cache && (tf32 || x3 || !prefill_attention_stores_kv(pa))) {
+      PG_CUDA_TRY(launch_kv_scatter(ws.qkv, ws.d_slot, ws.d_pos, cache->layer_pool(l), cache->tables[0].d_table, cache->kv,
+                                    rows, pdl, s));
+    } else if (cache) {
+      pa.kv_pool = cache->layer_pool(l); pa.page_table = cache->tables[0].d_table; pa.row_slot = ws.d_slot; pa.kv = cache->kv;
+    }
+    if (tf32) PG_CUDA_TRY(launch_prefill_attention_tc(pa, rows, ws.d_error, s));
+    else if (x3) PG_CUDA_TRY(launch_prefill_attention_x3(pa, rows, ws.d_error, s));
+    else PG_CUDA_TRY(launch_prefill_attention(pa, pdl, s));
     PG_CUDA_TRY(gemm(w.w_proj, w.q_proj, w.b_proj, ws.attn, at, ws.x, none, C, C, EPI_RESID, ws.x));
-    PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln2_g, w.ln2_b, eps, ws.norm, rows, C, pdl, s, n2));
-    PG_CUDA_TRY(gemm(w.w_fc, w.q_fc, w.b_fc, ws.norm, n2, ws.h, hp, F, C, EPI_GELU, nullptr));
+    if (!fuse_norm) PG_CUDA_TRY(launch_layernorm_rows(ws.x, w.ln2_g, w.ln2_b, eps, ws.norm, rows, C, pdl, s, n2));
+    PG_CUDA_TRY(gemm(w.w_fc, w.q_fc, w.b_fc, fuse_norm ? ws.x : ws.norm, n2, ws.h, hp, F, C, EPI_GELU, nullptr, fuse_norm ? w.ln2_g : nullptr, w.ln2_b));
     PG_CUDA_TRY(gemm(w.w_proj2, w.q_proj2, w.b_proj2, ws.h, hp, ws.x, none, C, F, EPI_RESID, ws.x));
   }
   return PG_OK;

@@ -178,6 +178,30 @@ def test_kv_cache_contents_match_oracle(midi):
         assert not gk[:, 40:].any()
 
 
+# Prompts whose products make their own norms (up to 16 rows, with and without a tile of eight to fill up; k = 256 held in registers) and
+# whose attention is the one for at most 64 tokens: queries in eights and all together, keys at the edges of 32 and 64, and 65 tokens beside them.
+@pytest.mark.parametrize("lens", [[1], [2, 5], [8], [9], [3, 6, 7], [16], [17], [31, 1], [32, 33], [63], [64], [65], [64, 2, 65], [7] * 50, [40] * 40])
+def test_prompts_of_a_few_rows(midi, lens):
+    cfg, w, g, o = midi
+    prompts = [synthetic.uniform_prompt(300 + i, n, cfg["vocab_size"]) for i, n in enumerate(lens)]
+    cache = g.new_kv_cache(max_batch=len(lens))
+    logits, am = g.prefill_batch(prompts, cache, want_logits=True)
+    caches = [o.new_kv_cache() for _ in lens]
+    assert_logits_close(logits, np.stack([o.prefill(p, c) for p, c in zip(prompts, caches)]))
+    logits, _, _, _ = g.forward_one_batch(am, cache, want_logits=True)  # reads what the prompts left in the cache
+    assert_logits_close(logits, np.stack([o.forward_one(int(t), c) for t, c in zip(am, caches)]))
+
+
+# The same products at k = 1088, whose rows do not stay in registers.
+def test_prompts_of_a_few_wide_rows(oracle):
+    cfg = dict(synthetic.preset("mini"), n_embd=1088, n_head=17, n_inner=320, n_layer=1)
+    w = synthetic.perturbed_weights(cfg, 5)
+    g, o = pg.Gpt2Model(cfg, w), oracle.Model(cfg, w, threads=4)
+    for n in (3, 8, 11, 16):
+        ids = synthetic.uniform_prompt(n, n, cfg["vocab_size"])
+        assert_logits_close(g.prefill(ids, g.new_kv_cache()), o.prefill(ids, o.new_kv_cache()))
+
+
 def test_token_by_token_prefill_equals_batched_prefill(midi):
     """The reference prefills token by token (rust.rs:920-926); the GEMM prefill must agree."""
     cfg, w, g, o = midi
