@@ -82,6 +82,7 @@ struct PrefillAttnArgs {
   float* kv_pool;
   const int *page_table, *row_slot;  // row_slot [rows]; positions count from a sequence's first row
   KvLayout kv;
+  unsigned long long kv_rows;  // rows of head_dim values in the pool
 };
 // Whether launch_prefill_attention writes keys and values to the cache too.
 bool prefill_attention_stores_kv(const PrefillAttnArgs& a);
@@ -91,6 +92,7 @@ cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, bool pdl, cudaStr
 bool prefill_attention_tc_supported(const PrefillAttnArgs& a);
 cudaError_t launch_prefill_attention_tc(const PrefillAttnArgs& a, int rows, int* error_flag, cudaStream_t s);
 // The same at FP32 grade (three TF32 products per term, lo parts formed inside the kernel): the FP32-parity modes.
+bool prefill_attention_x3_stores_kv(const PrefillAttnArgs& a);
 cudaError_t launch_prefill_attention_x3(const PrefillAttnArgs& a, int rows, int* error_flag, cudaStream_t s);
 cudaError_t init_attn_tc_attributes();
 // Copies K,V of every prompt row into the paged cache.

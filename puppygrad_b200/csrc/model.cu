@@ -1036,11 +1036,14 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
     pa.qkv = ws.qkv; pa.out = ws.attn; pa.pair = at; pa.seq_start = ws.d_seq_start;
     pa.n_head = m->heads(); pa.head_dim = m->head_dim(); pa.batch = plan.batch; pa.max_len = plan.max_len;
     const bool tc = !no_tc_attn && ws.d_error && prefill_attention_tc_supported(pa), tf32 = tc && m->backend.math_mode == PG_MATH_TF32, x3 = tc && pairs;
-    if (cache && (tf32 || x3 || !prefill_attention_stores_kv(pa))) {
-      PG_CUDA_TRY(launch_kv_scatter(ws.qkv, ws.d_slot, ws.d_pos, cache->layer_pool(l), cache->tables[0].d_table, cache->kv,
-                                    rows, pdl, s));
-    } else if (cache) {
-      pa.kv_pool = cache->layer_pool(l); pa.page_table = cache->tables[0].d_table; pa.row_slot = ws.d_slot; pa.kv = cache->kv;
+    if (cache) {
+      pa.page_table = cache->tables[0].d_table; pa.row_slot = ws.d_slot; pa.kv = cache->kv;
+      pa.kv_rows = (unsigned long long)cache->tables[0].num_pages * 2 * cache->kv.n_head * cache->kv.page_tokens;
+      if (tf32 ? false : x3 ? prefill_attention_x3_stores_kv(pa) : prefill_attention_stores_kv(pa))
+        pa.kv_pool = cache->layer_pool(l);
+      else
+        PG_CUDA_TRY(launch_kv_scatter(ws.qkv, ws.d_slot, ws.d_pos, cache->layer_pool(l), cache->tables[0].d_table, cache->kv,
+                                      rows, pdl, s));
     }
     if (tf32) PG_CUDA_TRY(launch_prefill_attention_tc(pa, rows, ws.d_error, s));
     else if (x3) PG_CUDA_TRY(launch_prefill_attention_x3(pa, rows, ws.d_error, s));

@@ -178,6 +178,25 @@ def test_kv_cache_contents_match_oracle(midi):
         assert not gk[:, 40:].any()
 
 
+# The tensor-core attention of prompts writes the cache page by page: lengths at the edges of pages and of its tiles of 128.
+@pytest.mark.parametrize("page_tokens", [16, 32, 64])
+def test_prompts_on_the_tensor_cores_fill_the_cache(midi, page_tokens):
+    cfg, w, _, o = midi
+    g = pg.Gpt2Model(cfg, w, pg.Gpt2CudaConfig(math_mode="tf32x3", page_tokens=page_tokens))
+    prompts = [synthetic.uniform_prompt(400 + n, n, cfg["vocab_size"]) for n in (1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 200, 255)]
+    cache = g.new_kv_cache(max_batch=len(prompts))
+    _, am = g.prefill_batch(prompts, cache)
+    caches = [o.new_kv_cache() for _ in prompts]
+    for p, c in zip(prompts, caches):
+        o.prefill(p, c)
+    for slot, c in enumerate(caches):
+        for layer in (0, cfg["n_layer"] - 1):
+            for got, want in zip(cache.read_layer(layer, slot), c.read_layer(layer)):
+                np.testing.assert_allclose(got, want, rtol=1e-4, atol=2e-5)
+    logits, _, _, _ = g.forward_one_batch(am, cache, want_logits=True)
+    assert_logits_close(logits, np.stack([o.forward_one(int(t), c) for t, c in zip(am, caches)]))
+
+
 # Prompts whose products make their own norms (up to 16 rows, with and without a tile of eight to fill up; k = 256 held in registers) and
 # whose attention is the one for at most 64 tokens: queries in eights and all together, keys at the edges of 32 and 64, and 65 tokens beside them.
 @pytest.mark.parametrize("lens", [[1], [2, 5], [8], [9], [3, 6, 7], [16], [17], [31, 1], [32, 33], [63], [64], [65], [64, 2, 65], [7] * 50, [40] * 40])
