@@ -362,10 +362,14 @@ enum ScanMode {
   SCAN_OUTPUT = 3    // one segment from its known start state: outputs
 };
 constexpr int SCAN_WARPS = 8;   // at most: 32 CPL columns
+// Warps that finish outputs beside `warps` that scan: with the one that stages, twelve warps on an SM in one block or in two, and so up to 168
+// registers for each.
+__host__ __device__ constexpr int finish_warps(int warps) { return warps > 4 ? 3 : 1; }
+constexpr int FINISH_THREADS = (SCAN_WARPS + finish_warps(SCAN_WARPS) + 1) * 32;
 constexpr int SCAN_STAGES = 3;
 struct ScanArgs {
   RecurrenceScanArgs a;
-  int mode, tb;
+  int mode, tb, warps;  // warps: those that scan
   float *seg_state, *seg_trans;  // [nseq][max_segs][heads][dim][dvp], [nseq][max_segs][heads][dim][dkp] (GLA: [..][dim] decays)
   int dkp;
   const float *k, *q, *v, *g;  // rows of keys, queries, values and gates (heads side by side) and their pitches
@@ -380,7 +384,13 @@ __device__ __forceinline__ void bulk_row(float* dst, const float* src, uint32_t 
                "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void named_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// Outputs in shared memory: buffer i (of two) is full at barrier 1 + i and may be written again at barrier 3 + i. The side that goes on arrives,
+// the other one waits.
+__device__ __forceinline__ void barrier_arrive(int id, int threads) {
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void barrier_wait(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
 // Sums of N values over the eight lanes of a group, in every lane: halves are exchanged on the way down, totals on the
 // way back.
@@ -577,8 +587,16 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) recurrence_scan_kern
     float* os = os0 + (size_t)(b & 1) * TB * 8 * OP;
 
     auto values = [&](const float* x, float (&v)[CPL]) {
+      if constexpr (CPL >= 4) {
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) v[c] = x[NA * DKP + col0 + c];
+        for (int c = 0; c < CPL; c += 4) {
+          const float4 f = load4(x + NA * DKP + col0 + c);
+          v[c] = f.x; v[c + 1] = f.y; v[c + 2] = f.z; v[c + 3] = f.w;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) v[c] = x[NA * DKP + col0 + c];
+      }
     };
     auto fetch = [&](const float* x, int arr, Row (&r)[J]) {
 #pragma unroll
@@ -632,7 +650,10 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) recurrence_scan_kern
           unpack2(o[c], x, y);
           r[c] = x + y;
         }
-        if (CPL == 4) store4(po, make_float4(r[0], r[1 % CPL], r[2 % CPL], r[3 % CPL]));
+        if (CPL == 8) {
+          store4(po, make_float4(r[0], r[1 % CPL], r[2 % CPL], r[3 % CPL]));
+          store4(po + 4, make_float4(r[4 % CPL], r[5 % CPL], r[6 % CPL], r[7 % CPL]));
+        } else if (CPL == 4) store4(po, make_float4(r[0], r[1 % CPL], r[2 % CPL], r[3 % CPL]));
         else if (CPL == 2) *reinterpret_cast<float2*>(po) = make_float2(r[0], r[1 % CPL]);
         else po[0] = r[0];
       }
@@ -693,7 +714,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) recurrence_scan_kern
     }
     if (outputs) {
       // every warp's shares are in; this buffer is written again two blocks on, after the next barrier
-      named_barrier(1, W * 32);
+      barrier_wait(1, W * 32);
       for (int t = warp; t < n; t += W) {
         const float* po = os + (size_t)t * 8 * OP;
         const float* g = x0 + (size_t)t * stride + NA * DKP + COLS;
@@ -753,7 +774,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) recurrence_scan_kern
 
 // The channel delta rule, four tokens at a time (see channel_quads_kernel); blocks, lanes, stages and modes as above.
 template <int RPL, int CPL>
-__global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) channel_scan_kernel(ScanArgs sa) {
+__global__ void __launch_bounds__(FINISH_THREADS, 1) channel_scan_kernel(ScanArgs sa) {
   extern __shared__ __align__(16) float sm[];
   __shared__ uint64_t full[SCAN_STAGES], empty[SCAN_STAGES];
   __shared__ int failed_flag;
@@ -765,7 +786,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) channel_scan_kernel(
   const int head = blockIdx.x / sa.col_blocks, cb = blockIdx.x % sa.col_blocks, seq = blockIdx.y, seg = blockIdx.z;
   const int all_cols = trans ? dk : l.vdim, cbase = cb * sa.block_cols;
   const int dv = min(sa.block_cols, all_cols - cbase);  // columns of this block
-  const int W = (blockDim.x >> 5) - 1, COLS = W * 4 * CPL, TB = sa.tb;  // TB: tokens of a stage, a multiple of QUAD
+  const int W = sa.warps, E = (blockDim.x >> 5) - 1 - W, COLS = W * 4 * CPL, TB = sa.tb;  // TB: tokens of a stage, a multiple of QUAD
   // a staged quad: per token A, B, Q, v, gate; then W and the numbers
   const int stride = 3 * DKP + 2 * COLS, qstride = QUAD * stride + DKP + QUAD_NUMBERS, OP = COLS + 4, quads = TB / QUAD;
   float* stage = sm;                                            // [SCAN_STAGES][quads][qstride]
@@ -784,7 +805,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) channel_scan_kernel(
   if (tid == 0) {
     for (int i = 0; i < SCAN_STAGES; ++i) {
       mbar_init(&full[i], 1);
-      mbar_init(&empty[i], (uint32_t)W);
+      mbar_init(&empty[i], (uint32_t)(W + E));
     }
     failed_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -793,7 +814,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) channel_scan_kernel(
   __syncthreads();
   const int blocks = (t1 - t0 + TB - 1) / TB;
 
-  if (warp == W) {  // ---- stages rows; lane = (token, array) of a quad, then its W and its numbers
+  if (warp == W + E) {  // ---- stages rows; lane = (token, array) of a quad, then its W and its numbers
     const int tok = lane / 5, arr = lane % 5;
     const float* rows[5] = {a.decay + head * dk, a.writes + head * dk, a.unit_next + head * dk, sa.v + head * l.vdim + cbase, sa.g + head * l.vdim + cbase};
     const bool on = lane >= 20 ? lane < 22 : arr < 2 || (arr == 2 && outputs) || (arr == 3 && want_v) || (arr == 4 && want_g);
@@ -826,6 +847,70 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) channel_scan_kernel(
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[r.stage]);
       }
+    }
+    return;
+  }
+
+  if (warp >= W) {  // ---- finishes outputs, two tokens at a time
+    float norm[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) norm[i] = sa.col_blocks == 1 && lane + i * 32 < dv ? l.norm[lane + i * 32] : 0.f;
+    RingCursor ring;
+    for (int b = 0; b < blocks; ++b, ring.next(SCAN_STAGES)) {
+      const int tb0 = t0 + b * TB, n = min(TB, t1 - tb0);
+      mbar_wait(&full[ring.stage], ring.parity, failed, a.error_flag, 43);
+      barrier_wait(1 + (b & 1), (W + E) * 32);
+      const float* x0 = stage + (size_t)ring.stage * quads * qstride;
+      const float* os = os0 + (size_t)(b & 1) * TB * OP;
+      for (int ta = warp - W; ta < n; ta += 2 * E) {
+        float o[2][4], sq[2] = {0.f, 0.f};  // at most 128 columns
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float* po = os + (size_t)min(ta + h * E, n - 1) * OP;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int c = lane + i * 32;
+            o[h][i] = c < dv ? po[c] * l.q_scale : 0.f;
+            sq[h] += o[h][i] * o[h][i];
+          }
+        }
+        if (sa.col_blocks > 1) {  // recurrence_output_kernel finishes the rows
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (ta + h * E >= n) break;
+            float* out = a.out_raw + (size_t)(tb0 + ta + h * E) * (l.heads * l.vdim) + head * l.vdim + cbase;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (lane + i * 32 < dv) out[lane + i * 32] = o[h][i];
+          }
+          continue;
+        }
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) {
+          sq[0] += __shfl_xor_sync(ALL_LANES, sq[0], m);
+          sq[1] += __shfl_xor_sync(ALL_LANES, sq[1], m);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int t = ta + h * E;
+          if (t >= n) break;
+          const float* g = x0 + (size_t)(t / QUAD) * qstride + (t % QUAD) * stride + 3 * DKP + COLS;
+          const float rinv = 1.f / sqrtf(sq[h] / (float)dv + l.eps);
+          const size_t base = (size_t)(tb0 + t) * a.ldy + head * dv;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int c = lane + i * 32;
+            if (c < dv) {
+              const float y = o[h][i] * rinv * norm[i] * sigmoid_f(g[c]) * l.out_scale;
+              if (sa.y_bf16) static_cast<__nv_bfloat16*>(a.y)[base + c] = __float2bfloat16_rn(y);
+              else static_cast<float*>(a.y)[base + c] = y;
+            }
+          }
+        }
+      }
+      __syncwarp();
+      if (b + 2 < blocks) barrier_arrive(3 + (b & 1), (W + E) * 32);
+      if (lane == 0) mbar_arrive(&empty[ring.stage]);
     }
     return;
   }
@@ -864,6 +949,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) channel_scan_kernel(
     __syncwarp();
     const float* x0 = stage + (size_t)ring.stage * quads * qstride;
     float* os = os0 + (size_t)(b & 1) * TB * OP;
+    if (outputs && b >= 2) barrier_wait(3 + (b & 1), (W + E) * 32);
     for (int g = 0; g * QUAD < n; ++g) {
       const float* x = x0 + (size_t)g * qstride;
       const float* num = x + QUAD * stride + DKP;
@@ -954,39 +1040,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) channel_scan_kernel(
         }
       }
     }
-    if (outputs) {
-      // every warp's shares are in; this buffer is written again two blocks on, after the next barrier
-      named_barrier(1, W * 32);
-      for (int t = warp; t < n; t += W) {
-        const float* po = os + (size_t)t * OP;
-        const float* g = x0 + (size_t)(t / QUAD) * qstride + (t % QUAD) * stride + 3 * DKP + COLS;
-        float o[4], sq = 0.f;  // at most 128 columns
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int c = lane + i * 32;
-          o[i] = c < dv ? po[c] * l.q_scale : 0.f;
-          sq += o[i] * o[i];
-        }
-        if (sa.col_blocks > 1) {  // recurrence_output_kernel finishes the rows
-          float* out = a.out_raw + (size_t)(tb0 + t) * (l.heads * l.vdim) + head * l.vdim + cbase;
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (lane + i * 32 < dv) out[lane + i * 32] = o[i];
-        } else {
-          const float rinv = 1.f / sqrtf(lane_sum(sq) / (float)dv + l.eps);
-          const size_t base = (size_t)(tb0 + t) * a.ldy + head * dv;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int c = lane + i * 32;
-            if (c < dv) {
-              const float y = o[i] * rinv * l.norm[c] * sigmoid_f(g[c]) * l.out_scale;
-              if (sa.y_bf16) static_cast<__nv_bfloat16*>(a.y)[base + c] = __float2bfloat16_rn(y);
-              else static_cast<float*>(a.y)[base + c] = y;
-            }
-          }
-        }
-      }
-    }
+    if (outputs) barrier_arrive(1 + (b & 1), (W + E) * 32);  // this warp's shares are in
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[ring.stage]);
   }
@@ -1180,6 +1234,11 @@ size_t scan_smem(int kind, int rpl, int cpl, int warps, int tb) {
   return ((size_t)SCAN_STAGES * tb * (na * 8 * rpl + 2 * cols + 4) + (size_t)2 * tb * 8 * (cols + 4)) * sizeof(float);
 }
 
+// Whether blocks of at most four scanning warps are more than SMs, and so two of them share one.
+bool scan_two(int kind, int rpl, int warps, dim3 grid) {
+  return kind != KIND_CHANNEL && rpl <= 8 && warps <= 4 && (long long)grid.x * grid.y * grid.z > sm_count();
+}
+
 template <int KIND, int RPL, int CPL>
 auto scan_kernel() {
   if constexpr (KIND == KIND_CHANNEL) return channel_scan_kernel<RPL, CPL>;
@@ -1190,19 +1249,26 @@ template <int KIND, int RPL, int CPL>
 cudaError_t launch_scan(ScanArgs sa, dim3 grid, int cols, cudaStream_t s) {
   const int warps = (cols + 4 * CPL - 1) / (4 * CPL);
   if (warps > SCAN_WARPS) return cudaErrorInvalidValue;
-  const int least = KIND == KIND_CHANNEL ? QUAD : 2;
+  const int least = KIND == KIND_CHANNEL ? QUAD : 2, finish = KIND == KIND_CHANNEL && (sa.mode == SCAN_FULL || sa.mode == SCAN_OUTPUT) ? finish_warps(warps) : 0;
+  // Tokens of a stage: as many as fit, or as let two blocks share an SM.
+  sa.warps = warps;
   sa.tb = 16;
-  while (sa.tb > least && scan_smem(KIND, RPL, CPL, warps, sa.tb) > MAX_SMEM) sa.tb /= 2;
+  while (sa.tb > least && scan_smem(KIND, RPL, CPL, warps, sa.tb) > (scan_two(KIND, RPL, warps, grid) ? MAX_SMEM / 2 : MAX_SMEM)) sa.tb /= 2;
   const size_t smem = scan_smem(KIND, RPL, CPL, warps, sa.tb);
   if (smem > MAX_SMEM) return cudaErrorInvalidValue;
   auto kernel = scan_kernel<KIND, RPL, CPL>();
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM);
   if (e != cudaSuccess) return e;
-  return launch_kernel(kernel, grid, dim3((warps + 1) * 32), smem, s, false, sa);
+  return launch_kernel(kernel, grid, dim3((warps + finish + 1) * 32), smem, s, false, sa);
 }
 
 template <int KIND, int RPL>
 cudaError_t launch_scan_cols(const ScanArgs& sa, dim3 grid, int cols, int cpl, cudaStream_t s) {
+  // More blocks than SMs: half the warps with twice the columns each, where that makes two blocks of an SM. PLACEHOLDER
+  constexpr int WIDEST = KIND == KIND_GLA && RPL <= 8 ? 8 : 4;
+  if (cpl * 2 <= WIDEST && scan_two(KIND, RPL, (cols + 8 * cpl - 1) / (8 * cpl), grid)) cpl *= 2;
+  if constexpr (WIDEST == 8)
+    if (cpl == 8) return launch_scan<KIND, RPL, 8>(sa, grid, cols, s);
   if (cpl == 4) return launch_scan<KIND, RPL, 4>(sa, grid, cols, s);
   if (cpl == 2) return launch_scan<KIND, RPL, 2>(sa, grid, cols, s);
   return launch_scan<KIND, RPL, 1>(sa, grid, cols, s);
