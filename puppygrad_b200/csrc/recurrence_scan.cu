@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(256) channel_taps_kernel(RecurrenceScanArgs a)
 // TB tokens at a time in a ring of shared-memory stages (bulk copies where rows are 16-byte aligned); in the others
 // eight lanes share a column (lane l holds rows 32 j + 4 l + i), a group of eight has CPL columns, a warp four groups.
 // A lane's share of an output goes to shared memory; after TB tokens the shares are added and the head norm and output
-// gate applied.
+// gate applied, by the same warps, or (channel rule) by finishing warps while the others go on with the next TB tokens.
 enum ScanMode {
   SCAN_FULL = 0,     // whole sequence: start from the cached state (or zero), outputs, final state to the cache
   SCAN_LOCAL = 1,    // one segment from a zero state, no outputs: its contribution to the state
@@ -362,8 +362,9 @@ enum ScanMode {
   SCAN_OUTPUT = 3    // one segment from its known start state: outputs
 };
 constexpr int SCAN_WARPS = 8;   // at most: 32 CPL columns
-// Warps that finish outputs beside `warps` that scan: with the one that stages, twelve warps on an SM in one block or in two, and so up to 168
-// registers for each.
+// Warps that finish the channel rule's outputs beside `warps` that scan: with the one that stages twelve, so that each may have 168
+// registers. 8192 tokens of a document, 16 heads of 128 x 128 in segments: the pass with outputs 603 -> 497 us. For the other rules, whose
+// outputs are sums of eight shares, three warps are too few: 8 x 1024 tokens through a model of delta layers take 1.035 times as long.
 __host__ __device__ constexpr int finish_warps(int warps) { return warps > 4 ? 3 : 1; }
 constexpr int FINISH_THREADS = (SCAN_WARPS + finish_warps(SCAN_WARPS) + 1) * 32;
 constexpr int SCAN_STAGES = 3;
@@ -1264,7 +1265,10 @@ cudaError_t launch_scan(ScanArgs sa, dim3 grid, int cols, cudaStream_t s) {
 
 template <int KIND, int RPL>
 cudaError_t launch_scan_cols(const ScanArgs& sa, dim3 grid, int cols, int cpl, cudaStream_t s) {
-  // More blocks than SMs: half the warps with twice the columns each, where that makes two blocks of an SM. PLACEHOLDER
+  // More blocks than SMs: half the warps with twice the columns each, where two blocks then share an SM. A warp reads the rows of a token
+  // whatever the number of its columns, so this halves those reads; what one block waits for, the other fills. 8 x 1024 tokens of 32
+  // heads of 64 x 64 (delta) 772 -> 578 us, 3592 tokens of 64 sequences 426 -> 288, and of 16 gated heads of 64 x 128
+  // 210 -> 181. A block that has an SM to itself is the faster with eight warps: 8 x 1024 tokens of 16 gated heads (128 blocks) 357 us, with four 507.
   constexpr int WIDEST = KIND == KIND_GLA && RPL <= 8 ? 8 : 4;
   if (cpl * 2 <= WIDEST && scan_two(KIND, RPL, (cols + 8 * cpl - 1) / (8 * cpl), grid)) cpl *= 2;
   if constexpr (WIDEST == 8)

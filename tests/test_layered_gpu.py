@@ -82,6 +82,32 @@ def test_norms_of_wide_rows(width, n):
     many_sequences(Case(lo.config(61, width, [lo.gla(2, 8, 12, ff=64)]), 5, rank=3), n, "bf16")
 
 
+# More (sequence, head) blocks of a scan than SMs: two of them share an SM, with up to eight columns per lane and shorter stages. Sizes up to
+# the widest, whole groups of columns and remainders; portions of odd and even lengths, from an empty and from a filled state.
+CROWDED = {
+    "gla-odd": lo.config(61, 50, [lo.gla(16, 7, 9)]),
+    "gla-24": lo.config(61, 48, [lo.gla(16, 16, 24)]),
+    "gla-72": lo.config(61, 48, [lo.gla(15, 40, 72)]),
+    "gla-128": lo.config(61, 48, [lo.gla(13, 64, 128)]),
+    "gla-long-keys": lo.config(61, 48, [lo.gla(13, 65, 40)]),
+    "delta-odd": lo.config(61, 50, [lo.pair(1, 1, 8, 8, 5, 16, 9, left_scale=0.0)]),
+    "delta-40": lo.config(61, 48, [lo.pair(1, 1, 8, 8, 5, 14, 40, left_scale=0.0)]),
+    "delta-64": lo.config(61, 48, [lo.pair(1, 1, 8, 8, 5, 13, 64, left_scale=0.0)]),
+}
+
+
+@pytest.mark.parametrize("name", CROWDED)
+def test_prompts_of_many_sequences(name):
+    case, n = Case(CROWDED[name], 9, rank=9), 13
+    model = case.model("fp32")
+    cache = model.new_kv_cache(max_batch=n)
+    ids, cuts = [case.ids(38 + i % 4, seed=i) for i in range(n)], [1 + (7 * i) % 19 for i in range(n)]
+    for part in (lambda x, t: x[:t], lambda x, t: x[t:]):
+        pieces = [part(x, t) for x, t in zip(ids, cuts)]
+        got = model.extend(range(n), pieces, cache, range(sum(map(len, pieces))))
+        assert_rows(got, np.concatenate([part(case.want(x), t) for x, t in zip(ids, cuts)]), "fp32")
+
+
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("name", ALONE)
 def test_mechanism_alone(name, mode):
