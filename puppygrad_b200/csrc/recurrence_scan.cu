@@ -262,10 +262,12 @@ __global__ void __launch_bounds__(256) channel_conv_vec_kernel(RecurrenceScanArg
 //   u_i = beta_i (v_i - A_i^T S - sum_{j < i} c_ij u_j),  out_i = Q_i^T S + sum_{j <= i} r_ij u_j,  S = W S + sum_j B_j u_j^T
 // with c_ij = k_i . D_ij k_j, r_ij = q_i . D_ij k_j, B_j = D_3j k_j, W = P_3. Quads are counted from a portion's first row; tokens
 // past its end count as decay 1 and zeros. A warp makes the rows and numbers of one head of one quad.
+// Bound by latency, from rows asked for to reductions: up to 128 rows of a head at 85 registers or fewer, three blocks on an SM, 8192 tokens of 16
+// heads of 128 163 -> 135 us.
 constexpr int QUAD = 4, QUAD_NUMBERS = 20;  // c (6), r (10), beta (4)
 __device__ __forceinline__ size_t first_quad(const RecurrenceScanArgs& a, int seq) { return (size_t)(a.seq_start[seq] / QUAD + seq); }
 template <int NE>
-__global__ void __launch_bounds__(256) channel_quads_kernel(RecurrenceScanArgs a) {
+__global__ void __launch_bounds__(256, NE <= 4 ? 3 : 1) channel_quads_kernel(RecurrenceScanArgs a) {
   const RecurrenceLayer& l = a.l;
   const int lane = threadIdx.x & 31, K = l.heads * l.dim, rep = l.heads / l.kv_heads, kv_pitch = l.kv_heads * l.dim;
   const int seq = blockIdx.y, first = a.seq_start[seq], len = a.seq_start[seq + 1] - first;
@@ -454,6 +456,7 @@ struct GroupScatter<N, 0> {
 // u'^T S_t = e - (u' . b) d + (u' . k) v, so that both reads come from one reduction over the state before the pair.
 template <int KIND, int RPL, int CPL>
 __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) recurrence_scan_kernel(ScanArgs sa) {
+  if (sa.mode == SCAN_LOCAL) grid_dep_launch();  // the transitions' blocks come up as these leave SMs
   extern __shared__ __align__(16) float sm[];
   __shared__ uint64_t full[SCAN_STAGES], empty[SCAN_STAGES];
   __shared__ int failed_flag;
@@ -481,7 +484,7 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) recurrence_scan_kern
   if (sa.mode != SCAN_FULL) {
     t0 += seg * a.seg_tokens;
     t1 = min(t1, t0 + a.seg_tokens);
-    if (t0 >= t1) return;
+    if (t0 >= t1) return;  // in front of any wait: other blocks hold the grid open
   }
   for (int i = tid; i < SCAN_STAGES * TB * stride; i += blockDim.x) stage[i] = 0.f;  // the padding stays zero
   if (tid == 0) {
@@ -771,11 +774,13 @@ __global__ void __launch_bounds__((SCAN_WARPS + 1) * 32, 1) recurrence_scan_kern
       for (int e = 0; e < 2; ++e)
         if (row_of(r + e) < dk && col0 + c < dv) fin[(size_t)row_of(r + e) * pitch + cbase + col0 + c] = v[e];
     }
+  if (trans) grid_dep_wait();  // what follows this grid also needs the contributions, which it overlaps
 }
 
 // The channel delta rule, four tokens at a time (see channel_quads_kernel); blocks, lanes, stages and modes as above.
 template <int RPL, int CPL>
 __global__ void __launch_bounds__(FINISH_THREADS, 1) channel_scan_kernel(ScanArgs sa) {
+  if (sa.mode == SCAN_LOCAL) grid_dep_launch();  // the transitions' blocks come up as these leave SMs
   extern __shared__ __align__(16) float sm[];
   __shared__ uint64_t full[SCAN_STAGES], empty[SCAN_STAGES];
   __shared__ int failed_flag;
@@ -800,7 +805,7 @@ __global__ void __launch_bounds__(FINISH_THREADS, 1) channel_scan_kernel(ScanArg
   if (sa.mode != SCAN_FULL) {
     t0 += seg * a.seg_tokens;
     t1 = min(t1, t0 + a.seg_tokens);
-    if (t0 >= t1) return;
+    if (t0 >= t1) return;  // in front of any wait: other blocks hold the grid open
   }
   for (int i = tid; i < SCAN_STAGES * quads * qstride; i += blockDim.x) stage[i] = 0.f;  // the padding stays zero
   if (tid == 0) {
@@ -1061,6 +1066,7 @@ __global__ void __launch_bounds__(FINISH_THREADS, 1) channel_scan_kernel(ScanArg
       for (int e = 0; e < 2; ++e)
         if (row_of(r + e) < dk && col0 + c < dv) fin[(size_t)row_of(r + e) * pitch + cbase + col0 + c] = v[e];
     }
+  if (trans) grid_dep_wait();  // what follows this grid also needs the contributions, which it overlaps
 }
 
 // Head norm, gate and branch scale of scan outputs that left in several column blocks; a warp per (row, head), at most
@@ -1260,7 +1266,9 @@ cudaError_t launch_scan(ScanArgs sa, dim3 grid, int cols, cudaStream_t s) {
   auto kernel = scan_kernel<KIND, RPL, CPL>();
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM);
   if (e != cudaSuccess) return e;
-  return launch_kernel(kernel, grid, dim3((warps + finish + 1) * 32), smem, s, false, sa);
+  // Transitions come behind the contributions, need nothing of theirs and write elsewhere: their blocks fill the SMs that the last, nearly empty
+  // wave of the other leaves idle. 8192 tokens, 16 heads of 128 x 128 in segments: both together 690 -> 576 us.
+  return launch_kernel(kernel, grid, dim3((warps + finish + 1) * 32), smem, s, sa.mode == SCAN_TRANS, sa);
 }
 
 template <int KIND, int RPL>
