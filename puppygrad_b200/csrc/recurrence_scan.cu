@@ -1117,8 +1117,11 @@ __global__ void __launch_bounds__(256) segment_decay_kernel(ScanArgs sa) {
 
 // Turns the segments' own contributions into their start states, in order: start[0] = cached state (or zero),
 // start[i + 1] = transition[i] start[i] + local[i]; the last one goes to the cache. Block = 16 columns of one head of
-// one sequence; the running state stays in shared memory, the next segment's numbers load one segment ahead.
-constexpr int COMBINE_COLS = 16, COMBINE_THREADS = 256, ROW_STEP = COMBINE_THREADS / COMBINE_COLS;
+// one sequence; the running state stays in shared memory, the next segment's numbers load one segment ahead. A thread has four columns of
+// PER rows: bound by the reads of transition rows and states in shared memory, 8 of 16 bytes for 64 multiply-adds (PER 4).
+// With one column and sixteen rows a thread, five reads for every sixteen multiply-adds, it took 171 us at 8192 tokens of 16 heads of
+// 128 x 128 in 32 segments; a document of that length through four such layers 14.35 ms, and 14.23 now.
+constexpr int COMBINE_COLS = 16, COMBINE_THREADS = 128, ROW_STEP = COMBINE_THREADS / (COMBINE_COLS / 4);
 template <int KIND, int PER>  // PER: rows of a thread, PER * ROW_STEP >= dim
 __global__ void __launch_bounds__(COMBINE_THREADS) recurrence_combine_kernel(ScanArgs sa) {
   extern __shared__ __align__(16) float sm[];
@@ -1133,8 +1136,8 @@ __global__ void __launch_bounds__(COMBINE_THREADS) recurrence_combine_kernel(Sca
   float* tr = sm + 2 * dk * COMBINE_COLS;  // delta: [2][dk][tp], the next one loading
   float* cached = a.state + ((size_t)a.seq_slot[seq] * l.heads + head) * dk * l.dvp;
   const bool fresh = a.seq_pos[seq] == 0;
-  const int c = tid % COMBINE_COLS, row0 = tid / COMBINE_COLS;  // this thread: one column, rows row0 + q * ROW_STEP
-  int at[PER];                                                  // where its rows of a transition matrix start
+  const int c = tid % (COMBINE_COLS / 4) * 4, row0 = tid / (COMBINE_COLS / 4);  // this thread: columns c..c + 3, rows row0 + q * ROW_STEP
+  int at[PER];                                                                  // where its rows of a transition matrix start
 #pragma unroll
   for (int q = 0; q < PER; ++q) at[q] = min(row0 + q * ROW_STEP, dk - 1) * tp;
   auto seg_at = [&](int g) { return ((size_t)seq * a.max_segs + g) * l.heads + head; };
@@ -1146,31 +1149,39 @@ __global__ void __launch_bounds__(COMBINE_THREADS) recurrence_combine_kernel(Sca
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + r * tp + x * 4)), "l"(src + (size_t)i * 4) : "memory");
     }
   };
-  float loc[PER], dec[PER];
+  float4 loc[PER];
+  float dec[PER];
   auto load_next = [&](int g) {
     const float* p = sa.seg_state + seg_at(g) * dk * l.dvp;
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
       const int r = row0 + q * ROW_STEP;
       if (r < dk) {
-        loc[q] = c < nc ? p[(size_t)r * l.dvp + c0 + c] : 0.f;
+        loc[q] = c < nc ? load4(p + (size_t)r * l.dvp + c0 + c) : make_float4(0, 0, 0, 0);  // rows are padded to fours
         if (KIND == KIND_GLA) dec[q] = sa.seg_trans[seg_at(g) * dk + r];
       }
     }
   };
   for (int i = tid; i < dk * COMBINE_COLS; i += COMBINE_THREADS) {
-    const int r = i / COMBINE_COLS, c = i % COMBINE_COLS;
-    cur[i] = (!fresh && c < nc) ? cached[(size_t)r * l.dvp + c0 + c] : 0.f;
+    const int r = i / COMBINE_COLS, x = i % COMBINE_COLS;
+    cur[i] = (!fresh && x < nc) ? cached[(size_t)r * l.dvp + c0 + x] : 0.f;
+  }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    loc[q] = make_float4(0, 0, 0, 0);
+    dec[q] = 0.f;
   }
   load_next(0);
   if (KIND == KIND_DELTA) load_trans(0, tr);
   asm volatile("cp.async.commit_group;" ::: "memory");
   for (int g = 0; g < segs; ++g) {
-    float v[PER], w[PER];
+    unsigned long long lo[PER], hi[PER];  // columns c, c + 1 and c + 2, c + 3
+    float w[PER];
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
-      v[q] = loc[q];
-      w[q] = KIND == KIND_GLA ? dec[q] : 0.f;
+      lo[q] = pack2(loc[q].x, loc[q].y);
+      hi[q] = pack2(loc[q].z, loc[q].w);
+      w[q] = dec[q];
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -1182,30 +1193,46 @@ __global__ void __launch_bounds__(COMBINE_THREADS) recurrence_combine_kernel(Sca
     float* start = sa.seg_state + seg_at(g) * dk * l.dvp;
     const float* m = tr + (size_t)(g & 1) * dk * tp;
     if (KIND == KIND_DELTA) {
+      auto add = [&](int q, float t, const ulonglong2& x) {
+        const unsigned long long t2 = pack2(t, t);
+        lo[q] = fma2(t2, x.x, lo[q]);
+        hi[q] = fma2(t2, x.y, hi[q]);
+      };
+      auto row = [&](int j) { return *reinterpret_cast<const ulonglong2*>(cur + j * COMBINE_COLS + c); };
       int j = 0;
       for (; j + 3 < dk; j += 4) {
-        const float x0 = cur[j * COMBINE_COLS + c], x1 = cur[(j + 1) * COMBINE_COLS + c], x2 = cur[(j + 2) * COMBINE_COLS + c], x3 = cur[(j + 3) * COMBINE_COLS + c];
+        const ulonglong2 x0 = row(j), x1 = row(j + 1), x2 = row(j + 2), x3 = row(j + 3);
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
           const float4 t = load4(m + at[q] + j);
-          v[q] = fmaf(t.x, x0, v[q]);
-          v[q] = fmaf(t.y, x1, v[q]);
-          v[q] = fmaf(t.z, x2, v[q]);
-          v[q] = fmaf(t.w, x3, v[q]);
+          add(q, t.x, x0);
+          add(q, t.y, x1);
+          add(q, t.z, x2);
+          add(q, t.w, x3);
         }
       }
       for (; j < dk; ++j)
 #pragma unroll
-        for (int q = 0; q < PER; ++q)
-          v[q] = fmaf(m[at[q] + j], cur[j * COMBINE_COLS + c], v[q]);
+        for (int q = 0; q < PER; ++q) add(q, m[at[q] + j], row(j));
     }
 #pragma unroll
     for (int q = 0; q < PER; ++q) {
-      const int r = row0 + q * ROW_STEP, i = r * COMBINE_COLS + c;
+      const int r = row0 + q * ROW_STEP;
       if (r < dk) {
-        const float old = cur[i];
-        if (c < nc) start[(size_t)r * l.dvp + c0 + c] = old;
-        nxt[i] = KIND == KIND_GLA ? fmaf(w[q], old, v[q]) : v[q];
+        const float4 old = load4(cur + r * COMBINE_COLS + c);
+        float* to = start + (size_t)r * l.dvp + c0 + c;
+        if (c + 3 < nc) {
+          store4(to, old);
+        } else {
+          if (c < nc) to[0] = old.x;
+          if (c + 1 < nc) to[1] = old.y;
+          if (c + 2 < nc) to[2] = old.z;
+        }
+        float4 v;
+        unpack2(lo[q], v.x, v.y);
+        unpack2(hi[q], v.z, v.w);
+        if (KIND == KIND_GLA) v = make_float4(fmaf(w[q], old.x, v.x), fmaf(w[q], old.y, v.y), fmaf(w[q], old.z, v.z), fmaf(w[q], old.w, v.w));
+        store4(nxt + r * COMBINE_COLS + c, v);
       }
     }
     __syncthreads();
@@ -1214,8 +1241,8 @@ __global__ void __launch_bounds__(COMBINE_THREADS) recurrence_combine_kernel(Sca
     nxt = t;
   }
   for (int i = tid; i < dk * COMBINE_COLS; i += COMBINE_THREADS) {
-    const int r = i / COMBINE_COLS, c = i % COMBINE_COLS;
-    if (c < nc) cached[(size_t)r * l.dvp + c0 + c] = cur[i];
+    const int r = i / COMBINE_COLS, x = i % COMBINE_COLS;
+    if (x < nc) cached[(size_t)r * l.dvp + c0 + x] = cur[i];
   }
 }
 
@@ -1406,9 +1433,9 @@ cudaError_t launch_recurrence_scan(const RecurrenceScanArgs& a, bool y_bf16, cud
     return r != cudaSuccess ? r : launch_kernel(kernel, cgrid, dim3(COMBINE_THREADS), csmem, s, false, sa);
   };
 #define PG_COMBINE(KIND_)                                                              \
-  (l.dim <= 4 * ROW_STEP   ? combine(recurrence_combine_kernel<KIND_, 4>)              \
-   : l.dim <= 8 * ROW_STEP ? combine(recurrence_combine_kernel<KIND_, 8>)              \
-                           : combine(recurrence_combine_kernel<KIND_, 16>))
+  (l.dim <= 2 * ROW_STEP   ? combine(recurrence_combine_kernel<KIND_, 2>)              \
+   : l.dim <= 4 * ROW_STEP ? combine(recurrence_combine_kernel<KIND_, 4>)              \
+                           : combine(recurrence_combine_kernel<KIND_, 8>))
   e = l.kind != KIND_GLA ? PG_COMBINE(KIND_DELTA) : PG_COMBINE(KIND_GLA);
 #undef PG_COMBINE
   if (e != cudaSuccess) return e;

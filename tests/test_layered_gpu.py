@@ -161,6 +161,19 @@ def test_long_prompt_in_segments_and_long_decoding(mixed, mode):
     assert_rows(got, want, mode)
 
 
+# States between segments: 64, 128 and 256 rows of a block at most, whole and cut fours of columns, one block of 16 columns and several.
+STATES = [lo.gla(2, 7, 9), lo.gla(2, 64, 18), lo.gla(1, 65, 35), lo.gla(1, 129, 16), lo.gla(1, 256, 3)] + [
+    lo.pair(1, 1, 8, 8, 5, 1, dim, left_scale=0.0) for dim in (1, 7, 31, 63, 66, 129, 144)]
+
+
+@pytest.mark.parametrize("layer", STATES, ids=lambda x: "%s-%d" % (x["type"], (x["mixer"].get("right") or x["mixer"])["dim"]))
+def test_states_between_segments(layer):
+    case = Case(lo.config(61, 48, [layer]), 13, rank=3)
+    ids = case.ids(1040)
+    model = case.model("fp32")
+    assert_rows(run_portions(model, model.new_kv_cache(1), 0, [ids[:515], ids[515:]]), case.want(ids), "fp32")
+
+
 @pytest.mark.parametrize("page_tokens", [16, 64])
 def test_page_sizes(mixed, page_tokens):
     ids = mixed.ids(90, 3)
