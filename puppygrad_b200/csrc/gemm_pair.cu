@@ -29,6 +29,7 @@ namespace {
 
 constexpr int PK = 64;   // FP16 elements per k block: one 128-byte swizzle row
 constexpr int PBN = 128; // columns of an output tile
+constexpr int PAIR_DRAIN = 8, PAIR_THREADS = (2 + PAIR_DRAIN) * 32;  // epilogue warps, two per quarter of the tensor-memory lanes
 
 // EXACT_W: the weights are BF16 values that their hi parts hold, the lo parts are not read (PAIR_FIT_HI).
 template <bool EXACT_W>
@@ -36,7 +37,7 @@ struct PairSmem {
   static constexpr int TILE_BYTES = TILE_M * PK * 2;  // 16 KB; 128 rows of weights are a tile too
   static constexpr int TILES = EXACT_W ? 3 : 4, STAGES = EXACT_W ? 4 : 3;
   static constexpr int STAGE_BYTES = TILES * TILE_BYTES;  // x hi, x lo, w hi, w lo
-  static constexpr int EPI_BYTES = 4 * 32 * 33 * 4;       // one padded 32x32 transpose tile per epilogue warp
+  static constexpr int EPI_BYTES = PAIR_DRAIN * 32 * 33 * 4;  // one padded 32x32 transpose tile per epilogue warp
   static constexpr size_t BYTES = (size_t)STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 
@@ -44,17 +45,19 @@ struct PairSmem {
 // row tile (launch_tile_pairs): one box per block, and the same copy serves the decode step (gemm_chain.cu).
 //
 // Persistent over 128 x 128 output tiles (column tiles of one row panel are neighbours, so the activation panel is reused
-// from L2). Warp 0 loads by TMA, one thread of warp 1 issues the MMAs, warps 2..5 drain. Tensor memory holds two buffers of
-// two accumulators, so that a tile is drained while the next one is multiplied: the tensor core adds with truncation, a bias
-// that grows with the MMAs into one accumulator, so the hi.hi products have one of their own and the small terms another.
-// hi_x times the hi and the lo weight tile, which lie next to each other, is one MMA of N = 256 into both.
+// from L2). Warp 0 loads by TMA, one thread of warp 1 issues the MMAs, warps 2..9 drain, half of a tile's columns each.
+// Tensor memory holds two buffers of two accumulators, so that a tile is drained while the next one is multiplied: the tensor core
+// adds with truncation, a bias that grows with the MMAs into one accumulator, so the hi.hi products have one of their own and the
+// small terms another. hi_x times the hi and the lo weight tile, which lie next to each other, is one MMA of N = 256 into both.
+// Four warps did not drain a tile with GELU while the next one was multiplied: 8192 x 3072 x 768 with GELU 126.6 us with four and
+// 96.2 with eight, 8192 x 768 x 768 36.1 and 32.5; 8192 x 4096 x 1024 with GELU 170.6 and 149.6.
 //
 // Bound by the tensor pipe where k is long: 82% of its active cycles at 8192 x 4800 x 1600; 66% at 8192 x 2304 x 768, where L2 (38%)
 // and shared memory (28% of its reads, 23% of its writes) are no nearer their limits. Mean of a layer's four products, useful
 // TFLOP/s (a third of the FP16 rate is 530): 8192 rows of GPT-2 small 343 (three TF32 products of FP32 words: 184), 16384 rows of
 // GPT-2 XL 448 (207). Relative error against 64 bits of 16384 x 4800 x 1600: 1.9e-6.
 template <bool EXACT_W>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
     tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_constant__ CUtensorMap map_xl,
                         const __grid_constant__ CUtensorMap map_w, PairGemmArgs a) {
   using S = PairSmem<EXACT_W>;
@@ -84,7 +87,7 @@ __global__ void __launch_bounds__(192, 1)
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&d_full[i], 1);
-      mbar_init(&d_empty[i], 4);
+      mbar_init(&d_empty[i], PAIR_DRAIN);
     }
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -147,8 +150,8 @@ __global__ void __launch_bounds__(192, 1)
   } else {
     // TMEM lane = output row, but a row-per-thread store touches 32 cache lines per instruction: every 32x32 block goes
     // through a padded shared-memory tile and leaves column-per-lane (pairs: two columns per lane, two rows at a time).
-    const int q = warp & 3;
-    float* tile = epi_tiles + q * (32 * 33);
+    const int q = warp & 3, first_col = (warp - 2) / 4 * (PBN / 2);
+    float* tile = epi_tiles + (warp - 2) * (32 * 33);
     uint32_t ti = 0;
     bool ok = true;
     for (int tile_id = blockIdx.x; tile_id < tiles && ok; tile_id += gridDim.x)
@@ -161,7 +164,7 @@ __global__ void __launch_bounds__(192, 1)
         if (!ok) break;
         tc_fence_after();
 #pragma unroll 1
-        for (int c0 = 0; c0 < PBN && n0 + c0 < a.n; c0 += 32) {
+        for (int c0 = first_col; c0 < first_col + PBN / 2 && n0 + c0 < a.n; c0 += 32) {
           const int col = n0 + c0 + lane;
           // residual values (or what the chunks before left in `out`) are asked for before the accumulator is read: one
           // by one between the stores, which may alias them, each would cost a memory round trip
@@ -309,7 +312,7 @@ cudaError_t launch_pair(const PairGemmArgs& a, cudaStream_t s) {
       w_rows > 0x7fffffffull || !make_map_f16(&w, a.w, w_rows, PK, (EXACT_W ? 1 : 2) * TILE_M))
     return cudaErrorInvalidValue;
   const int tiles = ((a.n + PBN - 1) / PBN) * ((a.m + TILE_M - 1) / TILE_M);
-  tc_gemm_pair_kernel<EXACT_W><<<std::min(tiles, sm_count()), 192, PairSmem<EXACT_W>::BYTES, s>>>(xh, xl, w, a);
+  tc_gemm_pair_kernel<EXACT_W><<<std::min(tiles, sm_count()), PAIR_THREADS, PairSmem<EXACT_W>::BYTES, s>>>(xh, xl, w, a);
   return cudaGetLastError();
 }
 

@@ -70,6 +70,13 @@ def test_linear_tf32x3_matches_oracle(oracle, m, n, k, epilogue):
     np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
 
 
+# Two warps drain a quarter of a tile's rows, half of its columns each: ends inside and between the halves and their groups of 32.
+@pytest.mark.parametrize("n", [31, 33, 64, 65, 96, 97, 127, 161, 193])
+@pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
+def test_linear_pairs_of_cut_column_tiles(oracle, n, epilogue):
+    test_linear_tf32x3_matches_oracle(oracle, 130, n, 96, epilogue)
+
+
 def hi_part(a):
     """Rounded to the 11 significant bits of an FP16 number."""
     m, e = np.frexp(a)
