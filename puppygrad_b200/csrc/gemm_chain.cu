@@ -62,6 +62,10 @@ constexpr size_t CH_SMEM = (size_t)CH_W_RING + (size_t)CH_X_STAGES * CH_ACT_BYTE
 static_assert(CH_SMEM <= 232448, "shared memory of one CTA");
 static_assert(sizeof(ChainPhase) % 8 == 0 && 384 + 2 * sizeof(ChainPhase) <= 1024, "two phase descriptors behind the barriers");
 constexpr size_t CH_PART_TILE = (size_t)CH_BN * TILE_M;  // floats of one partial tile: [token][row]
+// The partial tiles of a phase: one of two sets.
+__device__ __forceinline__ float* part_tiles(const ChainArgs& a, const ChainPhase& ph) {
+  return a.partials + (ph.part ? (size_t)gridDim.x * CH_MAX_SEG * CH_PART_TILE : 0);
+}
 
 // Share of one CTA in units: [g0, g1) of the phase's tiles * nkb units (row tile major); per = units per CTA.
 struct ChRange {
@@ -111,10 +115,10 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 // is passed when it reaches grid * b. Returns the same verdict to every worker thread.
 __device__ __forceinline__ bool chain_grid_barrier(unsigned* counter, unsigned target, volatile int* failed, int* err,
                                                    int wt, volatile int* verdict, int fence_first, uint64_t* go,
-                                                   const int* next_kind) {
-  // thread 0 alone needs to know whether a GEMM follows; the load overlaps the CTA barrier
+                                                   const ChainPhase* next) {
+  // thread 0 alone needs to know whether a GEMM follows whose input the activation producer loads; the loads overlap the CTA barrier
   uint64_t* go_next = nullptr;
-  if (wt == 0 && next_kind && !(fence_first & 16) && *next_kind == CH_GEMM) go_next = go;
+  if (wt == 0 && next && !(fence_first & 16) && next->kind == CH_GEMM && next->act >= 0) go_next = go;
   workers_sync();
   if (wt == 0) {
     if (!*failed) {
@@ -287,8 +291,8 @@ __device__ __forceinline__ void chain_rows_phase(const ChainArgs& a, const Chain
       const float4 xv = __ldcg(xrow + u);
       float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
       if (ph.bias) b = __ldg(reinterpret_cast<const float4*>(ph.bias) + u);
-      const float4 acc = aligned ? sum_partials_aligned<16>(a.partials, u * 4, j, cnt)
-                                 : sum_partials<16>(a.partials, u * 4, j, r.nkb, FastDiv{ph.r_magic_per, (unsigned)r.per}, FastDiv{ph.r_magic_nkb, (unsigned)r.nkb});
+      const float4 acc = aligned ? sum_partials_aligned<16>(part_tiles(a, ph), u * 4, j, cnt)
+                                 : sum_partials<16>(part_tiles(a, ph), u * 4, j, r.nkb, FastDiv{ph.r_magic_per, (unsigned)r.per}, FastDiv{ph.r_magic_nkb, (unsigned)r.nkb});
       v[i].x = xv.x + (b.x + acc.x);
       v[i].y = xv.y + (b.y + acc.y);
       v[i].z = xv.z + (b.z + acc.z);
@@ -419,6 +423,38 @@ __device__ __forceinline__ void chain_elem_phase(const ChainArgs& a, const Chain
     workers_sync();
     if (wt < a.m && best_s[wt]) atomicMax(ph.best + wt, best_s[wt]);
   }
+}
+
+// Input of a GEMM phase with act CH_ACT_SUMS: the GELU of the sums of the GEMM before it, for this CTA's units u0, u0 + 1, ..., as pairs
+// straight into the activation ring (128-byte swizzle; rows past the batch keep what they hold, their products go nowhere). In the place of
+// an ELEM phase: one grid barrier and a trip of the pairs through L2 less, but every value is made by as many CTAs as there are row tiles,
+// and nothing is multiplied meanwhile (chain_makes_input). 32 steps of 8 sequences of GPT-2 medium with BF16 weights 35.9 -> 34.5 ms.
+__device__ __forceinline__ bool chain_sums_input(const ChainArgs& a, const ChainPhase& ph, const ChRange& r, uint32_t u0, int wt, uint8_t* act_ring,
+                                                 int act_bytes, uint64_t* ready, uint64_t* done, bool ok, volatile int* failed) {
+  const int units = r.g1 - r.g0;
+  for (int i = 0; i < units && ok; ++i) {
+    const uint32_t u = u0 + i;
+    if (u >= CH_X_STAGES) ok = warp_wait(&done[u % CH_X_STAGES], ((u / CH_X_STAGES) - 1) & 1, failed, a.error_flag, 36);
+  }
+  const bool aligned = ph.in_nkb % ph.in_per == 0;
+  const int cnt = ph.in_nkb / ph.in_per, per_unit = a.m * 16, total = units * per_unit;
+  if (ok) {
+    for (int idx = wt; idx < total; idx += CH_WORKERS) {
+      const int i = idx / per_unit, at = idx - i * per_unit, j = at >> 4, f4 = at & 15;
+      const int f = ((r.g0 + i) % r.nkb) * CH_K + f4 * 4;
+      const float4 bias = ph.in_bias ? __ldg(reinterpret_cast<const float4*>(ph.in_bias + f)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 acc = aligned ? sum_partials_aligned<8>(a.partials, f, j, cnt)
+                                 : sum_partials<8>(a.partials, f, j, ph.in_nkb, FastDiv{ph.in_magic_per, (unsigned)ph.in_per}, FastDiv{ph.in_magic_nkb, (unsigned)ph.in_nkb});
+      uint8_t* tile = act_ring + (size_t)((u0 + i) % CH_X_STAGES) * CH_ACT_BYTES + j * 128 + (((f4 >> 1) ^ (j & 7)) << 4) + (f4 & 1) * 8;
+      store_pair4(reinterpret_cast<uint16_t*>(tile), reinterpret_cast<uint16_t*>(tile + act_bytes / 2),
+                  make_float4(gelu_ref(bias.x + acc.x), gelu_ref(bias.y + acc.y), gelu_ref(bias.z + acc.z), gelu_ref(bias.w + acc.w)), ph.in_scale);
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // read by the tensor cores
+  workers_sync();
+  if (wt == 0 && ok)
+    for (int i = 0; i < units; ++i) mbar_arrive(&ready[(u0 + i) % CH_X_STAGES]);
+  return ok;
 }
 
 // FINAL phase: end of a decode step for token j (finalize_kernel's work): the row arg-max the lm_head's
@@ -882,6 +918,10 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
         if (phase_at(a, p).kind != CH_GEMM) continue;
         const ChRange r = chain_range_ph(phase_at(a, p), cta);
         const int act = phase_at(a, p).act;
+        if (act < 0) {  // the workers make this input
+          u += r.g1 - r.g0;
+          continue;
+        }
         const CUtensorMap* mh = act == 0 ? &map_hi0 : act == 1 ? &map_hi1 : &map_hi2;
         const CUtensorMap* ml = act == 0 ? &map_lo0 : act == 1 ? &map_lo1 : &map_lo2;
         ok = mbar_wait(go, gp & 1, failed, a.error_flag, 25);
@@ -907,7 +947,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
     const int q = ww & 3, half = ww >> 2;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const int row = q * 32 + lane;
-    uint32_t si = 0, barriers = 0;
+    uint32_t si = 0, barriers = 0, units = 0;  // units: of this CTA in the GEMM phases so far
     bool ok = true;     // this warp's drains
     bool live = true;   // same for all workers of the CTA: decided at the grid barriers
     if (wt == 0) chain_trace(a, 31);
@@ -947,12 +987,14 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
       if (kind == CH_GEMM) {
         // inputs of this phase exist: previous kernel (first phase), or the barrier just passed, whose polling
         // thread has told the activation producer already
-        if (wt == 0 && (p == 0 || (a.tune_fence & 16))) mbar_arrive(go);
+        if (wt == 0 && ph.act >= 0 && (p == 0 || (a.tune_fence & 16))) mbar_arrive(go);
         if (live && p + 1 < a.n_phases && phase_at(a, p + 1).kind == CH_ATTN) {
           chain_attn_prepare(a, ww, lane, at_cur, at_consumed);
           at_prepared = true;
         }
         const ChRange r = chain_range_ph(ph, cta);
+        if (ph.act < 0) ok = chain_sums_input(a, ph, r, units, wt, act_ring, act_bytes, ready, done, ok && live, failed) && ok;
+        units += r.g1 - r.g0;
         unsigned long long* best_s = reinterpret_cast<unsigned long long*>(at_scratch);
         if (ph.whole_tiles && ph.best) {
           if (wt < CH_BN) best_s[wt] = 0ull;
@@ -995,7 +1037,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
             }
           } else if (ok) {
             tc_fence_after();
-            float* dst = a.partials + ((size_t)(cta * CH_MAX_SEG + seg) * CH_BN) * TILE_M + row;
+            float* dst = part_tiles(a, ph) + ((size_t)(cta * CH_MAX_SEG + seg) * CH_BN) * TILE_M + row;
 #pragma unroll
             for (int cc = 0; cc < 32; cc += 16) {
               const int c0 = half * 32 + cc;
@@ -1041,7 +1083,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
           reinterpret_cast<uint32_t*>(&ph_s[(p + 1) & 1])[wt] = reinterpret_cast<const uint32_t*>(&phase_at(a, p + 1))[wt];
         ++barriers;
         live = chain_grid_barrier(a.barrier, (unsigned)grid * barriers, failed, a.error_flag, wt, verdict, a.tune_fence, go,
-                                  &phase_at(a, p + 1).kind);
+                                  &phase_at(a, p + 1));
         ok = ok && live;
       }
       if (wt == 0 && p < 10) chain_trace(a, p);
@@ -1088,7 +1130,16 @@ int chain_grid(int num_sms) {
   return cached;
 }
 
-size_t chain_partial_floats(int grid) { return (size_t)grid * CH_MAX_SEG * CH_PART_TILE; }
+size_t chain_partial_floats(int grid) { return 2 * (size_t)grid * CH_MAX_SEG * CH_PART_TILE; }
+
+// Where making the input is little work: by rows and units of a CTA. us a step with an ELEM phase and without: width 768 (2 units) 9 rows 502 and 462,
+// 24 rows 525 and 505, 32 rows 522 and 524; width 1024 (4 units) 9 rows 987 and 966, 12 rows 983 and 966, 16 rows 999 and 1001, 24 rows
+// 1026 and 1082; width 1600 (9 units) 9 rows 2731 and 2758.
+bool chain_makes_input(int n, int k, int m, int grid) {
+  if (grid <= 0 || k % CH_K != 0) return false;
+  const int per = chain_range(n, k, 0, grid).per;
+  return m <= 24 && per <= 4 && per * m <= 48;
+}
 
 unsigned long long chain_argmax_init() { return argmax_key(0xff800000u, 0u); }
 
@@ -1103,6 +1154,10 @@ void chain_prepare_phases(ChainPhase* phases, int n_phases, int grid) {
     ph.r_per = r.per;
     ph.r_magic_per = r.per > 1 ? (unsigned)((0x100000000ull + (unsigned)r.per - 1) / (unsigned)r.per) : 0u;
     ph.r_magic_nkb = r.nkb > 1 ? (unsigned)((0x100000000ull + (unsigned)r.nkb - 1) / (unsigned)r.nkb) : 0u;
+    if (ph.kind == CH_GEMM && ph.act == CH_ACT_SUMS && p > 0) {
+      const ChainPhase& in = phases[p - 1];
+      ph.in_nkb = in.r_nkb; ph.in_per = in.r_per; ph.in_magic_per = in.r_magic_per; ph.in_magic_nkb = in.r_magic_nkb;
+    }
   }
 }
 
@@ -1137,14 +1192,19 @@ bool chain_supported(const ChainArgs& a, int grid, const ChainPhase* host_phases
     if (whole && (ph.bias || ph.gelu || ph.out_hi || (p + 1 < a.n_phases && phs[p + 1].kind != CH_FINAL))) return false;
     if (!whole && ph.kind == CH_GEMM && (ph.best || ph.out)) return false;
     if (ph.kind == CH_GEMM) {
-      if (ph.act < 0 || ph.act > 2 || !a.act_hi[ph.act] || !a.act_lo[ph.act] || a.act_k[ph.act] != ph.k) return false;
+      if (ph.act == CH_ACT_SUMS) {  // behind the GEMM it reads, whose partial tiles it leaves alone
+        if (p == 0 || whole || phs[p - 1].kind != CH_GEMM || phs[p - 1].whole_tiles || phs[p - 1].n != ph.k || phs[p - 1].part != 0 || ph.part != 1) return false;
+        if (r.per > CH_X_STAGES) return false;  // all of a CTA's units are staged at once
+      } else {
+        if (ph.act < 0 || ph.act > 2 || !a.act_hi[ph.act] || !a.act_lo[ph.act] || a.act_k[ph.act] != ph.k || ph.part != 0) return false;
+      }
       const unsigned long long rows =
           ((unsigned long long)ph.w_block0 + (unsigned long long)((ph.n + TILE_M - 1) / TILE_M) * r.nkb) * (a.exact ? 1 : 2) * TILE_M;
       if (rows > 0x7fffffffull || rows * CH_K > a.arena_halves) return false;
     } else if (ph.kind == CH_ROWS) {
       if (ph.n % 4 != 0 || ph.n > 4 * 4 * CH_WORKERS || !ph.x) return false;
       if (ph.ln_g && (!ph.ln_b || !ph.out_hi || !ph.out_lo)) return false;
-      if (p == 0 || phs[p - 1].kind != CH_GEMM || phs[p - 1].n != ph.n || phs[p - 1].k != ph.k) return false;
+      if (p == 0 || phs[p - 1].kind != CH_GEMM || phs[p - 1].n != ph.n || phs[p - 1].k != ph.k || phs[p - 1].part != ph.part) return false;
     } else if (ph.kind == CH_ELEM) {
       if (ph.out_hi && (!ph.out_lo || ph.n % 4 != 0)) return false;
       if (p == 0 || phs[p - 1].kind != CH_GEMM || phs[p - 1].n != ph.n || phs[p - 1].k != ph.k) return false;

@@ -201,7 +201,7 @@ enum ChainAct { CH_ACT_NORM = 0, CH_ACT_ATTN = 1, CH_ACT_H = 2 };
 struct ChainPhase {
   int kind;
   int n, k;           // GEMM: output features and reduction length; ROWS / ELEM / ATTN: those of the GEMM being reduced
-  int act;            // GEMM: which pair of activations is the input (ChainAct)
+  int act;            // GEMM: which pair of activations is the input (ChainAct), or CH_ACT_SUMS
   unsigned w_block0;  // GEMM: index of the first 128 x 64 block of this matrix inside the arena
   float inv_x, inv_w; // GEMM: reciprocals of the scales of its activations and weights
   float out_scale;    // phases with out_hi: scale of the pairs
@@ -222,7 +222,16 @@ struct ChainPhase {
   // GEMM without a reduce phase behind it (the lm_head): every CTA takes whole row tiles, so an accumulator holds
   // finished sums, and the drain stores them to `out` (or nowhere) and folds them into `best`; no bias, no partial tiles
   int whole_tiles;
+  // GEMM with act CH_ACT_SUMS, right behind the GEMM whose results are its input: the CTAs make their units' input themselves, as the ELEM phase
+  // that it spares would: tanh-GELU of in_bias + the sums, as pairs of scale in_scale; in_*: share arithmetic of that GEMM (derived)
+  const float* in_bias;
+  float in_scale;
+  int in_nkb, in_per;
+  unsigned in_magic_per, in_magic_nkb;
+  int part;  // which half of the partial tiles this phase (GEMM: writes, else: reads): 1 behind an input made from those in half 0
 };
+constexpr int CH_ACT_SUMS = -1;
+bool chain_makes_input(int n, int k, int m, int grid);  // whether that is the faster way for m tokens
 constexpr int CHAIN_MAX_PHASES = 10;
 struct ChainArgs {
   ChainPhase ph[CHAIN_MAX_PHASES];  // the phases, when phases_dev is nullptr

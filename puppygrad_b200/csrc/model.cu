@@ -625,6 +625,7 @@ static int ensure_chain_program(pg_cache* c, int batch, int chunk = 0) {
     ph.push_back(p);
     bucket.push_back(B_LAYER_NORM);
   }
+  const bool sums = chain_makes_input(C, F, batch, c->chain_ctas);
   for (int l = 0; l < L; ++l) {
     const LayerWeights& w = m->layers[l];
     cur_b = B_QKV;
@@ -639,11 +640,17 @@ static int ensure_chain_program(pg_cache* c, int batch, int chunk = 0) {
     rows(C, C, w.b_proj, w.ln2_g, w.ln2_b, w.x_norm2);
     cur_b = B_MLP_FC;
     gemm(w.q_fc, w.x_norm2, F, C, CH_ACT_NORM);
-    elem(F, C, w.b_fc, 1, nullptr, halves_of(c->hbuf), halves_of(c->h_lo), w.x_h);
+    if (!sums) elem(F, C, w.b_fc, 1, nullptr, halves_of(c->hbuf), halves_of(c->h_lo), w.x_h);
     cur_b = B_MLP_PROJ;
-    gemm(w.q_proj2, w.x_h, C, F, CH_ACT_H);
+    gemm(w.q_proj2, w.x_h, C, F, sums ? CH_ACT_SUMS : CH_ACT_H);
+    if (sums) {
+      ph.back().in_bias = w.b_fc;
+      ph.back().in_scale = w.x_h;
+      ph.back().part = 1;
+    }
     if (l + 1 < L) rows(C, F, w.b_proj2, m->layers[l + 1].ln1_g, m->layers[l + 1].ln1_b, m->layers[l + 1].x_norm1);
     else rows(C, F, w.b_proj2, m->lnf_g, m->lnf_b, m->x_normf);
+    ph.back().part = sums ? 1 : 0;
   }
   cur_b = B_LOGITS;
   gemm(m->q_wte, m->x_normf, V, C, CH_ACT_NORM);

@@ -937,6 +937,27 @@ def test_persistent_step_chooses_the_kernels_of_bf16_steps(batch):
     assert_logits_close(got[True], got[False])
 
 
+# In steps of few sequences the MLP's second product makes its own input from the partial sums of the first: widths whose k blocks lie
+# in one part, in equal and in unequal ones, one to four units of a block: up to 24 sequences, 16 at width 832, 12 at 960.
+@pytest.mark.parametrize("n_embd,n_head", [(64, 1), (192, 3), (448, 7), (832, 13), (960, 15)])
+@pytest.mark.parametrize("batch,math_mode", [(9, "tf32x3"), (12, "tf32x3"), (17, "tf32x3"), (24, "tf32x3"), (25, "tf32x3"), (5, "bf16"), (12, "bf16"), (16, "bf16")])
+def test_persistent_steps_of_widths(oracle, n_embd, n_head, batch, math_mode):
+    cfg = dict(synthetic.preset("mini"), n_embd=n_embd, n_head=n_head, n_inner=4 * n_embd)
+    w = synthetic.perturbed_weights(cfg, 61)
+    g = pg.Gpt2Model(cfg, w, pg.Gpt2CudaConfig(math_mode=math_mode))
+    o = oracle.Model(cfg, synthetic.bf16_rounded_weights(w) if math_mode == "bf16" else w, threads=4)
+    prompts = [synthetic.uniform_prompt(1500 + i, 3 + i % 4, cfg["vocab_size"]) for i in range(batch)]
+    cache = g.new_kv_cache(max_batch=batch)
+    _, cur = g.prefill_batch(prompts, cache)
+    ocaches = [o.new_kv_cache() for _ in prompts]
+    for p, c in zip(prompts, ocaches):
+        o.prefill(p, c)
+    for _ in range(2):
+        logits, am, _, _ = g.forward_one_batch(cur, cache, want_logits=True)
+        assert_logits_close(logits, np.stack([o.forward_one(int(t), c) for t, c in zip(cur, ocaches)]))
+        cur = am.copy()
+
+
 def test_narrow_weight_modes_exclude_each_other():
     cfg, w = tiny()
     with pytest.raises(pg.Gpt2Error, match="exclude each other"):
