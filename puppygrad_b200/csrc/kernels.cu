@@ -1495,6 +1495,15 @@ __global__ void __launch_bounds__(1024) topk_rows_kernel(const float* logits, in
   }
 }
 
+// One launch in the place of two copies of four bytes per sequence, 3 to 8 us each.
+__global__ void portion_end_kernel(PortionEndArgs a) {
+  for (int i = threadIdx.x; i < a.n; i += blockDim.x) {
+    const int slot = a.slot ? a.slot[i] : i;
+    a.pos[slot] = (a.start_pos ? a.start_pos[i] : 0) + a.seq_start[i + 1] - a.seq_start[i];
+    if (a.argmax) a.ids[slot] = a.argmax[i];
+  }
+}
+
 // ------------------------------------------------------------------ launch helper
 template <typename... KArgs, typename... Args>
 cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl,
@@ -1708,6 +1717,10 @@ cudaError_t launch_gather_rows(const float* src, const int* rows, float* dst, in
 
 cudaError_t launch_finalize(const FinalizeArgs& a, bool pdl, cudaStream_t s) {
   return launch(finalize_kernel, dim3(a.m), dim3(256), 0, s, pdl, a);
+}
+
+cudaError_t launch_portion_end(const PortionEndArgs& a, cudaStream_t s) {
+  return launch(portion_end_kernel, dim3(1), dim3(128), 0, s, false, a);
 }
 
 cudaError_t init_kernel_attributes() {

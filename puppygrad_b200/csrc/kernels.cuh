@@ -57,6 +57,14 @@ cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cuda
 // dst[o, i] = src[i, o]
 cudaError_t launch_transpose(const float* src, float* dst, int in_f, int out_f, cudaStream_t s);
 
+// After a portion of a prompt: position (and, with argmax, next id) of every sequence's slot. seq_start [n + 1] row offsets; slot nullptr:
+// sequence i in slot i; start_pos nullptr: zeros.
+struct PortionEndArgs {
+  const int *seq_start, *slot, *start_pos, *argmax;
+  int *pos, *ids, n;
+};
+cudaError_t launch_portion_end(const PortionEndArgs& a, cudaStream_t s);
+
 struct DecodeAttnArgs {
   const float* qkv;       // [batch, 3c]
   float* out;             // [batch, c]

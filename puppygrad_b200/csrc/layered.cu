@@ -529,6 +529,7 @@ int build_layer(Builder& b, const LayerSpec& spec, const std::string& p, int pag
 
 int alloc_rows(const LayeredModel* m, LayeredRows* r, size_t rows, bool step) {
   if (rows <= r->rows) return PG_OK;
+  PG_CUDA_TRY(cudaDeviceSynchronize());  // queued work may still use them
   for (void** p : r->buffers()) {
     if (*p) cudaFree(*p);
     *p = nullptr;
@@ -574,6 +575,7 @@ int alloc_rows(const LayeredModel* m, LayeredRows* r, size_t rows, bool step) {
 template <typename P>
 int grow(P** p, size_t* have, size_t want, size_t bytes_each) {
   if (want <= *have) return PG_OK;
+  PG_CUDA_TRY(cudaDeviceSynchronize());  // queued work may still use it
   if (*p) cudaFree((void*)*p);
   *p = nullptr;
   *have = 0;
@@ -1157,11 +1159,10 @@ cudaError_t enqueue_portions(pg_cache* c, const PortionPlan& plan, const Portion
 
 }  // namespace
 
-int layered_run_portions(pg_cache* c, const PortionPlan& plan, float* logits, StepProfiler* prof) {
+int layered_run_portions(pg_cache* c, const PortionPlan& plan, float* logits, StepProfiler* prof, PortionEndArgs* end) {
   const LayeredModel* m = c->model->layered.get();
   LayeredCache* lc = c->layered.get();
   const int rows = plan.rows(), ns = plan.n();
-  PG_CUDA_TRY(cudaStreamSynchronize(c->stream));  // workspaces may be replaced below
   if (int r = alloc_rows(m, &lc->portion, std::max<size_t>(rows, 64), false)) return r;
   // key / value workspace rows per page table: the cached keys a sequence still sees, then its own
   PortionDevice d;
@@ -1231,11 +1232,14 @@ int layered_run_portions(pg_cache* c, const PortionPlan& plan, float* logits, St
   }
   if (seg)
     if (int r = grow(&lc->segments, &lc->seg_floats, seg, sizeof(float))) return r;
-  PG_CUDA_TRY(cudaMemcpyAsync(lc->meta, meta.data(), meta.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  PG_CUDA_TRY(cudaStreamSynchronize(c->stream));  // `meta` is a pageable temporary
+  int* staged = nullptr;
+  if (int r = stage_ints(c, meta.size(), &staged)) return r;
+  std::copy(meta.begin(), meta.end(), staged);
+  if (int r = upload_ints(c, staged, meta.size(), lc->meta)) return r;
   d.ids = lc->meta + o_ids; d.pos = lc->meta + o_pos; d.row_seq = lc->meta + o_rs; d.seq_start = lc->meta + o_ss;
   d.slot = lc->meta + o_sl; d.start_pos = lc->meta + o_sp; d.out_rows = lc->meta + o_or;
   for (size_t o : o_ks) d.key_start.push_back(lc->meta + o);
+  end->seq_start = d.seq_start; end->slot = d.slot; end->start_pos = d.start_pos;
   size_t half = 0;
   for (const Rotation& r : m->rotations) half += r.dims / 2;
   if (half)

@@ -27,7 +27,8 @@ struct PortionPlan {
   int n() const { return (int)slot.size(); }
   int rows() const { return (int)ids.size(); }
 };
-int layered_run_portions(pg_cache* c, const PortionPlan& plan, float* logits, StepProfiler* prof);
+// `end` receives where the device has the plan's sequences.
+int layered_run_portions(pg_cache* c, const PortionPlan& plan, float* logits, StepProfiler* prof, PortionEndArgs* end);
 // Device buffer for the logits of `rows` rows (grow-only).
 int layered_logits_buffer(pg_cache* c, size_t rows, float** out);
 

@@ -96,6 +96,7 @@ pg_cache::~pg_cache() {
   if (t1) cudaEventDestroy(t1);
   if (h_ids) cudaFreeHost(h_ids);
   if (h_out) cudaFreeHost(h_out);
+  if (h_stage) cudaFreeHost(h_stage);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -385,6 +386,29 @@ static int build_model(const pg_gpt2_config& cfg, const float* const* tensors, c
   return PG_OK;
 }
 
+int stage_ints(pg_cache* c, size_t n, int** out) {
+  if (c->stage_used + n > c->stage_ints) {
+    PG_CUDA_TRY(cudaStreamSynchronize(c->stream));  // queued copies still read what is there
+    c->stage_used = 0;
+    if (n > c->stage_ints) {
+      if (c->h_stage) cudaFreeHost(c->h_stage);
+      c->h_stage = nullptr;
+      c->stage_ints = 0;
+      const size_t want = std::max<size_t>(2 * n, 16 * 1024);
+      PG_CUDA_TRY(cudaMallocHost(&c->h_stage, want * sizeof(int)));
+      c->stage_ints = want;
+    }
+  }
+  *out = c->h_stage + c->stage_used;
+  return PG_OK;
+}
+
+int upload_ints(pg_cache* c, const int* staged, size_t n, int* dev) {
+  c->stage_used = staged - c->h_stage + n;
+  PG_CUDA_TRY(cudaMemcpyAsync(dev, staged, n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  return PG_OK;
+}
+
 }  // namespace pg
 
 namespace pg {
@@ -534,14 +558,17 @@ static int ensure_pages(pg_cache* c, int slot, int upto) {
   return PG_OK;
 }
 
+// What was staged has been copied: the stream has nothing left to do.
+static void stream_idle(pg_cache* c) { c->stage_used = 0; }
+
 static int sync_table(pg_cache* c) {
   for (PageTable& t : c->tables) {
     if (!t.dirty) continue;
     // unassigned entries are uploaded as page 0; kernels never index past a slot's seq_len
-    std::vector<int> up(t.h_table.size());
-    for (size_t i = 0; i < up.size(); ++i) up[i] = std::max(t.h_table[i], 0);
-    PG_CUDA_TRY(cudaMemcpyAsync(t.d_table, up.data(), up.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    PG_CUDA_TRY(cudaStreamSynchronize(c->stream));  // `up` is a pageable temporary
+    int* up = nullptr;
+    if (int r = stage_ints(c, t.h_table.size(), &up)) return r;
+    for (size_t i = 0; i < t.h_table.size(); ++i) up[i] = std::max(t.h_table[i], 0);
+    if (int r = upload_ints(c, up, t.h_table.size(), t.d_table)) return r;
     t.dirty = false;
   }
   return PG_OK;
@@ -956,7 +983,7 @@ static int run_decode_step(pg_cache* c, int batch) {
 // ------------------------------------------------------------------ prefill (batched, GEMM path)
 struct PrefillPlan {
   int rows = 0, batch = 0, max_len = 0;
-  std::vector<int> ids, pos, slot, seq_start, last_rows;
+  std::vector<int> seq_start, last_rows;
 };
 
 static int grow_prefill_workspace(pg_cache* c, size_t rows) {
@@ -1127,6 +1154,7 @@ static int recover_after_timeout(pg_cache* c, int code) {
 static int check_device_error(pg_cache* c) {
   PG_CUDA_TRY(cudaMemcpyAsync(c->h_out, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   PG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  stream_idle(c);
   if (c->h_out[0]) return recover_after_timeout(c, c->h_out[0]);
   return PG_OK;
 }
@@ -1145,6 +1173,7 @@ static int fetch_outputs(pg_cache* c, int batch, float* logits_out, int32_t* arg
   const size_t words = lists ? at + 2 * list : argmax_out ? 1 + (size_t)batch : 1;
   PG_CUDA_TRY(cudaMemcpyAsync(c->h_out, c->d_results, words * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   PG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  stream_idle(c);
   if (c->h_out[0]) return recover_after_timeout(c, c->h_out[0]);
   if (argmax_out) memcpy(argmax_out, c->h_out + 1, batch * sizeof(int));
   if (lists && topk_vals) memcpy(topk_vals, c->h_out + at, list * sizeof(float));
@@ -1171,7 +1200,8 @@ static int run_layered_portions(const pg_model* m, pg_cache* c, PortionPlan& pla
   float* logits = nullptr;
   if (!plan.out_rows.empty())
     if (int r = layered_logits_buffer(c, plan.out_rows.size(), &logits)) return r;
-  if (int r = layered_run_portions(c, plan, logits, prof)) return r;
+  PortionEndArgs end{};
+  if (int r = layered_run_portions(c, plan, logits, prof, &end)) return r;
   cudaStream_t s = c->stream;
   if (need_last) {
     PG_CUDA_TRY(cudaMemcpyAsync(c->logits, logits + (size_t)n_want * V, (size_t)n * V * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -1179,15 +1209,11 @@ static int run_layered_portions(const pg_model* m, pg_cache* c, PortionPlan& pla
   }
   if (n_want && want_logits)
     PG_CUDA_TRY(cudaMemcpyAsync(want_logits, logits, (size_t)n_want * V * sizeof(float), cudaMemcpyDeviceToHost, s));
-  std::vector<int> pos(n);
-  for (int i = 0; i < n; ++i) {
-    pos[i] = plan.start_pos[i] + plan.seq_start[i + 1] - plan.seq_start[i];
-    PG_CUDA_TRY(cudaMemcpyAsync(c->d_pos + plan.slot[i], &pos[i], sizeof(int), cudaMemcpyHostToDevice, s));
-    if (need_last)  // the next id of the slot, should a greedy step follow without ids
-      PG_CUDA_TRY(cudaMemcpyAsync(c->d_ids + plan.slot[i], c->d_argmax + i, sizeof(int), cudaMemcpyDeviceToDevice, s));
-  }
+  end.pos = c->d_pos; end.ids = c->d_ids; end.n = n;
+  end.argmax = need_last ? c->d_argmax : nullptr;  // the next id of the slot, should a greedy step follow without ids
+  PG_CUDA_TRY(launch_portion_end(end, s));
   if (int r = check_device_error(c)) return r;  // waits for the stream
-  for (int i = 0; i < n; ++i) c->seq_len[plan.slot[i]] = pos[i];
+  for (int i = 0; i < n; ++i) c->seq_len[plan.slot[i]] = plan.start_pos[i] + plan.seq_start[i + 1] - plan.seq_start[i];
   return PG_OK;
 }
 
@@ -1267,24 +1293,24 @@ static int do_prefill(const pg_model* m, pg_cache* c, const int32_t* ids, const 
     if (int r = ensure_pages(c, b, lens[b])) return r;
   if (int r = sync_table(c)) return r;
   if (int r = grow_prefill_workspace(c, plan.rows)) return r;
-  plan.ids.assign(ids, ids + plan.rows);
+  const size_t R = plan.rows, words = 3 * R + 2 * batch + 1;
+  int* staged = nullptr;
+  if (int r = stage_ints(c, words, &staged)) return r;
+  memcpy(staged, ids, R * sizeof(int));
   for (int b = 0; b < batch; ++b)
     for (int t = 0; t < lens[b]; ++t) {
-      plan.pos.push_back(t);
-      plan.slot.push_back(b);
+      staged[R + plan.seq_start[b] + t] = t;
+      staged[2 * R + plan.seq_start[b] + t] = b;
     }
-  const size_t R = plan.rows;
+  memcpy(staged + 3 * R, plan.seq_start.data(), (batch + 1) * sizeof(int));
+  memcpy(staged + 3 * R + batch + 1, plan.last_rows.data(), batch * sizeof(int));
   int* d_ids = c->prow;
   int* d_pos = c->prow + R;
   int* d_slot = c->prow + 2 * R;
   int* d_start = c->prow + 3 * R;
   int* d_last = d_start + batch + 1;
   cudaStream_t s = c->stream;
-  PG_CUDA_TRY(cudaMemcpyAsync(d_ids, plan.ids.data(), R * sizeof(int), cudaMemcpyHostToDevice, s));
-  PG_CUDA_TRY(cudaMemcpyAsync(d_pos, plan.pos.data(), R * sizeof(int), cudaMemcpyHostToDevice, s));
-  PG_CUDA_TRY(cudaMemcpyAsync(d_slot, plan.slot.data(), R * sizeof(int), cudaMemcpyHostToDevice, s));
-  PG_CUDA_TRY(cudaMemcpyAsync(d_start, plan.seq_start.data(), (batch + 1) * sizeof(int), cudaMemcpyHostToDevice, s));
-  PG_CUDA_TRY(cudaMemcpyAsync(d_last, plan.last_rows.data(), batch * sizeof(int), cudaMemcpyHostToDevice, s));
+  if (int r = upload_ints(c, staged, words, c->prow)) return r;
   PG_CUDA_TRY(launch_embed(m->wte, m->wpe, d_ids, d_pos, c->px, plan.rows, m->c(), false, s));
   BlockWorkspace ws{c->px, c->pnorm, c->pqkv, c->pattn, c->ph, d_slot, d_pos, d_start, c->d_error};
   if (int r = run_blocks(m, ws, plan, c, s)) return r;
@@ -1297,8 +1323,9 @@ static int do_prefill(const pg_model* m, pg_cache* c, const int32_t* ids, const 
   PG_CUDA_TRY(launch_linear_rows(a, EPI_NONE, false, s));
   PG_CUDA_TRY(launch_argmax_rows(c->logits, batch, m->v(), c->d_argmax, s));
   // device-side sequence state: pos = lens, next id = argmax
-  PG_CUDA_TRY(cudaMemcpyAsync(c->d_pos, lens, batch * sizeof(int), cudaMemcpyHostToDevice, s));
-  PG_CUDA_TRY(cudaMemcpyAsync(c->d_ids, c->d_argmax, batch * sizeof(int), cudaMemcpyDeviceToDevice, s));
+  PortionEndArgs end{};
+  end.seq_start = d_start; end.argmax = c->d_argmax; end.pos = c->d_pos; end.ids = c->d_ids; end.n = batch;
+  PG_CUDA_TRY(launch_portion_end(end, s));
   if (int r = fetch_outputs(c, batch, logits_out, argmax_out, nullptr, nullptr, 0)) return r;
   for (int b = 0; b < batch; ++b) c->seq_len[b] = lens[b];
   return PG_OK;

@@ -174,6 +174,23 @@ def test_states_between_segments(layer):
     assert_rows(run_portions(model, model.new_kv_cache(1), 0, [ids[:515], ids[515:]]), case.want(ids), "fp32")
 
 
+def test_calls_of_growing_and_shrinking_size():
+    """The ids, positions and page tables of calls reach the device as they should when a call outgrows the memory they are copied
+    from, and when calls follow one another without a wait between them."""
+    case, n = Case(lo.config(61, 48, [lo.gla(2, 8, 12), lo.pair(2, 1, 8, 8, 9, 2, 8)]), 17, rank=3), 7
+    model = case.model("fp32")
+    cache = model.new_kv_cache(max_batch=n)
+    ids, at = [case.ids(1300, seed=i) for i in range(n)], [0] * n
+    for size in (3, 1, 1100, 2, 160, 1):
+        size = [size + (i % 3 if size > 1 else 0) for i in range(n)]
+        got = model.extend(range(n), [x[t:t + k] for x, t, k in zip(ids, at, size)], cache, range(sum(size)))
+        assert_rows(got, np.concatenate([case.want(x)[t:t + k] for x, t, k in zip(ids, at, size)]), "fp32")
+        at = [t + k for t, k in zip(at, size)]
+    order = list(range(n))[::-1]  # slots in another order
+    got = model.extend(order, [ids[i][at[i]:at[i] + 1 + i] for i in order], cache, range(sum(1 + i for i in order)))
+    assert_rows(got, np.concatenate([case.want(ids[i])[at[i]:at[i] + 1 + i] for i in order]), "fp32")
+
+
 @pytest.mark.parametrize("page_tokens", [16, 64])
 def test_page_sizes(mixed, page_tokens):
     ids = mixed.ids(90, 3)
