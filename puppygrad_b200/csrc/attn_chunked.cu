@@ -37,9 +37,35 @@ __device__ __forceinline__ void warp_norm_row(const float* x, int n, int np, con
 // the same change to the recurrent steps, 24 steps of 64 sequences of Dirurax of width 2048 with their prompts 25.1 -> 24.2 ms (the first keys
 // and values in registers instead of L2: 24.3; two blocks of 102 registers had taken two waves for the 512 of a step).
 constexpr int STEP_THREADS = 256, STEP_KEYS = 256, RB = 4;
+// No more blocks than SMs (FEW): registers for the first HELD rows of keys and values that a thread reads, asked for ahead of the dependency
+// wait; and the parts are a cluster, whose blocks merge them out of each other's shared memory. PLACEHOLDER
+constexpr int HELD = 4, MAX_CLUSTER = 8;
 
+// Eight elements of a row as they lie in memory.
 template <typename T>
-__global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(AttentionStepArgs a, int y_bf16) {
+struct Raw8 {
+  float4 v[sizeof(T) / 2];
+  __device__ __forceinline__ void load(const T* p) {
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T) / 2; ++i) v[i] = load4(reinterpret_cast<const float*>(p) + 4 * i);
+  }
+  __device__ __forceinline__ void get(float (&out)[8]) const { load8(reinterpret_cast<const T*>(v), out); }
+};
+
+__device__ __forceinline__ float cluster_load(const float* p, uint32_t rank) {
+  uint32_t at;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename T, bool FEW>
+__global__ void __launch_bounds__(STEP_THREADS, FEW ? 2 : 4) attention_step_kernel(AttentionStepArgs a, int y_bf16, int clustered) {
   extern __shared__ __align__(16) float sm[];
   __shared__ int last_flag;
   const AttentionLayer& l = a.l;
@@ -50,6 +76,10 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
   float* vn = kn + l.dimp;                   // [vdimp] new value as stored
   float* sc = vn + l.vdimp;                  // [RB][STEP_KEYS]
   float* acc_s = sc + RB * STEP_KEYS;        // [groups][RB][vdimp] cross-thread sums
+  const int nvec = l.vdimp / 8, groups = STEP_THREADS / nvec;  // value phase: thread = (8 columns, key subset)
+  const int vc = tid % nvec, vg = tid / nvec;
+  const int sub = lane >> 3, l8 = lane & 7;
+  float* part_s = acc_s + (size_t)groups * RB * l.vdimp;  // [rep][vdim + 2]: this part's maxima, sums, sums of values, for the cluster
   __shared__ float red_m[RB], red_l[RB], corr_s[RB];
 
   grid_dep_launch();
@@ -60,6 +90,15 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
   const int* table = a.page_table + (size_t)seq * l.pages_per_seq;
   T* pool = static_cast<T*>(a.pool);
   const bool owner = k0 <= last && last < k1;
+  Raw8<T> held_k[FEW ? HELD : 1], held_v[FEW ? HELD : 1];
+  if (FEW) {
+#pragma unroll
+    for (int u = 0; u < HELD; ++u) {
+      const int jk = k0 + u * (STEP_THREADS / 8) + warp * 4 + sub, jv = k0 + u * groups + vg;
+      if (jk < min(k1, last) && l8 * 8 < l.dimp) held_k[u].load(page_row(l, pool, table, jk, kvh, 0) + l8 * 8);
+      if (jv < min(k1, last) && vg < groups) held_v[u].load(page_row(l, pool, table, jv, kvh, 1) + vc * 8);
+    }
+  }
   for (int j = k0 + tid; j < min(last, min(k1, k0 + STEP_KEYS)); j += STEP_THREADS) {
     const T *kr = page_row(l, pool, table, j, kvh, 0), *vr = page_row(l, pool, table, j, kvh, 1);
     for (int c = 0; c < l.dimp; c += 128 / (int)sizeof(T)) asm volatile("prefetch.global.L2 [%0];" ::"l"(kr + c));
@@ -89,10 +128,6 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
   }
   __syncthreads();
 
-  const int nvec = l.vdimp / 8, groups = STEP_THREADS / nvec;  // value phase: thread = (8 columns, key subset)
-  const int vc = tid % nvec, vg = tid / nvec;
-  const int sub = lane >> 3, l8 = lane & 7;
-
   for (int r0 = 0; r0 < rep; r0 += RB) {
     const int nr = min(RB, rep - r0);
     float m_run[RB], l_run[RB], acc[RB][8];
@@ -105,7 +140,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
     }
     for (int kb = k0; kb < k1; kb += STEP_KEYS) {
       const int n = min(STEP_KEYS, k1 - kb);
-      for (int j0 = warp * 4; j0 < n; j0 += STEP_THREADS / 32 * 4) {
+      auto scores = [&](int j0, const Raw8<T>* held) {  // of keys j0 .. j0 + 3
         const int j = j0 + sub;
         float dot[RB];
 #pragma unroll
@@ -116,6 +151,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
           for (int c = l8 * 8; c < l.dimp; c += 64) {
             float kv[8];
             if (self) load8(kn + c, kv);
+            else if (held && c < 64) held->get(kv);
             else load8(krow + c, kv);
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
@@ -137,7 +173,14 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
           for (int r = 0; r < RB; ++r)
             if (r < nr) sc[r * STEP_KEYS + j] = dot[r] * l.scale;
         }
+      };
+      int j0 = warp * 4;
+      if (FEW && kb == k0) {
+#pragma unroll
+        for (int u = 0; u < HELD; ++u, j0 += STEP_THREADS / 8)
+          if (j0 < n) scores(j0, &held_k[u]);
       }
+      for (; j0 < n; j0 += STEP_THREADS / 8) scores(j0, nullptr);
       __syncthreads();
       if (warp < nr) {  // one warp per query head: running maximum, probabilities, sum
         float mx = -FLT_MAX;
@@ -171,9 +214,10 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
           for (int c = 0; c < 8; ++c) acc[r][c] *= corr_s[r];
         }
       if (vg < groups) {
-        for (int j = vg; j < n; j += groups) {
+        auto values = [&](int j, const Raw8<T>* held) {
           float vv[8];
           if (kb + j == last) load8(vn + vc * 8, vv);
+          else if (held) held->get(vv);
           else load8(page_row(l, pool, table, kb + j, kvh, 1) + vc * 8, vv);
 #pragma unroll
           for (int r = 0; r < RB; ++r)
@@ -182,7 +226,14 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
 #pragma unroll
               for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(pr, vv[e], acc[r][e]);
             }
+        };
+        int j = vg;
+        if (FEW && kb == k0) {
+#pragma unroll
+          for (int u = 0; u < HELD; ++u, j += groups)
+            if (j < n) values(j, &held_v[u]);
         }
+        for (; j < n; j += groups) values(j, nullptr);
       }
       __syncthreads();
     }
@@ -213,7 +264,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
         if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[at] = __float2bfloat16_rn(y);
         else static_cast<float*>(a.y)[at] = y;
       } else {
-        float* pt = a.part + (((size_t)seq * l.heads + h) * a.splits + split) * (l.vdim + 2);
+        float* pt = FEW && clustered ? part_s + (r0 + r) * (l.vdim + 2) : a.part + (((size_t)seq * l.heads + h) * a.splits + split) * (l.vdim + 2);
         pt[2 + c] = s;
         if (c == 0) {
           pt[0] = mr;
@@ -224,6 +275,39 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
     __syncthreads();
   }
   if (a.splits == 1) return;
+  auto store = [&](int i, float y) {
+    const size_t at = (size_t)seq * a.ldy + (kvh * rep + i / l.vdim) * l.vdim + i % l.vdim;
+    if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[at] = __float2bfloat16_rn(y);
+    else static_cast<float*>(a.y)[at] = y;
+  };
+  if (FEW && clustered) {  // part s is in the block of rank s
+    cluster_sync();
+    for (int i = split * STEP_THREADS + tid; i < rep * l.vdim; i += a.splits * STEP_THREADS) {
+      const int c = i % l.vdim;
+      const float* pt = part_s + i / l.vdim * (l.vdim + 2);
+      float m[MAX_CLUSTER], sum[MAX_CLUSTER], v[MAX_CLUSTER], top = -FLT_MAX, num = 0.f, den = 0.f;
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s)
+        if (s < a.splits) {
+          m[s] = cluster_load(pt, s);
+          sum[s] = cluster_load(pt + 1, s);
+          v[s] = cluster_load(pt + 2 + c, s);
+        }
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s)
+        if (s < a.splits) top = fmaxf(top, m[s]);
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s)
+        if (s < a.splits) {
+          const float w = expf(m[s] - top);
+          num += w * v[s];
+          den += w * sum[s];
+        }
+      store(i, num / den * l.out_scale);
+    }
+    cluster_sync();  // nobody leaves before the others have read
+    return;
+  }
   __threadfence();
   __syncthreads();
   if (tid == 0) {
@@ -245,10 +329,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) attention_step_kernel(Attenti
       num += w * pt[s * (l.vdim + 2) + 2 + c];
       den += w * pt[s * (l.vdim + 2) + 1];
     }
-    const float y = num / den * l.out_scale;
-    const size_t at = (size_t)seq * a.ldy + h * l.vdim + c;
-    if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[at] = __float2bfloat16_rn(y);
-    else static_cast<float*>(a.y)[at] = y;
+    store(i, num / den * l.out_scale);
   }
 }
 
@@ -507,6 +588,44 @@ size_t step_smem(const AttentionLayer& l) {
   return ((size_t)(l.heads / l.kv_heads) * l.dimp + l.dimp + l.vdimp + RB * STEP_KEYS + (size_t)groups * RB * l.vdimp) * sizeof(float);
 }
 
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 148;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) v = 148;
+    return v;
+  }();
+  return n;
+}
+
+template <typename T, bool FEW>
+cudaError_t launch_step(const AttentionStepArgs& a, size_t smem, bool y_bf16, bool pdl, cudaStream_t s) {
+  const AttentionLayer& l = a.l;
+  const bool clustered = FEW && a.splits > 1 && a.splits <= MAX_CLUSTER;
+  auto kernel = attention_step_kernel<T, FEW>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(l.kv_heads, a.batch, a.splits);
+  cfg.blockDim = dim3(STEP_THREADS);
+  cfg.dynamicSmemBytes = smem + (clustered ? (size_t)(l.heads / l.kv_heads) * (l.vdim + 2) * sizeof(float) : 0);
+  if (cfg.dynamicSmemBytes > 208 * 1024) return cudaErrorInvalidValue;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  if (clustered) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim = {1, 1, (unsigned)a.splits};
+    ++cfg.numAttrs;
+  }
+  if (pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, a, y_bf16 ? 1 : 0, clustered ? 1 : 0);
+}
+
 }  // namespace
 
 size_t attention_page_elems(const AttentionLayer& l) { return (size_t)l.kv_heads * l.page_tokens * (l.dimp + l.vrow); }
@@ -517,15 +636,9 @@ cudaError_t launch_attention_step(const AttentionStepArgs& a, bool bf16, bool y_
   const AttentionLayer& l = a.l;
   const size_t smem = step_smem(l);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  const dim3 grid(l.kv_heads, a.batch, a.splits);
-  const int yb = y_bf16 ? 1 : 0;
-  cudaError_t e;
-  if (bf16) {
-    e = cudaFuncSetAttribute(attention_step_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return e != cudaSuccess ? e : launch_kernel(attention_step_kernel<__nv_bfloat16>, grid, dim3(STEP_THREADS), smem, s, pdl, a, yb);
-  }
-  e = cudaFuncSetAttribute(attention_step_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  return e != cudaSuccess ? e : launch_kernel(attention_step_kernel<float>, grid, dim3(STEP_THREADS), smem, s, pdl, a, yb);
+  const bool few = (long long)l.kv_heads * a.batch * a.splits <= sm_count();
+  if (bf16) return few ? launch_step<__nv_bfloat16, true>(a, smem, y_bf16, pdl, s) : launch_step<__nv_bfloat16, false>(a, smem, y_bf16, pdl, s);
+  return few ? launch_step<float, true>(a, smem, y_bf16, pdl, s) : launch_step<float, false>(a, smem, y_bf16, pdl, s);
 }
 
 cudaError_t launch_attention_context(const AttentionPortionArgs& a, bool bf16, cudaStream_t s) {

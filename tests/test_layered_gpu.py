@@ -174,6 +174,19 @@ def test_states_between_segments(layer):
     assert_rows(run_portions(model, model.new_kv_cache(1), 0, [ids[:515], ids[515:]]), case.want(ids), "fp32")
 
 
+# Parts of the keys as a cluster (up to 8) and beyond; more rows than a block holds in registers; groups of one, four and nine query
+# heads; rows of one piece of 64 and of several, values of 8 to 256.
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("splits", [1, 3, 8, 11])
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(9, 1, 72, 40), (4, 4, 7, 3), (8, 2, 64, 64), (2, 1, 200, 256)])
+def test_parts_of_a_step(mode, splits, heads, kv_heads, dim, vdim):
+    case = Case(lo.config(67, 48, [lo.pair(heads, kv_heads, dim, vdim, 400, 1, 8, right_scale=0.0)]), 6)
+    ids = case.ids(408)
+    model = case.model(mode, attn_splits=splits)
+    cache = model.new_kv_cache(1)
+    assert_rows(run_portions(model, cache, 0, [ids[:1], ids[1:2], ids[2:3], ids[3:130], ids[130:131], ids[131:390]] + [[t] for t in ids[390:]]), case.want(ids), mode)
+
+
 def test_calls_of_growing_and_shrinking_size():
     """The ids, positions and page tables of calls reach the device as they should when a call outgrows the memory they are copied
     from, and when calls follow one another without a wait between them."""
