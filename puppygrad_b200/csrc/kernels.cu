@@ -1369,8 +1369,8 @@ __device__ __forceinline__ float value_of_key(int k) { return __int_as_float(k ^
 // 50257 at k = 40: 17.6 us (the rounds: 123 us). Bound by latency: the row once (loads issued ROW_LOADS at a time: the arg-max
 // of such rows takes 10 us, one load at a time 27 us), 32 counting barriers, one pass over the keys of the winners' threads.
 constexpr int TOPK_CAND = 512;
-__global__ void __launch_bounds__(1024) topk_rows_kernel(const float* logits, int m, int n, int k, float* vals,
-                                                         int* idx) {
+__global__ void __launch_bounds__(1024) topk_rows_kernel(const float* logits, int m, int n, int k, const int* k_at,
+                                                         int* lists) {
   extern __shared__ float4 dyn_smem4[];
   int* keys = reinterpret_cast<int*>(dyn_smem4);  // [n] total-order keys, INT_MIN = removed
   __shared__ int sk[32];
@@ -1380,6 +1380,10 @@ __global__ void __launch_bounds__(1024) topk_rows_kernel(const float* logits, in
   __shared__ int cand_i[TOPK_CAND];
   __shared__ int n_cand;
   const int r = blockIdx.x;
+  if (k_at) k = *k_at;  // written before this step began
+  float* vals = reinterpret_cast<float*>(lists);
+  int* idx = lists + (size_t)m * k;
+  pdl_wait();
   const float* row = logits + (size_t)r * n;
   int my_k = INT_MIN, my_i = INT_MAX;  // best of this thread's keys; scanning upwards keeps the lower index on ties
   for (int i0 = threadIdx.x; i0 < n; i0 += ROW_LOADS * 1024) {
@@ -1769,11 +1773,11 @@ cudaError_t launch_argmax_rows(const float* logits, int m, int n, int* out, cuda
   return cudaGetLastError();
 }
 
-cudaError_t launch_topk_rows(const float* logits, int m, int n, int k, float* vals, int* idx, cudaStream_t s) {
-  size_t smem = ((size_t)n * sizeof(int) + 15) & ~(size_t)15;
-  if (smem > 220 * 1024) return cudaErrorInvalidValue;
-  topk_rows_kernel<<<m, 1024, smem, s>>>(logits, m, n, k, vals, idx);
-  return cudaGetLastError();
+bool topk_rows_supported(int n) { return (((size_t)n * sizeof(int) + 15) & ~(size_t)15) <= 220 * 1024; }
+
+cudaError_t launch_topk_rows(const float* logits, int m, int n, int k, const int* k_at, int* lists, bool pdl, cudaStream_t s) {
+  if (!topk_rows_supported(n)) return cudaErrorInvalidValue;
+  return launch(topk_rows_kernel, dim3(m), dim3(1024), ((size_t)n * sizeof(int) + 15) & ~(size_t)15, s, pdl, logits, m, n, k, k_at, lists);
 }
 
 }  // namespace pg

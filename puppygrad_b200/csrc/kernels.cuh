@@ -344,6 +344,9 @@ cudaError_t launch_round_bf16(float* w, size_t n, uint16_t* packed, cudaStream_t
 // Plain argmax over rows of a [m, n] matrix (first strict maximum).
 cudaError_t launch_argmax_rows(const float* logits, int m, int n, int* out, cudaStream_t s);
 // k largest per row, descending, ties by lower index; k <= 64.
-cudaError_t launch_topk_rows(const float* logits, int m, int n, int k, float* vals, int* idx, cudaStream_t s);
+// The k largest of every row: lists is [m][k] values, then [m][k] indices. k_at: where the device has k (nullptr: k itself), so that a
+// graph serves every k.
+bool topk_rows_supported(int n);
+cudaError_t launch_topk_rows(const float* logits, int m, int n, int k, const int* k_at, int* lists, bool pdl, cudaStream_t s);
 
 }  // namespace pg

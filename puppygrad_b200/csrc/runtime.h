@@ -144,6 +144,7 @@ struct pg_cache {
   std::vector<PageTable> tables;  // GPT-2: one; layered models: one per distinct key lifetime
   float* kv_pool = nullptr;    // [layer][page][2][head][page_tokens][head_dim]
   std::vector<int> seq_len;    // host mirror of d_pos
+  int* d_call = nullptr;  // what comes with a call: [3] length of the lists, [4..] d_ids
   int *d_ids = nullptr, *d_pos = nullptr, *d_argmax = nullptr, *d_token_log = nullptr;
   float *x = nullptr, *norm = nullptr, *qkv = nullptr, *attn = nullptr, *hbuf = nullptr, *logits = nullptr;
   float* part_val = nullptr;
@@ -173,6 +174,7 @@ struct pg_cache {
     unsigned long long* d_times = nullptr;  // n + 1 time stamps, written in profiling runs
   };
   std::map<int, ChainProgram> chain_programs;
+  bool step_lists = false;  // the step makes lists of its largest logits, into d_results
   bool step_wants_logits = true;  // false: the caller of this step only reads the arg-max (greedy decoding)
   // single-kernel decode step (at most 8 sequences): layer table, tagged exchange buffers, tag counter
   unsigned long long* d_stream_ll = nullptr;  // ll_x | ll_qkv | ll_attn | ll_h | ll_part | ll_best
@@ -182,7 +184,7 @@ struct pg_cache {
 #ifdef PG_DEV_TRACE
   unsigned long long* d_stream_trace = nullptr;
 #endif
-  int *h_ids = nullptr, *h_out = nullptr;  // pinned staging
+  int *h_call = nullptr, *h_out = nullptr;  // pinned staging; h_call as d_call
   // Pinned memory that the numbers of a call (ids, positions, page tables) are copied from without waiting for the copies: pieces are
   // taken one after the other, and over again once the stream has been waited for (upload_ints, stream_idle). GPT-2 small's first token
   // 616 -> 602 us, 64 prompts and 24 steps of Dirurax of width 2048 24.26 -> 24.00 ms.

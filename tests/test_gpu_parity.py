@@ -558,6 +558,19 @@ def test_device_topk_of_equal_logits(vocab, run, k):
         assert am2[r] == order[0]
 
 
+@pytest.mark.parametrize("batch", [1, 3])
+def test_device_topk_of_changing_length(midi, batch):
+    """One graph of the step serves lists of every length; none, and logits alone, in between."""
+    cfg, w, g, o = midi
+    cache = g.new_kv_cache(max_batch=batch)
+    _, cur = g.prefill_batch([synthetic.uniform_prompt(700 + i, 5, cfg["vocab_size"]) for i in range(batch)], cache)
+    for k in (40, 1, 0, 64, 7, 40):
+        logits, cur, tv, ti = g.forward_one_batch(cur, cache, want_logits=True, top_k=k)
+        for r in range(batch if k else 0):
+            order = sorted(range(cfg["vocab_size"]), key=lambda i: (-float(logits[r, i]), i))[:k]
+            assert list(ti[r]) == order and np.array_equal(tv[r], logits[r, order])
+
+
 @pytest.mark.parametrize("kw", [dict(temperature=0.8, top_k=40), dict(temperature=0.9, top_p=0.95),
                                 dict(temperature=0.0, repeat_penalty=1.4), dict(temperature=0.0)])
 def test_generate_with_config_matches_oracle_loop(midi, oracle, kw):
