@@ -586,6 +586,7 @@ cudaError_t rows_core(const AttentionPortionArgs& a, cudaStream_t s) {
   return e == cudaSuccess && l.v_rot ? launch_attention_turn_back(a, s) : e;
 }
 
+constexpr size_t STEP_SMEM = 200 * 1024;
 size_t step_smem(const AttentionLayer& l) {
   const int groups = STEP_THREADS / (l.vdimp / 8);
   return ((size_t)(l.heads / l.kv_heads) * l.dimp + l.dimp + l.vdimp + RB * STEP_KEYS + (size_t)groups * RB * l.vdimp) * sizeof(float);
@@ -604,16 +605,16 @@ int sm_count() {
 template <typename T, bool FEW>
 cudaError_t launch_step(const AttentionStepArgs& a, size_t smem, bool y_bf16, bool pdl, cudaStream_t s) {
   const AttentionLayer& l = a.l;
-  const bool clustered = FEW && a.splits > 1 && a.splits <= MAX_CLUSTER;
+  const size_t parts = (size_t)(l.heads / l.kv_heads) * (l.vdim + 2) * sizeof(float);
+  const bool clustered = FEW && a.splits > 1 && a.splits <= MAX_CLUSTER && smem + parts <= STEP_SMEM;
   auto kernel = attention_step_kernel<T, FEW>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEP_SMEM);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(l.kv_heads, a.batch, a.splits);
   cfg.blockDim = dim3(STEP_THREADS);
-  cfg.dynamicSmemBytes = smem + (clustered ? (size_t)(l.heads / l.kv_heads) * (l.vdim + 2) * sizeof(float) : 0);
-  if (cfg.dynamicSmemBytes > 208 * 1024) return cudaErrorInvalidValue;
+  cfg.dynamicSmemBytes = smem + (clustered ? parts : 0);
   cfg.stream = s;
   cfg.attrs = attr;
   if (clustered) {
@@ -633,12 +634,12 @@ cudaError_t launch_step(const AttentionStepArgs& a, size_t smem, bool y_bf16, bo
 
 size_t attention_page_elems(const AttentionLayer& l) { return (size_t)l.kv_heads * l.page_tokens * (l.dimp + l.vrow); }
 
-bool attention_supported(const AttentionLayer& l) { return step_smem(l) <= 200 * 1024; }
+bool attention_supported(const AttentionLayer& l) { return step_smem(l) <= STEP_SMEM; }
 
 cudaError_t launch_attention_step(const AttentionStepArgs& a, bool bf16, bool y_bf16, bool pdl, cudaStream_t s) {
   const AttentionLayer& l = a.l;
   const size_t smem = step_smem(l);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > STEP_SMEM) return cudaErrorInvalidValue;
   const bool few = (long long)l.kv_heads * a.batch * a.splits <= sm_count();
   if (bf16) return few ? launch_step<__nv_bfloat16, true>(a, smem, y_bf16, pdl, s) : launch_step<__nv_bfloat16, false>(a, smem, y_bf16, pdl, s);
   return few ? launch_step<float, true>(a, smem, y_bf16, pdl, s) : launch_step<float, false>(a, smem, y_bf16, pdl, s);

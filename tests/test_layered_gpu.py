@@ -175,10 +175,10 @@ def test_states_between_segments(layer):
 
 
 # Parts of the keys as a cluster (up to 8) and beyond; more rows than a block holds in registers; groups of one, four and nine query
-# heads; rows of one piece of 64 and of several, values of 8 to 256.
+# heads; rows of one piece of 64 and of several, values of 8 to 256; a group whose parts do not fit beside the rest of shared memory.
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("splits", [1, 3, 8, 11])
-@pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(9, 1, 72, 40), (4, 4, 7, 3), (8, 2, 64, 64), (2, 1, 200, 256)])
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim", [(9, 1, 72, 40), (4, 4, 7, 3), (8, 2, 64, 64), (2, 1, 200, 256), (120, 1, 256, 256)])
 def test_parts_of_a_step(mode, splits, heads, kv_heads, dim, vdim):
     case = Case(lo.config(67, 48, [lo.pair(heads, kv_heads, dim, vdim, 400, 1, 8, right_scale=0.0)]), 6)
     ids = case.ids(408)
