@@ -55,9 +55,15 @@ inline size_t step_floats(const RecurrenceLayer& l, int buffers) {
 // and four columns of the state, so that nothing is asked per row.
 enum { STEP_ONE = 0, STEP_MANY = 1, STEP_FULL = 2 };
 constexpr int step_blocks(int nr) { return nr <= 4 ? 4 : nr <= 8 ? 3 : 2; }  // on an SM
+// With several items to a block the weights that a thread needs for each of them, all of one head, stay in shared memory, in words that it
+// copies and reads itself, where sizes allow (held_at; 0: not). They came from L2 for every item, three round trips of its chain:
+// 64 sequences, 16 heads of 64 x 128 20.8 -> 17.6 us, 32 of 64 x 64 29.8 -> 26.0; 24 steps of Dirurax of width 2048 with their prompts
+// 23.66 -> 23.13 ms. In registers, for a block's only item, they took 17.37 ms instead of 17.22 (64 steps of one sequence of width 1024: loads in
+// front of the dependency wait stand in the way of the product's), and held taps and gates gain the channel rule nothing (21.96 and 21.92).
+constexpr int HELD_W = 16, STEP_HELD = HELD_W + 3;  // rows of the decay projection; its bias, bias of the removal rate, norm
 
 template <int NR, int MODE>
-__global__ void __launch_bounds__(STEP_THREADS, MODE != STEP_ONE ? step_blocks(NR) : 1) recurrence_step_kernel(RecurrenceStepArgs a, int y_bf16, int ahead_at) {
+__global__ void __launch_bounds__(STEP_THREADS, MODE != STEP_ONE ? step_blocks(NR) : 1) recurrence_step_kernel(RecurrenceStepArgs a, int y_bf16, int ahead_at, int held_at) {
   constexpr bool MANY = MODE != STEP_ONE, FULL = MODE == STEP_FULL;
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[33];
@@ -110,6 +116,16 @@ __global__ void __launch_bounds__(STEP_THREADS, MODE != STEP_ONE ? step_blocks(N
     for (int i = 0; i < NRR; ++i)
       if (kg + i * KG < own) st[i] = quad(load4(from + (size_t)i * KG * dvp));
   }
+  const bool hold = MANY && held_at > 0;
+  float* held = sm + held_at + tid;
+  if (hold) {
+    const int RG = STEP_THREADS / dk;  // as below
+    if (tid < RG * dk)
+      for (int r = tid / dk, at = 0; r < l.rank; r += RG, at += STEP_THREADS) async_copy1(held + at, l.w2 + (size_t)r * K + head * dk + tid % dk);
+    if (tid < dk) async_copy1(held + HELD_W * STEP_THREADS, l.b2 + head * dk + tid);
+    if (tid < dk && delta) async_copy1(held + (HELD_W + 1) * STEP_THREADS, l.a_bias + head * dk + tid);
+    if (tid < dv) async_copy1(held + (HELD_W + 2) * STEP_THREADS, l.norm + (delta ? head * dv : 0) + tid);
+  }
   grid_dep_wait();
   fetch(first, sm);
   int flip = 0;
@@ -143,24 +159,33 @@ __global__ void __launch_bounds__(STEP_THREADS, MODE != STEP_ONE ? step_blocks(N
     const float inv_norm = 1.f / sqrtf(kk + UNIT_EPS);
     // second half of the decay projection: RG threads share a channel, so that its weights arrive in one round trip or two
     const int RG = dk >= STEP_THREADS ? 1 : STEP_THREADS / dk;
-    for (int i = tid; i < RG * dk; i += STEP_THREADS) {
-      const int c = i % dk, g = i / dk;
-      const float* __restrict__ w2 = l.w2 + head * dk + c;
-      float z = 0.f;
+    if (hold) {
+      if (tid < RG * dk) {
+        float z = 0.f;
+#pragma unroll 8
+        for (int r = tid / dk, at = 0; r < l.rank; r += RG, at += STEP_THREADS) z = fmaf(held[at], ts[r], z);
+        zs[tid] = z;
+      }
+    } else {
+      for (int i = tid; i < RG * dk; i += STEP_THREADS) {
+        const int c = i % dk, g = i / dk;
+        const float* __restrict__ w2 = l.w2 + head * dk + c;
+        float z = 0.f;
 #pragma unroll 16
-      for (int r = g; r < l.rank; r += RG) z = fmaf(w2[(size_t)r * K], ts[r], z);
-      zs[i] = z;
+        for (int r = g; r < l.rank; r += RG) z = fmaf(w2[(size_t)r * K], ts[r], z);
+        zs[i] = z;
+      }
     }
     __syncthreads();
     for (int c = tid; c < dk; c += STEP_THREADS) {
       const int ch = head * dk + c;
-      float z = l.b2[ch];
+      float z = hold ? held[HELD_W * STEP_THREADS] : l.b2[ch];
       for (int g = 0; g < RG; ++g) z += zs[g * dk + c];
       float b = 0.f;
       if (delta) {
         const float u = ks[c] * inv_norm;
         us[c] = u;
-        b = sigmoid_f(as[c] + l.a_bias[ch]) * u;
+        b = sigmoid_f(as[c] + (hold ? held[(HELD_W + 1) * STEP_THREADS] : l.a_bias[ch])) * u;
       }
       rp[c] = make_float4(decay_of(l.kind, z, l.inv_tau), ks[c], qs[c], b);
     }
@@ -215,7 +240,7 @@ __global__ void __launch_bounds__(STEP_THREADS, MODE != STEP_ONE ? step_blocks(N
     const float rinv = 1.f / sqrtf(sq / (float)dv + l.eps);
     for (int c = tid; c < dv; c += STEP_THREADS) {
       const float gate = delta ? sigmoid_f(gs[c]) : silu_f(gs[c]);
-      const float y = os[c] * rinv * l.norm[delta ? head * dv + c : c] * gate * l.out_scale;
+      const float y = os[c] * rinv * (hold ? held[(HELD_W + 2) * STEP_THREADS] : l.norm[delta ? head * dv + c : c]) * gate * l.out_scale;
       const size_t at = (size_t)seq * a.ldy + head * dv + c;
       if (y_bf16) static_cast<__nv_bfloat16*>(a.y)[at] = __float2bfloat16_rn(y);
       else static_cast<float*>(a.y)[at] = y;
@@ -239,7 +264,7 @@ inline size_t channel_floats(const RecurrenceLayer& l, int buffers) {
 constexpr int channel_blocks(int nr) { return nr > 0 && nr <= 8 ? 2 : 1; }
 
 template <int NR, int MODE>
-__global__ void __launch_bounds__(CH_THREADS, channel_blocks(NR)) channel_step_kernel(RecurrenceStepArgs a, int y_bf16, int ahead_at) {
+__global__ void __launch_bounds__(CH_THREADS, channel_blocks(NR)) channel_step_kernel(RecurrenceStepArgs a, int y_bf16, int ahead_at, int) {
   constexpr bool MANY = MODE != STEP_ONE, FULL = MODE == STEP_FULL;
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[CH_WARPS], lengths[3];  // of key and query; write strength
@@ -417,7 +442,7 @@ int sm_count() {
 constexpr size_t step_smem_limit(int per_sm) { return (size_t)227 * 1024 / per_sm - 1024; }
 
 // The instances that hold NR rows of the state per thread.
-typedef void (*StepKernel)(RecurrenceStepArgs, int, int);
+typedef void (*StepKernel)(RecurrenceStepArgs, int, int, int);
 struct StepKernels {
   StepKernel one, some, full;
   int nr, threads, per_sm;
@@ -444,9 +469,13 @@ cudaError_t launch_step(const StepKernels& k, const RecurrenceStepArgs& a, int y
   const int items = l.heads * a.batch, resident = k.per_sm * sm_count() / l.heads * l.heads;
   const size_t smem = floats(1) * sizeof(float), ahead = (floats(2) + 3) / 4 * 16, bytes = ahead + (size_t)k.nr * k.threads * 16;
   if (k.nr == 0 || resident == 0 || items <= resident || bytes > step_smem_limit(k.per_sm))
-    return launch_kernel(k.one, dim3(items), dim3(k.threads), smem, s, pdl, a, yb, 0);
+    return launch_kernel(k.one, dim3(items), dim3(k.threads), smem, s, pdl, a, yb, 0, 0);
+  const bool fits = l.kind != KIND_CHANNEL && l.dim <= STEP_THREADS && l.vdim <= STEP_THREADS && l.rank <= HELD_W * (STEP_THREADS / l.dim);
+  const size_t held = (size_t)STEP_HELD * STEP_THREADS * sizeof(float);
+  const bool hold = fits && bytes + held <= step_smem_limit(k.per_sm);
   const bool full = l.dim == k.nr * (k.threads / (l.dvp / 4)) && k.threads % (l.dvp / 4) == 0;
-  return launch_kernel(full ? k.full : k.some, dim3(resident), dim3(k.threads), bytes, s, pdl, a, yb, (int)(ahead / sizeof(float)));
+  return launch_kernel(full ? k.full : k.some, dim3(resident), dim3(k.threads), bytes + (hold ? held : 0), s, pdl, a, yb, (int)(ahead / sizeof(float)),
+                       hold ? (int)(bytes / sizeof(float)) : 0);
 }
 
 cudaError_t launch_channel_step(const RecurrenceStepArgs& a, int yb, bool pdl, cudaStream_t s) {

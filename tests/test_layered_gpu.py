@@ -68,6 +68,13 @@ def test_steps_of_many_sequences(name):
     many_sequences(Case(MANY[name], 7, rank=9))
 
 
+# The most columns of the decay projection that such a block keeps (16 for each of the threads that share a channel), and one more.
+@pytest.mark.parametrize("name, rank", [("gla-16", 256), ("gla-10-wide", 64), ("gla-10-wide", 65), ("gla-5-wider", 32), ("delta-13", 64), ("delta-13", 66),
+                                        ("delta-8-wide", 32), ("delta-8-wide", 33)])
+def test_steps_of_many_sequences_and_ranks(name, rank):
+    many_sequences(Case(MANY[name], 7, rank=rank))
+
+
 # Products of 9 to 64 rows take tiles of 64 weight rows: one row, whole and half tiles, and a row or two beside them; two tiles of 128 to a tile
 # of the weights' layout; input rows at the edges of 16, 32 and 64; k in one part and in several.
 @pytest.mark.parametrize("vocab", [63, 64, 65, 127, 129, 193])
