@@ -88,7 +88,8 @@ constexpr int LIN_WARPS = LIN_THREADS / 32;
 constexpr int LIN_ROWS = 4;
 
 // ------------------------------------------------------------------ decode linear
-// CTA: LIN_ROWS weight rows per group, the 128 threads split K; grid-stride over row groups.
+// CTA: LIN_ROWS weight rows per group, the 128 threads split K; grid-stride over row groups and, where there are more than MT input rows,
+// over groups of MT of them.
 // Replaces linear_block_into / transposed_dense_projection_into / logits_from_hidden_into
 // (src/models/gpt2/rust.rs:1481-1532, 1767-1813; src/models/cpu.rs:58-75) and, fused,
 // layer_norm_in_place, gelu_in_place, add_in_place (cpu.rs:119-171).
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_decode_kernel(LinearArgs a
   // 128-bit chunks per weight row that every thread requests before the dependency wait
   constexpr int PRE = MT <= 2 ? 3 : 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int k4 = a.k >> 2;
+  const int k4 = a.k >> 2, m_first = blockIdx.y * MT;
   const int groups = (a.n + LIN_ROWS - 1) / LIN_ROWS;
   const float4* w4 = reinterpret_cast<const float4*>(a.w);
 
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_decode_kernel(LinearArgs a
 
   float resid_pre = 0.f;
   if (EPI == EPI_RESID && tid < NV) {
-    const int row = blockIdx.x * LIN_ROWS + tid / MT, m = tid % MT;
+    const int row = blockIdx.x * LIN_ROWS + tid / MT, m = m_first + tid % MT;
     if (row < a.n && m < a.m) resid_pre = a.resid[(size_t)m * a.n + row];
   }
 
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_decode_kernel(LinearArgs a
 #pragma unroll
     for (int r = 0; r < LIN_ROWS; ++r) wrow[r] = w4 + (size_t)min(row0 + r, a.n - 1) * k4;
 
-    for (int m0 = 0; m0 < a.m; m0 += MT) {
+    for (int m0 = m_first; m0 < a.m; m0 += MT * gridDim.y) {
       float acc[NV];
 #pragma unroll
       for (int i = 0; i < NV; ++i) acc[i] = 0.f;
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_decode_kernel(LinearArgs a
       };
 
       int cstart = tid;
-      if (first_group && m0 == 0) {
+      if (first_group && m0 == m_first) {
 #pragma unroll
         for (int j = 0; j < PRE; ++j) {
           const int c = tid + j * LIN_THREADS;
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(LIN_THREADS) linear_decode_kernel(LinearArgs a
           const float b = (first_group || !a.bias) ? bias_pre : a.bias[row];
           float v = a.bias ? b + dotv : dotv;
           if (EPI == EPI_GELU) v = gelu_ref(v);
-          if (EPI == EPI_RESID) v = ((first_group && m0 == 0) ? resid_pre : a.resid[(size_t)m * a.n + row]) + v;
+          if (EPI == EPI_RESID) v = ((first_group && m0 == m_first) ? resid_pre : a.resid[(size_t)m * a.n + row]) + v;
           a.out[(size_t)m * a.n + row] = v;
           if (a.part_val && v > run_best) {
             run_best = v;
@@ -1525,6 +1526,11 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// More input rows than eight: a CTA per eight of them, instead of one that takes eight after eight, up to this many output features: the kernel is
+// bound by latency, and the second read of the weights comes from L2. 9 to 16 rows, us, one after the other / side by side: a prompt of 11
+// tokens of GPT-2 small 569 / 534, of XL 6055 / 5218, a step of 12 sequences 648 / 613 and 7314 / 6930, of 9 638 / 629. For the lm_head of 9 rows
+// (50257) the second read costs more than it gives: the last of these 664.
+constexpr int LIN_PARTS_MAX_N = 16384;
 template <int MT, int EPI>
 cudaError_t launch_linear_mt(const LinearArgs& a, bool ln, int grid, bool pdl, cudaStream_t s) {
   if (ln) {
@@ -1532,7 +1538,8 @@ cudaError_t launch_linear_mt(const LinearArgs& a, bool ln, int grid, bool pdl, c
     auto kern = linear_decode_kernel<MT, EPI, true>;
     return launch(kern, dim3(grid), dim3(LIN_THREADS), smem, s, pdl, a);
   }
-  return launch(linear_decode_kernel<MT, EPI, false>, dim3(grid), dim3(LIN_THREADS), 0, s, pdl, a);
+  const int parts = MT == 8 && a.m > MT && a.n <= LIN_PARTS_MAX_N ? (a.m + MT - 1) / MT : 1;
+  return launch(linear_decode_kernel<MT, EPI, false>, dim3(grid, parts), dim3(LIN_THREADS), 0, s, pdl, a);
 }
 
 template <int EPI>

@@ -49,6 +49,14 @@ def test_linear_fp32_tiles_match_oracle(oracle, m, n, k, epilogue):
     np.testing.assert_allclose(got, oracle_linear(oracle, x, w, b, epilogue, r), rtol=1e-3, atol=1e-4)
 
 
+# Nine to sixteen rows: a block per eight of them up to 16384 output features, one after the other above; groups of four features cut short;
+# k within, at and past what is read ahead.
+@pytest.mark.parametrize("m,n,k", [(9, 1, 4), (9, 16387, 36), (10, 16384, 36), (15, 5, 1024), (16, 1187, 1028), (16, 130, 1020), (11, 4739, 64)])
+@pytest.mark.parametrize("epilogue", ["none", "gelu", "resid"])
+def test_linear_fp32_of_two_groups_of_rows(oracle, m, n, k, epilogue):
+    test_linear_fp32_tiles_match_oracle(oracle, m, n, k, epilogue)
+
+
 def test_linear_fp32_of_more_rows_than_a_grid_dimension_holds():
     """One row more than 65535 tiles of 64."""
     m = 65535 * 64 + 1
