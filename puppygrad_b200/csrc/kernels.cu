@@ -305,8 +305,8 @@ constexpr int LR_WARPS = LR_THREADS / 32;
 constexpr int LR_ROWS = 4;
 constexpr size_t LR_MAX_SMEM = 208 * 1024;  // [MT][k] floats
 // Rows of one launch: eight, or sixteen where it makes their LayerNorm. 11 rows of GPT-2 small behind a norm, us, in a prompt: norm and
-// linear_decode_kernel, which reads the weights once per eight rows, 11.2 (2304 x 768) and 14.1 (3072 x 768), this one about 8.5; without a norm that
-// kernel is the faster one (whole FP32 steps of 9 and 16 sequences 639 and 676 us, with this one for all products 677 and 740).
+// linear_decode_kernel, eight rows after eight, 11.2 (2304 x 768) and 14.1 (3072 x 768), this one about 8.5; without a norm that kernel is the
+// faster one (whole FP32 steps of 9 and 16 sequences 629 and 640 us, with this one for all products 677 and 740).
 constexpr int LR_NORM_ROWS = 16, LR_PLAIN_ROWS = 8;
 constexpr int LR_ONE_ROW_MIN_N = 16384;      // one input row takes this kernel only for the lm_head
 
