@@ -62,9 +62,11 @@ constexpr size_t CH_SMEM = (size_t)CH_W_RING + (size_t)CH_X_STAGES * CH_ACT_BYTE
 static_assert(CH_SMEM <= 232448, "shared memory of one CTA");
 static_assert(sizeof(ChainPhase) % 8 == 0 && 384 + 2 * sizeof(ChainPhase) <= 1024, "two phase descriptors behind the barriers");
 constexpr size_t CH_PART_TILE = (size_t)CH_BN * TILE_M;  // floats of one partial tile: [token][row]
-// The partial tiles of a phase: one of two sets.
+// The partial tiles of a phase: one of two sets. SUMS: the launch has phases with act CH_ACT_SUMS. The others take a kernel without what goes
+// with them: a step of GPT-2 XL with 32 sequences 4.24 ms (one kernel for both: 4.37), of medium with 64 1.38 to 1.41 (1.39 to 1.41).
+template <bool SUMS>
 __device__ __forceinline__ float* part_tiles(const ChainArgs& a, const ChainPhase& ph) {
-  return a.partials + (ph.part ? (size_t)gridDim.x * CH_MAX_SEG * CH_PART_TILE : 0);
+  return a.partials + (SUMS && ph.part ? (size_t)gridDim.x * CH_MAX_SEG * CH_PART_TILE : 0);
 }
 
 // Share of one CTA in units: [g0, g1) of the phase's tiles * nkb units (row tile major); per = units per CTA.
@@ -113,12 +115,13 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 
 // Grid barrier of the worker warps: arrival count only grows during a launch, barrier b (1-based)
 // is passed when it reaches grid * b. Returns the same verdict to every worker thread.
+template <bool SUMS>
 __device__ __forceinline__ bool chain_grid_barrier(unsigned* counter, unsigned target, volatile int* failed, int* err,
                                                    int wt, volatile int* verdict, int fence_first, uint64_t* go,
                                                    const ChainPhase* next) {
   // thread 0 alone needs to know whether a GEMM follows whose input the activation producer loads; the loads overlap the CTA barrier
   uint64_t* go_next = nullptr;
-  if (wt == 0 && next && !(fence_first & 16) && next->kind == CH_GEMM && next->act >= 0) go_next = go;
+  if (wt == 0 && next && !(fence_first & 16) && next->kind == CH_GEMM && (!SUMS || next->act >= 0)) go_next = go;
   workers_sync();
   if (wt == 0) {
     if (!*failed) {
@@ -269,6 +272,7 @@ __device__ __forceinline__ float warp_sum_f(float v) {
 
 // ROWS phase: x[j, :] += bias + sum of partials, then optional LayerNorm of the updated row written
 // as FP16 pairs. One CTA per token; wt = worker thread 0..255; n % 4 == 0, n <= 4096.
+template <bool SUMS>
 __device__ __forceinline__ void chain_rows_phase(const ChainArgs& a, const ChainPhase& ph, int j, int wt, float* red, bool embed) {
   const int n = ph.n, n4 = n >> 2;
   const ChRange r = chain_range_ph(ph, 0);
@@ -291,8 +295,8 @@ __device__ __forceinline__ void chain_rows_phase(const ChainArgs& a, const Chain
       const float4 xv = __ldcg(xrow + u);
       float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
       if (ph.bias) b = __ldg(reinterpret_cast<const float4*>(ph.bias) + u);
-      const float4 acc = aligned ? sum_partials_aligned<16>(part_tiles(a, ph), u * 4, j, cnt)
-                                 : sum_partials<16>(part_tiles(a, ph), u * 4, j, r.nkb, FastDiv{ph.r_magic_per, (unsigned)r.per}, FastDiv{ph.r_magic_nkb, (unsigned)r.nkb});
+      const float4 acc = aligned ? sum_partials_aligned<16>(part_tiles<SUMS>(a, ph), u * 4, j, cnt)
+                                 : sum_partials<16>(part_tiles<SUMS>(a, ph), u * 4, j, r.nkb, FastDiv{ph.r_magic_per, (unsigned)r.per}, FastDiv{ph.r_magic_nkb, (unsigned)r.nkb});
       v[i].x = xv.x + (b.x + acc.x);
       v[i].y = xv.y + (b.y + acc.y);
       v[i].z = xv.z + (b.z + acc.z);
@@ -781,6 +785,7 @@ __device__ __forceinline__ void chain_attn_phase(const ChainArgs& a, const Chain
   }
 }
 
+template <bool SUMS>
 __global__ void __launch_bounds__(CH_THREADS, 1)
     chain_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_hi0,
                  const __grid_constant__ CUtensorMap map_lo0, const __grid_constant__ CUtensorMap map_hi1,
@@ -918,7 +923,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
         if (phase_at(a, p).kind != CH_GEMM) continue;
         const ChRange r = chain_range_ph(phase_at(a, p), cta);
         const int act = phase_at(a, p).act;
-        if (act < 0) {  // the workers make this input
+        if (SUMS && act < 0) {  // the workers make this input
           u += r.g1 - r.g0;
           continue;
         }
@@ -987,14 +992,16 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
       if (kind == CH_GEMM) {
         // inputs of this phase exist: previous kernel (first phase), or the barrier just passed, whose polling
         // thread has told the activation producer already
-        if (wt == 0 && ph.act >= 0 && (p == 0 || (a.tune_fence & 16))) mbar_arrive(go);
+        if (wt == 0 && (!SUMS || ph.act >= 0) && (p == 0 || (a.tune_fence & 16))) mbar_arrive(go);
         if (live && p + 1 < a.n_phases && phase_at(a, p + 1).kind == CH_ATTN) {
           chain_attn_prepare(a, ww, lane, at_cur, at_consumed);
           at_prepared = true;
         }
         const ChRange r = chain_range_ph(ph, cta);
-        if (ph.act < 0) ok = chain_sums_input(a, ph, r, units, wt, act_ring, act_bytes, ready, done, ok && live, failed) && ok;
-        units += r.g1 - r.g0;
+        if (SUMS) {
+          if (ph.act < 0) ok = chain_sums_input(a, ph, r, units, wt, act_ring, act_bytes, ready, done, ok && live, failed) && ok;
+          units += r.g1 - r.g0;
+        }
         unsigned long long* best_s = reinterpret_cast<unsigned long long*>(at_scratch);
         if (ph.whole_tiles && ph.best) {
           if (wt < CH_BN) best_s[wt] = 0ull;
@@ -1037,7 +1044,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
             }
           } else if (ok) {
             tc_fence_after();
-            float* dst = part_tiles(a, ph) + ((size_t)(cta * CH_MAX_SEG + seg) * CH_BN) * TILE_M + row;
+            float* dst = part_tiles<SUMS>(a, ph) + ((size_t)(cta * CH_MAX_SEG + seg) * CH_BN) * TILE_M + row;
 #pragma unroll
             for (int cc = 0; cc < 32; cc += 16) {
               const int c0 = half * 32 + cc;
@@ -1063,7 +1070,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
         chain_attn_phase(a, ph, wt, act_ring, kv_full, at_scratch, at_consumed, at_cur, at_prepared, failed, live);
         at_prepared = false;
       } else if (kind == CH_ROWS || kind == CH_EMBED) {
-        if (live && cta < a.m) chain_rows_phase(a, ph, cta, wt, red, kind == CH_EMBED);
+        if (live && cta < a.m) chain_rows_phase<SUMS>(a, ph, cta, wt, red, kind == CH_EMBED);
       } else if (kind == CH_FINAL) {
         if (live && cta == 0 && wt < a.m) chain_final_phase(a, wt);
       } else {
@@ -1082,7 +1089,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1)
         if (wt < PH_WORDS)  // the next phase's descriptor; the barrier's first CTA barrier orders it before its readers
           reinterpret_cast<uint32_t*>(&ph_s[(p + 1) & 1])[wt] = reinterpret_cast<const uint32_t*>(&phase_at(a, p + 1))[wt];
         ++barriers;
-        live = chain_grid_barrier(a.barrier, (unsigned)grid * barriers, failed, a.error_flag, wt, verdict, a.tune_fence, go,
+        live = chain_grid_barrier<SUMS>(a.barrier, (unsigned)grid * barriers, failed, a.error_flag, wt, verdict, a.tune_fence, go,
                                   &phase_at(a, p + 1));
         ok = ok && live;
       }
@@ -1114,12 +1121,13 @@ int chain_grid(int num_sms) {
   if (cached >= 0) return cached;
   cached = 0;
   if (!encode_fn()) return 0;
-  if (cudaFuncSetAttribute(chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM) != cudaSuccess) {
+  if (cudaFuncSetAttribute(chain_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(chain_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chain_kernel, CH_THREADS, CH_SMEM) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chain_kernel<true>, CH_THREADS, CH_SMEM) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -1229,7 +1237,10 @@ cudaError_t launch_chain(const ChainArgs& a, int grid, cudaStream_t s) {
       return cudaErrorInvalidValue;
   }
   ChainArgs args = a;
-  if (!args.phases_dev) chain_prepare_phases(args.ph, args.n_phases, grid);
+  if (!args.phases_dev) {
+    chain_prepare_phases(args.ph, args.n_phases, grid);
+    for (int p = 0; p < args.n_phases; ++p) args.sums |= args.ph[p].kind == CH_GEMM && args.ph[p].act == CH_ACT_SUMS;
+  }
   void* params[9] = {&maps[0], &maps[1], &maps[2], &maps[3], &maps[4], &maps[5], &maps[6], &args, const_cast<int*>(&bn)};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -1241,7 +1252,7 @@ cudaError_t launch_chain(const ChainArgs& a, int grid, cudaStream_t s) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(chain_kernel), params);
+  return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(args.sums ? chain_kernel<true> : chain_kernel<false>), params);
 }
 
 }  // namespace pg

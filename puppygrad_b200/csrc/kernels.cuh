@@ -244,6 +244,7 @@ constexpr int CHAIN_MAX_PHASES = 10;
 struct ChainArgs {
   ChainPhase ph[CHAIN_MAX_PHASES];  // the phases, when phases_dev is nullptr
   const ChainPhase* phases_dev;     // or: the phases in device memory (any number of them)
+  int sums;  // with phases_dev: whether any of them has act CH_ACT_SUMS
   int n_phases;
   // ATTN phases: causal attention of one new token per sequence over the paged cache (head_dim 64),
   // appending the new K and V; key / value rows are staged in shared memory by bulk async copies

@@ -714,6 +714,7 @@ static int ensure_chain_program(pg_cache* c, int batch, int chunk = 0) {
     std::vector<ChainPhase> lean = ph;
     for (ChainPhase& p : lean)
       if (p.best) p.out = nullptr;
+    prog.sums = sums ? 1 : 0;
     PG_CUDA_TRY(cudaMalloc(&prog.dev_argmax_only, lean.size() * sizeof(ChainPhase)));
     PG_CUDA_TRY(cudaMemcpy(prog.dev_argmax_only, lean.data(), lean.size() * sizeof(ChainPhase), cudaMemcpyHostToDevice));
   }
@@ -814,6 +815,7 @@ static cudaError_t enqueue_decode_step(pg_cache* c, int batch, int splits, cudaS
         const auto& prog = c->chain_programs[chain_program_key(rows, k)];
         ChainArgs a = chain_base_args(c, rows, k);
         a.phases_dev = c->step_wants_logits ? prog.dev : prog.dev_argmax_only;
+        a.sums = prog.sums;
         a.n_phases = prog.n;
         cur_bucket = B_OTHER;
         PG_E(launch_chain(a, c->chain_ctas, s));
@@ -828,6 +830,7 @@ static cudaError_t enqueue_decode_step(pg_cache* c, int batch, int splits, cudaS
       // the whole step, from the embedding to the token fed back, as one persistent cooperative kernel
       ChainArgs a = chain_base_args(c, batch);
       a.phases_dev = (c->step_wants_logits || prof) ? prog->second.dev : prog->second.dev_argmax_only;
+      a.sums = prog->second.sums;
       a.n_phases = prog->second.n;
       if (prof) a.phase_times = prog->second.d_times;  // per-phase time stamps for the operation profile
       cur_bucket = B_OTHER;

@@ -168,6 +168,7 @@ struct pg_cache {
   int chain_min_batch = 9;
   struct ChainProgram {  // whole-step phase list of the persistent chain kernel for one batch size
     ChainPhase* dev = nullptr;            // in device memory (nullptr: this batch size is not supported)
+    int sums = 0;                           // ChainArgs::sums
     ChainPhase* dev_argmax_only = nullptr;  // the same list whose lm_head reduce phase keeps the row arg-max but stores no logits
     int n = 0;
     std::vector<int> bucket;              // profile bucket of every phase
