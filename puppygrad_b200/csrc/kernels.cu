@@ -1534,6 +1534,7 @@ constexpr int LIN_PARTS_MAX_N = 16384;
 template <int MT, int EPI>
 cudaError_t launch_linear_mt(const LinearArgs& a, bool ln, int grid, bool pdl, cudaStream_t s) {
   if (ln) {
+    if (a.m > MT) return cudaErrorInvalidValue;  // it normalises MT rows
     size_t smem = (size_t)MT * a.k * sizeof(float);
     auto kern = linear_decode_kernel<MT, EPI, true>;
     return launch(kern, dim3(grid), dim3(LIN_THREADS), smem, s, pdl, a);
@@ -1571,20 +1572,22 @@ int linear_decode_grid(int n, int sms) {
   return groups < cap ? groups : cap;
 }
 
-// smallest row count class (1, 2, 4, 8) that takes the shared-memory kernel (one input row is faster on the
-// kernel above: GPT-2 medium steps of 1 / 2 / 4 / 8 sequences took 747 / 893 / 1113 / 1580 us with it and
+// smallest row count class (1, 2, 4, 8; 16: more than eight rows, behind a LayerNorm) that takes the shared-memory kernel (one
+// input row is faster on the kernel above: GPT-2 medium steps of 1 / 2 / 4 / 8 sequences took 747 / 893 / 1113 / 1580 us with it and
 // 758 / 789 / 921 / 1091 us with the shared-memory kernel); PG_LR_MIN_MT overrides it for tuning
 static int g_lr_min_mt = [] { const char* e = getenv("PG_LR_MIN_MT"); return e ? atoi(e) : 2; }();
 
+static int linear_rows_class(int m) { return m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : m <= 8 ? 8 : 16; }
 // Shared memory of linear_rows_smem_kernel: rows of zeros fill a tile of at most eight, no room is spent on them above.
-static size_t linear_rows_smem(int m, int k) {
-  const int rows = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : m <= 8 ? 8 : m;
-  return (size_t)rows * k * sizeof(float);
+static size_t linear_rows_smem(int m, int k) { return (size_t)(m <= 8 ? linear_rows_class(m) : m) * k * sizeof(float); }
+static bool linear_rows_in_smem(int m, int n, int k, bool norm) {
+  return m <= (norm ? LR_NORM_ROWS : LR_PLAIN_ROWS) && linear_rows_smem(m, k) <= LR_MAX_SMEM &&
+         (linear_rows_class(m) >= g_lr_min_mt || (m <= LR_PLAIN_ROWS && n >= LR_ONE_ROW_MIN_N));
 }
-static bool linear_rows_in_smem(int m, int k, bool norm) { return m <= (norm ? LR_NORM_ROWS : LR_PLAIN_ROWS) && linear_rows_smem(m, k) <= LR_MAX_SMEM; }
 
+// More than eight rows: only that kernel makes their norms.
 bool linear_decode_fuses_norm(int m, int k) {
-  return k % 4 == 0 && k <= 2048 && (m <= 8 || linear_rows_in_smem(m, k, true));
+  return k % 4 == 0 && k <= 2048 && (m <= 8 || linear_rows_in_smem(m, 0, k, true));
 }
 
 cudaError_t launch_linear_decode(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s, int* grid_out) {
@@ -1594,8 +1597,8 @@ cudaError_t launch_linear_decode(const LinearArgs& a, int epilogue, bool pdl, cu
     if (grid_out) *grid_out = 0;
     return launch(linear_generic_kernel, dim3((unsigned)((total + 127) / 128)), dim3(128), 0, s, pdl, a, epilogue);
   }
-  const int mt = a.m <= 1 ? 1 : a.m <= 2 ? 2 : a.m <= 4 ? 4 : 8;
-  if (linear_rows_in_smem(a.m, a.k, a.ln_g != nullptr) && (mt >= g_lr_min_mt || a.n >= LR_ONE_ROW_MIN_N)) {
+  const int mt = std::min(linear_rows_class(a.m), 8);
+  if (linear_rows_in_smem(a.m, a.n, a.k, a.ln_g != nullptr)) {
     // activations staged in shared memory, one persistent CTA per SM; k is shared out over the warps of a
     // CTA when the matrix has too few rows to give every warp of the chip a row group
     const int groups = (a.n + LR_ROWS - 1) / LR_ROWS, k4 = a.k / 4;

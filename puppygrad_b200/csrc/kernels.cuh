@@ -34,7 +34,7 @@ struct LinearArgs {
 // *grid_out (the stride of part_val / part_idx).
 cudaError_t launch_linear_decode(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s, int* grid_out);
 int linear_decode_grid(int n, int num_sms);
-// Whether it makes the LayerNorm of m rows of k itself.
+// Whether it makes the LayerNorm of m rows of k itself; above eight rows only without the residual epilogue.
 bool linear_decode_fuses_norm(int m, int k);
 
 // out[r, :] = wte[ids[r]] + wpe[pos[r]]
@@ -52,7 +52,8 @@ cudaError_t launch_layernorm_rows(const float* x, const float* g, const float* b
 // General FP32 GEMM out[m,n] = x[m,k] . w[n,k]^T (+bias)(+GELU | +resid), CUDA-core FMA (gemm_f32.cu); k % 4 == 0.
 cudaError_t launch_gemm_f32_tiles(const LinearArgs& a, int epilogue, cudaStream_t s);
 cudaError_t init_gemm_f32_attributes();
-// The faster of the two FP32 products for any number of rows (no arg-max partials; LayerNorm prologue: at most 16 rows).
+// The faster of the two FP32 products for any number of rows (no arg-max partials; LayerNorm prologue:
+// as linear_decode_fuses_norm says).
 cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s);
 // dst[o, i] = src[i, o]
 cudaError_t launch_transpose(const float* src, float* dst, int in_f, int out_f, cudaStream_t s);

@@ -5,6 +5,8 @@ for the FP32 path); greedy token streams must be identical.
 """
 import json
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -219,6 +221,24 @@ def test_prompts_of_a_few_wide_rows(oracle):
     for n in (3, 8, 11, 16):
         ids = synthetic.uniform_prompt(n, n, cfg["vocab_size"])
         assert_logits_close(g.prefill(ids, g.new_kv_cache()), o.prefill(ids, o.new_kv_cache()))
+
+
+# PG_LR_MIN_MT, read once per process, keeps rows off the kernel that alone makes the norms of more than eight of them.
+@pytest.mark.parametrize("min_class", [9, 17])
+def test_prompts_of_a_few_rows_off_the_shared_memory_kernel(midi, tmp_path, min_class):
+    cfg, w, _, o = midi
+    code = """if 1:
+        import sys, numpy as np, puppygrad_b200 as pg
+        from puppygrad_b200 import synthetic
+        cfg = synthetic.preset("midi")
+        g = pg.Gpt2Model(cfg, synthetic.perturbed_weights(cfg, 11))
+        np.save(sys.argv[1], np.stack([g.prefill(synthetic.uniform_prompt(n, n, cfg["vocab_size"]), g.new_kv_cache()) for n in (8, 9, 12, 16)]))
+    """
+    out = tmp_path / "logits.npy"
+    subprocess.run([sys.executable, "-c", code, str(out)], check=True, env=dict(os.environ, PG_LR_MIN_MT=str(min_class)),
+                   cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    for n, logits in zip((8, 9, 12, 16), np.load(out)):
+        assert_logits_close(logits, o.prefill(synthetic.uniform_prompt(n, n, cfg["vocab_size"]), o.new_kv_cache()))
 
 
 def test_token_by_token_prefill_equals_batched_prefill(midi):
