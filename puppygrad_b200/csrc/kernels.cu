@@ -1688,13 +1688,21 @@ cudaError_t launch_decode_attention(const DecodeAttnArgs& a, bool pdl, cudaStrea
   return launch(kern, dim3(a.kv.n_head, a.batch, 1), dim3(ATT_THREADS), smem, s, pdl, a);
 }
 
-bool prefill_attention_stores_kv(const PrefillAttnArgs& a) { return a.head_dim == 64 && a.max_len <= PS_KEYS; }
+// Eight queries per block of the kernel for short prompts, a warp each, while that leaves an SM at most four blocks; else a block per head and
+// sequence, whose warps read the keys from shared memory again for each of their queries.
+static bool short_prompts_in_eights(const PrefillAttnArgs& a) { return (long long)a.n_head * a.batch * ((a.max_len + 7) / 8) <= 4ll * num_sms(); }
+
+// Up to PS_KEYS tokens in eights, up to 40 with a block per head and sequence. us a layer of FP32 prompts, that kernel / tiles and the kernel that
+// fills the cache: in eights 1 x 64 tokens of 12 heads 6.0 / 13.0, 8 x 48 9.4 / 13.9, 4 x 64 of 16 heads 9.7 / 14.8; a block per head and sequence, 12 heads:
+// 32 x 40 17.7 / 21.6, 64 x 40 37.4 / 38.5, 64 x 44 42.4 / 39.5, 64 x 48 45.8 / 40.6, 64 x 64 66.3 / 46.2; 25 heads, 32 sequences of 40, 44 and 64
+// 37.5 / 40.3, 44.7 / 41.9, 74.7 / 49.7.
+bool prefill_attention_stores_kv(const PrefillAttnArgs& a) {
+  return a.head_dim == 64 && a.max_len <= (short_prompts_in_eights(a) ? PS_KEYS : 40);
+}
 
 cudaError_t launch_prefill_attention(const PrefillAttnArgs& a, bool pdl, cudaStream_t s) {
   if (prefill_attention_stores_kv(a)) {
-    // eight queries per block, a warp each, while that leaves an SM at most four blocks; else a block per head and sequence
-    const long long fine = (long long)a.n_head * a.batch * ((a.max_len + 7) / 8);
-    const int per_block = fine <= 4ll * num_sms() ? 8 : PS_KEYS;
+    const int per_block = short_prompts_in_eights(a) ? 8 : PS_KEYS;
     return launch(prefill_attention_small_kernel, dim3(a.n_head, (a.max_len + per_block - 1) / per_block, a.batch), dim3(PS_THREADS), 0, s, pdl, a, per_block);
   }
   if (a.head_dim == 64) {

@@ -200,8 +200,9 @@ def test_prompts_on_the_tensor_cores_fill_the_cache(midi, page_tokens):
 
 
 # Prompts whose products make their own norms (up to 16 rows, with and without a tile of eight to fill up; k = 256 held in registers) and
-# whose attention is the one for at most 64 tokens: queries in eights and all together, keys at the edges of 32 and 64, and 65 tokens beside them.
-@pytest.mark.parametrize("lens", [[1], [2, 5], [8], [9], [3, 6, 7], [16], [17], [31, 1], [32, 33], [63], [64], [65], [64, 2, 65], [7] * 50, [40] * 40])
+# whose attention is the one for short prompts: queries in eights (up to 64 tokens) and all together (up to 40), keys at the edges of 32 and 64,
+# and the lengths beside them that take tiles.
+@pytest.mark.parametrize("lens", [[1], [2, 5], [8], [9], [3, 6, 7], [16], [17], [31, 1], [32, 33], [63], [64], [65], [64, 2, 65], [7] * 50, [40] * 40, [41] * 40, [64] * 18, [64] * 19])
 def test_prompts_of_a_few_rows(midi, lens):
     cfg, w, g, o = midi
     prompts = [synthetic.uniform_prompt(300 + i, n, cfg["vocab_size"]) for i, n in enumerate(lens)]
