@@ -62,7 +62,7 @@ constexpr size_t CH_SMEM = (size_t)CH_W_RING + (size_t)CH_X_STAGES * CH_ACT_BYTE
 static_assert(CH_SMEM <= 232448, "shared memory of one CTA");
 static_assert(sizeof(ChainPhase) % 8 == 0 && 384 + 2 * sizeof(ChainPhase) <= 1024, "two phase descriptors behind the barriers");
 constexpr size_t CH_PART_TILE = (size_t)CH_BN * TILE_M;  // floats of one partial tile: [token][row]
-// The partial tiles of a phase: one of two sets. SUMS: the launch has phases with act CH_ACT_SUMS. The others take a kernel without what goes
+// The partial tiles of a phase: one of two sets, the second where there are such phases. SUMS: the launch has phases with act CH_ACT_SUMS. The others take a kernel without what goes
 // with them: a step of GPT-2 XL with 32 sequences 4.24 ms (one kernel for both: 4.37), of medium with 64 1.38 to 1.41 (1.39 to 1.41).
 template <bool SUMS>
 __device__ __forceinline__ float* part_tiles(const ChainArgs& a, const ChainPhase& ph) {
@@ -1138,7 +1138,7 @@ int chain_grid(int num_sms) {
   return cached;
 }
 
-size_t chain_partial_floats(int grid) { return 2 * (size_t)grid * CH_MAX_SEG * CH_PART_TILE; }
+size_t chain_partial_floats(int grid, int sets) { return (size_t)sets * grid * CH_MAX_SEG * CH_PART_TILE; }
 
 // Where making the input is little work: by rows and units of a CTA. us a step with an ELEM phase and without: width 768 (2 units) 9 rows 502 and 462,
 // 24 rows 525 and 505, 32 rows 522 and 524; width 1024 (4 units) 9 rows 987 and 966, 12 rows 983 and 966, 16 rows 999 and 1001, 24 rows

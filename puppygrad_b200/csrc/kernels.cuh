@@ -271,7 +271,7 @@ struct ChainArgs {
   const uint16_t* act_hi[3];  // activation pairs by ChainAct: [m, k] each
   const uint16_t* act_lo[3];
   int act_k[3];
-  float* partials;     // chain_partial_floats(grid) floats
+  float* partials;     // chain_partial_floats(grid, 1) floats, with CH_ACT_SUMS phases (grid, 2)
   unsigned* barrier;   // one word, zero before the first launch (the kernel leaves it zero)
   int* error_flag;     // set non-zero when a bounded wait expired
   int tune_fence;      // tuning: bit 0 = a separate __threadfence(), bit 1 = a proxy fence before the arrival at the grid barrier
@@ -284,7 +284,7 @@ struct ChainArgs {
 };
 // Cooperative grid of the chain kernel on this device (0: not launchable) and the scratch it needs.
 int chain_grid(int num_sms);
-size_t chain_partial_floats(int grid);
+size_t chain_partial_floats(int grid, int sets);
 // Value of an empty row arg-max accumulator: (-inf, index 0), the start of argmax_logits (generation.rs:269-279).
 unsigned long long chain_argmax_init();
 // True when every phase fits the kernel's limits for a grid of `grid` CTAs. `host_phases` is the

@@ -496,7 +496,9 @@ static int cache_new(const pg_model* m, int max_batch, pg_cache** out) {
     PG_CUDA_TRY(cudaMalloc(&c->h_lo, (size_t)bmax * F * sizeof(float)));
     if (m->pair_arena && !env_flag("PG_NO_CHAIN") && chain_grid(m->num_sms) > 0) {
       c->chain_ctas = chain_grid(m->num_sms);
-      PG_CUDA_TRY(cudaMalloc(&c->chain_partials, chain_partial_floats(c->chain_ctas) * sizeof(float)));
+      // the fewest sequences of a launch; more make the input of the MLP's second product themselves only where these do
+      c->chain_sums = chain_makes_input(C, F, max_batch > 64 ? 1 : c->chain_min_batch, c->chain_ctas);
+      PG_CUDA_TRY(cudaMalloc(&c->chain_partials, chain_partial_floats(c->chain_ctas, c->chain_sums ? 2 : 1) * sizeof(float)));
       PG_CUDA_TRY(cudaMalloc(&c->d_chain_barrier, sizeof(unsigned)));
       PG_CUDA_TRY(cudaMemsetAsync(c->d_chain_barrier, 0, sizeof(unsigned), c->stream));
       {
@@ -654,7 +656,7 @@ static int ensure_chain_program(pg_cache* c, int batch, int chunk = 0) {
     ph.push_back(p);
     bucket.push_back(B_LAYER_NORM);
   }
-  const bool sums = chain_makes_input(C, F, batch, c->chain_ctas);
+  const bool sums = c->chain_sums && chain_makes_input(C, F, batch, c->chain_ctas);
   for (int l = 0; l < L; ++l) {
     const LayerWeights& w = m->layers[l];
     cur_b = B_QKV;

@@ -172,7 +172,7 @@ extern "C" int pg_op_linear(const float* x, const float* w, const float* bias, c
       chain.arena = dwlo.as<uint16_t>();
       chain.act_hi[0] = dhi.as<uint16_t>(); chain.act_lo[0] = dlo.as<uint16_t>(); chain.act_k[0] = k;
       chain.error_flag = derr.as<int>();
-      PG_OP_TRY(cudaMalloc(&dpart.p, chain_partial_floats(g) * 4));
+      PG_OP_TRY(cudaMalloc(&dpart.p, chain_partial_floats(g, 1) * 4));
       PG_OP_TRY(cudaMalloc(&dbar.p, 4));
       PG_OP_TRY(cudaMemsetAsync(dbar.p, 0, 4, s));
       chain.partials = dpart.as<float>(); chain.barrier = dbar.as<unsigned>();

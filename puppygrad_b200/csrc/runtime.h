@@ -166,6 +166,7 @@ struct pg_cache {
   // multiply-adds (as the chain kernel / as one kernel per operation 8 would take, us: GPT-2 small 506 / 488, medium 1018 / 1064, XL
   // 2816 / 3717), 5 with BF16 weights (enqueue_decode_step).
   int chain_min_batch = 9;
+  bool chain_sums = false;  // some batch has phases with act CH_ACT_SUMS: chain_partials holds two sets
   struct ChainProgram {  // whole-step phase list of the persistent chain kernel for one batch size
     ChainPhase* dev = nullptr;            // in device memory (nullptr: this batch size is not supported)
     int sums = 0;                           // ChainArgs::sums

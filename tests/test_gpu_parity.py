@@ -992,6 +992,20 @@ def test_persistent_steps_of_widths(oracle, n_embd, n_head, batch, math_mode):
         cur = am.copy()
 
 
+def test_memory_of_the_persistent_step():
+    """One set of partial tiles (19.4 MB) where no step of the model takes two: 13 x 100 blocks of the MLP's second product are nine to an SM."""
+    import torch
+    cfg = dict(synthetic.preset("mini"), n_embd=1600, n_head=25, n_inner=6400, n_layer=1, n_positions=64)
+    g = pg.Gpt2Model(cfg, synthetic.random_init_weights(cfg, 1), pg.Gpt2CudaConfig(math_mode="tf32x3"))
+    used = {}
+    for batch in (8, 9):  # without and with the state of that kernel
+        free = torch.cuda.mem_get_info()[0]
+        caches = [g.new_kv_cache(max_batch=batch) for _ in range(4)]
+        used[batch] = (free - torch.cuda.mem_get_info()[0]) / 4
+        del caches
+    assert used[9] - used[8] < 1.5 * 148 * 4 * 64 * 128 * 4
+
+
 def test_narrow_weight_modes_exclude_each_other():
     cfg, w = tiny()
     with pytest.raises(pg.Gpt2Error, match="exclude each other"):
