@@ -318,8 +318,9 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
   constexpr int SH = (NV >= 32) ? 0 : (NV == 16) ? 1 : (NV == 8) ? 2 : 3;  // 5 - log2(NV)
   constexpr int FOLDS = NV > 32 ? NV / 32 : 1, FV = NV / FOLDS;             // sums are folded over a warp's lanes 32 at a time
   __shared__ float part[LR_WARPS][NV];
-  __shared__ float best_v[LR_WARPS][NV];
-  __shared__ int best_i[LR_WARPS][NV];
+  constexpr bool BEST = MT <= 8;  // arg-max partials: refused above
+  __shared__ float best_v[LR_WARPS][BEST ? NV : 1];
+  __shared__ int best_i[LR_WARPS][BEST ? NV : 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k4 = a.k >> 2;
   const int groups = (a.n + LR_ROWS - 1) / LR_ROWS;
@@ -419,13 +420,8 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
   const int own = kparts == 1 ? FOLDS : 1;               // sums a finisher has
   const int fs = kparts == 1 ? (lane >> SH) : tid % NV;  // number of its first one; the next is FV on
   const int fslot = kparts == 1 ? wg : tid / NV;         // group slot
-  float run_best[FOLDS];  // lm_head arg-max partial of this finisher's (row in group, input row) pairs
-  int run_idx[FOLDS];
-#pragma unroll
-  for (int h = 0; h < FOLDS; ++h) {
-    run_best[h] = -INFINITY;
-    run_idx[h] = INT_MAX;
-  }
+  float run_best = -INFINITY;  // lm_head arg-max partial of this finisher's (row in group, input row) pair
+  int run_idx = INT_MAX;
 
   // every warp of the CTA makes the same number of rounds (the CTA barrier inside needs all of them)
   const int rounds = (groups - (int)blockIdx.x * gpc + g_stride - 1) / g_stride;
@@ -502,27 +498,24 @@ __global__ void __launch_bounds__(LR_THREADS, 1) linear_rows_smem_kernel(LinearA
       if (EPI == EPI_GELU) v = gelu_ref(v);
       if (EPI == EPI_RESID) v = resid_v[h] + v;
       a.out[(size_t)fm * a.n + orow] = v;
-      if (a.part_val && v > run_best[h]) {
-        run_best[h] = v;
-        run_idx[h] = orow;
+      if (BEST && a.part_val && v > run_best) {
+        run_best = v;
+        run_idx = orow;
       }
     }
     if (kparts > 1) __syncthreads();  // `part` is rewritten in the next round
   }
 
-  if (a.part_val) {
+  if (BEST && a.part_val) {
     // finishers: kparts = 1: holder lanes of every warp, sum number lane >> SH; else threads t < gpc * NV
     if (kparts == 1) {
       if (holder) {
-#pragma unroll
-        for (int h = 0; h < FOLDS; ++h) {
-          best_v[warp][(lane >> SH) + h * FV] = run_best[h];
-          best_i[warp][(lane >> SH) + h * FV] = run_idx[h];
-        }
+        best_v[warp][lane >> SH] = run_best;
+        best_i[warp][lane >> SH] = run_idx;
       }
     } else if (tid < gpc * NV) {
-      best_v[tid / NV][tid % NV] = run_best[0];
-      best_i[tid / NV][tid % NV] = run_idx[0];
+      best_v[tid / NV][tid % NV] = run_best;
+      best_i[tid / NV][tid % NV] = run_idx;
     }
     __syncthreads();
     if (tid < MT && tid < a.m) {
