@@ -94,3 +94,16 @@ def many_sequences(case, n=61, mode="fp32"):
         got = model.forward_one_batch([x[t] for x, t in zip(ids, at)], cache, want_logits=True)[0]
         at = [t + 1 for t in at]
         assert_rows(got, np.stack([case.want(x[:t])[-1] for x, t in zip(ids, at)]), mode)
+
+
+def ragged_segments(case):
+    """Two calls with sequences of very different lengths, the longest of which make the recurrences run in segments: many of them, one, a
+    whole and a short last one, from empty and from filled states."""
+    lens = [(900, 2), (1, 640), (129, 1), (300, 128), (513, 385)]
+    model = case.model("fp32")
+    cache = model.new_kv_cache(len(lens))
+    ids = [case.ids(a + b, seed=i) for i, (a, b) in enumerate(lens)]
+    for part in (lambda x, n: x[:n], lambda x, n: x[n:]):
+        pieces = [part(x, a) for x, (a, _) in zip(ids, lens)]
+        got = model.extend(range(len(lens)), pieces, cache, range(sum(map(len, pieces))))
+        assert_rows(got, np.concatenate([part(case.want(x), a) for x, (a, _) in zip(ids, lens)]), "fp32")

@@ -214,12 +214,14 @@ def test_prompts_of_a_few_rows(midi, lens):
     assert_logits_close(logits, np.stack([o.forward_one(int(t), c) for t, c in zip(am, caches)]))
 
 
-# The same products at k = 1088, whose rows do not stay in registers.
-def test_prompts_of_a_few_wide_rows(oracle):
-    cfg = dict(synthetic.preset("mini"), n_embd=1088, n_head=17, n_inner=320, n_layer=1)
+# The same products at other widths: rows that do not stay in registers (1088); those and more row groups than the chip has warps, so that k is
+# in one part (1600); k in one part because it is short, and a last group of rows cut short (128).
+@pytest.mark.parametrize("n_embd,n_head,n_inner", [(1088, 17, 320), (1600, 25, 6400), (128, 2, 498)])
+def test_prompts_of_a_few_rows_of_other_widths(oracle, n_embd, n_head, n_inner):
+    cfg = dict(synthetic.preset("mini"), n_embd=n_embd, n_head=n_head, n_inner=n_inner, n_layer=1)
     w = synthetic.perturbed_weights(cfg, 5)
     g, o = pg.Gpt2Model(cfg, w), oracle.Model(cfg, w, threads=4)
-    for n in (3, 8, 11, 16):
+    for n in (3, 8, 9, 11, 16):
         ids = synthetic.uniform_prompt(n, n, cfg["vocab_size"])
         assert_logits_close(g.prefill(ids, g.new_kv_cache()), o.prefill(ids, o.new_kv_cache()))
 
@@ -579,10 +581,12 @@ def test_device_topk_of_equal_logits(vocab, run, k):
         assert am2[r] == order[0]
 
 
-@pytest.mark.parametrize("batch", [1, 3])
-def test_device_topk_of_changing_length(midi, batch):
+# More than 64 sequences: the lists follow several launches of the persistent kernel.
+@pytest.mark.parametrize("batch, math_mode", [(1, "fp32"), (3, "fp32"), (65, "tf32x3"), (130, "bf16")])
+def test_device_topk_of_changing_length(midi, batch, math_mode):
     """One graph of the step serves lists of every length; none, and logits alone, in between."""
-    cfg, w, g, o = midi
+    cfg, w, _, _ = midi
+    g = pg.Gpt2Model(cfg, w, pg.Gpt2CudaConfig(math_mode=math_mode))
     cache = g.new_kv_cache(max_batch=batch)
     _, cur = g.prefill_batch([synthetic.uniform_prompt(700 + i, 5, cfg["vocab_size"]) for i in range(batch)], cache)
     for k in (40, 1, 0, 64, 7, 40):

@@ -12,7 +12,7 @@ import puppygrad_b200 as pg
 from puppygrad_b200 import trace
 from tests import layered_cases as cases
 from tests import layered_oracle as lo
-from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, many_sequences, row_errors, run_portions
+from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, many_sequences, ragged_segments, row_errors, run_portions
 
 pytestmark = pytest.mark.gpu
 
@@ -179,6 +179,12 @@ def test_states_between_segments(layer):
     ids = case.ids(1040)
     model = case.model("fp32")
     assert_rows(run_portions(model, model.new_kv_cache(1), 0, [ids[:515], ids[515:]]), case.want(ids), "fp32")
+
+
+@pytest.mark.parametrize("layer", [lo.gla(2, 64, 18), lo.gla(3, 65, 35), lo.pair(1, 1, 8, 8, 5, 3, 31, left_scale=0.0), lo.pair(1, 1, 8, 8, 5, 2, 64, left_scale=0.0),
+                                   lo.pair(1, 1, 8, 8, 5, 1, 144, left_scale=0.0)])
+def test_segments_of_sequences_of_different_lengths(layer):
+    ragged_segments(Case(lo.config(61, 48, [layer]), 13, rank=3))
 
 
 # Parts of the keys as a cluster (up to 8) and beyond; more rows than a block holds in registers; groups of one, four and nine query

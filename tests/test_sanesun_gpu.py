@@ -10,7 +10,7 @@ import puppygrad_b200 as pg
 from puppygrad_b200 import trace
 from tests import layered_cases as cases
 from tests import sanesun_oracle as so
-from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, many_sequences, row_errors, run_portions
+from tests.layered_cases import BOUND, MODES, assert_rows, assert_stream, cut, many_sequences, ragged_segments, row_errors, run_portions
 
 pytestmark = pytest.mark.gpu
 
@@ -78,6 +78,11 @@ ALONE = {
                                    so.delta(5, 5, 72, 40, 1)])
 def test_steps_of_many_sequences(layer):
     many_sequences(Case(so.config(61, 50, [layer]), 7, rank=9))
+
+
+@pytest.mark.parametrize("layer", [so.delta(3, 1, 31, 40, 4), so.delta(2, 2, 128, 128, 4), so.delta(1, 1, 66, 9, 1)])
+def test_segments_of_sequences_of_different_lengths(layer):
+    ragged_segments(Case(so.config(61, 50, [layer]), 13, rank=3))
 
 
 # One kernel with two sizes of shared memory in one model: heads of 128 x 128 behind four and behind three taps.
