@@ -31,7 +31,8 @@ __device__ __forceinline__ void warp_norm_row(const float* x, int n, int np, con
 // ------------------------------------------------------------------ one token per sequence
 // Block = one kv head of one sequence and one part of its visible keys, for RB query heads of the group at a time.
 // Eight lanes share a key (16-byte pieces of the row), the probabilities go through shared memory, and threads then own
-// eight value columns each for a subset of the keys. Partial results of the parts are merged by the last block.
+// eight value columns each for a subset of the keys. Partial results of the parts are merged by the blocks of a cluster, each
+// a share of the outputs (FEW, below), or, where the launch has no clusters, by the last block.
 //
 // Bound by a chain of round trips, so registers are cut for four blocks on an SM and cached rows are asked for ahead of the dependency wait: with
 // the same change to the recurrent steps, 24 steps of 64 sequences of Dirurax of width 2048 with their prompts 25.1 -> 24.2 ms (two blocks of

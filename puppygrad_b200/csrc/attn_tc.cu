@@ -410,7 +410,8 @@ __device__ __forceinline__ void kv_store_2d(const CUtensorMap* map, int x, int y
 
 // With a.kv_pool the CTA also writes its queries' keys and values to the cache: its last tile holds these rows, which the producer warp stores page
 // by page (the rows of a page that the sequence does not fill: one by one) while the tile is worked on. In the place of a kernel that read and wrote
-// them all (26 us a layer for 8 x 1024 rows of GPT-2 small, 106 for 32 x 512 of XL): 7.26 -> 7.09 ms, 281 -> 278 ms with 24 steps.
+// them all (26 us a layer for 8 x 1024 rows of GPT-2 small, 106 for 32 x 512 of XL): 8 x 1024 rows
+// 7.26 -> 7.09 ms; XL's 32 prompts with 24 steps gain less than two runs of them differ by.
 __global__ void __launch_bounds__(X3_THREADS, 1)
     prefill_attention_x3_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_kv, PrefillAttnArgs a, int* error_flag) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];

@@ -1651,10 +1651,11 @@ cudaError_t launch_layernorm_rows_split(const float* x, const float* g, const fl
 }
 
 // The decode kernels stream the weights once per 8 rows and start before the kernel in front of them has ended; the tiles read them
-// once. Whole steps on decode kernels and on tiles, us: 13 / 16 sequences of GPT-2 small 666 / 681 and 725 / 731, of medium 1515 / 1577 and
-// 1783 / 1798; with 17, a third round, 937 (20 sequences) and 739, 2136 and 1818. Prompts of 13 and 16 rows: small 757 / 778 and 869 / 869,
-// medium 1575 / 1635 and 2030 / 2033. The lm_head alone, the rest of the step on decode kernels: medium 1426 / 1449 / 1512 / 1524 / 1611 and
-// 1459 / 1474 / 1502 / 1515 / 1577 for 9 / 10 / 12 / 13 / 16 sequences.
+// once. Whole steps on decode kernels and on tiles, us: 9 / 12 / 16 sequences of GPT-2 small 634 / 627 / 650 and 719 / 719 / 725, of medium
+// 1415 / 1453 / 1518 and 1760 / 1766 / 1783; with 17, a third round, 728 and 735, 1922 and 1805, with 24 752 and 747, 1990 and 1838. Prompts of 9
+// and 16 rows: small 523 / 570 and 684 / 705, medium 1294 / 1365 and 1672 / 1731, of 17 843 and 848, 2102 and 2018. The lm_head alone, steps on decode
+// kernels and on tiles: 9 / 10 / 12 / 16 sequences of small 634 / 638 / 647 / 693 and 600 / 606 / 626 / 650, of medium 1415 / 1424 / 1462 / 1566 and
+// 1432 / 1460 / 1453 / 1518: at 9 and 10 the one gains what the other loses.
 cudaError_t launch_linear_rows(const LinearArgs& a, int epilogue, bool pdl, cudaStream_t s) {
   if (a.m <= (a.n <= 16384 ? 16 : 10) || a.k % 4 != 0 || a.ln_g) return launch_linear_decode(a, epilogue, pdl, s, nullptr);
   return launch_gemm_f32_tiles(a, epilogue, s);

@@ -1040,8 +1040,8 @@ static int run_blocks(const pg_model* m, const BlockWorkspace& ws, const Prefill
   // epilogue of the MLP's first product) writes pairs instead of FP32, into the same buffer: [rows, k] hi, then lo.
   const bool pairs = m->pair_arena && m->backend.math_mode != PG_MATH_TF32 && ws.d_error && rows >= 128 && m->head_dim() == 64 && C <= 4096;
   // A prompt of a few rows is a chain of launches of 2 to 10 us: the next one's blocks come up, and its first weights, while the last
-  // one ends (11 rows of GPT-2 small: 879 -> 749 us, 16: 902 -> 778; 585 and 614 with the norms made by the products). From 17 rows on the products are tiles (launch_linear_rows), which
-  // start when everything in front of them has ended.
+  // one ends (11 rows of GPT-2 small: 879 -> 749 us, 16: 902 -> 778; 535 and 570 since the products make the norms and take two groups of
+  // rows side by side). From 17 rows on the products are tiles (launch_linear_rows), which start when everything in front of them has ended.
   const bool pdl = m->use_pdl && rows <= 16;
   auto pair_of = [&](float* buf, int k, float scale) {
     PairOut p;

@@ -105,7 +105,10 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_step_kernel(NormStepArgs a)
   }
 }
 
-constexpr int NORM_HELD_ROWS = 256;  // at most two blocks on an SM
+// The rows of a step, at most two blocks on an SM. us between the ends of a norm and of the kernel in front of it inside a greedy step of Dirurax of
+// width 2048, held / not held: 12 rows 4.0 / 5.7, 64 4.3 / 5.8, 128 4.3 / 5.8, 256 4.6 / 6.1. The line could lie higher (300 rows 4.7 / 7.4, 400
+// 4.8 / 7.6; from 512 on 8.2 / 8.0) and take rows of 4096 too (64 rows 8.0 / 10.8, a step 1310 / 1351).
+constexpr int NORM_HELD_ROWS = 256;
 
 template <typename T>
 cudaError_t launch_norm_step_t(const NormStepArgs& a, int rows, bool pdl, cudaStream_t s) {

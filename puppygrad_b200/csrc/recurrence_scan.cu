@@ -1119,8 +1119,8 @@ __global__ void __launch_bounds__(256) segment_decay_kernel(ScanArgs sa) {
 // start[i + 1] = transition[i] start[i] + local[i]; the last one goes to the cache. Block = 16 columns of one head of
 // one sequence; the running state stays in shared memory, the next segment's numbers load one segment ahead. A thread has four columns of
 // PER rows: bound by the reads of transition rows and states in shared memory, 8 of 16 bytes for 64 multiply-adds (PER 4).
-// With one column and sixteen rows a thread, five reads for every sixteen multiply-adds, it took 171 us at 8192 tokens of 16 heads of
-// 128 x 128 in 32 segments; a document of that length through four such layers 14.35 ms, and 14.23 now.
+// With one column and eight rows a thread, three reads (two of them of 16 bytes) for every eight multiply-adds, it took 171 us at 8192 tokens
+// of 16 heads of 128 x 128 in 32 segments; a document of that length through four such layers 14.35 ms, and 14.23 now.
 constexpr int COMBINE_COLS = 16, COMBINE_THREADS = 128, ROW_STEP = COMBINE_THREADS / (COMBINE_COLS / 4);
 template <int KIND, int PER>  // PER: rows of a thread, PER * ROW_STEP >= dim
 __global__ void __launch_bounds__(COMBINE_THREADS) recurrence_combine_kernel(ScanArgs sa) {
